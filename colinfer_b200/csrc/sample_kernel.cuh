@@ -30,8 +30,17 @@
 
 namespace smp {
 
-constexpr int NT = 512, NW = NT / 32;
-constexpr int CTAS_PER_SM = 2;
+#ifdef COLINFER_PROFILE
+// Profiling builds only: cycles per phase, summed over rows and CTAs (thread 0's clock).
+__device__ unsigned long long g_prof[16];
+#define SM_PROF(slot) do { if (tid == 0) { const long long t_ = clock64(); atomicAdd(&g_prof[slot], (unsigned long long)(t_ - prof_last)); prof_last = clock64(); } } while (0)
+#else
+#define SM_PROF(slot) do { } while (0)
+#endif
+
+constexpr int NT = 256, NW = NT / 32;
+constexpr int NUM_SM = 148;          // (a B200's; only says from how many rows on their order matters)
+constexpr int CTAS_PER_SM = 3;
 constexpr int CHUNK = 512;           // logits per chunk: 16 per lane
 constexpr int RING = 4096;           // bytes of ring per warp: fp32 two stages of 2 KB; bf16 two of 1 KB and one chunk in fp32
 constexpr int NB1 = 4096;            // histogram buckets
@@ -41,17 +50,17 @@ constexpr int FASTK = 100;           // largest top_k finished from the sample's
 constexpr int BINS = 512;            // bins of the sample and of the selections on lists
 constexpr int BINS_PAD = BINS + BINS / 16;   // one spare word per sixteen: a lane reading its sixteen bins hits a bank of its own
 constexpr float FAST_SCALE = 32.0f;  // sample bins per unit logit (16 units)
-constexpr int KCAP = 208;            // list entries per warp: rows without a histogram,
-constexpr int KCAP_CL = 144;         // the same in a CTA of a cluster (behind the pushed candidates),
-constexpr int WCAP = 80;             // rows with a histogram
-constexpr int GCAP = 128;            // list entries per warp gathered from all CTAs of a cluster
+constexpr int U_BYTES = 22528;       // lists, or histogram and lists
 constexpr int FCAP = 128;            // candidates of the one-warp finish
+constexpr int KCAP = U_BYTES / 8 / NW;                       // list entries per warp: rows without a histogram,
+constexpr int KCAP_CL = (U_BYTES - 8 * FCAP * 8) / 8 / NW;   // the same in a CTA of a cluster (behind the candidates of all CTAs),
+constexpr int WCAP = (U_BYTES - NB1 * 4) / 8 / NW;           // rows with one
+constexpr int GCAP = NB1 * 4 / 8 / NW;                       // entries per warp gathered from all CTAs of a cluster
 constexpr int FIN_CAND = 64;         // entries of one bin compared pairwise
 constexpr int FB_NB = 256;           // radix buckets per level of the fallback select
 constexpr int PEN_TABLE = 2048;      // distinct history ids with an O(1) count
 constexpr int LIST_MAX = 1400;       // logits a list selection may hold
 constexpr int BAL_ROWS = 16384;      // launches up to this many rows deal their rows to the CTAs by cost class
-constexpr int BAL_MINE = BAL_ROWS / 128 + 8;
 constexpr int MAX_V = 524288;
 constexpr long long WAIT_CYCLES = 400000000LL;
 #define SM_FLT_MAX 3.402823466e38f
@@ -66,7 +75,6 @@ struct Args {
     int64_t* out; colinfer_row_stats* stats; int32_t* status;
     int B, R, V; int flags;
     int cluster;                       // CTAs per row
-    int smem_bins, smem_csum, smem_bars, smem_sc, smem_pen;   // offsets of the shared-memory parts behind the ring and the lists
 };
 
 template <bool B> struct BoolTag { static constexpr bool value = B; };
@@ -77,28 +85,98 @@ struct RowP {
     float T; int kk; float topp, lmp; long long seed; float rp, pp, fp; int hlen; long long pos; float u; int pad;
 };
 
+// A row at hand.  What the phases of a row hand on lives here, not in registers: at 64 registers per thread anything that
+// stays alive across a pass is spilled, and with 226 KB of an SM's 256 in shared memory a spill is a round trip to L2.
+struct RowS {
+    const char* base; uint32_t end;    // the 16-byte boundary at or below its first logit; the low word of the one at or above its end
+    int row, key;                      // its index, and that plus 1
+    int a, Nc;                         // position of the first logit, chunks
+    const int32_t* mrow;               // grammar mask (NULL: none)
+    int pen_on, pen_cap;               // penalties; entries in the tables (tokens beyond are counted by scanning the history)
+    const int32_t* hist; int hlen; float rp, pp, fp;
+    int cls;                           // ROW_* below
+    float tc, topp, lmp, u; int kk;
+    float scw;                         // histogram buckets per unit logit
+    float lref; int count_hist;        // the sample's maximum (the group's); pass 1 counts the histogram
+    float L; int aidx, status;         // the row's maximum, the lowest token that has it
+    int hist_ready;
+    float lcut, horizon; int minp;     // smallest kept logit; the mass horizon; the cut lies above it
+    MassFn mass;
+    float href; int hoff;              // histogram: bucket b holds the logits in (href - (b + 1 - hoff) / scw, href - (b - hoff) / scw]
+    int path; float t_hi, t_lo; int band_top, band_bot;   // how a wide row is cut; its band, in logits and in buckets
+    int drawn; long long token; u64 total;                // the draw's warp stores the token itself
+    int listed;                        // the lists of pass 1 hold everything that can be kept
+    int hist_slow;                     // the history has more tokens than the tables
+};
+enum { ROW_SAMPLED = 1, ROW_FASTK = 2, ROW_WIDE = 4 };
+enum { PATH_PURE = 0, PATH_LIST = 1, PATH_BAND = 2, PATH_FALLBACK = 3 };
+
+// A warp's ring between passes: chunks consumed, chunks under way, and of which row (index + 1; 0: none) they are.
+struct WarpRing { int cons, out, key; };
+
+// Where the row after the one at hand lies (key 0: none).
+struct NextRow { const char* base; uint32_t end; int key, Nc; };
+
 struct Sc {
     RowP rp[2];
+    RowS rows[2];                      // the row at hand and the one after it, by the parity of the row's number in the CTA
+    NextRow next[2];
+    WarpRing ring[NW];
+    int V, W, GW, rank;                // logits per row; mask words per row; warps that share a row; this CTA among them
+    int drop, dead;                    // test flag; a wait ran out
+    __align__(16) uint4 clc; u64 clc_bar;   // the answer of the hardware's work queue, its barrier
+    int cls_tot[3]; unsigned short cls_pre[3][NT];   // rows per cost class: all, before each thread's
+    int pen_off;                       // offset of the penalty tables in shared memory
     // published to the CTAs of the cluster (or to the CTA's own warps): the sample's maxima; the row's maximum and argmax per
     // warp; the CTA's list bound and flags; the warps' list lengths; mass sums
     float swf[NW];
     float wf[NW]; int wi[NW];
+    int in_klist;                      // the lists of the row at hand take the histogram's place
     float tw; int flags;               // 1 list overflow or no bound, 2 a wait ran out, 4 histogram not counted
     int wn[NW];
     u64 g_all[NW], g_keep[NW];
     u64 t_cnt, t_est;                  // totals of the CTA's share of the histogram
-    int npush; float push_lo;          // candidates pushed to the leader, the value down to which they are complete
+    int nsel;                          // candidates selected
+    int npush; float push_lo;          // candidates sent to the group's first CTA, the value down to which they are complete
     int ok; float fin_cut; u64 fin_total; int fin_token;
     int fb[3]; u64 fe[3];              // finds of fine_decide
     // CTA-local
-    u64 wsum[NW], woff[NW], wtotal, wsum2[NW], woff2[NW], wtotal2;
+    u64 wsum[NW], woff[NW], wtotal, wsum2[NW], woff2[NW];
     int found; u64 found_excl;
     int ncand; float res_f; int sel_ok; uint32_t cand_kmin, cand_kmax;
     float cand_l[FIN_CAND]; u64 cand_w[FIN_CAND];
-    uint32_t fo_idx[FCAP]; float fo_l[FCAP];
-    int nsel; int aidx; int hist_slow; int x_chunk; u64 x_before;
-    int my_rows[BAL_MINE]; int my_count;
+    int x_chunk; u64 x_before;
 };
+
+// Candidates: as selected (over the sample's bins); by descending logit and by ascending token, with masses (over those of the
+// selection too, once every warp has read them).
+struct Fin {
+    uint32_t fc_idx[FCAP]; float fc_l[FCAP];
+    float sv_l[FCAP]; uint32_t sv_q[FCAP];
+    uint32_t so_idx[FCAP]; float so_l[FCAP]; uint32_t so_q[FCAP];
+    int ties[FCAP];
+};
+static_assert(sizeof(Fin) <= 2 * BINS_PAD * 4 && 2 * FCAP * 4 <= BINS_PAD * 4, "candidates over the bins");
+
+// Shared memory: rings, scratch, lists (or histogram and lists), bins, barriers, chunk sums, penalty tables (launches with
+// histories).  The history bitmap, a bit per position, lies over lists, bins and chunk sums while the tables are built.
+constexpr int OFF_SC = NW * RING;
+constexpr int OFF_BARS = (OFF_SC + (int)sizeof(Sc) + 15) & ~15;
+constexpr int OFF_U = (OFF_BARS + NW * 16 + 127) & ~127;
+constexpr int OFF_BINS = OFF_U + U_BYTES;
+constexpr int OFF_CSUM = OFF_BINS + 2 * BINS_PAD * 4;
+static_assert(2 * BINS_PAD * 4 >= BINS * 8 && BINS_PAD * 4 >= CHUNK * 4, "what lies over the bins");
+__host__ __device__ inline int max_chunks(int V) { return (V + 7 + CHUNK - 1) / CHUNK; }   // a row may start seven logits into its first chunk
+__host__ __device__ inline int pen_offset(int V, bool pen) {
+    const int nc = max_chunks(V);
+    const int over = pen ? nc * 64 - U_BYTES - 2 * BINS_PAD * 4 : 0;      // what of the bitmap reaches into the chunk sums
+    return (OFF_CSUM + (nc * 8 > over ? nc * 8 : over) + 15) & ~15;
+}
+__host__ __device__ inline int smem_bytes(int V, bool pen) { return pen_offset(V, pen) + (pen ? 4 * PEN_TABLE + (max_chunks(V) + 1) * 4 : 0); }
+
+extern __shared__ __align__(128) unsigned char smem[];
+__device__ __forceinline__ Sc* scratch() { return reinterpret_cast<Sc*>(smem + OFF_SC); }
+__device__ __forceinline__ Fin* fin_area() { return reinterpret_cast<Fin*>(smem + OFF_BINS); }
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
@@ -211,27 +289,6 @@ __device__ __forceinline__ int warp_count_bin(const uint32_t* hist, uint32_t kk,
     return hl * PERB + bl;
 }
 
-// Sorts 128 ordered keys held four per lane (element lane * 4 + t) into descending order across the warp: a bitonic
-// network of 28 compare-exchange stages, the wide ones by shuffle.
-__device__ __forceinline__ void warp_sort_desc4(uint32_t (&a)[4], int lane) {
-#pragma unroll
-    for (int k = 2; k <= 128; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            uint32_t b[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int i = lane * 4 + t;
-                const uint32_t o = j >= 4 ? __shfl_xor_sync(0xffffffffu, a[t], j >> 2) : a[t ^ (j & 3)];
-                const bool take_max = ((i & j) == 0) == ((i & k) == 0);
-                b[t] = take_max ? max(a[t], o) : min(a[t], o);
-            }
-#pragma unroll
-            for (int t = 0; t < 4; ++t) a[t] = b[t];
-        }
-    }
-}
-
 // ------------------------------------------------------------------------------------------------ packed fp32 pairs
 __device__ __forceinline__ u64 pk2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ void up2(u64 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
@@ -239,123 +296,36 @@ __device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0,
 __device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
-// The masses of MassFn for pairs of logits, each as two integers: mass = (hi - HI0) * 2^15 + (lo - LO0).  The arithmetic is
-// MassFn's, operation by operation, two logits per instruction; rounding the exponential to a multiple of 2^-30 takes
-// two rounding additions instead of a conversion, which would double the load of the exponentials' pipe.
+// The masses of MassFn for pairs of logits, each as two floats: mass = (hi * 2^15 + lo * 2^-15) * 2^15 with hi a multiple of
+// 2^-15 and lo an integer, |lo| <= 2^14.  The arithmetic is MassFn's, operation by operation, two logits per instruction;
+// rounding the exponential to a multiple of 2^-30 takes two rounding additions instead of a conversion, which would double
+// the load of the exponentials' pipe.  A logit of -inf gives NaN.
 struct Mass2 {
-    static constexpr uint32_t HI0 = 0x43C00000u, LO0 = 0x4B400000u;    // the bits of 384 = 1.5 * 2^8 and of 1.5 * 2^23
     u64 rinv, ntc, nm;
     __device__ __forceinline__ void init(const MassFn& f) { rinv = pk2(f.rinv, f.rinv); ntc = pk2(-f.tc, -f.tc); nm = pk2(-f.m, -f.m); }
-    __device__ __forceinline__ void operator()(float l0, float l1, uint32_t& hi0, uint32_t& hi1, uint32_t& lo0, uint32_t& lo1) const {
+    __device__ __forceinline__ void operator()(float l0, float l1, u64& hi, u64& lo) const {
         const u64 l = pk2(l0, l1);
         const u64 q0 = mul2(l, rinv);
         const u64 z = fma2(fma2(q0, ntc, l), rinv, q0);
-        float y0, y1, e0, e1, a, b;
+        float y0, y1, e0, e1;
         up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(y1));
         const u64 e = pk2(e0, e1);
-        const u64 t1 = add2(e, pk2(384.0f, 384.0f));                   // e rounded to a multiple of 2^-15
-        const u64 h = add2(t1, pk2(-384.0f, -384.0f));
-        const u64 r = fma2(h, pk2(-1.0f, -1.0f), e);                   // the rest, exactly
-        const u64 t2 = fma2(r, pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f));   // in units of 2^-30, to the nearest integer
-        up2(t1, a, b); hi0 = __float_as_uint(a); hi1 = __float_as_uint(b);
-        up2(t2, a, b); lo0 = __float_as_uint(a); lo1 = __float_as_uint(b);
+        hi = add2(add2(e, pk2(384.0f, 384.0f)), pk2(-384.0f, -384.0f));        // e rounded to a multiple of 2^-15
+        const u64 r = fma2(hi, pk2(-1.0f, -1.0f), e);                           // the rest, exactly
+        lo = add2(fma2(r, pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f)), pk2(-12582912.0f, -12582912.0f));   // to the nearest 2^-30
     }
 };
 
 // ------------------------------------------------------------------------------------------------ the row as its warps read it
 // L2 policies: rows that are read twice ask to be kept on their first pass; everything else asks to go first.
-__device__ __forceinline__ u64 l2_keep() { u64 p; asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p)); return p; }
-__device__ __forceinline__ u64 l2_stream() { u64 p; asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p)); return p; }
-
-// A warp's ring: two stages, filled in the order of the passes.  `np` is the next chunk to ask for, `rem` how many are
-// left in this pass, nnp / nrem the same for the pass that follows.
-struct Ring {
-    uint32_t buf, bar;                 // shared-memory addresses of the stages and of their barriers
-    const char* np; const char* nnp;
-    int next_key;                      // the row the next pass reads (its index + 1; 0: unknown)
-    uint32_t end, nend;                // low words of the rows' end addresses (16-byte aligned)
-    int rem, nrem;
-    int cons, iss;                     // chunks consumed and asked for
-    bool keep, nkeep;
-    bool dead, drop;
-};
-
-template <int ELT>
-struct Reader {
-    static constexpr int CHB = CHUNK * ELT;
-    Ring g;
-    int stride;                        // bytes between a warp's chunks
-    int lane;
-
-    __device__ __forceinline__ void issue_one(const char* p, uint32_t end, bool keep) {
-        if (lane == 0) {
-            const uint32_t left = end - (uint32_t)reinterpret_cast<u64>(p);
-            const uint32_t bytes = left < (uint32_t)CHB ? left : (uint32_t)CHB;
-            const uint32_t s = (uint32_t)g.iss & 1u;
-            const u64 pol = keep ? l2_keep() : l2_stream();
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(g.bar + 8 * s), "r"(bytes) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-                         ::"r"(g.buf + s * CHB), "l"(p), "r"(bytes), "r"(g.bar + 8 * s), "l"(pol) : "memory");
-        }
-    }
-    // Asks for chunks until both stages are under way.
-    __device__ __forceinline__ void fill() {
-        while (g.iss - g.cons < 2) {
-            if (g.rem > 0) {
-                if (!g.drop && !g.dead) issue_one(g.np, g.end, g.keep);
-                g.np += stride; --g.rem;
-            } else if (g.nrem > 0) {
-                if (!g.drop && !g.dead) issue_one(g.nnp, g.nend, g.nkeep);
-                g.nnp += stride; --g.nrem;
-            } else break;
-            ++g.iss;
-        }
-    }
-    // The stage of the next chunk; waits for its bytes.
-    __device__ __forceinline__ void wait() {
-        if (g.dead) return;
-        const uint32_t bar = g.bar + 8 * ((uint32_t)g.cons & 1u), par = ((uint32_t)g.cons >> 1) & 1u;
-        auto test = [&]() {
-            uint32_t ok;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok) : "r"(bar), "r"(par), "r"(20000u) : "memory");
-            return ok != 0;
-        };
-        if (!test()) {
-            const long long t0 = clock64();
-            bool late = false;
-            while (!test()) if (clock64() - t0 > WAIT_CYCLES) { late = true; break; }
-            g.dead = __any_sync(0xffffffffu, late);
-        }
-    }
-    // Gives the stage back.  `wrote`: the warp changed it with ordinary stores.
-    __device__ __forceinline__ void release(bool wrote) {
-        if (wrote) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        ++g.cons;
-        fill();
-    }
-    // Begins a pass over row `key`: n chunks from `first`, the row's last byte before `end`.  Chunks that were asked for
-    // ahead are used when they belong to this pass.
-    __device__ __forceinline__ void begin(int key, const char* first, u64 end, int n, bool keep) {
-        if (g.next_key == key) {
-            g.np = g.nnp; g.rem = g.nrem;
-        } else {
-            while (g.iss != g.cons) { wait(); ++g.cons; }            // something else was on its way: let it land
-            g.np = first; g.rem = n;
-        }
-        g.end = (uint32_t)end; g.keep = keep;
-        g.next_key = 0; g.nrem = 0;
-        fill();
-    }
-    __device__ __forceinline__ void then(int key, const char* first, u64 end, int n, bool keep) {
-        g.next_key = key; g.nnp = first; g.nend = (uint32_t)end; g.nrem = n; g.nkeep = keep;
-    }
-    __device__ __forceinline__ uint32_t stage() const { return g.buf + ((uint32_t)g.cons & 1u) * CHB; }
-};
-
+__device__ __forceinline__ u64 l2_policy(bool keep) {
+    u64 p;
+    if (keep) asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    else asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
 __device__ __forceinline__ float lds32(uint32_t a) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory"); return v; }
 __device__ __forceinline__ void sts32(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ void sts16(uint32_t a, unsigned short v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(v) : "memory"); }
@@ -368,268 +338,641 @@ __device__ __forceinline__ void sts128(uint32_t a, float4 v) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
-// Position in the chunk of a lane's e-th logit (e = 0 .. 15).
-template <int ELT> __device__ __forceinline__ int pos_of(int e, int lane) {
-    return ELT == 4 ? (e >> 2) * 128 + lane * 4 + (e & 3) : (e >> 3) * 256 + lane * 8 + (e & 7);
-}
+// Position in the chunk of a lane's e-th logit (e = 0 .. 15): groups of four, a group of every lane side by side.
+__device__ __forceinline__ int pos_of(int e, int lane) { return (e >> 2) * 128 + lane * 4 + (e & 3); }
 
 // The penalties of a row: its history's tokens among the CTA's chunks, in ascending order, with their counts.
-struct Pen {
-    bool on;
-    const uint32_t* pre;               // [chunks + 1] first entry of every chunk
-    const unsigned short* pos;         // [PEN_TABLE] position in its chunk
-    const unsigned short* cnt;         // [PEN_TABLE]
-    int cap;                           // entries in the tables; tokens beyond are counted by scanning the history
-    const int32_t* hist; int hlen; float rp, pp, fp;
+struct PenTab {
+    uint32_t* ent;                     // [PEN_TABLE] position in its chunk (low half), occurrences (high half)
+    uint32_t* pre;                     // [chunks + 1] first entry of every chunk
 };
+__device__ __forceinline__ PenTab pen_tab(const Sc* sc) {
+    PenTab t;
+    t.ent = reinterpret_cast<uint32_t*>(smem + sc->pen_off);
+    t.pre = t.ent + PEN_TABLE;
+    return t;
+}
+// The entries of one chunk, and a lane's first one, fetched a chunk ahead.
+struct PenPeek { uint32_t r0, r1, ent; };
+__device__ __forceinline__ PenPeek pen_peek(const PenTab& t, int cap, int c, int lane) {
+    PenPeek k;
+    k.r0 = t.pre[c]; k.r1 = t.pre[c + 1];
+    k.ent = k.r0 + lane < min(k.r1, (uint32_t)cap) ? t.ent[k.r0 + lane] : 0u;
+    return k;
+}
 
-// Replaces the penalised logits of chunk c (fp32, at shared address `at`) by their penalised values.  A warp calls.
-static __device__ __noinline__ void pen_patch_slow(const Pen& pen, uint32_t at, int c, int a, int V, int lane, int* hist_slow) {
-    // tokens without a table entry: every first occurrence in the history whose rank lies beyond the tables
-    *hist_slow = 1;
-    const int t_lo = max(c * CHUNK - a, 0), t_hi = min(c * CHUNK - a + CHUNK, V);
-    for (int i = lane; i < pen.hlen; i += 32) {
-        const int v = __ldg(pen.hist + i);
+// Entries beyond the warp's first 32, and tokens without a table entry (every first occurrence in the history that the tables
+// do not hold).
+static __device__ __noinline__ void pen_patch_more(RowS& rw, uint32_t at, int c, uint32_t r0, uint32_t r1) {
+    const Sc* sc = scratch();
+    const PenTab t = pen_tab(sc);
+    const int lane = lane_id();
+    const uint32_t rt = min(r1, (uint32_t)rw.pen_cap);
+    for (uint32_t r = r0 + 32 + lane; r < rt; r += 32) {
+        const uint32_t q = at + 4 * (t.ent[r] & 0xFFFFu);
+        const float x = lds32(q);
+        if (x > CI_NEG_INF) sts32(q, apply_penalty(x, (int)(t.ent[r] >> 16), rw.rp, rw.pp, rw.fp));
+    }
+    if (r1 <= rt) return;
+    rw.hist_slow = 1;
+    const int t_lo = max(c * CHUNK - rw.a, 0), t_hi = min(c * CHUNK - rw.a + CHUNK, sc->V);
+    for (int i = lane; i < rw.hlen; i += 32) {
+        const int v = __ldg(rw.hist + i);
         if (v < t_lo || v >= t_hi) continue;
         int count = 0; bool first = true;
-        for (int j = 0; j < pen.hlen; ++j) {
-            if (__ldg(pen.hist + j) == v) { if (j < i) { first = false; break; } ++count; }
+        for (int j = 0; j < rw.hlen; ++j) {
+            if (__ldg(rw.hist + j) == v) { if (j < i) { first = false; break; } ++count; }
         }
         if (!first) continue;
-        const int pos = v + a - c * CHUNK;
+        const uint32_t pos = (uint32_t)(v + rw.a - c * CHUNK);
         bool tabled = false;
-        for (uint32_t r = pen.pre[c]; r < pen.pre[c + 1] && (int)r < pen.cap; ++r) tabled |= (int)pen.pos[r] == pos;
+        for (uint32_t r = r0; r < rt; ++r) tabled |= (t.ent[r] & 0xFFFFu) == pos;
         if (tabled) continue;
         const float x = lds32(at + 4 * pos);
-        if (x > CI_NEG_INF) sts32(at + 4 * pos, apply_penalty(x, count, pen.rp, pen.pp, pen.fp));
+        if (x > CI_NEG_INF) sts32(at + 4 * pos, apply_penalty(x, count, rw.rp, rw.pp, rw.fp));
     }
 }
-__device__ __forceinline__ void pen_patch(const Pen& pen, uint32_t at, int c, int a, int V, int lane, int* hist_slow) {
-    const uint32_t r0 = pen.pre[c], r1 = pen.pre[c + 1];
-    const uint32_t rt = min(r1, (uint32_t)pen.cap);
-    for (uint32_t r = r0 + lane; r < rt; r += 32) {
-        const uint32_t q = at + 4 * (uint32_t)pen.pos[r];
+// Replaces the penalised logits of chunk c (fp32, at shared address `at`) by their penalised values.  A warp calls.
+__device__ __forceinline__ void pen_patch(RowS& rw, uint32_t at, int c, const PenPeek& k) {
+    if (k.ent) {                                                         // (an entry counts at least one occurrence)
+        const uint32_t q = at + 4 * (k.ent & 0xFFFFu);
         const float x = lds32(q);
-        if (x > CI_NEG_INF) sts32(q, apply_penalty(x, (int)pen.cnt[r], pen.rp, pen.pp, pen.fp));
+        if (x > CI_NEG_INF) sts32(q, apply_penalty(x, (int)(k.ent >> 16), rw.rp, rw.pp, rw.fp));
     }
-    if (r1 > rt) pen_patch_slow(pen, at, c, a, V, lane, hist_slow);
+    if (k.r1 - k.r0 > 32 || k.r1 > (uint32_t)rw.pen_cap) pen_patch_more(rw, at, c, k.r0, k.r1);
+    __syncwarp();
 }
 
-// What the passes need to know of a row.
-struct RowV {
-    int V, a, Nc;                      // logits, position of the first one, chunks
-    const int32_t* mrow; int W;        // grammar mask (NULL: none)
-    Pen pen;
+// The logits of the first and last chunk that lie outside the row read as -inf.
+template <int ELT>
+static __device__ __noinline__ void mend_edges(uint32_t st, int c, int a) {
+    const int lane = lane_id(), lo = c == 0 ? a : 0, hi = scratch()->V + a - c * CHUNK;
+    for (int p = lane; p < CHUNK; p += 32)
+        if (p < lo || p >= hi) { if (ELT == 4) sts32(st + 4 * p, CI_NEG_INF); else sts16(st + 2 * p, 0xFF80u); }
+    __syncwarp();
+}
+
+// A warp's two-stage ring.  While a pass runs its state lives in registers, between passes in Sc.
+template <int ELT>
+struct Pipe {
+    static constexpr int CHB = CHUNK * ELT;
+    uint32_t buf, bar;                 // shared-memory addresses of the stages and of their barriers
+    int cons, out;                     // chunks consumed, chunks under way
+    bool asks;                         // the lane that asks for chunks (none once a wait ran out)
+
+    __device__ __forceinline__ Pipe() {
+        const int warp = warp_id();
+        buf = smem_u32(smem) + warp * RING;
+        bar = smem_u32(smem) + OFF_BARS + warp * 16;
+        const Sc* sc = scratch();
+        cons = sc->ring[warp].cons; out = sc->ring[warp].out;
+        asks = lane_id() == 0 && !(sc->drop | sc->dead);
+    }
+    __device__ __forceinline__ uint32_t conv() const { return buf + 2 * CHB; }          // bf16: an fp32 copy of one chunk
+    __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) & 1u) * CHB; }
+    __device__ __forceinline__ void issue(const char* p, uint32_t bytes, u64 pol) {
+        if (asks) {
+            const uint32_t s = (uint32_t)(cons + out) & 1u;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * s), "r"(bytes) : "memory");
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                         ::"r"(buf + s * CHB), "l"(p), "r"(bytes), "r"(bar + 8 * s), "l"(pol) : "memory");
+        }
+        ++out;
+    }
+    // The bytes of the chunk j places from the next one to consume are there.
+    __device__ __forceinline__ void wait(int j = 0) {
+        const uint32_t b = bar + 8 * ((uint32_t)(cons + j) & 1u), par = ((uint32_t)(cons + j) >> 1) & 1u;
+        auto test = [&]() {
+            uint32_t ok;
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok) : "r"(b), "r"(par), "r"(20000u) : "memory");
+            return ok != 0;
+        };
+        if (!test()) {
+            // (with the test flag nothing was asked for: the wait runs out, once per CTA and warp)
+            Sc* sc = scratch();
+            if (*(volatile int*)&sc->dead) return;
+            const long long t0 = clock64();
+            while (!test()) if (clock64() - t0 > WAIT_CYCLES) { sc->dead = 1; asks = false; break; }
+            __syncwarp();
+        }
+    }
+    // Between passes: what was asked for ahead stays when it belongs to row `key`, else it is let land and dropped.
+    __device__ __forceinline__ void expect(int key) {
+        Sc* sc = scratch();
+        if (out > 0 && sc->ring[warp_id()].key != key)
+            while (out > 0) { wait(); ++cons; --out; }
+    }
+    __device__ __forceinline__ void save(int key) {
+        __syncwarp();
+        if (lane_id() == 0) { WarpRing& r = scratch()->ring[warp_id()]; r.cons = cons; r.out = out; r.key = key; }
+        __syncwarp();
+    }
 };
 
+// Bytes of chunk c of a row of Nc chunks that ends at `end` (low word, as all of it: rows are short).
+template <int ELT>
+__device__ __forceinline__ uint32_t chunk_bytes(const char* p, uint32_t end) {
+    const uint32_t left = end - (uint32_t)reinterpret_cast<u64>(p);
+    return left < (uint32_t)(CHUNK * ELT) ? left : (uint32_t)(CHUNK * ELT);
+}
+
+// Asks for the first chunks of row `key`, as far as they are not under way.
+template <int ELT>
+__device__ __forceinline__ void ring_start(int key, const char* base, uint32_t end, int Nc, int gw, int GW) {
+    Pipe<ELT> p;
+    p.expect(key);
+    while (p.out < 2 && gw + p.out * GW < Nc) {
+        const char* q = base + (size_t)(gw + p.out * GW) * Pipe<ELT>::CHB;
+        p.issue(q, chunk_bytes<ELT>(q, end), l2_policy(true));
+    }
+    p.save(key);
+}
+
 // The mask word of one lane for chunk c: words (512 c - a) / 32 + lane, lanes 0 .. 16.
-__device__ __forceinline__ uint32_t mask_word(const RowV& rw, int c, int lane) {
-    const int w = ((c * CHUNK - rw.a) >> 5) + lane;
-    return (lane <= 16 && w >= 0 && w < rw.W) ? (uint32_t)__ldg(rw.mrow + w) : 0u;
+__device__ __forceinline__ uint32_t mask_word(const int32_t* mrow, int W, int a, int c, int lane) {
+    const int w = ((c * CHUNK - a) >> 5) + lane;
+    return (lane <= 16 && w >= 0 && w < W) ? (uint32_t)__ldg(mrow + w) : 0u;
 }
 
-// The chunk at the reader's current stage as 16 effective logits per lane.  fresh: the stage has just arrived (its edges and,
-// for fp32, its penalties are still to be applied).  mw: the lane's mask word.  wrote: the stage was changed.
-template <int ELT>
-__device__ __forceinline__ void read_chunk(const RowV& rw, uint32_t st, uint32_t conv, int c, bool fresh, uint32_t mw, float (&v)[16], int lane,
-                                           bool& wrote, int* hist_slow) {
+// A chunk as a pass reads it: group k (0 .. 3) of the lane's effective logits.
+template <int ELT, bool MASK>
+struct Chunk {
+    uint32_t at;                       // the lane's first group: in the stage, or (bf16 chunks with penalties) in the fp32 copy
+    bool wide;                         // fp32 values
+    uint32_t mw; int sh;               // the lane's mask word, the bit of position 0
+    int c;
+
+    __device__ __forceinline__ float4 stored(int k) const {
+        if (ELT == 4 || wide) return lds128(at + k * 512);
+        uint32_t x, y;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(at + k * 256) : "memory");
+        return make_float4(__uint_as_float(x << 16), __uint_as_float(x & 0xFFFF0000u), __uint_as_float(y << 16), __uint_as_float(y & 0xFFFF0000u));
+    }
+    __device__ __forceinline__ float4 group(int k, float none) const {
+        float4 v = stored(k);
+        if (MASK) {
+            const int bit = sh + k * 128 + lane_id() * 4;
+            uint32_t bits = __shfl_sync(0xffffffffu, mw, bit >> 5);
+            if (sh & 3) bits = __funnelshift_r(bits, __shfl_sync(0xffffffffu, mw, (bit >> 5) + 1), bit & 31);   // groups straddle words (an unaligned row)
+            else bits >>= bit & 31;
+            if (!(bits & 1u)) v.x = none;
+            if (!(bits & 2u)) v.y = none;
+            if (!(bits & 4u)) v.z = none;
+            if (!(bits & 8u)) v.w = none;
+        }
+        return v;
+    }
+    // logit e of the lane as stored (penalties; not the mask, which only removes)
+    __device__ __forceinline__ float one(int e) const {
+        if (ELT == 4 || wide) return lds32(at + (e >> 2) * 512 + (e & 3) * 4);
+        unsigned short h;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(at + (e >> 2) * 256 + (e & 3) * 2) : "memory");
+        return __uint_as_float((uint32_t)h << 16);
+    }
+};
+
+// Prepares the chunk at stage `st`.  fresh: it has just arrived (its edges and, for fp32, its penalties are still to be
+// applied); wrote: the stage was changed.
+template <int ELT, bool MASK>
+__device__ __forceinline__ Chunk<ELT, MASK> open_chunk(RowS& rw, uint32_t st, uint32_t conv, int c, bool fresh, bool pen, const PenPeek& pk, uint32_t mw, bool& wrote) {
+    const int lane = lane_id();
+    Chunk<ELT, MASK> k;
+    k.c = c; k.mw = mw; k.sh = (-rw.a) & 31; k.wide = ELT == 4;
     wrote = false;
-    if (fresh) {
-        if ((c == 0 && rw.a > 0) || c == rw.Nc - 1) {
-            const int lo = c == 0 ? rw.a : 0, hi = rw.V + rw.a - c * CHUNK;
-            for (int p = lane; p < CHUNK; p += 32)
-                if (p < lo || p >= hi) { if (ELT == 4) sts32(st + 4 * p, CI_NEG_INF); else sts16(st + 2 * p, 0xFF80u); }
-            wrote = true;
+    if (fresh && (c == 0 || c == rw.Nc - 1)) { mend_edges<ELT>(st, c, rw.a); wrote = true; }
+    k.at = st + lane * 4 * ELT;
+    if (pen) {
+        if (ELT == 4) { if (fresh) { pen_patch(rw, st, c, pk); wrote = true; } }
+        else {                                                           // penalised values are fp32: through an fp32 copy of the chunk
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sts128(conv + lane * 16 + j * 512, k.stored(j));
             __syncwarp();
-        }
-        if (ELT == 4 && rw.pen.on && rw.pen.pre[c] != rw.pen.pre[c + 1]) {
-            pen_patch(rw.pen, st, c, rw.a, rw.V, lane, hist_slow);
-            wrote = true;
-            __syncwarp();
+            pen_patch(rw, conv, c, pk);
+            k.at = conv + lane * 16; k.wide = true;
         }
     }
-    if (ELT == 4) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 x = lds128(st + k * 512 + lane * 16);
-            v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float4 x = lds128(st + k * 512 + lane * 16);           // eight bf16: upper halves of floats
-            const uint32_t u[4] = {__float_as_uint(x.x), __float_as_uint(x.y), __float_as_uint(x.z), __float_as_uint(x.w)};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { v[8 * k + 2 * j] = __uint_as_float(u[j] << 16); v[8 * k + 2 * j + 1] = __uint_as_float(u[j] & 0xFFFF0000u); }
-        }
-        if (rw.pen.on && rw.pen.pre[c] != rw.pen.pre[c + 1]) {           // penalised values are fp32: through an fp32 copy of the chunk
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                sts128(conv + ((k >> 1) * 256 + lane * 8 + (k & 1) * 4) * 4, make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]));
-            __syncwarp();
-            pen_patch(rw.pen, conv, c, rw.a, rw.V, lane, hist_slow);
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float4 x = lds128(conv + ((k >> 1) * 256 + lane * 8 + (k & 1) * 4) * 4);
-                v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
-            }
-            __syncwarp();
-        }
-    }
-    if (rw.mrow != nullptr) {
-        constexpr int GE = ELT == 4 ? 4 : 8;                             // consecutive logits per lane
-        const int sh = (-rw.a) & 31;                                     // bit of position 0 in the lanes' words
-#pragma unroll
-        for (int k = 0; k < 16 / GE; ++k) {
-            const int bit = sh + k * (32 * GE) + lane * GE;
-            const uint32_t lo = __shfl_sync(0xffffffffu, mw, bit >> 5);
-            uint32_t bits = lo >> (bit & 31);
-            if (sh % GE) {                                               // groups straddle words (an unaligned row)
-                const uint32_t hi = __shfl_sync(0xffffffffu, mw, (bit >> 5) + 1);
-                bits = __funnelshift_r(lo, hi, bit & 31);
-            }
-#pragma unroll
-            for (int j = 0; j < GE; ++j) if (!(bits & (1u << j))) v[k * GE + j] = CI_NEG_INF;
-        }
-    }
+    return k;
 }
 
-// A lane's logit e of the current chunk, as the pass saw it (penalties; not the mask, which only removes).
-template <int ELT>
-__device__ __forceinline__ float peek(const RowV& rw, uint32_t st, uint32_t conv, int c, int pos) {
-    if (ELT == 4) return lds32(st + 4 * pos);
-    if (rw.pen.on && rw.pen.pre[c] != rw.pen.pre[c + 1]) return lds32(conv + 4 * pos);
-    unsigned short h;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(st + 2 * pos) : "memory");
-    return __uint_as_float((uint32_t)h << 16);
+// What the ring asks for when a pass has asked for all of its own chunks.
+enum { THEN_NOTHING = 0, THEN_AGAIN = 1, THEN_NEXT_ROW = 2 };
+
+// One pass of the calling warp over its chunks of the row at hand: f(chunk) on every one.  keep: the row's L2
+// policy; seen: how many of its
+// first chunks have been read before (and lie in the ring as they were left).
+template <bool CL, int ELT, bool MASK, class F>
+__device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep, int seen, int then, F f) {
+    constexpr int CHB = CHUNK * ELT;
+    Sc* sc = scratch();
+    Pipe<ELT> p;
+    p.expect(rw.key);
+    const int GW = CL ? sc->GW : NW;
+    const int gw = (CL ? sc->rank * NW : 0) + warp_id();
+    const int Nc = rw.Nc;
+    const bool pen_on = rw.pen_on != 0;
+    const u64 pol = l2_policy(keep);
+    int cn = gw + p.out * GW;                                            // the next chunk to ask for
+    const char* next = rw.base + (size_t)cn * CHB;
+    while (p.out < 2 && cn < Nc) { p.issue(next, chunk_bytes<ELT>(next, rw.end), pol); next += GW * CHB; cn += GW; }
+    uint32_t mw[MASK ? 3 : 1];                                           // mask words of this chunk and the next two
+    if (MASK) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) mw[MASK ? j : 0] = gw + j * GW < Nc ? mask_word(rw.mrow, sc->W, rw.a, gw + j * GW, lane_id()) : 0u;
+    }
+    PenPeek pk = {0, 0, 0};
+    if (pen_on && gw < Nc) pk = pen_peek(pen_tab(sc), rw.pen_cap, gw, lane_id());
+#pragma unroll 1
+    for (int c = gw; c < Nc; c += GW) {
+        if (seen == 0) p.wait();
+        bool wrote = false;
+        const PenPeek pcur = pk;
+        if (pen_on && c + GW < Nc) pk = pen_peek(pen_tab(sc), rw.pen_cap, c + GW, lane_id());
+        f(open_chunk<ELT, MASK>(rw, p.stage(), p.conv(), c, seen == 0, pen_on && pcur.r0 != pcur.r1, pcur, mw[0], wrote));
+        if (MASK) {
+            mw[0] = mw[MASK ? 1 : 0]; mw[MASK ? 1 : 0] = mw[MASK ? 2 : 0];
+            if (c + 3 * GW < Nc) mw[MASK ? 2 : 0] = mask_word(rw.mrow, sc->W, rw.a, c + 3 * GW, lane_id());
+        }
+        // gives the stage back (what the warp changed in it with ordinary stores comes before the next copy) and asks for more
+        if (wrote || seen) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        seen = max(seen - 1, 0);
+        __syncwarp();
+        ++p.cons; --p.out;
+        if (cn < Nc) { p.issue(next, cn == Nc - 1 ? chunk_bytes<ELT>(next, rw.end) : CHB, pol); next += GW * CHB; cn += GW; }
+    }
+    // the first chunks of what comes next
+    const bool other = then == THEN_NEXT_ROW;
+    const int nkey = *(volatile const int*)&nx.key;
+    __threadfence_block();
+    const int nnc = then == THEN_NOTHING ? 0 : !other ? Nc : nkey ? nx.Nc : 0;
+    for (int c = gw; p.out < 2 && c < nnc; c += GW) {
+        const char* q = (other ? nx.base : rw.base) + (size_t)c * CHB;
+        p.issue(q, chunk_bytes<ELT>(q, other ? nx.end : rw.end), l2_policy(other));
+    }
+    p.save(other ? nkey : rw.key);
 }
 
 // Appends the logits of the chunk selected by the lanes' masks mk to the warp's list (no particular order).
-template <int ELT>
-__device__ __forceinline__ void list_append(const RowV& rw, Cand* list, int cap, int* wn, unsigned mk, uint32_t st, uint32_t conv, int c, int lane) {
+template <class C>
+__device__ __forceinline__ void list_append(int a, Cand* list, int cap, unsigned mk, const C& k) {
     if (mk) {
-        int at = atomicAdd(wn, __popc(mk));
+        Sc* sc = scratch();
+        int at = atomicAdd(&sc->wn[warp_id()], __popc(mk));
+        const int t0 = k.c * CHUNK - a;
         do {
             const int e = __ffs(mk) - 1;
             mk &= mk - 1;
-            const int pos = pos_of<ELT>(e, lane);
-            if (at < cap) { list[at].idx = (uint32_t)(c * CHUNK - rw.a + pos); list[at].l = peek<ELT>(rw, st, conv, c, pos); }
+            if (at < cap) { list[at].idx = (uint32_t)(t0 + pos_of(e, lane_id())); list[at].l = k.one(e); }
             ++at;
         } while (mk);
     }
+}
+// The same for the logits >= t (looked for again: few lanes have any).
+template <class C>
+__device__ __forceinline__ void list_above(int a, Cand* list, int cap, float t, bool any, const C& k) {
+    if (__any_sync(0xffffffffu, any)) {
+        unsigned mk = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = k.group(j, CI_NEG_INF);
+            mk |= ((v.x >= t ? 1u : 0u) | (v.y >= t ? 2u : 0u) | (v.z >= t ? 4u : 0u) | (v.w >= t ? 8u : 0u)) << (4 * j);
+        }
+        list_append(a, list, cap, mk, k);
+    }
+}
+__device__ __forceinline__ float max4(float4 v, float m) { return fmax3(fmax3(v.x, v.y, v.z), v.w, m); }
+
+// The passes.
+struct Top { float l; int idx; };
+
+// Maximum of the warp's chunks and the lowest token that has it.
+template <bool CL, int ELT, bool MASK>
+__device__ __forceinline__ Top pass_max(RowS& rw, const NextRow& nx, bool keep, int then) {
+    float lmax = CI_NEG_INF;
+    int lidx = 0x7fffffff;
+    run_pass<CL, ELT, MASK>(rw, nx, keep, 0, then, [&](const auto& k) {
+        float m = CI_NEG_INF;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m = max4(k.group(j, CI_NEG_INF), m);
+        if (__any_sync(0xffffffffu, m > lmax)) {
+            int e = 15;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                const float4 v = k.group(j, CI_NEG_INF);
+                e = v.w == m ? 4 * j + 3 : e; e = v.z == m ? 4 * j + 2 : e; e = v.y == m ? 4 * j + 1 : e; e = v.x == m ? 4 * j : e;
+            }
+            if (m > lmax) { lmax = m; lidx = k.c * CHUNK - rw.a + pos_of(e, lane_id()); }   // strict: the first (lowest) position of the maximum stays
+        }
+    });
+    return Top{lmax, lidx};
+}
+
+// Lists the logits >= t of the warp's chunks; returns their maximum.
+template <bool CL, int ELT, bool MASK>
+__device__ __forceinline__ float pass_list(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap) {
+    float lmax = CI_NEG_INF;
+    run_pass<CL, ELT, MASK>(rw, nx, keep, seen, then, [&](const auto& k) {
+        float m = CI_NEG_INF;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m = max4(k.group(j, CI_NEG_INF), m);
+        lmax = fmaxf(lmax, m);
+        list_above(rw.a, list, cap, t, m >= t, k);
+    });
+    return lmax;
+}
+
+// Histogram bucket of a logit: floor((href - x) * scale) + hoff clamped to [0, NB1).  The clamp is a saturating
+// multiply-add, the conversion a rounding addition (neither the ALU nor the conversion pipe is asked).  A logit exactly on an
+// edge may land in either neighbour; every user keeps a whole bucket of margin.
+struct Buckets {
+    float href, s, c;                  // saturate((href - x) * s + c) in units of NB1 - 1 buckets
+    __device__ __forceinline__ Buckets(float h, float scale, int hoff) : href(h), s(scale / (float)(NB1 - 1)), c(((float)hoff - 0.5f) / (float)(NB1 - 1)) {}
+    __device__ __forceinline__ float sat(float d) const { float r; asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(d), "f"(s), "f"(c)); return r; }
+    __device__ __forceinline__ int operator()(float x) const {
+        return __float_as_int(fmaf(sat(href - x), (float)(NB1 - 1), 8388608.0f)) - 0x4B000000;
+    }
+};
+
+// The same with a count of every logit's bucket; masked (-inf) logits are not counted.
+template <bool CL, int ELT, bool MASK>
+__device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap, float href, float scale, int hoff) {
+    float lmax = CI_NEG_INF;
+    const Buckets bk(href, scale, hoff);
+    const uint32_t h0 = smem_u32(smem) + OFF_U - (0x4B000000u << 2);
+    const u64 hr = pk2(href, href), k4 = pk2((float)(NB1 - 1), (float)(NB1 - 1)), mg = pk2(8388608.0f, 8388608.0f), neg = pk2(-1.0f, -1.0f);
+    run_pass<CL, ELT, MASK>(rw, nx, keep, seen, then, [&](const auto& k) {
+        float m = CI_NEG_INF;
+        auto count = [&](float x, float b) {
+            const uint32_t at = h0 + (__float_as_uint(b) << 2);
+            if (!MASK || x > CI_NEG_INF) asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory");
+        };
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = k.group(j, CI_NEG_INF);
+            m = max4(v, m);
+            float d0, d1, d2, d3, b0, b1, b2, b3;
+            up2(fma2(pk2(v.x, v.y), neg, hr), d0, d1);
+            up2(fma2(pk2(v.z, v.w), neg, hr), d2, d3);
+            up2(fma2(pk2(bk.sat(d0), bk.sat(d1)), k4, mg), b0, b1);
+            up2(fma2(pk2(bk.sat(d2), bk.sat(d3)), k4, mg), b2, b3);
+            count(v.x, b0); count(v.y, b1); count(v.z, b2); count(v.w, b3);
+        }
+        lmax = fmaxf(lmax, m);
+        list_above(rw.a, list, cap, t, m >= t, k);
+    });
+    return lmax;
+}
+
+// The mass pass: per chunk the mass of the logits >= lk (BAND: of those above t_hi) into csum, and, BAND, the logits of
+// [tl, t_hi] into the warp's list and the mass of all logits >= lk.  MINP: lk may lie above the mass horizon.
+// What bounds it: ~ 12 issue slots and one exponential per logit (an SM has 4 and 1/2 per cycle and 32 logits).
+struct Masses { u64 all, keep; };
+template <bool CL, int ELT, bool MASK, bool BAND, bool MINP>
+__device__ __forceinline__ Masses pass_mass(RowS& rw, const NextRow& nx, int then, MassFn mass, float lk, float t_hi, float tl, Cand* list, u64* csum) {
+    Mass2 m2;
+    m2.init(mass);
+    u64 keep = 0;
+    int all_h = 0, all_l = 0;
+    run_pass<CL, ELT, MASK>(rw, nx, false, 0, then, [&](const auto& k) {
+        bool mend = MINP;
+        u64 sh, sl;                                                      // sums of the chunk: exact (multiples of 2^-15 up to 16, integers up to 2^18)
+        float ah, al, s0, s1;
+        unsigned mk;
+        while (true) {
+            sh = sl = 0; ah = al = 0.0f; mk = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float4 v = k.group(j, SM_LOW);
+                if (mend) {                                              // logits without mass
+                    v.x = v.x >= lk ? v.x : SM_LOW; v.y = v.y >= lk ? v.y : SM_LOW;
+                    v.z = v.z >= lk ? v.z : SM_LOW; v.w = v.w >= lk ? v.w : SM_LOW;
+                }
+                u64 hi, lo;
+                float h0, h1, l0, l1;
+                m2(v.x, v.y, hi, lo);
+                sh = add2(sh, hi); sl = add2(sl, lo);
+                if (BAND) {
+                    up2(hi, h0, h1); up2(lo, l0, l1);
+                    if (v.x > t_hi) { ah += h0; al += l0; } else if (v.x >= tl) mk |= 1u << (4 * j);
+                    if (v.y > t_hi) { ah += h1; al += l1; } else if (v.y >= tl) mk |= 2u << (4 * j);
+                }
+                m2(v.z, v.w, hi, lo);
+                sh = add2(sh, hi); sl = add2(sl, lo);
+                if (BAND) {
+                    up2(hi, h0, h1); up2(lo, l0, l1);
+                    if (v.z > t_hi) { ah += h0; al += l0; } else if (v.z >= tl) mk |= 4u << (4 * j);
+                    if (v.w > t_hi) { ah += h1; al += l1; } else if (v.w >= tl) mk |= 8u << (4 * j);
+                }
+            }
+            up2(sh, s0, s1);
+            if (MINP || mend || !__any_sync(0xffffffffu, !(s0 + s1 < 1e9f))) break;
+            mend = true;                                                 // a logit of -inf: once more
+        }
+        float r0, r1;
+        up2(sl, r0, r1);
+        const int ch = __float2int_rn((s0 + s1) * 32768.0f), cl = __float2int_rn(r0 + r1);
+        if (BAND) { all_h += ch; all_l += cl; }
+        const uint32_t wh = __reduce_add_sync(0xffffffffu, (unsigned)(BAND ? __float2int_rn(ah * 32768.0f) : ch));
+        const int wl = (int)__reduce_add_sync(0xffffffffu, (unsigned)(BAND ? __float2int_rn(al) : cl));
+        const u64 q = ((u64)wh << 15) + (u64)(long long)wl;
+        if (lane_id() == 0) csum[k.c] = q;
+        keep += q;
+        if (BAND) list_append(rw.a, list, CL ? WCAP : KCAP, mk, k);
+    });
+    Masses r;
+    r.keep = keep;
+    r.all = BAND ? ((u64)__reduce_add_sync(0xffffffffu, (unsigned)all_h) << 15) + (u64)(long long)(int)__reduce_add_sync(0xffffffffu, (unsigned)all_l) : keep;
+    return r;
+}
+
+// One level of the exact radix select over the order-preserving keys of the logits >= lk: the bins of the keys that begin with
+// `prefix`, by count or by mass.
+template <bool CL, int ELT, bool MASK>
+static __device__ __noinline__ void pass_radix(RowS& rw, const NextRow& nx, MassFn mass, float lk, int lvl, uint32_t prefix, bool by_mass, u64* bins) {
+    const int lane = lane_id(), shift = 24 - 8 * lvl;
+    run_pass<CL, ELT, MASK>(rw, nx, false, 0, THEN_NOTHING, [&](const auto& k) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = k.group(j, CI_NEG_INF);
+#pragma unroll 1
+            for (int e = 0; e < 4; ++e) {
+                const float l = e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w;
+                int bin = -1;
+                if (l >= lk) {
+                    const uint32_t f = f2key(l);
+                    if (lvl == 0 || (f >> (shift + 8)) == prefix) bin = FB_NB - 1 - (int)((f >> shift) & 0xFFu);
+                }
+                // lanes of one bin add once (most keys of a level share a few bins: plain atomics would serialise)
+                const unsigned peers = __match_any_sync(0xffffffffu, bin);
+                const uint32_t w = bin < 0 ? 0u : (by_mass ? mass(l) : 1u);
+                const uint32_t lo = __reduce_add_sync(peers, w & 0xFFFFu), hi = __reduce_add_sync(peers, w >> 16);
+                if (bin >= 0 && lane == __ffs(peers) - 1) atomicAdd(&bins[bin], ((u64)hi << 16) + lo);
+            }
+        }
+    });
+}
+
+// Exact masses of the buckets [w0, w0 + BINS), and the warp's mass above them.
+template <bool CL, int ELT, bool MASK>
+static __device__ __noinline__ u64 pass_window(RowS& rw, const NextRow& nx, MassFn mass, float lk, float href, float scale, int hoff, int w0, u64* bins) {
+    u64 hi = 0;
+    const Buckets bk(href, scale, hoff);
+    run_pass<CL, ELT, MASK>(rw, nx, false, 0, THEN_NOTHING, [&](const auto& k) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = k.group(j, CI_NEG_INF);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (x[e] >= lk) {
+                    const int bb = bk(x[e]);
+                    if (bb < w0) hi += (u64)mass(x[e]);
+                    else if (bb < w0 + BINS) atomicAdd(&bins[bb - w0], (u64)mass(x[e]));
+                }
+            }
+        }
+    });
+    return warp_sum_u64(hi);
+}
+
+// The rarer uses of the passes, as functions of their own.
+// The lowest token of the warp's chunks whose logit is L.
+template <bool CL, int ELT, bool MASK>
+static __device__ __noinline__ int argmax_pass(RowS& rw, const NextRow& nx, float L) {
+    Top m = pass_max<CL, ELT, MASK>(rw, nx, false, THEN_NOTHING);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const float om = __shfl_xor_sync(0xffffffffu, m.l, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, m.idx, o);
+        if (om > m.l || (om == m.l && oi < m.idx)) { m.l = om; m.idx = oi; }
+    }
+    return m.l == L ? m.idx : 0x7fffffff;
+}
+// The histogram counted from the row's maximum.
+template <bool CL, int ELT, bool MASK>
+static __device__ __noinline__ void recount_pass(RowS& rw, const NextRow& nx) {
+    pass_hist<CL, ELT, MASK>(rw, nx, true, 0, THEN_AGAIN, SM_POS_INF, nullptr, 0, rw.L, rw.scw, 0);
+}
+// The logits a large top-k can keep.
+template <bool CL, int ELT, bool MASK>
+static __device__ __noinline__ void relist_pass(RowS& rw, const NextRow& nx, Cand* list, int cap) {
+    pass_list<CL, ELT, MASK>(rw, nx, false, 0, THEN_NEXT_ROW, fmaxf(fmaxf(rw.t_lo, rw.lcut), -SM_FLT_MAX), list, cap);
 }
 
 // A warp's share of a set of listed logits: entries start, start + step, ... below n.
 struct View { const Cand* p; int start, n, step; };
 
-// Selects the logits of the warps' views that can belong to the top kk: BINS linear bins over [max(bound, cut), L] give the
-// bin of the kk-th largest, everything down to it goes to `dst` (at most FCAP, no particular order).  Returns how many, or
-// -1 when the views cannot decide.  Every logit >= bound of the row (CTA's share) is in the views.  complete: nothing that
-// could tie with the kk-th lies outside dst; all_cut: dst holds everything >= cut.  bins zeroed by the caller before its last
-// barrier.  Two __syncthreads.
-__device__ __forceinline__ int select_top(const View& w, float bound, bool bound_is_cut, float cut, float L, int kk, uint32_t* bins, Cand* dst, Sc* sc,
-                                          float& lo_out, float& scale_out, int& bstar_out, bool& complete, bool& all_cut, bool may_be_empty) {
+// Selects the listed logits that can belong to the top kk: BINS linear bins over [max(bound, cut), L] give the bin of the
+// kk-th largest, everything down to it goes to the CTA's candidates (at most FCAP, no particular order).  Returns how many,
+// or -1 when the lists cannot decide.  Every logit >= bound (of the row, or of the CTA's share of it) is in the lists; `few`:
+// fewer than kk of them may reach max(bound, cut).  bins and nsel are zeroed before the caller's last barrier.
+// Two __syncthreads.
+__device__ __forceinline__ int select_top(const View& w, float bound, float cut, float L, int kk, bool few, uint32_t* bins, Sc* sc, float& scale, int& bstar) {
     const int lane = lane_id();
     const float lo = fmaxf(bound, cut);
-    const float scale = L > lo ? (float)(BINS - 2) / (L - lo) : 0.0f;
+    scale = L > lo ? (float)(BINS - 2) / (L - lo) : 0.0f;
     auto bin_of = [&](float l) { return max(0, min(BINS - 1, __float2int_rz((L - l) * scale))); };
     for (int j = w.start; j < w.n; j += w.step) { const float l = w.p[j].l; if (l >= lo) atomicAdd(&bins[padbin(bin_of(l))], 1u); }
-    if (threadIdx.x == 0) sc->nsel = 0;
     __syncthreads();
     uint32_t run_b;
-    int bstar = warp_count_bin(bins, (uint32_t)kk, lane, run_b);     // every warp scans the bins itself
-    lo_out = lo; scale_out = scale;
-    all_cut = false;
+    bstar = warp_count_bin(bins, (uint32_t)kk, lane, run_b);         // every warp scans the bins itself
     int n = (int)run_b;
-    if (!(lo <= L)) { n = may_be_empty ? 0 : -1; bstar = BINS - 1; complete = all_cut = true; }
-    else if (bstar < 0) {
+    if (bstar < 0) {
         // fewer than kk listed logits reach lo: if lo is the cut, fewer than kk logits survive it and top-k removes nothing
-        if (!(lo > bound || bound_is_cut) || (run_b == 0 && !may_be_empty)) n = -1;
+        if (!(lo > bound || few)) n = -1;
         bstar = BINS - 1;
-        complete = all_cut = true;
-    } else {
-        complete = true;                                             // every logit >= lo is listed, every listed one down to bstar taken
     }
-    bstar_out = bstar;
-    if (n > FCAP) n = -1;
+    if (n > FCAP || !(lo <= L)) n = -1;
     if (n > 0) {
         for (int j = w.start; j < w.n; j += w.step) {
             const Cand c = w.p[j];
-            if (c.l >= lo && bin_of(c.l) <= bstar) { const int at = atomicAdd(&sc->nsel, 1); if (at < FCAP) dst[at] = c; }
+            if (c.l >= lo && bin_of(c.l) <= bstar) { const int at = atomicAdd(&sc->nsel, 1); if (at < FCAP) { fin_area()->fc_idx[at] = c.idx; fin_area()->fc_l[at] = c.l; } }
         }
     }
     __syncthreads();
     return n;
 }
 
-// Top-k, top-p and the draw on nc <= FCAP candidates (sc->fo_*, token order), by warp 0.  Writes sc->ok / fin_*.
-static __device__ __noinline__ void finish_warp(int nc, float lo, float scale, int bstar, bool complete, float L, float lcut_in, float tc, const MassFn mass,
-                                                int kk, float topp, float u, Sc* sc) {
+// Candidates in order: every one's rank by descending logit (equal logits: as selected) and by token, a few threads per
+// candidate, and its mass.
+static __device__ __noinline__ void order_candidates(int nc, const MassFn mass) {
+    Sc* sc = scratch();
+    constexpr int TPC = NT / FCAP;                                   // threads per candidate
+    const int i = threadIdx.x / TPC, part = threadIdx.x % TPC;
+    if (threadIdx.x < FCAP) {
+        const int t = threadIdx.x;
+        if (t >= nc) { fin_area()->fc_idx[t] = 0xFFFFFFu; fin_area()->fc_l[t] = CI_NEG_INF; fin_area()->sv_l[t] = CI_NEG_INF; fin_area()->sv_q[t] = 0; fin_area()->so_l[t] = CI_NEG_INF; fin_area()->so_q[t] = 0; }
+        fin_area()->ties[t] = 0;
+    }
+    __syncthreads();
+    // (tokens: their difference saturated to 1; equal logits share a rank and are told apart by arrival)
+    const float my_l = fin_area()->fc_l[i], my_i = (float)fin_area()->fc_idx[i];
+    int rv = 0; float rif = 0.0f;
+    auto sat = [](float d) { float r; asm("add.rn.sat.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(d)); return r; };
+    for (int j = part * 4; j < nc; j += 4 * TPC) {
+        const float4 l = *reinterpret_cast<const float4*>(&fin_area()->fc_l[j]);
+        const uint4 d = *reinterpret_cast<const uint4*>(&fin_area()->fc_idx[j]);
+        rv += (l.x > my_l) + (l.y > my_l) + (l.z > my_l) + (l.w > my_l);
+        rif += sat(my_i - (float)d.x) + sat(my_i - (float)d.y); rif += sat(my_i - (float)d.z) + sat(my_i - (float)d.w);
+    }
+#pragma unroll
+    for (int o = 1; o < TPC; o <<= 1) { rv += __shfl_xor_sync(0xffffffffu, rv, o); rif += __shfl_xor_sync(0xffffffffu, rif, o); }
+    const int ri = (int)rif;
+    const uint32_t q = my_l > CI_NEG_INF ? mass(my_l) : 0u;
+    if (i < nc) {
+        if (part == 0) { rv += atomicAdd(&fin_area()->ties[rv], 1); fin_area()->sv_l[rv] = my_l; fin_area()->sv_q[rv] = q; }
+        else if (part == 1) { fin_area()->so_idx[ri] = fin_area()->fc_idx[i]; fin_area()->so_l[ri] = my_l; fin_area()->so_q[ri] = q; }
+    }
+    __syncthreads();
+}
+
+// Top-k, top-p and the draw on the ordered candidates (every logit of the row >= lo in the bins down to bstar), by one
+// warp.  Writes ok, fin_*.
+static __device__ __noinline__ void finish_warp(float lo, float L, float scale, int bstar, float lcut_in, float tc, int kk, float topp, float u) {
+    Sc* sc = scratch();
     const int lane = lane_id();
-    auto bin_of = [&](float l) { return max(0, min(BINS - 1, __float2int_rz((L - l) * scale))); };
     constexpr int PERC = FCAP / 32;
-    float l[PERC]; uint32_t q[PERC];
-    static_assert(PERC == 4, "the warp sort holds four keys per lane");
-    uint32_t sk[PERC];
+    static_assert(PERC == 4, "128-bit loads");
+    const float4 l4 = *reinterpret_cast<const float4*>(&fin_area()->sv_l[lane * 4]);
+    const uint4 q4 = *reinterpret_cast<const uint4*>(&fin_area()->sv_q[lane * 4]);
+    const float l[4] = {l4.x, l4.y, l4.z, l4.w}; const uint32_t q[4] = {q4.x, q4.y, q4.z, q4.w};
     int surv = 0;
 #pragma unroll
-    for (int t = 0; t < PERC; ++t) {
-        const int e = lane * PERC + t;
-        l[t] = e < nc ? sc->fo_l[e] : CI_NEG_INF;
-        sk[t] = e < nc ? f2key(l[t]) : 0u;
-        surv += (e < nc && l[t] >= lcut_in) ? 1 : 0;
-    }
+    for (int t = 0; t < PERC; ++t) surv += l[t] >= lcut_in && l[t] > CI_NEG_INF ? 1 : 0;
     surv = (int)__reduce_add_sync(0xffffffffu, (unsigned)surv);
-    // the candidates' keys in descending order (absent entries, key 0, come last): the kk-th largest is read off, the
-    // top-p pivot is where the running mass of the sorted candidates reaches its target
-    warp_sort_desc4(sk, lane);
-    auto sorted_at = [&](int pos) {                                  // key at sorted position pos (warp-uniform pos)
-        const int t = pos & 3;
-        const uint32_t mine = t == 0 ? sk[0] : t == 1 ? sk[1] : t == 2 ? sk[2] : sk[3];
-        return __shfl_sync(0xffffffffu, mine, pos >> 2);
-    };
     float cut = lcut_in;
     bool ok = surv > 0;
     if (ok && kk <= surv) {                                          // else fewer than k survive min-p: top-k removes nothing
-        const float lk = key2f(sorted_at(kk - 1));
+        const float lk = fin_area()->sv_l[kk - 1];
         const float ck = lower_logit_for(scale_logit(lk, tc), tc, lk);
-        ok = complete && ck >= lo && bin_of(ck) <= bstar;            // else a tie partner could lie outside the candidates
+        ok = ck >= lo && __float2int_rz((L - ck) * scale) <= bstar;  // else a tie partner could lie outside the candidates
         cut = fmaxf(cut, ck);
-    } else {
-        ok = ok && complete;                                         // every logit >= the min-p cut is a candidate
     }
-#pragma unroll
-    for (int t = 0; t < PERC; ++t) q[t] = l[t] >= cut ? mass(l[t]) : 0u;
     if (ok && topp < 1.0f) {
-        u64 sq[PERC], s = 0;
+        u64 s = 0;
 #pragma unroll
-        for (int t = 0; t < PERC; ++t) {
-            const float sl = sk[t] ? key2f(sk[t]) : CI_NEG_INF;
-            sq[t] = sl >= cut ? (u64)mass(sl) : 0ull;
-            s += sq[t];
-        }
+        for (int t = 0; t < PERC; ++t) s += l[t] >= cut ? (u64)q[t] : 0ull;
         const u64 incl = warp_incl_scan_u64(s, lane);
         const u64 s1 = __shfl_sync(0xffffffffu, incl, 31);
         ok = s1 > 0;
         const u64 target = ceil_target(topp, s1);
         const unsigned hit = __ballot_sync(0xffffffffu, incl >= target);
-        int pos = 0;
-        if (hit) {
-            const int hl = __ffs(hit) - 1;
-            u64 run = incl - s; int tt = 0;
+        const int hl = hit ? __ffs(hit) - 1 : 0;
+        u64 run = incl - s; int tt = 0;
 #pragma unroll
-            for (int t = 0; t < PERC; ++t) { run += sq[t]; if (run >= target) { tt = t; break; } }
-            pos = hl * PERC + __shfl_sync(0xffffffffu, tt, hl);
+        for (int t = PERC - 1; t >= 0; --t) {                        // the first t whose running mass reaches the target
+            u64 r = run;
+#pragma unroll
+            for (int k = 0; k <= t; ++k) r += l[k] >= cut ? (u64)q[k] : 0ull;
+            if (r >= target) tt = t;
         }
-        const float lp = key2f(sorted_at(pos));
+        const float lp = fin_area()->sv_l[hl * PERC + __shfl_sync(0xffffffffu, tt, hl)];
         if (ok) cut = fmaxf(cut, lower_logit_for(scale_logit(lp, tc), tc, lp));
-#pragma unroll
-        for (int t = 0; t < PERC; ++t) q[t] = l[t] >= cut ? q[t] : 0u;
     }
-    u64 s = 0;
-#pragma unroll
-    for (int t = 0; t < PERC; ++t) s += q[t];
+    const float4 ol4 = *reinterpret_cast<const float4*>(&fin_area()->so_l[lane * 4]);
+    const uint4 oq4 = *reinterpret_cast<const uint4*>(&fin_area()->so_q[lane * 4]);
+    const uint32_t o[4] = {ol4.x >= cut ? oq4.x : 0u, ol4.y >= cut ? oq4.y : 0u, ol4.z >= cut ? oq4.z : 0u, ol4.w >= cut ? oq4.w : 0u};
+    const u64 s = ((u64)o[0] + o[1]) + ((u64)o[2] + o[3]);
     const u64 incl = warp_incl_scan_u64(s, lane);
     const u64 tot = __shfl_sync(0xffffffffu, incl, 31);
     ok = ok && tot > 0;
@@ -638,22 +981,10 @@ static __device__ __noinline__ void finish_warp(int nc, float lo, float scale, i
     if (lane == 0) sc->ok = 0;
     __syncwarp();
     if (ok && lane == __ffs(hit) - 1) {
-        u64 run = incl - s; int e = lane * PERC;
-#pragma unroll
-        for (int t = 0; t < PERC; ++t) { run += q[t]; if (run >= target) { e = lane * PERC + t; break; } }
-        sc->fin_token = (int)sc->fo_idx[e]; sc->fin_cut = cut; sc->fin_total = tot; sc->ok = 1;
+        u64 run = incl - s; int e = PERC - 1;
+        for (int t = 0; t < PERC - 1; ++t) { run += o[t]; if (run >= target) { e = t; break; } }
+        sc->fin_token = (int)fin_area()->so_idx[lane * PERC + e]; sc->fin_cut = cut; sc->fin_total = tot; sc->ok = 1;
     }
-}
-
-// Candidates in token order: every candidate's rank among the indices, four threads per candidate.  src: nc <= FCAP entries.
-__device__ __forceinline__ void order_candidates(const Cand* src, int nc, Sc* sc) {
-    const int i = threadIdx.x >> 2, part = threadIdx.x & 3;          // NT / 4 = FCAP candidates
-    const Cand me = i < nc ? src[i] : Cand{0xFFFFFFFFu, 0.0f};
-    int r = 0;
-    for (int j = part; j < nc; j += 4) r += src[j].idx < me.idx ? 1 : 0;
-    r += __shfl_xor_sync(0xffffffffu, r, 1);
-    r += __shfl_xor_sync(0xffffffffu, r, 2);
-    if (part == 0 && i < nc) { sc->fo_idx[r] = me.idx; sc->fo_l[r] = me.l; }
 }
 
 // Exact weighted selection among the listed logits of the warps' views: the value v with W(l > v) < target <= W(l >= v).
@@ -823,10 +1154,64 @@ __device__ __forceinline__ float row_uniform(const Args& a, const RowP* rp, int 
     return 1.0f;
 }
 
-// CL: the launch uses clusters (a.cluster > 1 CTAs per row); ELT: bytes per logit (4 fp32, 2 bf16).
-template <bool CL, int ELT>
+// Where a row lies.
+template <int ELT>
+__device__ __forceinline__ const char* place_row(const Args& a, int row, int& al, uint32_t& end, int& nc) {
+    const u64 addr = reinterpret_cast<u64>(a.logits) + (u64)row * (u64)a.V * ELT;
+    al = (int)((addr & 15) / ELT);
+    end = (uint32_t)((addr + (u64)a.V * ELT + 15) & ~15ull);
+    nc = (a.V + al + CHUNK - 1) / CHUNK;
+    return reinterpret_cast<const char*>(addr & ~15ull);
+}
+// Fills in row number `it` of the CTA from its parameters.  One thread.
+template <int ELT>
+static __device__ __noinline__ void derive_row(const Args& a, int it, int row) {
+    Sc* sc = scratch();
+    const RowP* rp = &sc->rp[it & 1];
+    RowS& rw = sc->rows[it & 1];
+    const int b = a.R == 1 ? row : row / a.R, r = row - b * a.R;
+    rw.base = place_row<ELT>(a, row, rw.a, rw.end, rw.Nc);
+    rw.row = row; rw.key = row + 1;
+    rw.mrow = a.mask ? a.mask + ((size_t)b * a.mask_rows + r) * a.W : nullptr;
+    const int hlen = max(0, min(rp->hlen, a.p.hist_stride));
+    rw.hist = a.p.history ? a.p.history + (size_t)b * a.p.hist_stride : nullptr;
+    rw.hlen = hlen; rw.rp = rp->rp; rw.pp = rp->pp; rw.fp = rp->fp;
+    rw.pen_on = a.p.history != nullptr && hlen > 0 && !(rp->rp == 1.0f && rp->pp == 0.0f && rp->fp == 0.0f);
+    rw.pen_cap = hlen <= 65535 ? PEN_TABLE : 0;                  // (the counts are 16 bits)
+    const int kk = rp->kk;
+    const bool sampled = (rp->T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION);
+    const bool fastk = sampled && kk > 0 && kk <= FASTK && kk < a.V;
+    const bool wide = sampled && !fastk && ((kk > 0 && kk < a.V) || rp->topp < 1.0f);
+    rw.cls = (sampled ? ROW_SAMPLED : 0) | (fastk ? ROW_FASTK : 0) | (wide ? ROW_WIDE : 0);
+    rw.tc = fmaxf(rp->T, 1e-6f); rw.kk = kk; rw.topp = rp->topp; rw.lmp = rp->lmp;
+    rw.scw = (float)NB1 / (RANGE * rw.tc);
+    rw.u = row_uniform(a, rp, r);
+    rw.hist_slow = 0;
+}
+
+// The hardware's queue of the grid's CTAs that have not started: a running CTA asks for the index of one of them, which then
+// never starts (cluster launch control).  One thread; the answer lands in sc->clc.
+__device__ __forceinline__ void queue_ask(Sc* sc) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // (the last answer has been read)
+    mbar_expect_tx(&sc->clc_bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(&sc->clc)), "r"(smem_u32(&sc->clc_bar)) : "memory");
+}
+// The index, -1 when none was left (or the answer does not come).
+__device__ __forceinline__ int queue_answer(Sc* sc, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_test(&sc->clc_bar, parity)) if (clock64() - t0 > WAIT_CYCLES) { sc->dead = 1; return -1; }
+    uint32_t ok, x;
+    asm volatile("{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tld.shared.b128 h, [%2];\n\t"
+                 "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+                 "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+                 : "=r"(ok), "=r"(x) : "r"(smem_u32(&sc->clc)) : "memory");
+    return ok ? (int)x : -1;
+}
+
+// CL: the launch uses clusters (a.cluster > 1 CTAs per row); ELT: bytes per logit (4 fp32, 2 bf16); MASK: it has a grammar mask.
+template <bool CL, int ELT, bool MASK>
 __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constant__ Args a) {
-    constexpr int CHB = CHUNK * ELT;
     const int tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     const int V = a.V;
     Grp<CL> g;
@@ -834,496 +1219,470 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     g.rank = CL ? (int)(blockIdx.x % a.cluster) : 0;
     const int GW = NW * g.C, gw = g.rank * NW + warp;            // warps of the group, this warp among them
 
-    extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char* U = smem + NW * RING;
-    Cand* klist = reinterpret_cast<Cand*>(U);                    // [NW][KCAP]: rows without a histogram, one CTA per row
-    uint32_t* hist = reinterpret_cast<uint32_t*>(U);             // [NB1], else
-    Cand* wlist = reinterpret_cast<Cand*>(U + NB1 * 4);          // [NW][WCAP]
-    Cand* gath = reinterpret_cast<Cand*>(U);                     // [NW][GCAP] lists of all CTAs, over the histogram
-    Cand* push = reinterpret_cast<Cand*>(U);                     // [8][FCAP] candidates of all CTAs, over the histogram
-    uint32_t* bitmap = reinterpret_cast<uint32_t*>(U);           // history bitmap while the tables are built (may reach into bins, csum)
-    uint32_t* sbins = reinterpret_cast<uint32_t*>(smem + a.smem_bins);   // [BINS_PAD] sample
+    Sc* sc = scratch();
+    Cand* klist = reinterpret_cast<Cand*>(smem + OFF_U);         // [NW][KCAP]: rows without a histogram,
+    uint32_t* hist = reinterpret_cast<uint32_t*>(smem + OFF_U);  // or [NB1],
+    Cand* wlist = reinterpret_cast<Cand*>(smem + OFF_U + NB1 * 4);       // [NW][WCAP]
+    Cand* push = reinterpret_cast<Cand*>(smem + OFF_U);          // [8][FCAP] candidates of all CTAs, over the histogram
+    Cand* gath = reinterpret_cast<Cand*>(smem + OFF_U);          // [NW][GCAP] lists of all CTAs, over the histogram
+    uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem + OFF_U);        // history bitmap while the tables are built (may reach over bins and csum)
+    uint32_t* sbins = reinterpret_cast<uint32_t*>(smem + OFF_BINS);      // [BINS_PAD] sample
     uint32_t* fbins = sbins + BINS_PAD;                          // [BINS_PAD] selection
-    Cand* fc = reinterpret_cast<Cand*>(sbins);                   // [FCAP] candidates, over the sample's bins
     u64* bins = reinterpret_cast<u64*>(sbins);                   // [BINS] weighted selections, radix levels
     float* xbuf = reinterpret_cast<float*>(sbins);               // [CHUNK] the chunk the draw falls into
-    u64* csum = reinterpret_cast<u64*>(smem + a.smem_csum);      // [chunks] kept mass per chunk (the CTA's own)
-    Sc* sc = reinterpret_cast<Sc*>(smem + a.smem_sc);
-    unsigned short* pcnt = reinterpret_cast<unsigned short*>(smem + a.smem_pen);   // [PEN_TABLE] (launches with histories)
-    unsigned short* ppos = pcnt + PEN_TABLE;                     // [PEN_TABLE]
-    uint32_t* cpre = reinterpret_cast<uint32_t*>(ppos + PEN_TABLE);    // [chunks + 1]
+    u64* csum = reinterpret_cast<u64*>(smem + OFF_CSUM);         // [chunks] kept mass per chunk (the CTA's own)
 
-    Reader<ELT> rd;
-    rd.lane = lane;
-    rd.stride = GW * CHB;
-    rd.g.buf = smem_u32(smem + warp * RING);
-    rd.g.bar = smem_u32(smem + a.smem_bars) + 16 * warp;
-    rd.g.rem = rd.g.nrem = 0; rd.g.cons = rd.g.iss = 0;
-    rd.g.np = rd.g.nnp = nullptr; rd.g.next_key = 0; rd.g.end = rd.g.nend = 0;
-    rd.g.keep = rd.g.nkeep = false;
-    rd.g.dead = false; rd.g.drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0;
-    const uint32_t conv = rd.g.buf + 2 * CHB;                    // bf16: an fp32 copy of one chunk
+    if (tid == 0) {
+        sc->V = V; sc->W = a.W; sc->GW = GW; sc->rank = g.rank;
+        sc->drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0; sc->dead = 0;
+        sc->pen_off = pen_offset(V, a.p.history != nullptr);
+        sc->flags = 0; sc->nsel = 0;
+    }
     if (lane == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rd.g.bar) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rd.g.bar + 8) : "memory");
+        const uint32_t bar = smem_u32(smem) + OFF_BARS + warp * 16;
+        sc->ring[warp].cons = 0; sc->ring[warp].out = 0; sc->ring[warp].key = 0;
+        sc->wn[warp] = 0; sc->swf[warp] = CI_NEG_INF;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8) : "memory");
         fence_mbar_init();
     }
-    __syncwarp();
+    __syncthreads();
 
     // ---------------------------------------------------------------------------------------- which rows are this group's
-    const long long n_rows = (long long)a.B * a.R;
-    const long long grp = CL ? blockIdx.x / a.cluster : blockIdx.x, n_grp = CL ? gridDim.x / a.cluster : gridDim.x;
-    long long my_n = n_rows > grp ? (n_rows - grp + n_grp - 1) / n_grp : 0;
-    // Rows differ in cost (a wide row takes two or three passes, any other one): every CTA orders them by cost class with one
-    // scan -- the same order in all CTAs -- and takes every gridDim-th entry.
-    const bool dealt = !CL && n_rows > n_grp && n_rows <= BAL_ROWS && gridDim.x >= 128;
+    const int n_rows = a.B * a.R;
+    const int grp = CL ? blockIdx.x / a.cluster : blockIdx.x, n_grp = CL ? gridDim.x / a.cluster : gridDim.x;
+    // Without clusters the grid has a CTA per row, of which as many start as fit; a CTA that is through with its row takes the
+    // next one off the hardware's queue.  Rows differ in cost (a wide row takes two or three passes, any other one): the CTAs'
+    // indices are positions in an order of the rows by cost class, dearest first, which every CTA works out for itself.
+    const bool dealt = !CL && n_rows > 2 * NUM_SM && n_rows <= BAL_ROWS;
+    auto row_class = [&](int row) {
+        const int b = a.R == 1 ? row : row / a.R;
+        const float T = a.p.temperature[b];
+        const int k = a.p.top_k[b];
+        if (!((T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION))) return 2;
+        return (k > 0 && k <= FASTK && k < V) ? 1 : 0;
+    };
+    const int per_thread = (n_rows + NT - 1) / NT;               // consecutive rows per thread
     if (dealt) {
-        auto row_class = [&](int row) {
-            const int b = row / a.R;
-            const float T = a.p.temperature[b];
-            const int k = a.p.top_k[b];
-            if (!((T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION))) return 2;
-            return (k > 0 && k <= FASTK && k < V) ? 1 : 0;
-        };
-        const int per = ((int)n_rows + NT - 1) / NT;             // consecutive rows per thread
-        const int lo = min(tid * per, (int)n_rows), hi = min(lo + per, (int)n_rows);
-        u64 packed = 0;
-        for (int row = lo; row < hi; ++row) packed += 1ull << (21 * row_class(row));
-        if (tid == 0) sc->my_count = 0;
-        u64 tot;
-        u64 ex = block_excl_scan(packed, sc, tot);
-        const int G = (int)gridDim.x;
-        const long long n0 = (long long)(tot & 0x1FFFFFull), n1 = (long long)((tot >> 21) & 0x1FFFFFull);
-        // Wide rows go round the CTAs first; where that round ends some CTAs hold one fewer: those get two small-top-k rows each
-        // before the rest of that class (and then the greedy rows) continue round the CTAs from there.
-        const int r0 = (int)(n0 % G), n_short = r0 ? G - r0 : 0;
-        const long long extra = min(2ll * n_short, n1);
-        for (int row = lo; row < hi; ++row) {
-            const int j = row_class(row);
-            const long long q = (long long)((ex >> (21 * j)) & 0x1FFFFFull);     // position inside the class
-            ex += 1ull << (21 * j);
-            int cta;
-            if (j == 0) cta = (int)(q % G);
-            else if (j == 1) cta = q < extra ? r0 + (int)(q % n_short) : (int)((r0 + q - extra) % G);
-            else cta = (int)((r0 + n1 - extra + q) % G);
-            if (cta == (int)blockIdx.x) sc->my_rows[atomicAdd(&sc->my_count, 1)] = row;   // any order
+        u64 packed = 0, tot;
+#pragma unroll 4
+        for (int j = 0; j < per_thread; ++j) { const int row = tid * per_thread + j; if (row < n_rows) packed += 1ull << (21 * row_class(row)); }
+        const u64 ex = block_excl_scan(packed, sc, tot);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            sc->cls_pre[j][tid] = (unsigned short)((ex >> (21 * j)) & 0x1FFFFFull);
+            if (tid == 0) sc->cls_tot[j] = (int)((tot >> (21 * j)) & 0x1FFFFFull);
         }
         __syncthreads();
-        my_n = sc->my_count;
     }
-    auto row_at = [&](long long it) { return dealt ? (long long)sc->my_rows[it] : grp + it * n_grp; };
-    auto row_base = [&](long long row, int& al, u64& end) {
-        const u64 addr = reinterpret_cast<u64>(a.logits) + (u64)row * (u64)V * ELT;
-        al = (int)((addr & 15) / ELT);
-        end = (addr + (u64)V * ELT + 15) & ~15ull;
-        return reinterpret_cast<const char*>(addr & ~15ull);
+    // The row at a position of that order.  One warp.
+    auto row_of = [&](int pos) {
+        if (!dealt) return pos;
+        int j = 0;
+        while (j < 2 && pos >= sc->cls_tot[j]) { pos -= sc->cls_tot[j]; ++j; }
+        int t = 0;                                               // the last thread with at most pos rows of class j before its own
+#pragma unroll
+        for (int step = NT / 2; step; step >>= 1) if (sc->cls_pre[j][t + step] <= pos) t += step;
+        int left = pos - sc->cls_pre[j][t], row = 0;
+        for (int j0 = 0; j0 < per_thread; j0 += 32) {
+            const int k = t * per_thread + j0 + lane;
+            const unsigned is = __ballot_sync(0xffffffffu, j0 + lane < per_thread && k < n_rows && row_class(k) == j);
+            const int c = __popc(is);
+            if (left < c) {
+                unsigned m = is;
+                for (int q = 0; q < left; ++q) m &= m - 1;
+                row = t * per_thread + j0 + __ffs(m) - 1;
+                break;
+            }
+            left -= c;
+        }
+        return row;
     };
-    auto chunks_of = [&](int al) { return (V + al + CHUNK - 1) / CHUNK; };
-    auto mine_of = [&](int nc) { return gw < nc ? (nc - gw + GW - 1) / GW : 0; };
-
-    if (warp == 0 && my_n > 0) { fetch_params(a, row_at(0), &sc->rp[0], lane); asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-    for (long long it = 0; it < my_n; ++it) {
-        const long long row = row_at(it);
-        const int b = (int)(row / a.R), r = (int)(row % a.R);
-        RowV rw;
-        u64 row_end;
-        const char* base = row_base(row, rw.a, row_end);
-        rw.V = V; rw.Nc = chunks_of(rw.a); rw.W = a.W;
-        rw.mrow = a.mask ? a.mask + ((size_t)b * a.mask_rows + r) * a.W : nullptr;
-        const int nch = mine_of(rw.Nc);
-        const char* first = base + (size_t)gw * CHB;
-        const int key = (int)row + 1;
-        rd.begin(key, first, row_end, nch, true);
-        RowP* rp = &sc->rp[it & 1];
-        if (warp == 0) {
+    // The last warp looks after the row that comes next: takes it off the queue early in the first pass of the row at hand, notes
+    // where it lies, fetches its parameters, and derives the rest before the row at hand ends.
+    constexpr int PW = NW - 1;
+    int next_row = -1;                                           // (the last warp's)
+    auto fetch_row = [&](int it) { fetch_params(a, next_row, &sc->rp[it & 1], lane); asm volatile("cp.async.commit_group;" ::: "memory"); };
+    auto find_next = [&](int it) {                               // number it + 1
+        if (CL) { const int row = grp + (it + 1) * n_grp; next_row = row < n_rows ? row : -1; }
+        else {
+            int pos = -1;
+            if (lane == 0) pos = queue_answer(sc, it & 1);
+            pos = __shfl_sync(0xffffffffu, pos, 0);
+            next_row = pos >= 0 ? row_of(pos) : -1;
+        }
+        if (next_row >= 0) {
+            fetch_row(it + 1);
+            if (lane == 0) {
+                NextRow& nx = sc->next[it & 1];
+                int al;
+                nx.base = place_row<ELT>(a, next_row, al, nx.end, nx.Nc);
+                __threadfence_block();
+                *(volatile int*)&nx.key = next_row + 1;
+            }
+        }
+        __syncwarp();
+    };
+    auto derive = [&](int it) {
+        if (next_row >= 0) {
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncwarp();
-            if (lane == 0) { rp->u = row_uniform(a, rp, r); sc->hist_slow = 0; sc->flags = 0; }
+            if (lane == 0) derive_row<ELT>(a, it, next_row);
         }
-        if (tid < NW) { sc->wn[tid] = 0; sc->swf[tid] = CI_NEG_INF; }
-        __syncthreads();                                         // parameters are here, the previous row's shared memory is free
-        const float T = rp->T;
-        const bool sampled = (T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION);
-        const float tc = fmaxf(T, 1e-6f);
-        const int kk = rp->kk;
-        const float topp = rp->topp;
-        const bool fastk = sampled && kk > 0 && kk <= FASTK && kk < V;
-        bool need_topk = kk > 0 && kk < V;
-        const bool need_topp = topp < 1.0f;
-        const bool wide = sampled && !fastk && (need_topk || need_topp);
-        const bool lists = fastk || wide;
-        Cand* mylist = !fastk ? wlist + warp * WCAP : CL ? push + 8 * FCAP + warp * KCAP_CL : klist + warp * KCAP;
-        const int lcap = !fastk ? WCAP : CL ? KCAP_CL : KCAP;
+    };
+#ifdef COLINFER_PROFILE
+    long long prof_last = clock64();
+#endif
+    if (warp == PW) {
+        next_row = row_of(grp);
+        fetch_row(0);
+        if (lane == 0) { sc->next[0].key = sc->next[1].key = 0; mbar_init(&sc->clc_bar, 1); fence_mbar_init(); }
+        derive(0);
+    }
+    __syncthreads();
+
+    for (int it = 0; ; ++it) {
+        RowS& rw = sc->rows[it & 1];
+        const NextRow& nx = sc->next[it & 1];
+        ring_start<ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW);
+        if (!CL && tid == PW * 32) queue_ask(sc);
+        bool found = false, derived = false;                     // (the last warp's)
+        auto look_ahead = [&]() { if (warp == PW && !found) { find_next(it); found = true; } };
+        auto derive_next = [&]() { if (warp == PW && !derived) { look_ahead(); derive(it + 1); derived = true; if (lane == 0) sc->next[(it + 1) & 1].key = 0; } };
+        SM_PROF(0);
 
         // ------------------------------------------------------------------------------------ penalty tables
-        {
-            const int hlen = max(0, min(rp->hlen, a.p.hist_stride));
-            Pen& pen = rw.pen;
-            pen.hist = a.p.history ? a.p.history + (size_t)b * a.p.hist_stride : nullptr;
-            pen.hlen = hlen;
-            pen.rp = rp->rp; pen.pp = rp->pp; pen.fp = rp->fp;
-            pen.on = pen.hist != nullptr && hlen > 0 && !(pen.rp == 1.0f && pen.pp == 0.0f && pen.fp == 0.0f);
-            pen.pre = cpre; pen.pos = ppos; pen.cnt = pcnt;
-            pen.cap = hlen <= 65535 ? PEN_TABLE : 0;             // (the counts are 16 bits)
-            if (pen.on) {
-                // A bitmap of the history's tokens among the CTA's chunks (position order), popcounts per chunk, their prefix: a
-                // token's rank is its table entry.  The first four ids per thread stay in registers.
-                constexpr int HP = 4;
-                int ht[HP];
+        if (rw.pen_on) {
+            // A bitmap of the history's tokens among the CTA's chunks (position order), popcounts per chunk, their prefix: a
+            // token's rank is its table entry.  The first four ids per thread stay in registers.
+            const PenTab pt = pen_tab(sc);
+            const int hlen = rw.hlen, Nc = rw.Nc, al = rw.a;
+            const int32_t* h = rw.hist;
+            constexpr int HP = 4;
+            int ht[HP];
 #pragma unroll
-                for (int j = 0; j < HP; ++j) { const int i = tid + j * NT; ht[j] = i < hlen ? __ldg(pen.hist + i) : -1; }
-                for (int i = tid; i < rw.Nc * 4; i += NT) reinterpret_cast<uint4*>(bitmap)[i] = make_uint4(0, 0, 0, 0);
-                for (int i = tid; i < PEN_TABLE / 8; i += NT) reinterpret_cast<uint4*>(pcnt)[i] = make_uint4(0, 0, 0, 0);
-                auto mine = [&](int v, int& p) {
-                    if (v < 0 || v >= V) return false;
-                    p = v + rw.a;
-                    return !CL || ((p >> 13) % g.C) == g.rank;   // chunk / 16 mod C
-                };
-                __syncthreads();
-                auto mark = [&](int v) { int p; if (mine(v, p)) atomicOr(&bitmap[p >> 5], 1u << (p & 31)); };
+            for (int j = 0; j < HP; ++j) { const int i = tid + j * NT; ht[j] = i < hlen ? __ldg(h + i) : -1; }
+            for (int i = tid; i < Nc * 4; i += NT) reinterpret_cast<uint4*>(bitmap)[i] = make_uint4(0, 0, 0, 0);
+            for (int i = tid; i < PEN_TABLE / 4; i += NT) reinterpret_cast<uint4*>(pt.ent)[i] = make_uint4(0, 0, 0, 0);
+            auto mine = [&](int v, int& p) {
+                if (v < 0 || v >= V) return false;
+                p = v + al;
+                return !CL || ((p / (CHUNK * NW)) % g.C) == g.rank;
+            };
+            __syncthreads();
+            auto mark = [&](int v) { int p; if (mine(v, p)) atomicOr(&bitmap[p >> 5], 1u << (p & 31)); };
 #pragma unroll
-                for (int j = 0; j < HP; ++j) mark(ht[j]);
-                for (int i = tid + HP * NT; i < hlen; i += NT) mark(__ldg(pen.hist + i));
-                __syncthreads();
-                const int per = (rw.Nc + NT - 1) / NT;
-                const int lo = min(tid * per, rw.Nc), hi = min(lo + per, rw.Nc);
-                auto chunk_pop = [&](int c) {
-                    uint32_t s = 0;
+            for (int j = 0; j < HP; ++j) mark(ht[j]);
+            for (int i = tid + HP * NT; i < hlen; i += NT) mark(__ldg(h + i));
+            __syncthreads();
+            const int per = (Nc + NT - 1) / NT;
+            const int lo = min(tid * per, Nc), hi = min(lo + per, Nc);
+            auto chunk_pop = [&](int c) {
+                uint32_t s = 0;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) { const uint4 x = reinterpret_cast<const uint4*>(bitmap)[c * 4 + k]; s += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w); }
-                    return s;
-                };
-                u64 local = 0, total_bits;
-                for (int c = lo; c < hi; ++c) local += chunk_pop(c);
-                uint32_t run = (uint32_t)block_excl_scan(local, sc, total_bits);
-                for (int c = lo; c < hi; ++c) { cpre[c] = run; run += chunk_pop(c); }
-                if (tid == 0) cpre[rw.Nc] = (uint32_t)total_bits;
-                __syncthreads();
-                auto enter = [&](int v) {
-                    int p;
-                    if (!mine(v, p)) return;
-                    const int c = p >> 9, w = p >> 5;
-                    uint32_t rk = cpre[c] + __popc(bitmap[w] & ((1u << (p & 31)) - 1u));
-                    for (int i = c * 16; i < w; ++i) rk += __popc(bitmap[i]);
-                    if ((int)rk < pen.cap) {
-                        ppos[rk] = (unsigned short)(p & (CHUNK - 1));
-                        atomicAdd(reinterpret_cast<uint32_t*>(pcnt) + (rk >> 1), (rk & 1) ? 65536u : 1u);
-                    }
-                };
+                for (int k = 0; k < 4; ++k) { const uint4 x = reinterpret_cast<const uint4*>(bitmap)[c * 4 + k]; s += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w); }
+                return s;
+            };
+            u64 local = 0, total_bits;
+            for (int c = lo; c < hi; ++c) local += chunk_pop(c);
+            uint32_t run = (uint32_t)block_excl_scan(local, sc, total_bits);
+            for (int c = lo; c < hi; ++c) { pt.pre[c] = run; if (c + 1 < hi) run += chunk_pop(c); }
+            if (tid == 0) pt.pre[Nc] = (uint32_t)total_bits;
+            __syncthreads();
+            const int cap = rw.pen_cap;
+            auto enter = [&](int v) {
+                int p;
+                if (!mine(v, p)) return;
+                const int c = p >> 9, w = p >> 5;
+                uint32_t rk = pt.pre[c] + __popc(bitmap[w] & ((1u << (p & 31)) - 1u));
+                for (int i = c * 16; i < w; ++i) rk += __popc(bitmap[i]);
+                if ((int)rk < cap) {                             // the first to come brings the position along
+                    if (atomicAdd(&pt.ent[rk], 65536u) < 65536u) atomicAdd(&pt.ent[rk], (uint32_t)(p & (CHUNK - 1)));
+                }
+            };
 #pragma unroll
-                for (int j = 0; j < HP; ++j) enter(ht[j]);
-                for (int i = tid + HP * NT; i < hlen; i += NT) enter(__ldg(pen.hist + i));
-                __syncthreads();
-            }
+            for (int j = 0; j < HP; ++j) enter(ht[j]);
+            for (int i = tid + HP * NT; i < hlen; i += NT) enter(__ldg(h + i));
+            __syncthreads();
         }
+        SM_PROF(1);
 
-        // ------------------------------------------------------------------------------------ what the passes ask for next
-        const long long nrow = it + 1 < my_n && !CL ? row_at(it + 1) : -1;
-        if (warp == 0 && it + 1 < my_n) { fetch_params(a, row_at(it + 1), &sc->rp[(it + 1) & 1], lane); asm volatile("cp.async.commit_group;" ::: "memory"); }
-        auto then_next_row = [&]() {
-            if (nrow >= 0) {
-                int al; u64 e2;
-                const char* nb = row_base(nrow, al, e2);
-                rd.then((int)nrow + 1, nb + (size_t)gw * CHB, e2, mine_of(chunks_of(al)), true);
-            }
-        };
-        auto then_this_row = [&]() { rd.then(key, first, row_end, nch, false); };
-
-        // ------------------------------------------------------------------------------------ the sample: list bound, histogram layout
-        float tw = -SM_FLT_MAX;                                  // the CTA's list bound
-        float lref = CI_NEG_INF;                                 // the sample's maximum (the group's): buckets hang from it
-        bool count_hist = false;
-        bool fresh0 = true;                                      // the first chunk has not been read yet
-        const float SCW = (float)NB1 / (RANGE * tc);
-        if (lists) {
-            for (int i = tid; i < 2 * BINS_PAD; i += NT) sbins[i] = 0u;
-            if (wide) for (int i = tid; i < NB1 / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
-            float gm[4] = {CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF};
-            if (nch > 0) {
-                float v[16];
-                bool wrote;
-                const uint32_t mw = rw.mrow ? mask_word(rw, gw, lane) : 0u;
-                rd.wait();
-                read_chunk<ELT>(rw, rd.stage(), conv, gw, true, mw, v, lane, wrote, &sc->hist_slow);
-                fresh0 = false;
+        // ------------------------------------------------------------------------------------ pass 1
+        {
+            const int cls = rw.cls;
+            const bool fastk = (cls & ROW_FASTK) != 0, wide = (cls & ROW_WIDE) != 0, lists = fastk || wide;
+            Cand* list = wlist + warp * WCAP;
+            int lcap = WCAP;
+            float tw = -SM_FLT_MAX;                              // the CTA's list bound
+            float lref = CI_NEG_INF;                             // the sample's maximum (the group's): buckets hang from it
+            bool count_hist = false;
+            int seen = 0;                                        // first chunks of the warp that have been read
+            bool in_klist = fastk;
+            if (lists) {
+                // The sample, the first two chunks of every warp: list bound, histogram layout.
+                for (int i = tid; i < 2 * BINS_PAD; i += NT) sbins[i] = 0u;
+                if (wide) for (int i = tid; i < NB1 / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
+                float gm[8], sm = CI_NEG_INF;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) gm[k] = fmaxf(fmaxf(v[4 * k], v[4 * k + 1]), fmaxf(v[4 * k + 2], v[4 * k + 3]));
-                float sm = fmaxf(fmaxf(gm[0], gm[1]), fmaxf(gm[2], gm[3]));
+                for (int j = 0; j < 8; ++j) gm[j] = CI_NEG_INF;
+                {
+                    Pipe<ELT> p;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int c = gw + j * GW;
+                        if (c >= rw.Nc) continue;
+                        const uint32_t mw = MASK ? mask_word(rw.mrow, a.W, rw.a, c, lane) : 0u;
+                        PenPeek pk = {0, 0, 0};
+                        if (rw.pen_on) pk = pen_peek(pen_tab(sc), rw.pen_cap, c, lane);
+                        bool wrote;
+                        p.wait(j);
+                        const auto k = open_chunk<ELT, MASK>(rw, p.stage(j), p.conv(), c, true, pk.r0 != pk.r1, pk, mw, wrote);
+                        ++seen;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) { gm[4 * j + e] = max4(k.group(e, CI_NEG_INF), CI_NEG_INF); sm = fmaxf(sm, gm[4 * j + e]); }
+                        __syncwarp();
+                    }
+                }
 #pragma unroll
                 for (int o = 16; o; o >>= 1) sm = fmaxf(sm, __shfl_xor_sync(0xffffffffu, sm, o));
                 if (lane == 0) sc->swf[warp] = sm;
+                if (CL && wide) g.sync(); else __syncthreads();
+                // the bins of the bound hang from the smallest finite warp maximum plus 4: a few dominant tokens in the sample
+                // must not stretch them beyond the bulk
+                float hi = CI_NEG_INF, lo = SM_POS_INF;
+                for (int i = lane; i < ((CL && wide) ? GW : NW); i += 32) {
+                    const float x = (CL && wide) ? g.at(sc, i / NW)->swf[i % NW] : sc->swf[i];
+                    hi = fmaxf(hi, x);
+                    if (x > CI_NEG_INF) lo = fminf(lo, x);
+                }
+#pragma unroll
+                for (int o = 16; o; o >>= 1) {
+                    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+                    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                }
+                lref = hi;
+                const float top = fminf(lo + 4.0f, hi);          // +inf when no warp saw a finite logit
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (gm[k] > CI_NEG_INF && top < SM_POS_INF)
+                        atomicAdd(&sbins[padbin(max(0, min(BINS - 1, __float2int_rz((top - gm[k]) * FAST_SCALE))))], 1u);
+                __syncthreads();
+                auto bound = [&](int k) {                        // what at least k logits of the CTA's share reach (-FLT_MAX: unknown)
+                    uint32_t have;
+                    const int bk = warp_count_bin(sbins, (uint32_t)k, lane, have);
+                    return bk >= 0 && bk < BINS - 1 ? top - ((float)(bk + 1) + 0.01f) / FAST_SCALE - fabsf(top) * 1e-6f : -SM_FLT_MAX;
+                };
+                tw = bound(fastk ? rw.kk : 8);
+                if (wide && lref > CI_NEG_INF && lref < SM_POS_INF) {
+                    // A wide row does without a histogram where a list is sure to hold all the mass: what can be kept lies above the
+                    // min-p cut, or the mass horizon, of the sample's maximum (the row's can only be larger), and the sample says
+                    // that this is at most half of what the lists hold.
+                    const float tc = rw.tc;
+                    const float sure = fmaxf(lref + rw.lmp * tc, lref - 22.0f * tc) - fabsf(lref) * 1e-5f - 1e-5f * tc;
+                    const int share = (rw.Nc + g.C - 1) / g.C;   // chunks of the CTA
+                    const float t2 = bound(max(1, (CL ? KCAP_CL : KCAP) * NW * NW / share));
+                    count_hist = !(t2 > -SM_FLT_MAX && t2 < sure);
+                    if (!count_hist) { tw = sure; in_klist = true; }
+                }
+                if (in_klist) { list = CL ? push + 8 * FCAP + warp * KCAP_CL : klist + warp * KCAP; lcap = CL ? KCAP_CL : KCAP; }
+                if (tid == 0) sc->in_klist = in_klist;
+                if (tid == 0) { rw.lref = lref; rw.count_hist = count_hist; }
             }
-            if (CL && wide) g.sync(); else __syncthreads();
-            // the bins of the bound hang from the smallest finite warp maximum plus 4: a few dominant tokens in the sample
-            // must not stretch them beyond the bulk
-            float hi = CI_NEG_INF, lo = SM_POS_INF;
-            for (int i = lane; i < ((CL && wide) ? GW : NW); i += 32) {
-                const float x = (CL && wide) ? g.at(sc, i >> 4)->swf[i & 15] : sc->swf[i];
-                hi = fmaxf(hi, x);
-                if (x > CI_NEG_INF) lo = fminf(lo, x);
+            SM_PROF(2);
+            look_ahead();
+            if (tid == 0) sc->tw = tw;
+            const bool one_pass = !(cls & ROW_SAMPLED) || in_klist;
+            const int then = one_pass ? THEN_NEXT_ROW : THEN_AGAIN;
+            const float t = tw > -SM_FLT_MAX ? tw : SM_POS_INF;  // no bound: nothing is listed
+            const int bad = (lists && !(tw > -SM_FLT_MAX) ? 1 : 0) | (wide && !count_hist ? 4 : 0);
+            Top top1{CI_NEG_INF, 0x7fffffff};
+            if (!lists) top1 = pass_max<CL, ELT, MASK>(rw, nx, !one_pass, then);
+            else if (count_hist) top1.l = pass_hist<CL, ELT, MASK>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF);
+            else top1.l = pass_list<CL, ELT, MASK>(rw, nx, !one_pass, seen, then, t, list, lcap);
+            SM_PROF(3);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                const float om = __shfl_xor_sync(0xffffffffu, top1.l, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, top1.idx, o);
+                if (om > top1.l || (om == top1.l && oi < top1.idx)) { top1.l = om; top1.idx = oi; }
+            }
+            if (lane == 0) {
+                sc->wf[warp] = top1.l; sc->wi[warp] = top1.idx;
+                const int f = bad | (lists && sc->wn[warp] > lcap ? 1 : 0);
+                if (f) atomicOr(&sc->flags, f);
+            }
+        }
+        g.sync();
+
+        // ------------------------------------------------------------------------------------ the row's maximum and cut
+        bool done = true;                                        // the row needs no further pass
+        {
+            const int cls = rw.cls;
+            const bool sampled = (cls & ROW_SAMPLED) != 0, fastk = (cls & ROW_FASTK) != 0, lists = (cls & (ROW_FASTK | ROW_WIDE)) != 0;
+            const bool in_klist = sc->in_klist != 0;
+            Cand* list = !in_klist ? wlist + warp * WCAP : CL ? push + 8 * FCAP + warp * KCAP_CL : klist + warp * KCAP;
+            const int lcap = !in_klist ? WCAP : CL ? KCAP_CL : KCAP;
+            float L = CI_NEG_INF, lo_all = -SM_FLT_MAX;
+            int aidx = 0x7fffffff, fl = 0;
+            for (int i = lane; i < GW; i += 32) {
+                const Sc* ps = g.at(sc, i / NW);
+                const float om = ps->wf[i % NW]; const int oi = ps->wi[i % NW];
+                if (om > L || (om == L && oi < aidx)) { L = om; aidx = oi; }
+                lo_all = fmaxf(lo_all, ps->tw);
+                fl |= ps->flags;
             }
 #pragma unroll
             for (int o = 16; o; o >>= 1) {
-                hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-                lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                const float om = __shfl_xor_sync(0xffffffffu, L, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, aidx, o);
+                if (om > L || (om == L && oi < aidx)) { L = om; aidx = oi; }
+                lo_all = fmaxf(lo_all, __shfl_xor_sync(0xffffffffu, lo_all, o));
+                fl |= __shfl_xor_sync(0xffffffffu, fl, o);
             }
-            lref = hi;
-            const float top = fminf(lo + 4.0f, hi);              // +inf when no warp saw a finite logit
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (gm[k] > CI_NEG_INF && top < SM_POS_INF)
-                    atomicAdd(&sbins[padbin(max(0, min(BINS - 1, __float2int_rz((top - gm[k]) * FAST_SCALE))))], 1u);
-            __syncthreads();
-            uint32_t have;
-            const int bk = warp_count_bin(sbins, (uint32_t)(fastk ? kk : 8), lane, have);
-            if (bk >= 0 && bk < BINS - 1) tw = top - ((float)(bk + 1) + 0.01f) / FAST_SCALE - fabsf(top) * 1e-6f;
-            if (wide && lref > CI_NEG_INF && lref < SM_POS_INF) {
-                // no histogram where the list is sure to hold all the mass: the bound lies below the min-p cut, or the mass
-                // horizon, of the sample's maximum already (the row's can only be larger)
-                const float sure = fmaxf(lref + rp->lmp * tc, lref - 22.0f * tc) - fabsf(lref) * 1e-5f - 1e-5f * tc;
-                count_hist = !(tw > -SM_FLT_MAX && tw < sure);
-            }
-        }
-
-        // ------------------------------------------------------------------------------------ pass 1
-        float lmax = CI_NEG_INF;
-        int lidx = 0x7fffffff;
-        // One pass of the warp over its chunks: f(v, chunk, stage) on every chunk.
-        auto pass = [&](auto f) {
-            uint32_t mw = (rw.mrow && nch > 0) ? mask_word(rw, gw, lane) : 0u;
-            for (int i = 0, c = gw; i < nch; ++i, c += GW) {
-                const uint32_t mcur = mw;
-                if (rw.mrow && i + 1 < nch) mw = mask_word(rw, c + GW, lane);
-                float v[16];
-                bool wrote;
-                const bool fresh = i > 0 || fresh0;
-                if (fresh) rd.wait();
-                const uint32_t st = rd.stage();
-                read_chunk<ELT>(rw, st, conv, c, fresh, mcur, v, lane, wrote, &sc->hist_slow);
-                f(v, c, st);
-                rd.release(wrote || !fresh);
-            }
-            fresh0 = true;
-        };
-        auto pass_max = [&]() {
-            lmax = CI_NEG_INF; lidx = 0x7fffffff;
-            pass([&](const float (&v)[16], int c, uint32_t) {
-                const float m = max16(v);
-                if (m > lmax) {                                  // strict: the first (lowest) position of the maximum stays
-                    lmax = m;
-                    int e = 15;
-#pragma unroll
-                    for (int j = 14; j >= 0; --j) e = v[j] == m ? j : e;
-                    lidx = c * CHUNK - rw.a + pos_of<ELT>(e, lane);
+            const bool lists_ok = lists && !(fl & 1);
+            const bool finite_max = (L > CI_NEG_INF) && (L < SM_POS_INF);
+            if (lists && (a.stats || !finite_max)) {
+                // the lowest index of the maximum, for rows whose pass only listed: from the lists, else from one more pass
+                int x;
+                if (lists_ok && finite_max) {
+                    uint32_t best = 0x7fffffffu;
+                    for (int j = lane; j < min(sc->wn[warp], lcap); j += 32) if (list[j].l == L) best = min(best, list[j].idx);
+                    x = (int)__reduce_min_sync(0xffffffffu, best);
+                } else {
+                    x = argmax_pass<CL, ELT, MASK>(rw, nx, L);
                 }
-            });
-        };
-        auto pass_list = [&](auto hist_tag, float t) {
-            constexpr bool HIST = decltype(hist_tag)::value;
-            pass([&](const float (&v)[16], int c, uint32_t st) {
-                const float m = max16(v);
-                lmax = fmaxf(lmax, m);
-                if (HIST) {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                        if (v[e] > CI_NEG_INF) atomicAdd(&hist[fine_bucket(v[e], lref, SCW, (float)HOFF - 0.5f)], 1u);
-                }
-                if (__ballot_sync(0xffffffffu, m >= t)) {
-                    unsigned mk = 0;
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) mk |= v[e] >= t ? 1u << e : 0u;
-                    list_append<ELT>(rw, mylist, lcap, &sc->wn[warp], mk, st, conv, c, lane);
-                }
-            });
-        };
-        const bool one_pass = !sampled || fastk || (wide && !count_hist && tw > -SM_FLT_MAX);
-        rd.g.keep = !one_pass;
-        if (one_pass) then_next_row(); else then_this_row();
-        if (!lists) pass_max();
-        else if (count_hist) pass_list(BoolTag<true>{}, tw > -SM_FLT_MAX ? tw : SM_POS_INF);
-        else pass_list(BoolTag<false>{}, tw > -SM_FLT_MAX ? tw : SM_POS_INF);
-
-        // ------------------------------------------------------------------------------------ the row's maximum
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const float om = __shfl_xor_sync(0xffffffffu, lmax, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, lidx, o);
-            if (om > lmax || (om == lmax && oi < lidx)) { lmax = om; lidx = oi; }
-        }
-        if (lane == 0) { sc->wf[warp] = lmax; sc->wi[warp] = lidx; }
-        if (lists) {
-            const int bad = (sc->wn[warp] > lcap || !(tw > -SM_FLT_MAX)) ? 1 : 0;
-            const int f = bad | (wide && !count_hist ? 4 : 0);
-            if (lane == 0 && f) atomicOr(&sc->flags, f);
-        }
-        if (lane == 0 && rd.g.dead) atomicOr(&sc->flags, 2);
-        if (tid == 0) sc->tw = tw;
-        g.sync();
-        float L = CI_NEG_INF, lo_all = -SM_FLT_MAX;
-        int aidx = 0x7fffffff, fl = 0;
-        for (int i = lane; i < GW; i += 32) {
-            const Sc* ps = g.at(sc, i >> 4);
-            const float om = ps->wf[i & 15]; const int oi = ps->wi[i & 15];
-            if (om > L || (om == L && oi < aidx)) { L = om; aidx = oi; }
-            lo_all = fmaxf(lo_all, ps->tw);
-            fl |= ps->flags;
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const float om = __shfl_xor_sync(0xffffffffu, L, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, aidx, o);
-            if (om > L || (om == L && oi < aidx)) { L = om; aidx = oi; }
-            lo_all = fmaxf(lo_all, __shfl_xor_sync(0xffffffffu, lo_all, o));
-            fl |= __shfl_xor_sync(0xffffffffu, fl, o);
-        }
-        const bool lists_ok = lists && !(fl & 1);
-        bool hist_ready = count_hist && !(fl & 4) && (L - lref) * SCW < (float)(HOFF - 2);   // the maximum lies inside the buckets
-
-        int status = 0;
-        const bool finite_max = (L > CI_NEG_INF) && (L < SM_POS_INF);
-        if (sampled && !finite_max) status |= COLINFER_ROW_DEGENERATE;
-        float lcut = CI_NEG_INF;
-        u64 total_mass = 0;
-        long long token = -1;
-        bool leader_wrote = false;                               // the draw's warp has stored the token itself
-
-        // The lowest index of the maximum, for rows whose pass only listed: from the lists, else from one more pass.
-        auto find_argmax = [&](bool from_lists) {
-            if (from_lists) {
-                uint32_t best = 0x7fffffffu;
-                for (int j = lane; j < min(sc->wn[warp], lcap); j += 32) if (mylist[j].l == L) best = min(best, mylist[j].idx);
-                lidx = (int)__reduce_min_sync(0xffffffffu, best);
-            } else {
-                rd.begin(key, first, row_end, nch, false);
-                pass_max();
-#pragma unroll
-                for (int o = 16; o; o >>= 1) {
-                    const float om = __shfl_xor_sync(0xffffffffu, lmax, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, lidx, o);
-                    if (om > lmax || (om == lmax && oi < lidx)) { lmax = om; lidx = oi; }
-                }
-                if (lmax != L) lidx = 0x7fffffff;
-            }
-            if (lane == 0) sc->wi[warp] = lidx;
-            g.sync();
-            int x = 0x7fffffff;
-            for (int i = lane; i < GW; i += 32) x = min(x, g.at(sc, i >> 4)->wi[i & 15]);
-            aidx = (int)__reduce_min_sync(0xffffffffu, (unsigned)x);
-        };
-        if (lists && (a.stats || !finite_max)) find_argmax(lists_ok && finite_max);
-        if (aidx == 0x7fffffff) aidx = 0;
-        if (!sampled || !finite_max) token = aidx;
-
-        if (sampled && finite_max) {
-            const float m = scale_logit(L, tc);
-            MassFn mass;
-            mass.init(tc, m);
-            const float thr = __fadd_rn(m, rp->lmp);
-            lcut = lower_logit_for(thr, tc, __fmul_rn(thr, tc));
-            const bool minp = lcut > L - 22.0f * tc - fabsf(L) * 1e-6f;
-            // Logits more than 22 temperatures below the maximum have integer mass 0 (2^30 exp(-22) < 1/2): they can never
-            // be drawn and add nothing to any sum, so every selection works above that horizon.  (A top-k whose k-th
-            // largest lies below it removes nothing that could be drawn.)
-            lcut = fmaxf(lcut, L - 22.0f * tc - fabsf(L) * 1e-6f);
-            const float u = rp->u;
-            bool done = false;
-
-            // -------------------------------------------------------------------------------- finish from the lists
-            // Small top-k rows; and any other row whose bound lies below the cut: every logit that carries mass is listed
-            // (top-k, if any, then removes nothing beyond the list).
-            if (lists_ok && (fastk || lo_all < lcut)) {
-                const int kq = need_topk ? kk : 0x7fffffff;
-                View w{mylist, lane, min(sc->wn[warp], lcap), 32};
-                float lo, scale; int bstar; bool complete, all_cut;
-                bool ok;
-                int n = select_top(w, tw, false, lcut, L, kq, fbins, CL ? push + g.rank * FCAP : fc, sc, lo, scale, bstar, complete, all_cut, CL);
-                const Cand* src = fc;
-                if constexpr (CL) {
-                    // every CTA selects its own top k, its candidates go to the first one, which selects among them
-                    float plo = SM_POS_INF;
-                    const Cand* own = push + g.rank * FCAP;
-                    if (n > 0 && g.rank != 0) for (int i = tid; i < n; i += NT) g.at(push, 0)[g.rank * FCAP + i] = own[i];
-                    if (all_cut) plo = lo;
-                    else for (int i = lane; i < n; i += 32) plo = fminf(plo, own[i].l);
-#pragma unroll
-                    for (int o = 16; o; o >>= 1) plo = fminf(plo, __shfl_xor_sync(0xffffffffu, plo, o));
-                    if (tid == 0) { sc->npush = all_cut || n < 0 || complete ? n : -1; sc->push_lo = plo; sc->ok = 0; }
-                    if (tid < BINS_PAD) fbins[tid] = 0u;
-                    if (NT < BINS_PAD && tid < BINS_PAD - NT) fbins[NT + tid] = 0u;
-                    g.sync();
-                    if (g.rank == 0) {
-                        float bound = CI_NEG_INF; bool every = true; bool good = true;
-                        for (int q = 0; q < g.C; ++q) {
-                            const Sc* ps = g.at(sc, q);
-                            good = good && ps->npush >= 0;
-                            bound = fmaxf(bound, ps->push_lo);
-                            every = every && ps->push_lo <= lcut;
-                        }
-                        if (good) {
-                            const int wpr = NW / g.C, q = warp / wpr, sub = warp % wpr;
-                            View w2{push + q * FCAP, sub * 32 + lane, g.at(sc, q)->npush, 32 * wpr};
-                            n = select_top(w2, bound, every, lcut, L, kq, fbins, fc, sc, lo, scale, bstar, complete, all_cut, false);
-                        } else n = -1;
-                    }
-                    ok = g.rank == 0 && n > 0;
-                } else ok = n > 0;
-                if (ok) {
-                    order_candidates(src, n, sc);
-                    __syncthreads();
-                    if (warp == 0) finish_warp(n, lo, scale, bstar, complete, L, lcut, tc, mass, kq, topp, u, sc);
-                } else if (tid == 0) sc->ok = 0;
+                if (lane == 0) sc->wi[warp] = x;
                 g.sync();
-                const Sc* ps = g.at(sc, 0);
-                done = ps->ok != 0;
-                if (done) { token = ps->fin_token; lcut = ps->fin_cut; total_mass = ps->fin_total; }
-                else hist_ready = hist_ready && !CL;             // (the candidates were pushed over the histogram)
-                if (!done && fastk) hist_ready = false;
-                // (what follows writes sc->ok / push again only after another barrier)
+                x = 0x7fffffff;
+                for (int i = lane; i < GW; i += 32) x = min(x, g.at(sc, i / NW)->wi[i % NW]);
+                aidx = (int)__reduce_min_sync(0xffffffffu, (unsigned)x);
             }
-
-            if (!done) {
-                enum { PATH_PURE = 0, PATH_LIST = 1, PATH_BAND = 2, PATH_FALLBACK = 3 };
-                int path = PATH_PURE;
-                float t_hi = CI_NEG_INF, t_lo = SM_POS_INF;
-                int band_top = 0, band_bot = 0;                  // buckets the band covers (from, to)
-                // Bucket b holds the logits in (edge(b + 1), edge(b)].
-                auto zero_hist = [&]() { for (int i = tid; i < NB1 / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0); };
-                float href = lref; int hoff = HOFF;
-                if (need_topk || need_topp) {
-                    if (!hist_ready) {
-                        // ------------------------------------------------------------------------ the histogram, from the row's maximum
-                        href = L; hoff = 0;
-                        if (CL) g.sync(); else __syncthreads();  // nobody reads the lists or candidates over it any more
-                        zero_hist();
-                        __syncthreads();
-                        rd.begin(key, first, row_end, nch, true);
-                        then_this_row();
-                        pass([&](const float (&v)[16], int, uint32_t) {
+            if (aidx == 0x7fffffff) aidx = 0;
+            const float tc = rw.tc;
+            float lcut = CI_NEG_INF, horizon = CI_NEG_INF;
+            MassFn mass;
+            mass.tc = tc; mass.rinv = 0.0f; mass.m = 0.0f;
+            const bool go = sampled && finite_max;
+            if (go) {
+                const float m = scale_logit(L, tc);
+                mass.init(tc, m);
+                if (rw.lmp > CI_NEG_INF) {
+                    const float thr = __fadd_rn(m, rw.lmp);
+                    lcut = lower_logit_for(thr, tc, __fmul_rn(thr, tc));
+                }
+                // Logits more than 22 temperatures below the maximum have integer mass 0 (2^30 exp(-22) < 1/2): they can never
+                // be drawn and add nothing to any sum, so every selection works above that horizon.  (A top-k whose k-th
+                // largest lies below it removes nothing that could be drawn.)
+                horizon = L - 22.0f * tc - fabsf(L) * 1e-6f;
+            }
+            if (tid == 0) {
+                rw.L = L; rw.aidx = aidx; rw.status = sampled && !finite_max ? COLINFER_ROW_DEGENERATE : 0;
+                rw.hist_ready = rw.count_hist && !(fl & 4) && !fastk && (L - rw.lref) * rw.scw < (float)(HOFF - 2);   // the maximum lies inside the buckets
+                rw.minp = lcut > horizon;
+                rw.lcut = fmaxf(lcut, horizon); rw.horizon = horizon; rw.mass = mass;
+                rw.drawn = 0; rw.token = aidx; rw.total = 0; rw.listed = 0;
+            }
+            lcut = fmaxf(lcut, horizon);
+            SM_PROF(4);
+            if (go) {
+                done = false;
+                // ---------------------------------------------------------------------------- finish from the lists
+                // Small top-k rows; and any other row whose bound lies below the cut: every logit that carries mass is listed
+                // (top-k, if any, then removes nothing beyond the list).
+                if (lists_ok && (fastk || lo_all < lcut)) {
+                    const int kq = rw.kk > 0 && rw.kk < V ? rw.kk : 0x7fffffff;
+                    const View w{list, lane, min(sc->wn[warp], lcap), 32};
+                    float scale, lo = fmaxf(lo_all, lcut); int bstar;
+                    const float tw = sc->tw;
+                    int n = select_top(w, tw, lcut, L, kq, CL && tw <= lcut, fbins, sc, scale, bstar);
+                    if constexpr (CL) {
+                        // every CTA selects its own top k; its candidates go to the first one, which selects among them
+                        if (n > 0) {
+                            Cand* to = g.at(push, 0) + g.rank * FCAP;
+                            for (int i = tid; i < n; i += NT) to[i] = Cand{fin_area()->fc_idx[i], fin_area()->fc_l[i]};
+                        }
+                        float plo = SM_POS_INF;                  // the value down to which they are complete
+                        if (bstar == BINS - 1) plo = fmaxf(tw, lcut);
+                        else for (int i = lane; i < n; i += 32) plo = fminf(plo, fin_area()->fc_l[i]);
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) if (v[e] > CI_NEG_INF) atomicAdd(&hist[fine_bucket(v[e], href, SCW, -0.5f)], 1u);
-                        });
+                        for (int o = 16; o; o >>= 1) plo = fminf(plo, __shfl_xor_sync(0xffffffffu, plo, o));
+                        for (int i = tid; i < BINS_PAD; i += NT) fbins[i] = 0u;
+                        __syncthreads();
+                        if (tid == 0) { sc->npush = n; sc->push_lo = plo; sc->nsel = 0; }
                         g.sync();
+                        if (g.rank == 0) {
+                            lo = lcut;
+                            bool good = true;
+                            for (int q = 0; q < g.C; ++q) { const Sc* ps = g.at(sc, q); good = good && ps->npush >= 0; lo = fmaxf(lo, ps->push_lo); }
+                            n = -1;
+                            if (good) {
+                                const int wpr = NW / g.C, q = warp / wpr;
+                                const View w2{push + q * FCAP, (warp % wpr) * 32 + lane, g.at(sc, q)->npush, 32 * wpr};
+                                n = select_top(w2, lo, lcut, L, kq, lo <= lcut, fbins, sc, scale, bstar);
+                            }
+                        }
                     }
-                    auto bucket1 = [&](float x) { return fine_bucket(x, href, SCW, (float)hoff - 0.5f); };
-                    auto edge = [&](int bb) { return href - (float)(bb - hoff) / SCW; };
-                    // the histogram counts every finite logit; buckets wholly below the cut are left out
-                    const int b_cut = bucket1(lcut);
-                    const float dL = (L - href) / tc;
-                    auto mass_est = [&](int i) {
-                        return (u64)__float2uint_rn(exp2f(fminf(0.0f, -(((float)(i - hoff) + 0.5f) * (RANGE / (float)NB1) + dL) * CI_LOG2E)) * CI_MASS_SCALE);
-                    };
-                    // 700: how far down the lists reach in a small nucleus (~ 44 per warp)
-                    const FineDecision fd = fine_decide<CL>(g, hist, mass_est, b_cut, need_topk ? (u64)kk : 0ull, 700ull, topp, need_topp, sc);
-                    if (need_topk && (u64)kk >= fd.total_cnt) need_topk = false;   // at most k reach the cut's bucket: top-k removes nothing
-                    if (need_topk) {
+                    if (g.rank == 0) {
+                        if (n > 0) {
+                            order_candidates(n, mass);
+                            if (warp == 0) finish_warp(lo, L, scale, bstar, lcut, tc, kq, rw.topp, rw.u);
+                        } else if (tid == 0) sc->ok = 0;
+                    }
+                    derive_next();
+                    g.sync();
+                    const Sc* ps = g.at(sc, 0);
+                    done = ps->ok != 0;
+                    if (tid == 0) {
+                        if (done) { rw.token = ps->fin_token; rw.lcut = ps->fin_cut; rw.total = ps->fin_total; }
+                        if (CL) rw.hist_ready = 0;               // (candidates lie over the histogram)
+                        // lists that hold all the mass, too long for the one-warp finish: selected on as they are
+                        if (!CL && !done && !fastk && in_klist) { rw.path = PATH_LIST; rw.listed = 1; rw.t_lo = lo_all; }
+                    }
+                }
+            }
+        }
+        SM_PROF(5);
+
+        if (!done) {
+            // -------------------------------------------------------------------------------- how the row is cut
+            __syncthreads();                                     // (the first thread's notes on the row)
+            auto need_topk = [&]() { return rw.kk > 0 && rw.kk < V; };
+            if (rw.listed) {
+            } else if (need_topk() || rw.topp < 1.0f) {
+                if (!rw.hist_ready) {
+                    // the histogram, from the row's maximum
+                    if (CL) g.sync(); else __syncthreads();      // nobody reads the lists over it any more
+                    for (int i = tid; i < NB1 / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
+                    __syncthreads();
+                    recount_pass<CL, ELT, MASK>(rw, nx);
+                    g.sync();
+                }
+                const bool ready = rw.hist_ready != 0;
+                const float href = ready ? rw.lref : rw.L; const int hoff = ready ? HOFF : 0;
+                const float lcut = rw.lcut, scw = rw.scw;
+                const Buckets bucket(href, scw, hoff);
+                // the histogram counts every logit; buckets wholly below the cut are left out
+                const int b_cut = bucket(lcut);
+                const float dL = (rw.L - href) / rw.tc;
+                auto mass_est = [&](int i) {                     // (the last bucket holds everything beyond)
+                    return i == NB1 - 1 ? 0ull : (u64)__float2uint_rn(exp2f(fminf(0.0f, -(((float)(i - hoff) + 0.5f) * (RANGE / (float)NB1) + dL) * CI_LOG2E)) * CI_MASS_SCALE);
+                };
+                // 500: how far down the lists reach in a small nucleus (they hold ~ 750)
+                const FineDecision fd = fine_decide<CL>(g, hist, mass_est, b_cut, need_topk() ? (u64)rw.kk : 0ull, 500ull, rw.topp, rw.topp < 1.0f, sc);
+                if (tid == 0) {
+                    auto edge = [&](int bb) { return href - (float)(bb - hoff) / scw; };
+                    int path = PATH_PURE;
+                    float t_hi = CI_NEG_INF, t_lo = SM_POS_INF;
+                    int band_top = 0, band_bot = 0;
+                    const bool topk = need_topk() && (u64)rw.kk < fd.total_cnt;  // else at most k reach the cut's bucket: top-k removes nothing
+                    if (topk) {
                         // (bucket 0 of a histogram laid out from the sample may hold logits from far above it)
-                        if (fd.b_k < (hist_ready ? 1 : 0) || fd.b_k >= NB1 - 3 || fd.n_upto > (u64)LIST_MAX) path = PATH_FALLBACK;
-                        else { path = PATH_LIST; t_lo = edge(fd.b_k + 2) - 0.01f / SCW - fabsf(href) * 1e-6f; }
-                    } else if (need_topp) {
+                        if (fd.b_k < (ready ? 1 : 0) || fd.b_k >= NB1 - 3 || fd.n_upto > (u64)LIST_MAX) path = PATH_FALLBACK;
+                        else { path = PATH_LIST; t_lo = edge(fd.b_k + 2) - 0.01f / scw - fabsf(href) * 1e-6f; }
+                    } else if (rw.topp < 1.0f) {
                         const int bp = fd.b_p, bcap = fd.b_cap;
-                        const int up = ELT == 2 ? 3 : 1, dn = ELT == 2 ? 4 : 2;
-                        if (fd.est_total == 0 || bp < (hist_ready ? 1 : 0)) path = PATH_FALLBACK;
+                        const int up = ELT == 2 ? 3 : 1, dn = ELT == 2 ? 4 : 1;
+                        if (fd.est_total == 0 || bp < (ready ? 1 : 0)) path = PATH_FALLBACK;
                         else if (bcap < 0 || bcap > bp + dn + 1) {
                             // small nucleus: list everything down to well below the estimated pivot; nothing is "above"
                             path = PATH_BAND;
@@ -1337,7 +1696,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                             t_lo = edge(bp + dn + 1);
                             band_top = max(0, bp - up); band_bot = bp + dn;
                             if (a.flags & COLINFER_TEST_MISS_BAND) {     // test hook: a band eight buckets off (above or below by row parity)
-                                const int s8 = (row & 1) ? 8 : -8;
+                                const int s8 = (rw.row & 1) ? 8 : -8;
                                 if (bp - up + s8 > 0 && bp + dn + s8 + 2 < NB1) {
                                     t_hi = edge(bp - up + s8); t_lo = edge(bp + dn + 1 + s8);
                                     band_top = bp - up + s8; band_bot = bp + dn + s8;
@@ -1345,349 +1704,318 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                             }
                         }
                     }
+                    rw.path = path; rw.t_hi = t_hi; rw.t_lo = t_lo; rw.band_top = band_top; rw.band_bot = band_bot; rw.href = href; rw.hoff = hoff;
                 }
-                const float lk = fmaxf(lcut, -SM_FLT_MAX);
-                if (CL) g.sync(); else __syncthreads();          // (the finds are read, the lists are free)
-                auto zero_csum = [&]() { for (int c = tid; c < rw.Nc; c += NT) csum[c] = 0; };
-                // adds the listed logits that survive `cut` to their chunks' kept masses (the CTA's own lists)
-                auto keep_listed = [&](const Cand* list, int n, float cut) {
-                    for (int j = lane; j < n; j += 32) {
-                        const Cand c = list[j];
-                        if (c.l >= cut) { const uint32_t q = mass(c.l); if (q) atomicAdd(&csum[(c.idx + rw.a) / CHUNK], (u64)q); }
-                    }
-                };
-                // the warps' view of the listed logits of all CTAs (n < 0: a list overflowed)
-                auto view_all = [&](Cand* list, int cap, bool& over) {
-                    View w{list, lane, 0, 32};
-                    over = false;
-                    if constexpr (CL) {
-                        int n = 0;
-                        for (int q = 0; q < g.C; ++q) {
-                            const int c = g.at(sc, q)->wn[warp];
-                            const Cand* src = g.at(list, q);
-                            if (c > cap) over = true;
-                            for (int j = lane; j < min(c, cap); j += 32) if (n + j < GCAP) gath[warp * GCAP + n + j] = src[j];
-                            n += min(c, cap);
-                        }
-                        if (n > GCAP) over = true;
-                        w.p = gath + warp * GCAP; w.n = min(n, GCAP);
-                        __syncwarp();
-                    } else {
-                        w.n = min(sc->wn[warp], cap);
-                        over = sc->wn[warp] > cap;
-                    }
-                    over = __syncthreads_or(over) != 0;
-                    return w;
-                };
+            } else if (tid == 0) { rw.path = PATH_PURE; rw.t_hi = CI_NEG_INF; rw.t_lo = SM_POS_INF; }
+            if (CL) g.sync(); else __syncthreads();              // (the path is known, the finds are read, the lists are free)
+            SM_PROF(6);
 
-                // ---------------------------------------------------------------------------- large top-k (then top-p) on a list
-                if (path == PATH_LIST) {
-                    const float tl = fmaxf(fmaxf(t_lo, lcut), -SM_FLT_MAX);
-                    mylist = CL ? wlist + warp * WCAP : klist + warp * KCAP;
-                    const int cap = CL ? WCAP : KCAP;
+            // adds the listed logits that survive `cut` to their chunks' kept masses (the warp's own list)
+            auto keep_listed = [&](const Cand* list, int cap, float cut, const MassFn& mass) {
+                for (int j = lane; j < min(sc->wn[warp], cap); j += 32) {
+                    const Cand c = list[j];
+                    if (c.l >= cut) { const uint32_t q = mass(c.l); if (q) atomicAdd(&csum[(c.idx + rw.a) / CHUNK], (u64)q); }
+                }
+            };
+            // the warps' view of the listed logits of all CTAs; over: a list overflowed
+            auto view_all = [&](Cand* list, int cap, bool& over) {
+                View w{list, lane, 0, 32};
+                over = false;
+                if constexpr (CL) {
+                    int n = 0;
+                    for (int q = 0; q < g.C; ++q) {
+                        const int c = g.at(sc, q)->wn[warp];
+                        const Cand* src = g.at(list, q);
+                        if (c > cap) over = true;
+                        for (int j = lane; j < min(c, cap); j += 32) if (n + j < GCAP) gath[warp * GCAP + n + j] = src[j];
+                        n += min(c, cap);
+                    }
+                    if (n > GCAP) over = true;
+                    w.p = gath + warp * GCAP; w.n = min(n, GCAP);
+                    __syncwarp();
+                } else {
+                    w.n = min(sc->wn[warp], cap);
+                    over = sc->wn[warp] > cap;
+                }
+                over = __syncthreads_or(over) != 0;
+                return w;
+            };
+            // Exact radix select over the keys, four 8-bit levels, one pass each, above lcut.  by_mass: the top-p pivot; else
+            // the kk-th largest.  False when the filter removes nothing.
+            auto radix_select = [&](bool by_mass, float& pivot) {
+                uint32_t prefix = 0;
+                u64 target = by_mass ? 0 : (u64)rw.kk;
+                for (int lvl = 0; lvl < 4; ++lvl) {
+                    g.sync();
+                    for (int i = tid; i < FB_NB; i += NT) bins[i] = 0;
+                    __syncthreads();
+                    pass_radix<CL, ELT, MASK>(rw, nx, rw.mass, fmaxf(rw.lcut, -SM_FLT_MAX), lvl, prefix, by_mass, bins);
+                    g.sync();
+                    auto level = [&](int i) { u64 s = 0; for (int q = 0; q < (CL ? g.C : 1); ++q) s += g.at(bins, q)[i]; return s; };
+                    int b_star; u64 before, grand;
+                    if (lvl == 0) {
+                        bins_find(level, FB_NB, 0, sc, b_star, before, grand);
+                        if (by_mass) target = ceil_target(rw.topp, grand);
+                        else if (target >= grand) return false;
+                        if (grand == 0) return false;
+                        __syncthreads();
+                    }
+                    bins_find(level, FB_NB, target, sc, b_star, before, grand);
+                    if (b_star < 0) return false;
+                    target -= before;
+                    prefix = (prefix << 8) | (uint32_t)(FB_NB - 1 - b_star);
+                }
+                pivot = key2f(prefix);
+                return true;
+            };
+            // raises the cut to a pivot (ties at the pivot are kept)
+            auto raise_cut = [&](float pivot) {
+                const float cut = fmaxf(rw.lcut, lower_logit_for(scale_logit(pivot, rw.tc), rw.tc, pivot));
+                __syncthreads();
+                if (tid == 0) rw.lcut = cut;
+                __syncthreads();
+            };
+
+            // -------------------------------------------------------------------------------- large top-k (then top-p) on a list
+            if (rw.path == PATH_LIST) {
+                Cand* list = CL ? wlist + warp * WCAP : klist + warp * KCAP;
+                constexpr int cap = CL ? WCAP : KCAP;
+                for (int c = tid; c < rw.Nc; c += NT) csum[c] = 0;
+                if (!rw.listed) {
                     if (lane == 0) sc->wn[warp] = 0;
                     __syncwarp();
-                    zero_csum();
-                    rd.begin(key, first, row_end, nch, false);
-                    then_next_row();
-                    pass([&](const float (&v)[16], int c, uint32_t st) {
-                        if (__ballot_sync(0xffffffffu, max16(v) >= tl)) {
-                            unsigned mk = 0;
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) mk |= v[e] >= tl ? 1u << e : 0u;
-                            list_append<ELT>(rw, mylist, cap, &sc->wn[warp], mk, st, conv, c, lane);
-                        }
-                    });
-                    g.sync();
-                    bool over;
-                    View w = view_all(mylist, cap, over);
-                    float cut = fmaxf(lcut, -SM_FLT_MAX);
-                    bool ok = !over;
-                    const float scale = (float)(BINS - 2) / fmaxf(L - tl, 1e-30f);
-                    if (ok) {
-                        u64 cnt = 0, surv;
-                        for (int j = w.start; j < w.n; j += w.step) cnt += w.p[j].l >= cut ? 1 : 0;
-                        block_excl_scan(cnt, sc, surv);
-                        ok = surv > 0;
-                        if (ok && (u64)kk <= surv) {             // else fewer than k survive min-p: top-k removes nothing
-                            float lkk; u64 tot;
-                            const float c0 = cut;
-                            ok = list_select(w, [&](float l) { return (u64)(l >= c0 ? 1 : 0); }, L, scale, (u64)kk, bins, sc, lkk, tot);
-                            if (ok) { cut = fmaxf(cut, lower_logit_for(scale_logit(lkk, tc), tc, lkk)); ok = cut >= tl; }   // else a tie partner could lie outside the list
-                        }
-                    }
-                    if (ok && need_topp) {
+                    relist_pass<CL, ELT, MASK>(rw, nx, list, cap);
+                }
+                g.sync();
+                const MassFn mass = rw.mass;
+                const float tc = rw.tc, tl = fmaxf(fmaxf(rw.t_lo, rw.lcut), -SM_FLT_MAX);
+                bool over;
+                const View w = view_all(list, cap, over);
+                float cut = fmaxf(rw.lcut, -SM_FLT_MAX);
+                bool ok = !over;
+                const float L = rw.L, scale = (float)(BINS - 2) / fmaxf(L - tl, 1e-30f);
+                if (ok) {
+                    u64 cnt = 0, surv;
+                    for (int j = w.start; j < w.n; j += w.step) cnt += w.p[j].l >= cut ? 1 : 0;
+                    block_excl_scan(cnt, sc, surv);
+                    ok = surv > 0;
+                    if (ok && need_topk() && (u64)rw.kk <= surv) {   // else fewer than k survive min-p: top-k removes nothing
+                        float lkk; u64 tot;
                         const float c0 = cut;
-                        u64 part = 0, s1;
-                        for (int j = w.start; j < w.n; j += w.step) part += w.p[j].l >= c0 ? (u64)mass(w.p[j].l) : 0ull;
-                        block_excl_scan(part, sc, s1);
-                        ok = s1 > 0;
-                        if (ok) {
-                            float lp; u64 tot;
-                            ok = list_select(w, [&](float l) { return l >= c0 ? (u64)mass(l) : 0ull; }, L, scale, ceil_target(topp, s1), bins, sc, lp, tot);
-                            if (ok) { cut = fmaxf(cut, lower_logit_for(scale_logit(lp, tc), tc, lp)); ok = cut >= tl; }
-                        }
-                    }
-                    if (ok) { lcut = cut; keep_listed(mylist, min(sc->wn[warp], cap), cut); }
-                    else path = PATH_FALLBACK;
-                }
-
-                // ---------------------------------------------------------------------------- exact radix select over the keys
-                // Four 8-bit levels, one pass each.  by_mass: the top-p pivot; else the kk-th largest.  False when the filter
-                // removes nothing.
-                auto radix_select = [&](bool by_mass, float& pivot) {
-                    const float lkr = fmaxf(lcut, -SM_FLT_MAX);
-                    uint32_t prefix = 0;
-                    u64 target = by_mass ? 0 : (u64)kk;
-                    for (int lvl = 0; lvl < 4; ++lvl) {
-                        const int shift = 24 - 8 * lvl;
-                        g.sync();
-                        for (int i = tid; i < FB_NB; i += NT) bins[i] = 0;
-                        __syncthreads();
-                        rd.begin(key, first, row_end, nch, false);
-                        pass([&](const float (&v)[16], int, uint32_t) {
-                            for (int e = 0; e < 16; ++e) {
-                                float l = v[0];
-#pragma unroll
-                                for (int j = 1; j < 16; ++j) l = e == j ? v[j] : l;
-                                int bin = -1;
-                                if (l >= lkr) {
-                                    const uint32_t key = f2key(l);
-                                    if (lvl == 0 || (key >> (shift + 8)) == prefix) bin = FB_NB - 1 - (int)((key >> shift) & 0xFFu);
-                                }
-                                // lanes of one bin add once (most keys of a level share a few bins: plain atomics would serialise)
-                                const unsigned peers = __match_any_sync(0xffffffffu, bin);
-                                const uint32_t w = bin < 0 ? 0u : (by_mass ? mass(l) : 1u);
-                                const uint32_t lo = __reduce_add_sync(peers, w & 0xFFFFu), hi = __reduce_add_sync(peers, w >> 16);
-                                if (bin >= 0 && lane == __ffs(peers) - 1) atomicAdd(&bins[bin], ((u64)hi << 16) + lo);
-                            }
-                        });
-                        g.sync();
-                        auto level = [&](int i) { u64 s = 0; for (int q = 0; q < (CL ? g.C : 1); ++q) s += g.at(bins, q)[i]; return s; };
-                        int b_star; u64 before, grand;
-                        if (lvl == 0) {
-                            bins_find(level, FB_NB, 0, sc, b_star, before, grand);
-                            if (by_mass) target = ceil_target(topp, grand);
-                            else if (target >= grand) return false;
-                            if (grand == 0) return false;
-                            __syncthreads();
-                        }
-                        bins_find(level, FB_NB, target, sc, b_star, before, grand);
-                        if (b_star < 0) return false;
-                        target -= before;
-                        prefix = (prefix << 8) | (uint32_t)(FB_NB - 1 - b_star);
-                    }
-                    pivot = key2f(prefix);
-                    return true;
-                };
-                if (path == PATH_FALLBACK) {
-                    status |= COLINFER_ROW_SELECT_SLOW;
-                    float lpiv;
-                    if (kk > 0 && kk < V && radix_select(false, lpiv)) lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
-                    if (need_topp && radix_select(true, lpiv)) lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
-                    path = PATH_PURE;
-                }
-
-                // ---------------------------------------------------------------------------- mass pass: kept mass per chunk
-                // What bounds it: ~ 14 issue slots and one exponential per logit.
-                if (path != PATH_LIST) {
-                    mylist = wlist + warp * WCAP;
-                    Mass2 m2;
-                    m2.init(mass);
-                    for (int attempt = 0; attempt < 3; ++attempt) {
-                        const float lk3 = fmaxf(lcut, -SM_FLT_MAX);
-                        const bool band = path == PATH_BAND;
-                        uint32_t all_hi = 0, all_lo = 0;
-                        u64 keep = 0;                            // lane 0: the warp's kept mass
-                        const float tl = fmaxf(t_lo, lk3);
-                        if (lane == 0) sc->wn[warp] = 0;
-                        __syncwarp();
-                        auto mass_pass = [&](auto band_tag, auto minp_tag) {
-                            constexpr bool BAND = decltype(band_tag)::value;
-                            constexpr bool MINP = decltype(minp_tag)::value;
-                            pass([&](const float (&v)[16], int c, uint32_t st) {
-                                uint32_t hi = 0, lo = 0, ahi = 0, alo = 0;
-                                unsigned mk = 0;
-#pragma unroll
-                                for (int e = 0; e < 16; e += 2) {
-                                    uint32_t h0, h1, l0, l1;
-                                    // logits without mass: below the cut, or -inf
-                                    const float x0 = MINP ? (v[e] >= lk3 ? v[e] : SM_LOW) : fmaxf(v[e], SM_LOW);
-                                    const float x1 = MINP ? (v[e + 1] >= lk3 ? v[e + 1] : SM_LOW) : fmaxf(v[e + 1], SM_LOW);
-                                    m2(x0, x1, h0, h1, l0, l1);
-                                    hi += h0 + h1; lo += l0 + l1;
-                                    if (BAND) {
-                                        if (x0 > t_hi) { ahi += h0 - Mass2::HI0; alo += l0 - Mass2::LO0; }
-                                        else if (x0 >= tl) mk |= 1u << e;
-                                        if (x1 > t_hi) { ahi += h1 - Mass2::HI0; alo += l1 - Mass2::LO0; }
-                                        else if (x1 >= tl) mk |= 2u << e;
-                                    }
-                                }
-                                hi -= 16 * Mass2::HI0; lo -= 16 * Mass2::LO0;
-                                if (BAND) { all_hi += hi; all_lo += lo; hi = ahi; lo = alo; }
-                                const uint32_t chi = __reduce_add_sync(0xffffffffu, hi);
-                                const int clo = (int)__reduce_add_sync(0xffffffffu, lo);
-                                if (lane == 0) { const u64 q = ((u64)chi << 15) + (u64)(long long)clo; csum[c] = q; keep += q; }
-                                if (BAND) list_append<ELT>(rw, mylist, WCAP, &sc->wn[warp], mk, st, conv, c, lane);
-                            });
-                        };
-                        rd.begin(key, first, row_end, nch, false);
-                        then_next_row();
-                        const bool mp = minp || path == PATH_PURE;   // after the fallback the cut is a pivot
-                        if (band) { if (mp) mass_pass(BoolTag<true>{}, BoolTag<true>{}); else mass_pass(BoolTag<true>{}, BoolTag<false>{}); }
-                        else { if (mp) mass_pass(BoolTag<false>{}, BoolTag<true>{}); else mass_pass(BoolTag<false>{}, BoolTag<false>{}); }
-                        if (!band) break;
-                        const u64 wall = ((u64)__reduce_add_sync(0xffffffffu, all_hi) << 15) + (u64)(long long)(int)__reduce_add_sync(0xffffffffu, all_lo);
-                        if (lane == 0) { sc->g_all[warp] = wall; sc->g_keep[warp] = keep; }
-                        g.sync();
-                        u64 s1 = 0, s_above = 0;
-                        for (int i = lane; i < GW; i += 32) { const Sc* ps = g.at(sc, i >> 4); s1 += ps->g_all[i & 15]; s_above += ps->g_keep[i & 15]; }
-                        s1 = warp_sum_u64(s1); s_above = warp_sum_u64(s_above);
-                        bool over;
-                        View w = view_all(mylist, WCAP, over);
-                        const u64 target = ceil_target(topp, s1);
-                        bool ok = !over && s1 > 0 && s_above < target;
-                        if (ok) {
-                            const float bs = t_hi < SM_POS_INF ? t_hi : L;
-                            // (a small nucleus lists everything above the cut: the bins span [cut, base], not [-max, base])
-                            const float scale = (float)(BINS - 2) / fmaxf(bs - fmaxf(t_lo, lk3), 1e-30f);
-                            float lp; u64 s_band;
-                            ok = list_select(w, [&](float l) { return (u64)mass(l); }, bs, scale, target - s_above, bins, sc, lp, s_band);
-                            if (ok) {
-                                const float cut2 = fmaxf(lcut, lower_logit_for(scale_logit(lp, tc), tc, lp));
-                                if (cut2 < t_lo) ok = false;     // a tie partner could lie below the band
-                                else { lcut = cut2; keep_listed(mylist, min(sc->wn[warp], WCAP), lcut); }
-                            }
-                        }
-                        if (ok) break;
-                        status |= COLINFER_ROW_SELECT_SLOW;
-                        bool found_band = false;
-                        if (attempt == 0 && !over && s1 > 0) {
-                            // The estimated band missed the pivot.  Exact masses of the BINS buckets next to the band, on the side
-                            // the pivot lies, give its bucket; the mass pass then runs again around it.
-                            const int w0 = target <= s_above ? max(0, band_top - BINS + 1) : max(0, band_bot);
-                            g.sync();
-                            for (int i = tid; i < BINS; i += NT) bins[i] = 0;
-                            __syncthreads();
-                            u64 hi = 0;
-                            rd.begin(key, first, row_end, nch, false);
-                            pass([&](const float (&v)[16], int, uint32_t) {
-#pragma unroll
-                                for (int e = 0; e < 16; ++e) {
-                                    if (v[e] >= lk3) {
-                                        const int bb = fine_bucket(v[e], href, SCW, (float)hoff - 0.5f);
-                                        if (bb < w0) hi += (u64)mass(v[e]);
-                                        else if (bb < w0 + BINS) atomicAdd(&bins[bb - w0], (u64)mass(v[e]));
-                                    }
-                                }
-                            });
-                            hi = warp_sum_u64(hi);
-                            if (lane == 0) sc->g_all[warp] = hi;
-                            g.sync();
-                            u64 s_hi = 0;
-                            for (int i = lane; i < GW; i += 32) s_hi += g.at(sc, i >> 4)->g_all[i & 15];
-                            s_hi = warp_sum_u64(s_hi);
-                            int bw = -1; u64 bef, tw2;
-                            auto win = [&](int i) { u64 s = 0; for (int q = 0; q < (CL ? g.C : 1); ++q) s += g.at(bins, q)[i]; return s; };
-                            if (target > s_hi) bins_find(win, BINS, target - s_hi, sc, bw, bef, tw2);
-                            g.sync();
-                            if (bw >= 0) {
-                                const int bstar = w0 + bw;
-                                t_hi = bstar - 1 <= 0 ? SM_POS_INF : href - (float)(bstar - 1 - hoff) / SCW;
-                                t_lo = href - (float)(bstar + 2 - hoff) / SCW;
-                                found_band = true;
-                            }
-                        }
-                        if (!found_band) {
-                            // a list overflowed, or the pivot lies far from the estimate: exact radix select by mass
-                            float lpiv;
-                            if (radix_select(true, lpiv)) lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
-                            path = PATH_PURE;
-                        }
-                        g.sync();
+                        ok = list_select(w, [&](float l) { return (u64)(l >= c0 ? 1 : 0); }, L, scale, (u64)rw.kk, bins, sc, lkk, tot);
+                        if (ok) { cut = fmaxf(cut, lower_logit_for(scale_logit(lkk, tc), tc, lkk)); ok = cut >= tl; }   // else a tie partner could lie outside the list
                     }
                 }
+                if (ok && rw.topp < 1.0f) {
+                    const float c0 = cut;
+                    u64 part = 0, s1;
+                    for (int j = w.start; j < w.n; j += w.step) part += w.p[j].l >= c0 ? (u64)mass(w.p[j].l) : 0ull;
+                    block_excl_scan(part, sc, s1);
+                    ok = s1 > 0;
+                    if (ok) {
+                        float lp; u64 tot;
+                        ok = list_select(w, [&](float l) { return l >= c0 ? (u64)mass(l) : 0ull; }, L, scale, ceil_target(rw.topp, s1), bins, sc, lp, tot);
+                        if (ok) { cut = fmaxf(cut, lower_logit_for(scale_logit(lp, tc), tc, lp)); ok = cut >= tl; }
+                    }
+                }
+                if (ok) keep_listed(list, cap, cut, mass);
+                __syncthreads();
+                if (tid == 0) { if (ok) rw.lcut = cut; else rw.path = PATH_FALLBACK; }
+                __syncthreads();
+            }
+            if (rw.path == PATH_FALLBACK) {
+                float lpiv;
+                if (need_topk() && radix_select(false, lpiv)) raise_cut(lpiv);
+                if (rw.topp < 1.0f && radix_select(true, lpiv)) raise_cut(lpiv);
+                __syncthreads();
+                if (tid == 0) { rw.path = PATH_PURE; rw.status |= COLINFER_ROW_SELECT_SLOW; }
+                __syncthreads();
+            }
+            SM_PROF(7);
 
-                // ---------------------------------------------------------------------------- the draw: chunk, then logit
-                g.sync();                                        // the chunks' kept masses are complete
+            // -------------------------------------------------------------------------------- mass pass: kept mass per chunk
+            for (int attempt = 0; rw.path != PATH_LIST && attempt < 3; ++attempt) {
+                // (with one CTA per row the band's list takes the histogram's place: the path is decided)
+                Cand* blist = CL ? wlist + warp * WCAP : klist + warp * KCAP;
+                constexpr int bcap = CL ? WCAP : KCAP;
+                if (lane == 0) sc->wn[warp] = 0;
+                __syncwarp();
                 {
-                    const int per = (rw.Nc + NT - 1) / NT;
-                    const int c_lo = min(tid * per, rw.Nc), c_hi = min(c_lo + per, rw.Nc);
-                    auto kept = [&](int c) { return g.at(csum, CL ? (c >> 4) % g.C : 0)[c]; };
-                    u64 s = 0;
-                    for (int c = c_lo; c < c_hi; ++c) s += kept(c);
-                    const u64 excl = block_excl_scan(s, sc, total_mass);
-                    const u64 target = ceil_target(u, total_mass);
-                    if (total_mass > 0 && excl < target && target <= excl + s) {
-                        u64 run = excl;
-                        for (int c = c_lo; c < c_hi; ++c) {
-                            const u64 q = kept(c);
-                            if (run + q >= target) { sc->x_chunk = c; sc->x_before = run; break; }
-                            run += q;
+                    const float lk3 = fmaxf(rw.lcut, -SM_FLT_MAX), tl = fmaxf(rw.t_lo, lk3), t_hi = rw.t_hi;
+                    const MassFn mass = rw.mass;
+                    const bool mp = rw.minp || lk3 > rw.horizon; // (after the fallback the cut is a pivot)
+                    Masses ms;
+                    if (rw.path == PATH_BAND) {
+                        if (!mp) ms = pass_mass<CL, ELT, MASK, true, false>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
+                        else ms = pass_mass<CL, ELT, MASK, true, true>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
+                        if (lane == 0) { sc->g_all[warp] = ms.all; sc->g_keep[warp] = ms.keep; }
+                    } else if (!mp) pass_mass<CL, ELT, MASK, false, false>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
+                    else pass_mass<CL, ELT, MASK, false, true>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
+                }
+                SM_PROF(8);
+                if (rw.path != PATH_BAND) break;
+                g.sync();
+                u64 s1 = 0, s_above = 0;
+                for (int i = lane; i < GW; i += 32) { const Sc* ps = g.at(sc, i / NW); s1 += ps->g_all[i % NW]; s_above += ps->g_keep[i % NW]; }
+                s1 = warp_sum_u64(s1); s_above = warp_sum_u64(s_above);
+                bool over;
+                const View w = view_all(blist, bcap, over);
+                const u64 target = ceil_target(rw.topp, s1);
+                bool ok = !over && s1 > 0 && s_above < target;
+                if (ok) {
+                    const float t_hi = rw.t_hi, t_lo = rw.t_lo, lcut = rw.lcut;
+                    const MassFn mass = rw.mass;
+                    const float bs = t_hi < SM_POS_INF ? t_hi : rw.L;
+                    // (a small nucleus lists everything above the cut: the bins span [cut, base], not [-max, base])
+                    const float scale = (float)(BINS - 2) / fmaxf(bs - fmaxf(t_lo, lcut), 1e-30f);
+                    float lp; u64 s_band;
+                    ok = list_select(w, [&](float l) { return (u64)mass(l); }, bs, scale, target - s_above, bins, sc, lp, s_band);
+                    if (ok) {
+                        const float cut2 = fmaxf(lcut, lower_logit_for(scale_logit(lp, mass.tc), mass.tc, lp));
+                        if (cut2 < t_lo) ok = false;             // a tie partner could lie below the band
+                        else {
+                            keep_listed(blist, bcap, cut2, mass);
+                            __syncthreads();
+                            if (tid == 0) rw.lcut = cut2;
                         }
                     }
+                }
+                if (ok) break;
+                bool found_band = false;
+                if (attempt == 0 && !over && s1 > 0) {
+                    // The estimated band missed the pivot.  Exact masses of the BINS buckets next to the band, on the side
+                    // the pivot lies, give its bucket; the mass pass then runs again around it.
+                    const int w0 = target <= s_above ? max(0, rw.band_top - BINS + 1) : max(0, rw.band_bot);
+                    g.sync();
+                    for (int i = tid; i < BINS; i += NT) bins[i] = 0;
                     __syncthreads();
-                    if (total_mass == 0) { status |= COLINFER_ROW_DEGENERATE; if (lists && !a.stats) find_argmax(false); token = aidx; }
-                    else {
-                        leader_wrote = true;
-                        const int c = sc->x_chunk;
-                        if (warp == 0 && (!CL || ((c >> 4) % g.C) == g.rank)) {
-                            // the chunk in fp32, penalties applied (its CTA has the tables), then masked
-                            const uint32_t xb = smem_u32(xbuf);
-                            for (int p = lane; p < CHUNK; p += 32) {
-                                const int t = c * CHUNK + p - rw.a;
-                                float x = CI_NEG_INF;
-                                if (t >= 0 && t < V)
-                                    x = ELT == 4 ? __ldcg(reinterpret_cast<const float*>(base) + c * CHUNK + p)
-                                                 : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(base)[c * CHUNK + p]);
-                                xbuf[p] = x;
-                            }
-                            __syncwarp();
-                            if (rw.pen.on) pen_patch(rw.pen, xb, c, rw.a, V, lane, &sc->hist_slow);
-                            __syncwarp();
-                            const float lkf = fmaxf(lcut, -SM_FLT_MAX);
-                            u64 q16 = 0; uint32_t q[16];
+                    const u64 hi = pass_window<CL, ELT, MASK>(rw, nx, rw.mass, fmaxf(rw.lcut, -SM_FLT_MAX), rw.href, rw.scw, rw.hoff, w0, bins);
+                    if (lane == 0) sc->g_all[warp] = hi;
+                    g.sync();
+                    u64 s_hi = 0;
+                    for (int i = lane; i < GW; i += 32) s_hi += g.at(sc, i / NW)->g_all[i % NW];
+                    s_hi = warp_sum_u64(s_hi);
+                    int bw = -1; u64 bef, tot;
+                    auto win = [&](int i) { u64 s = 0; for (int q = 0; q < (CL ? g.C : 1); ++q) s += g.at(bins, q)[i]; return s; };
+                    if (target > s_hi) bins_find(win, BINS, target - s_hi, sc, bw, bef, tot);
+                    g.sync();
+                    if (bw >= 0) {
+                        const int bst = w0 + bw;
+                        if (tid == 0) {
+                            rw.t_hi = bst - 1 <= 0 ? SM_POS_INF : rw.href - (float)(bst - 1 - rw.hoff) / rw.scw;
+                            rw.t_lo = rw.href - (float)(bst + 2 - rw.hoff) / rw.scw;
+                        }
+                        found_band = true;
+                    }
+                }
+                if (!found_band) {
+                    // a list overflowed, or the pivot lies far from the estimate: exact radix select by mass
+                    float lpiv;
+                    if (radix_select(true, lpiv)) raise_cut(lpiv);
+                    __syncthreads();
+                    if (tid == 0) rw.path = PATH_PURE;
+                }
+                if (tid == 0) rw.status |= COLINFER_ROW_SELECT_SLOW;
+                g.sync();
+            }
+            SM_PROF(9);
+
+            // -------------------------------------------------------------------------------- the draw: chunk, then logit
+            g.sync();                                            // the chunks' kept masses are complete
+            {
+                const int Nc = rw.Nc;
+                const int per = (Nc + NT - 1) / NT;
+                const int c_lo = min(tid * per, Nc), c_hi = min(c_lo + per, Nc);
+                auto kept = [&](int c) { return g.at(csum, CL ? (c / NW) % g.C : 0)[c]; };
+                u64 s = 0, total;
+                for (int c = c_lo; c < c_hi; ++c) s += kept(c);
+                const u64 excl = block_excl_scan(s, sc, total);
+                const u64 target = ceil_target(rw.u, total);
+                if (total > 0 && excl < target && target <= excl + s) {
+                    u64 run = excl;
+                    for (int c = c_lo; c < c_hi; ++c) {
+                        const u64 q = kept(c);
+                        if (run + q >= target) { sc->x_chunk = c; sc->x_before = run; break; }
+                        run += q;
+                    }
+                }
+                if (tid == 0) { rw.total = total; if (total > 0) rw.drawn = 1; else rw.status |= COLINFER_ROW_DEGENERATE; }
+                __syncthreads();
+                derive_next();
+                if (total == 0) {
+                    if ((rw.cls & ROW_WIDE) && !a.stats) {       // (a row without any kept mass emits its argmax)
+                        const int x = argmax_pass<CL, ELT, MASK>(rw, nx, rw.L);
+                        if (lane == 0) sc->wi[warp] = x;
+                        g.sync();
+                        int y = 0x7fffffff;
+                        for (int i = lane; i < GW; i += 32) y = min(y, g.at(sc, i / NW)->wi[i % NW]);
+                        y = (int)__reduce_min_sync(0xffffffffu, (unsigned)y);
+                        if (tid == 0) rw.token = y == 0x7fffffff ? 0 : y;
+                    }
+                } else if (warp == 0) {
+                    const int c = sc->x_chunk;
+                    if (!CL || ((c / NW) % g.C) == g.rank) {
+                        // the chunk in fp32, penalties applied (its CTA has the tables), then masked
+                        const char* base = rw.base;
+                        const int al = rw.a;
+                        for (int p = lane; p < CHUNK; p += 32) {
+                            const int t = c * CHUNK + p - al;
+                            float x = CI_NEG_INF;
+                            if (t >= 0 && t < V)
+                                x = ELT == 4 ? __ldcg(reinterpret_cast<const float*>(base) + c * CHUNK + p)
+                                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(base)[c * CHUNK + p]);
+                            xbuf[p] = x;
+                        }
+                        __syncwarp();
+                        if (rw.pen_on) { const PenPeek pk = pen_peek(pen_tab(sc), rw.pen_cap, c, lane); if (pk.r0 != pk.r1) pen_patch(rw, smem_u32(xbuf), c, pk); }
+                        const float lkf = fmaxf(rw.lcut, -SM_FLT_MAX);
+                        const MassFn mass = rw.mass;
+                        u64 q16 = 0; uint32_t q[16];
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) {       // sixteen consecutive logits per lane
-                                const int p = lane * 16 + e, t = c * CHUNK + p - rw.a;
-                                float x = xbuf[p];
-                                if (rw.mrow && t >= 0 && t < V && !((__ldg(rw.mrow + (t >> 5)) >> (t & 31)) & 1)) x = CI_NEG_INF;
-                                q[e] = x >= lkf ? mass(x) : 0u;
-                                q16 += q[e];
-                            }
-                            const u64 before = sc->x_before;
-                            const u64 incl = before + warp_incl_scan_u64(q16, lane);
-                            const unsigned hit = __ballot_sync(0xffffffffu, incl >= target);
-                            if (hit && lane == __ffs(hit) - 1) {
-                                u64 cum = incl - q16; int e = 15;
+                        for (int e = 0; e < 16; ++e) {           // sixteen consecutive logits per lane
+                            const int p = lane * 16 + e, t = c * CHUNK + p - al;
+                            float x = xbuf[p];
+                            if (MASK && t >= 0 && t < V && !((__ldg(rw.mrow + (t >> 5)) >> (t & 31)) & 1)) x = CI_NEG_INF;
+                            q[e] = x >= lkf ? mass(x) : 0u;
+                            q16 += q[e];
+                        }
+                        const u64 incl = sc->x_before + warp_incl_scan_u64(q16, lane);
+                        const unsigned hit = __ballot_sync(0xffffffffu, incl >= target);
+                        if (hit && lane == __ffs(hit) - 1) {
+                            u64 cum = incl; int e = 0;
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) { cum += q[j]; if (cum >= target) { e = j; break; } }
-                                if (a.out) a.out[row] = (long long)(c * CHUNK + lane * 16 + e - rw.a);
-                            }
+                            for (int j = 15; j >= 0; --j) { if (cum >= target) e = j; cum -= q[j]; }   // the first whose running mass reaches the target
+                            if (a.out) a.out[rw.row] = (long long)(c * CHUNK + lane * 16 + e - al);
                         }
                     }
                 }
             }
         }
-        if (lane == 0 && rd.g.dead) atomicOr(&sc->flags, 2);
+        SM_PROF(10);
+        derive_next();
+        // (nobody reads these of this row any more)
+        if (tid < NW) { sc->wn[tid] = 0; sc->swf[tid] = CI_NEG_INF; }
+        if (tid == 0) { sc->flags = 0; sc->nsel = 0; }
         if (CL) g.sync(); else __syncthreads();
         if (tid == 0 && g.rank == 0) {
+            int status = rw.status;
             for (int q = 0; q < g.C; ++q) {
-                const Sc* ps = g.at(sc, q);
-                if (ps->hist_slow) status |= COLINFER_ROW_HIST_SLOW;
-                if (ps->flags & 2) status |= COLINFER_ROW_TIMEOUT;
+                if (g.at(&rw, q)->hist_slow) status |= COLINFER_ROW_HIST_SLOW;
+                if (g.at(sc, q)->dead) status |= COLINFER_ROW_TIMEOUT;
             }
-            if (!leader_wrote && a.out) a.out[row] = token;
-            if (a.status) a.status[row] = status;
+            if (!rw.drawn && a.out) a.out[rw.row] = rw.token;
+            if (a.status) a.status[rw.row] = status;
             if (a.stats) {
                 colinfer_row_stats st;
-                st.lmax = L; st.lcut = lcut; st.tc = tc; st.status = status; st.argmax = aidx; st.mass_q = total_mass;
-                a.stats[row] = st;
+                st.lmax = rw.L; st.lcut = rw.lcut; st.tc = rw.tc; st.status = status; st.argmax = rw.aidx; st.mass_q = rw.total;
+                a.stats[rw.row] = st;
             }
         }
         if (CL) g.sync();                                        // nobody reads this CTA's shared memory any more
+        if (nx.key == 0) break;
     }
-    while (rd.g.iss != rd.g.cons) { rd.wait(); ++rd.g.cons; }    // nothing is on its way when the CTA ends
+    Pipe<ELT> p;
+    p.expect(-1);                                                // nothing is on its way when the CTA ends
 }
 
 }  // namespace smp
