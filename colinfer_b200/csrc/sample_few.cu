@@ -1,0 +1,26 @@
+// sample_few.cu -- the fused kernel with a cluster of 1, 2, 4 or 8 CTAs per row, for launches of at most as many rows as SMs: one
+// CTA of 512 threads per SM with four chunks under way per warp (a cluster of eight holds a row of 151,936 logits that way).
+#define SMP_NAME smp_few
+#define SMP_THREADS 512
+#define SMP_CTAS 1
+#define SMP_STAGES 4
+#define SMP_LISTS 45056
+#include "sample_kernel.cuh"
+
+const void* colinfer_few_kernel(int index) {
+    static const void* const k[4] = {(const void*)SMP_NAME::k_sample<true, 4, false>, (const void*)SMP_NAME::k_sample<true, 4, true>,
+                                     (const void*)SMP_NAME::k_sample<true, 2, false>, (const void*)SMP_NAME::k_sample<true, 2, true>};
+    return k[index];
+}
+int colinfer_few_smem(int V, bool pen) { return SMP_NAME::smem_bytes(V, pen); }
+int colinfer_few_threads() { return SMP_NAME::NT; }
+
+#ifdef COLINFER_PROFILE
+extern "C" int colinfer_profile_read_few(unsigned long long* out16) {
+    cudaDeviceSynchronize();
+    int e = (int)cudaMemcpyFromSymbol(out16, SMP_NAME::g_prof, 128);
+    unsigned long long z[16] = {};
+    if (!e) e = (int)cudaMemcpyToSymbol(SMP_NAME::g_prof, z, 128);
+    return e;
+}
+#endif

@@ -26,9 +26,9 @@
 // band misses the pivot, an exact select over the 32-bit keys runs (slower, same result).
 #pragma once
 #include "common.cuh"
-#include "../../include/colinfer_b200.h"
+#include "sample_host.h"
 
-namespace smp {
+namespace SMP_NAME {
 
 #ifdef COLINFER_PROFILE
 // Profiling builds only: cycles per phase, summed over rows and CTAs (thread 0's clock).
@@ -38,11 +38,12 @@ __device__ unsigned long long g_prof[16];
 #define SM_PROF(slot) do { } while (0)
 #endif
 
-constexpr int NT = 256, NW = NT / 32;
+constexpr int NT = SMP_THREADS, NW = NT / 32;
 constexpr int NUM_SM = 148;          // (a B200's; only says from how many rows on their order matters)
-constexpr int CTAS_PER_SM = 3;
+constexpr int CTAS_PER_SM = SMP_CTAS;
+constexpr int NST = SMP_STAGES;      // stages of a warp's ring
 constexpr int CHUNK = 512;           // logits per chunk: 16 per lane
-constexpr int RING = 4096;           // bytes of ring per warp: fp32 two stages of 2 KB; bf16 two of 1 KB and one chunk in fp32
+constexpr int RING = NST * 2048;     // bytes of ring per warp: a stage is 2 KB of fp32, or 1 KB of bf16 (and an fp32 copy of one chunk behind them)
 constexpr int NB1 = 4096;            // histogram buckets
 constexpr int HOFF = 1024;           // of these, above the sample's maximum
 constexpr float RANGE = 25.0f;       // they span RANGE temperatures
@@ -50,10 +51,11 @@ constexpr int FASTK = 100;           // largest top_k finished from the sample's
 constexpr int BINS = 512;            // bins of the sample and of the selections on lists
 constexpr int BINS_PAD = BINS + BINS / 16;   // one spare word per sixteen: a lane reading its sixteen bins hits a bank of its own
 constexpr float FAST_SCALE = 32.0f;  // sample bins per unit logit (16 units)
-constexpr int U_BYTES = 22528;       // lists, or histogram and lists
+constexpr int U_BYTES = SMP_LISTS;   // lists, or histogram and lists
 constexpr int FCAP = 128;            // candidates of the one-warp finish
 constexpr int KCAP = U_BYTES / 8 / NW;                       // list entries per warp: rows without a histogram,
-constexpr int KCAP_CL = (U_BYTES - 8 * FCAP * 8) / 8 / NW;   // the same in a CTA of a cluster (behind the candidates of all CTAs),
+constexpr int PUSH = 2048;           // candidates the CTAs of a cluster send to the first one, in equal shares
+constexpr int KCAP_CL = (U_BYTES - PUSH * 8) / 8 / NW;   // the same in a CTA of a cluster (behind the candidates of all CTAs),
 constexpr int WCAP = (U_BYTES - NB1 * 4) / 8 / NW;           // rows with one
 constexpr int GCAP = NB1 * 4 / 8 / NW;                       // entries per warp gathered from all CTAs of a cluster
 constexpr int FIN_CAND = 64;         // entries of one bin compared pairwise
@@ -67,15 +69,7 @@ constexpr long long WAIT_CYCLES = 400000000LL;
 #define SM_POS_INF (__int_as_float(0x7f800000))
 #define SM_LOW (-1e30f)              // stands in for logits without mass in the mass pass: finite through every step
 
-struct Args {
-    const void* logits;
-    const int32_t* mask; int mask_rows; int W;
-    colinfer_sampler_params p;
-    const void* pos; int pos_i64; const float* u;
-    int64_t* out; colinfer_row_stats* stats; int32_t* status;
-    int B, R, V; int flags;
-    int cluster;                       // CTAs per row
-};
+using Args = colinfer_sample_args;
 
 template <bool B> struct BoolTag { static constexpr bool value = B; };
 struct Cand { uint32_t idx; float l; };
@@ -132,12 +126,13 @@ struct Sc {
     float swf[NW];
     float wf[NW]; int wi[NW];
     int in_klist;                      // the lists of the row at hand take the histogram's place
+    float4 pub;                        // the CTA's maximum, its lowest token, tw and flags
     float tw; int flags;               // 1 list overflow or no bound, 2 a wait ran out, 4 histogram not counted
     int wn[NW];
     u64 g_all[NW], g_keep[NW];
-    u64 t_cnt, t_est;                  // totals of the CTA's share of the histogram
+    u64 t_cnt, t_est, sum_off;         // totals of the CTA's share of the histogram; what the estimates are off by
+    u64 sum_all, sum_keep;             // masses of the CTA's chunks
     int nsel;                          // candidates selected
-    int npush; float push_lo;          // candidates sent to the group's first CTA, the value down to which they are complete
     int ok; float fin_cut; u64 fin_total; int fin_token;
     int fb[3]; u64 fe[3];              // finds of fine_decide
     // CTA-local
@@ -162,7 +157,7 @@ static_assert(sizeof(Fin) <= 2 * BINS_PAD * 4 && 2 * FCAP * 4 <= BINS_PAD * 4, "
 // histories).  The history bitmap, a bit per position, lies over lists, bins and chunk sums while the tables are built.
 constexpr int OFF_SC = NW * RING;
 constexpr int OFF_BARS = (OFF_SC + (int)sizeof(Sc) + 15) & ~15;
-constexpr int OFF_U = (OFF_BARS + NW * 16 + 127) & ~127;
+constexpr int OFF_U = (OFF_BARS + NW * 8 * NST + 127) & ~127;
 constexpr int OFF_BINS = OFF_U + U_BYTES;
 constexpr int OFF_CSUM = OFF_BINS + 2 * BINS_PAD * 4;
 static_assert(2 * BINS_PAD * 4 >= BINS * 8 && BINS_PAD * 4 >= CHUNK * 4, "what lies over the bins");
@@ -186,6 +181,15 @@ __device__ __forceinline__ float max16(const float (&v)[16]) {
     const float a = fmax3(v[0], v[1], v[2]), b = fmax3(v[3], v[4], v[5]), c = fmax3(v[6], v[7], v[8]);
     const float d = fmax3(v[9], v[10], v[11]), e = fmax3(v[12], v[13], v[14]);
     return fmax3(fmax3(a, b, c), fmax3(d, e, v[15]), CI_NEG_INF);
+}
+
+// 64-bit addition in shared memory as a 32-bit one with a carry: the hardware has no 64-bit one there, it would be a
+// compare-and-swap loop.  (The sum is complete once every adder is through.)
+__device__ __forceinline__ void add64(u64* p, u64 v) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(p);
+    const uint32_t lo = (uint32_t)v, old = atomicAdd(w, lo);
+    const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(w + 1, hi);
 }
 
 // ------------------------------------------------------------------------------------------------ the CTAs that share a row
@@ -412,7 +416,7 @@ static __device__ __noinline__ void mend_edges(uint32_t st, int c, int a) {
     __syncwarp();
 }
 
-// A warp's two-stage ring.  While a pass runs its state lives in registers, between passes in Sc.
+// A warp's ring.  While a pass runs its state lives in registers, between passes in Sc.
 template <int ELT>
 struct Pipe {
     static constexpr int CHB = CHUNK * ELT;
@@ -423,16 +427,16 @@ struct Pipe {
     __device__ __forceinline__ Pipe() {
         const int warp = warp_id();
         buf = smem_u32(smem) + warp * RING;
-        bar = smem_u32(smem) + OFF_BARS + warp * 16;
+        bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
         const Sc* sc = scratch();
         cons = sc->ring[warp].cons; out = sc->ring[warp].out;
         asks = lane_id() == 0 && !(sc->drop | sc->dead);
     }
-    __device__ __forceinline__ uint32_t conv() const { return buf + 2 * CHB; }          // bf16: an fp32 copy of one chunk
-    __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) & 1u) * CHB; }
+    __device__ __forceinline__ uint32_t conv() const { return buf + NST * CHB; }          // bf16: an fp32 copy of one chunk
+    __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) % NST) * CHB; }
     __device__ __forceinline__ void issue(const char* p, uint32_t bytes, u64 pol) {
         if (asks) {
-            const uint32_t s = (uint32_t)(cons + out) & 1u;
+            const uint32_t s = (uint32_t)(cons + out) % NST;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * s), "r"(bytes) : "memory");
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                          ::"r"(buf + s * CHB), "l"(p), "r"(bytes), "r"(bar + 8 * s), "l"(pol) : "memory");
@@ -441,7 +445,7 @@ struct Pipe {
     }
     // The bytes of the chunk j places from the next one to consume are there.
     __device__ __forceinline__ void wait(int j = 0) {
-        const uint32_t b = bar + 8 * ((uint32_t)(cons + j) & 1u), par = ((uint32_t)(cons + j) >> 1) & 1u;
+        const uint32_t b = bar + 8 * ((uint32_t)(cons + j) % NST), par = ((uint32_t)(cons + j) / NST) & 1u;
         auto test = [&]() {
             uint32_t ok;
             asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -482,7 +486,7 @@ template <int ELT>
 __device__ __forceinline__ void ring_start(int key, const char* base, uint32_t end, int Nc, int gw, int GW) {
     Pipe<ELT> p;
     p.expect(key);
-    while (p.out < 2 && gw + p.out * GW < Nc) {
+    while (p.out < NST && gw + p.out * GW < Nc) {
         const char* q = base + (size_t)(gw + p.out * GW) * Pipe<ELT>::CHB;
         p.issue(q, chunk_bytes<ELT>(q, end), l2_policy(true));
     }
@@ -509,19 +513,48 @@ struct Chunk {
         asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(at + k * 256) : "memory");
         return make_float4(__uint_as_float(x << 16), __uint_as_float(x & 0xFFFF0000u), __uint_as_float(y << 16), __uint_as_float(y & 0xFFFF0000u));
     }
+    // the mask bits of group k (bit 0 .. 3)
+    __device__ __forceinline__ uint32_t bits4(int k) const {
+        const int bit = sh + k * 128 + lane_id() * 4;
+        const uint32_t w = __shfl_sync(0xffffffffu, mw, bit >> 5);
+        if (sh & 3) return __funnelshift_r(w, __shfl_sync(0xffffffffu, mw, (bit >> 5) + 1), bit & 31);   // groups straddle words (an unaligned row)
+        return w >> (bit & 31);
+    }
     __device__ __forceinline__ float4 group(int k, float none) const {
         float4 v = stored(k);
         if (MASK) {
-            const int bit = sh + k * 128 + lane_id() * 4;
-            uint32_t bits = __shfl_sync(0xffffffffu, mw, bit >> 5);
-            if (sh & 3) bits = __funnelshift_r(bits, __shfl_sync(0xffffffffu, mw, (bit >> 5) + 1), bit & 31);   // groups straddle words (an unaligned row)
-            else bits >>= bit & 31;
+            const uint32_t bits = bits4(k);
             if (!(bits & 1u)) v.x = none;
             if (!(bits & 2u)) v.y = none;
             if (!(bits & 4u)) v.z = none;
             if (!(bits & 8u)) v.w = none;
         }
         return v;
+    }
+    // the lane's largest logit; bf16 chunks two at a time, masked ones as NaN, which a maximum passes over
+    __device__ __forceinline__ float max16() const {
+        float m = CI_NEG_INF;
+        if (ELT == 2 && !wide) {
+            uint32_t r = 0xFF80FF80u;                                    // two bf16 of -inf
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                uint32_t x, y;
+                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(at + k * 256) : "memory");
+                if (MASK) {
+                    // the group's four bits spread to the top bits of four bytes (i to 7 + 8 i), those replicated to halves
+                    const uint32_t top = (~bits4(k) & 0xFu) * 0x10204080u;
+                    uint32_t h;
+                    asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(h) : "r"(top)); x |= h;
+                    asm("prmt.b32 %0, %1, 0, 0xBBAA;" : "=r"(h) : "r"(top)); y |= h;
+                }
+                asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(x));
+                asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(y));
+            }
+            return fmaxf(__uint_as_float(r << 16), __uint_as_float(r & 0xFFFF0000u));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { const float4 v = group(k, CI_NEG_INF); m = fmax3(fmax3(v.x, v.y, v.z), v.w, m); }
+        return m;
     }
     // logit e of the lane as stored (penalties; not the mask, which only removes)
     __device__ __forceinline__ float one(int e) const {
@@ -574,7 +607,7 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
     const u64 pol = l2_policy(keep);
     int cn = gw + p.out * GW;                                            // the next chunk to ask for
     const char* next = rw.base + (size_t)cn * CHB;
-    while (p.out < 2 && cn < Nc) { p.issue(next, chunk_bytes<ELT>(next, rw.end), pol); next += GW * CHB; cn += GW; }
+    while (p.out < NST && cn < Nc) { p.issue(next, chunk_bytes<ELT>(next, rw.end), pol); next += GW * CHB; cn += GW; }
     uint32_t mw[MASK ? 3 : 1];                                           // mask words of this chunk and the next two
     if (MASK) {
 #pragma unroll
@@ -605,7 +638,7 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
     const int nkey = *(volatile const int*)&nx.key;
     __threadfence_block();
     const int nnc = then == THEN_NOTHING ? 0 : !other ? Nc : nkey ? nx.Nc : 0;
-    for (int c = gw; p.out < 2 && c < nnc; c += GW) {
+    for (int c = gw; p.out < NST && c < nnc; c += GW) {
         const char* q = (other ? nx.base : rw.base) + (size_t)c * CHB;
         p.issue(q, chunk_bytes<ELT>(q, other ? nx.end : rw.end), l2_policy(other));
     }
@@ -645,36 +678,39 @@ __device__ __forceinline__ float max4(float4 v, float m) { return fmax3(fmax3(v.
 // The passes.
 struct Top { float l; int idx; };
 
-// Maximum of the warp's chunks and the lowest token that has it.
+// Maximum of the warp's chunks and the lowest token that has it (the same in all lanes).
+__device__ __forceinline__ float warp_max(float x) {
+    float m;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(x));
+    return m;
+}
 template <bool CL, int ELT, bool MASK>
 __device__ __forceinline__ Top pass_max(RowS& rw, const NextRow& nx, bool keep, int then) {
-    float lmax = CI_NEG_INF;
-    int lidx = 0x7fffffff;
+    float wmax = CI_NEG_INF;
+    int widx = 0x7fffffff;
     run_pass<CL, ELT, MASK>(rw, nx, keep, 0, then, [&](const auto& k) {
-        float m = CI_NEG_INF;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) m = max4(k.group(j, CI_NEG_INF), m);
-        if (__any_sync(0xffffffffu, m > lmax)) {
-            int e = 15;
-#pragma unroll
+        const float m = k.max16(), top = warp_max(m);
+        if (top > wmax) {                                                // strict: the first (lowest) position of the maximum stays
+            wmax = top;
+            unsigned p = 0x7fffffff;
+#pragma unroll 1
             for (int j = 3; j >= 0; --j) {
                 const float4 v = k.group(j, CI_NEG_INF);
-                e = v.w == m ? 4 * j + 3 : e; e = v.z == m ? 4 * j + 2 : e; e = v.y == m ? 4 * j + 1 : e; e = v.x == m ? 4 * j : e;
+                const int e = v.x == top ? 0 : v.y == top ? 1 : v.z == top ? 2 : v.w == top ? 3 : 4;
+                if (e < 4) p = min(p, (unsigned)(4 * j + e));
             }
-            if (m > lmax) { lmax = m; lidx = k.c * CHUNK - rw.a + pos_of(e, lane_id()); }   // strict: the first (lowest) position of the maximum stays
+            widx = (int)__reduce_min_sync(0xffffffffu, p == 0x7fffffffu ? p : (unsigned)(k.c * CHUNK - rw.a + pos_of(p, lane_id())));
         }
     });
-    return Top{lmax, lidx};
+    return Top{wmax, widx};
 }
 
-// Lists the logits >= t of the warp's chunks; returns their maximum.
+// Lists the logits >= t of the warp's chunks; returns the lane's maximum.
 template <bool CL, int ELT, bool MASK>
 __device__ __forceinline__ float pass_list(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap) {
     float lmax = CI_NEG_INF;
     run_pass<CL, ELT, MASK>(rw, nx, keep, seen, then, [&](const auto& k) {
-        float m = CI_NEG_INF;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) m = max4(k.group(j, CI_NEG_INF), m);
+        const float m = k.max16();
         lmax = fmaxf(lmax, m);
         list_above(rw.a, list, cap, t, m >= t, k);
     });
@@ -693,9 +729,9 @@ struct Buckets {
     }
 };
 
-// The same with a count of every logit's bucket; masked (-inf) logits are not counted.
+// The same with a count of the buckets of the logits >= from (what lies below, and -inf, cannot be kept).
 template <bool CL, int ELT, bool MASK>
-__device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap, float href, float scale, int hoff) {
+__device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap, float href, float scale, int hoff, float from) {
     float lmax = CI_NEG_INF;
     const Buckets bk(href, scale, hoff);
     const uint32_t h0 = smem_u32(smem) + OFF_U - (0x4B000000u << 2);
@@ -704,7 +740,7 @@ __device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool kee
         float m = CI_NEG_INF;
         auto count = [&](float x, float b) {
             const uint32_t at = h0 + (__float_as_uint(b) << 2);
-            if (!MASK || x > CI_NEG_INF) asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory");
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p red.shared.add.u32 [%0], 1;\n\t}" ::"r"(at), "f"(x), "f"(from) : "memory");
         };
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -806,7 +842,7 @@ static __device__ __noinline__ void pass_radix(RowS& rw, const NextRow& nx, Mass
                 const unsigned peers = __match_any_sync(0xffffffffu, bin);
                 const uint32_t w = bin < 0 ? 0u : (by_mass ? mass(l) : 1u);
                 const uint32_t lo = __reduce_add_sync(peers, w & 0xFFFFu), hi = __reduce_add_sync(peers, w >> 16);
-                if (bin >= 0 && lane == __ffs(peers) - 1) atomicAdd(&bins[bin], ((u64)hi << 16) + lo);
+                if (bin >= 0 && lane == __ffs(peers) - 1) add64(&bins[bin], ((u64)hi << 16) + lo);
             }
         }
     });
@@ -827,7 +863,7 @@ static __device__ __noinline__ u64 pass_window(RowS& rw, const NextRow& nx, Mass
                 if (x[e] >= lk) {
                     const int bb = bk(x[e]);
                     if (bb < w0) hi += (u64)mass(x[e]);
-                    else if (bb < w0 + BINS) atomicAdd(&bins[bb - w0], (u64)mass(x[e]));
+                    else if (bb < w0 + BINS) add64(&bins[bb - w0], (u64)mass(x[e]));
                 }
             }
         }
@@ -839,19 +875,13 @@ static __device__ __noinline__ u64 pass_window(RowS& rw, const NextRow& nx, Mass
 // The lowest token of the warp's chunks whose logit is L.
 template <bool CL, int ELT, bool MASK>
 static __device__ __noinline__ int argmax_pass(RowS& rw, const NextRow& nx, float L) {
-    Top m = pass_max<CL, ELT, MASK>(rw, nx, false, THEN_NOTHING);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const float om = __shfl_xor_sync(0xffffffffu, m.l, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, m.idx, o);
-        if (om > m.l || (om == m.l && oi < m.idx)) { m.l = om; m.idx = oi; }
-    }
+    const Top m = pass_max<CL, ELT, MASK>(rw, nx, false, THEN_NOTHING);
     return m.l == L ? m.idx : 0x7fffffff;
 }
 // The histogram counted from the row's maximum.
 template <bool CL, int ELT, bool MASK>
 static __device__ __noinline__ void recount_pass(RowS& rw, const NextRow& nx) {
-    pass_hist<CL, ELT, MASK>(rw, nx, true, 0, THEN_AGAIN, SM_POS_INF, nullptr, 0, rw.L, rw.scw, 0);
+    pass_hist<CL, ELT, MASK>(rw, nx, true, 0, THEN_AGAIN, SM_POS_INF, nullptr, 0, rw.L, rw.scw, 0, rw.lcut);
 }
 // The logits a large top-k can keep.
 template <bool CL, int ELT, bool MASK>
@@ -864,10 +894,9 @@ struct View { const Cand* p; int start, n, step; };
 
 // Selects the listed logits that can belong to the top kk: BINS linear bins over [max(bound, cut), L] give the bin of the
 // kk-th largest, everything down to it goes to the CTA's candidates (at most FCAP, no particular order).  Returns how many,
-// or -1 when the lists cannot decide.  Every logit >= bound (of the row, or of the CTA's share of it) is in the lists; `few`:
-// fewer than kk of them may reach max(bound, cut).  bins and nsel are zeroed before the caller's last barrier.
+// or -1 when the lists cannot decide.  Every logit >= bound of the row is in the lists.  bins and nsel are zeroed before the caller's last barrier.
 // Two __syncthreads.
-__device__ __forceinline__ int select_top(const View& w, float bound, float cut, float L, int kk, bool few, uint32_t* bins, Sc* sc, float& scale, int& bstar) {
+__device__ __forceinline__ int select_top(const View& w, float bound, float cut, float L, int kk, uint32_t* bins, Sc* sc, float& scale, int& bstar) {
     const int lane = lane_id();
     const float lo = fmaxf(bound, cut);
     scale = L > lo ? (float)(BINS - 2) / (L - lo) : 0.0f;
@@ -879,7 +908,7 @@ __device__ __forceinline__ int select_top(const View& w, float bound, float cut,
     int n = (int)run_b;
     if (bstar < 0) {
         // fewer than kk listed logits reach lo: if lo is the cut, fewer than kk logits survive it and top-k removes nothing
-        if (!(lo > bound || few)) n = -1;
+        if (!(lo > bound)) n = -1;
         bstar = BINS - 1;
     }
     if (n > FCAP || !(lo <= L)) n = -1;
@@ -1000,7 +1029,7 @@ __device__ bool list_select(const View& w, W wt, float base, float scale, u64 ta
     for (int i = w.start; i < w.n; i += w.step) {
         const float l = w.p[i].l;
         const u64 q = wt(l);
-        if (q) atomicAdd(&bins[bin_of(l)], q);
+        if (q) add64(&bins[bin_of(l)], q);
     }
     __syncthreads();
     int b_star; u64 before;
@@ -1084,15 +1113,21 @@ __device__ FineDecision fine_decide(const Grp<CL>& g, uint32_t* hist, W west, in
     g.sync();
     FineDecision o;
     u64 off_c = 0, off_e = 0;
+    long long off = 0;                                               // what the estimates are off by on the largest logits
     o.total_cnt = 0; o.est_total = 0;
     for (int r = 0; r < (CL ? g.C : 1); ++r) {
         const Sc* ps = g.at(sc, r);
         const u64 tc = ps->t_cnt, te = ps->t_est;
         if (r < g.rank) { off_c += tc; off_e += te; }
         o.total_cnt += tc; o.est_total += te;
+        off += (long long)ps->sum_off;
     }
     const u64 ex_c = off_c + sc->woff[warp] + in_c - sc_c, ex_e = off_e + sc->woff2[warp] + in_e - sc_e;
-    const u64 t_p = (want_p && o.est_total > 0) ? ceil_target(topp, o.est_total) : 0ull;
+    u64 t_p = 0;
+    if (want_p && o.est_total > 0 && (long long)o.est_total + off > 0) {
+        const long long t = (long long)ceil_target(topp, (u64)((long long)o.est_total + off)) - off;
+        t_p = t < 1 ? 1ull : min((u64)t, o.est_total);
+    }
     auto tell = [&](int k, int b, u64 v) { for (int r = 0; r < (CL ? g.C : 1); ++r) { Sc* ps = g.at(sc, r); ps->fb[k] = b; ps->fe[k] = v; } };
     if (kk_target && ex_c < kk_target && kk_target <= ex_c + sc_c) {
         u64 run = ex_c;
@@ -1223,7 +1258,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     Cand* klist = reinterpret_cast<Cand*>(smem + OFF_U);         // [NW][KCAP]: rows without a histogram,
     uint32_t* hist = reinterpret_cast<uint32_t*>(smem + OFF_U);  // or [NB1],
     Cand* wlist = reinterpret_cast<Cand*>(smem + OFF_U + NB1 * 4);       // [NW][WCAP]
-    Cand* push = reinterpret_cast<Cand*>(smem + OFF_U);          // [8][FCAP] candidates of all CTAs, over the histogram
+    Cand* push = reinterpret_cast<Cand*>(smem + OFF_U);          // [C][PUSH / C] candidates of all CTAs, over the histogram
     Cand* gath = reinterpret_cast<Cand*>(smem + OFF_U);          // [NW][GCAP] lists of all CTAs, over the histogram
     uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem + OFF_U);        // history bitmap while the tables are built (may reach over bins and csum)
     uint32_t* sbins = reinterpret_cast<uint32_t*>(smem + OFF_BINS);      // [BINS_PAD] sample
@@ -1236,14 +1271,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         sc->V = V; sc->W = a.W; sc->GW = GW; sc->rank = g.rank;
         sc->drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0; sc->dead = 0;
         sc->pen_off = pen_offset(V, a.p.history != nullptr);
-        sc->flags = 0; sc->nsel = 0;
+        sc->flags = 0; sc->nsel = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0;
     }
     if (lane == 0) {
-        const uint32_t bar = smem_u32(smem) + OFF_BARS + warp * 16;
+        const uint32_t bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
         sc->ring[warp].cons = 0; sc->ring[warp].out = 0; sc->ring[warp].key = 0;
         sc->wn[warp] = 0; sc->swf[warp] = CI_NEG_INF;
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8) : "memory");
+        for (int j = 0; j < NST; ++j) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * j) : "memory");
         fence_mbar_init();
     }
     __syncthreads();
@@ -1313,6 +1347,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         }
         if (next_row >= 0) {
             fetch_row(it + 1);
+            if (a.p.history) {                                   // the history's lines into L2
+                const char* h = reinterpret_cast<const char*>(a.p.history + (size_t)(a.R == 1 ? next_row : next_row / a.R) * a.p.hist_stride);
+                for (int i = lane * 128; i < min(a.p.hist_stride, 4096) * 4; i += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(h + i));
+            }
             if (lane == 0) {
                 NextRow& nx = sc->next[it & 1];
                 int al;
@@ -1336,16 +1374,24 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     if (warp == PW) {
         next_row = row_of(grp);
         fetch_row(0);
-        if (lane == 0) { sc->next[0].key = sc->next[1].key = 0; mbar_init(&sc->clc_bar, 1); fence_mbar_init(); }
-        derive(0);
+        if (lane == 0) {
+            RowS& rw = sc->rows[0];
+            rw.base = place_row<ELT>(a, next_row, rw.a, rw.end, rw.Nc);
+            sc->next[0].key = sc->next[1].key = 0;
+            sc->rows[0].key = next_row + 1;
+            mbar_init(&sc->clc_bar, 1);
+            fence_mbar_init();
+        }
     }
+    __syncthreads();
+    ring_start<ELT>(sc->rows[0].key, sc->rows[0].base, sc->rows[0].end, sc->rows[0].Nc, gw, GW);   // the logits travel while the parameters do
+    if (warp == PW) derive(0);
     __syncthreads();
 
     for (int it = 0; ; ++it) {
         RowS& rw = sc->rows[it & 1];
         const NextRow& nx = sc->next[it & 1];
         ring_start<ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW);
-        if (!CL && tid == PW * 32) queue_ask(sc);
         bool found = false, derived = false;                     // (the last warp's)
         auto look_ahead = [&]() { if (warp == PW && !found) { find_next(it); found = true; } };
         auto derive_next = [&]() { if (warp == PW && !derived) { look_ahead(); derive(it + 1); derived = true; if (lane == 0) sc->next[(it + 1) & 1].key = 0; } };
@@ -1393,9 +1439,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             auto enter = [&](int v) {
                 int p;
                 if (!mine(v, p)) return;
-                const int c = p >> 9, w = p >> 5;
-                uint32_t rk = pt.pre[c] + __popc(bitmap[w] & ((1u << (p & 31)) - 1u));
-                for (int i = c * 16; i < w; ++i) rk += __popc(bitmap[i]);
+                const int c = p >> 9;
+                uint32_t rk = pt.pre[c];
+                for (int i = c * 16; i < (p >> 5); ++i) rk += __popc(bitmap[i]);   // the chunk's bits before the token's
+                rk += __popc(bitmap[p >> 5] & ((1u << (p & 31)) - 1u));
                 if ((int)rk < cap) {                             // the first to come brings the position along
                     if (atomicAdd(&pt.ent[rk], 65536u) < 65536u) atomicAdd(&pt.ent[rk], (uint32_t)(p & (CHUNK - 1)));
                 }
@@ -1415,6 +1462,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             int lcap = WCAP;
             float tw = -SM_FLT_MAX;                              // the CTA's list bound
             float lref = CI_NEG_INF;                             // the sample's maximum (the group's): buckets hang from it
+            float from = -SM_FLT_MAX;                            // nothing below can be kept
             bool count_hist = false;
             int seen = 0;                                        // first chunks of the warp that have been read
             bool in_klist = fastk;
@@ -1482,13 +1530,15 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     const int share = (rw.Nc + g.C - 1) / g.C;   // chunks of the CTA
                     const float t2 = bound(max(1, (CL ? KCAP_CL : KCAP) * NW * NW / share));
                     count_hist = !(t2 > -SM_FLT_MAX && t2 < sure);
+                    from = fmaxf(from, sure);
                     if (!count_hist) { tw = sure; in_klist = true; }
                 }
-                if (in_klist) { list = CL ? push + 8 * FCAP + warp * KCAP_CL : klist + warp * KCAP; lcap = CL ? KCAP_CL : KCAP; }
+                if (in_klist) { list = CL ? push + PUSH + warp * KCAP_CL : klist + warp * KCAP; lcap = CL ? KCAP_CL : KCAP; }
                 if (tid == 0) sc->in_klist = in_klist;
                 if (tid == 0) { rw.lref = lref; rw.count_hist = count_hist; }
             }
             SM_PROF(2);
+            if (!CL && tid == PW * 32) queue_ask(sc);
             look_ahead();
             if (tid == 0) sc->tw = tw;
             const bool one_pass = !(cls & ROW_SAMPLED) || in_klist;
@@ -1497,22 +1547,28 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             const int bad = (lists && !(tw > -SM_FLT_MAX) ? 1 : 0) | (wide && !count_hist ? 4 : 0);
             Top top1{CI_NEG_INF, 0x7fffffff};
             if (!lists) top1 = pass_max<CL, ELT, MASK>(rw, nx, !one_pass, then);
-            else if (count_hist) top1.l = pass_hist<CL, ELT, MASK>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF);
+            else if (count_hist) top1.l = pass_hist<CL, ELT, MASK>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF, from);
             else top1.l = pass_list<CL, ELT, MASK>(rw, nx, !one_pass, seen, then, t, list, lcap);
             SM_PROF(3);
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const float om = __shfl_xor_sync(0xffffffffu, top1.l, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, top1.idx, o);
-                if (om > top1.l || (om == top1.l && oi < top1.idx)) { top1.l = om; top1.idx = oi; }
-            }
+            if (lists) top1.l = warp_max(top1.l);
             if (lane == 0) {
                 sc->wf[warp] = top1.l; sc->wi[warp] = top1.idx;
                 const int f = bad | (lists && sc->wn[warp] > lcap ? 1 : 0);
                 if (f) atomicOr(&sc->flags, f);
             }
         }
-        g.sync();
+        __syncthreads();
+        if constexpr (CL) {
+            // one record per CTA for the others to read
+            if (warp == 0) {
+                float l = lane < NW ? sc->wf[lane] : CI_NEG_INF;
+                int i = lane < NW ? sc->wi[lane] : 0x7fffffff;
+                const float m = warp_max(l);
+                i = (int)__reduce_min_sync(0xffffffffu, l == m ? (unsigned)i : 0x7fffffffu);
+                if (lane == 0) sc->pub = make_float4(m, __int_as_float(i), sc->tw, __int_as_float(sc->flags));
+            }
+            g.sync();
+        }
 
         // ------------------------------------------------------------------------------------ the row's maximum and cut
         bool done = true;                                        // the row needs no further pass
@@ -1520,24 +1576,18 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             const int cls = rw.cls;
             const bool sampled = (cls & ROW_SAMPLED) != 0, fastk = (cls & ROW_FASTK) != 0, lists = (cls & (ROW_FASTK | ROW_WIDE)) != 0;
             const bool in_klist = sc->in_klist != 0;
-            Cand* list = !in_klist ? wlist + warp * WCAP : CL ? push + 8 * FCAP + warp * KCAP_CL : klist + warp * KCAP;
+            Cand* list = !in_klist ? wlist + warp * WCAP : CL ? push + PUSH + warp * KCAP_CL : klist + warp * KCAP;
             const int lcap = !in_klist ? WCAP : CL ? KCAP_CL : KCAP;
             float L = CI_NEG_INF, lo_all = -SM_FLT_MAX;
             int aidx = 0x7fffffff, fl = 0;
-            for (int i = lane; i < GW; i += 32) {
-                const Sc* ps = g.at(sc, i / NW);
-                const float om = ps->wf[i % NW]; const int oi = ps->wi[i % NW];
-                if (om > L || (om == L && oi < aidx)) { L = om; aidx = oi; }
-                lo_all = fmaxf(lo_all, ps->tw);
-                fl |= ps->flags;
-            }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const float om = __shfl_xor_sync(0xffffffffu, L, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, aidx, o);
-                if (om > L || (om == L && oi < aidx)) { L = om; aidx = oi; }
-                lo_all = fmaxf(lo_all, __shfl_xor_sync(0xffffffffu, lo_all, o));
-                fl |= __shfl_xor_sync(0xffffffffu, fl, o);
+            {
+                float4 e = make_float4(CI_NEG_INF, __int_as_float(0x7fffffff), -SM_FLT_MAX, 0.0f);
+                if (CL) { if (lane < g.C) e = g.at(sc, lane)->pub; }
+                else if (lane < NW) e = make_float4(sc->wf[lane], __int_as_float(sc->wi[lane]), sc->tw, __int_as_float(sc->flags));
+                L = warp_max(e.x);
+                aidx = (int)__reduce_min_sync(0xffffffffu, e.x == L ? (unsigned)__float_as_int(e.y) : 0x7fffffffu);
+                lo_all = warp_max(e.z);
+                fl = (int)__reduce_or_sync(0xffffffffu, (unsigned)__float_as_int(e.w));
             }
             const bool lists_ok = lists && !(fl & 1);
             const bool finite_max = (L > CI_NEG_INF) && (L < SM_POS_INF);
@@ -1592,35 +1642,30 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 if (lists_ok && (fastk || lo_all < lcut)) {
                     const int kq = rw.kk > 0 && rw.kk < V ? rw.kk : 0x7fffffff;
                     const View w{list, lane, min(sc->wn[warp], lcap), 32};
-                    float scale, lo = fmaxf(lo_all, lcut); int bstar;
-                    const float tw = sc->tw;
-                    int n = select_top(w, tw, lcut, L, kq, CL && tw <= lcut, fbins, sc, scale, bstar);
+                    float scale; int bstar, n = -1;
+                    const float lo = fmaxf(lo_all, lcut);
                     if constexpr (CL) {
-                        // every CTA selects its own top k; its candidates go to the first one, which selects among them
-                        if (n > 0) {
-                            Cand* to = g.at(push, 0) + g.rank * FCAP;
-                            for (int i = tid; i < n; i += NT) to[i] = Cand{fin_area()->fc_idx[i], fin_area()->fc_l[i]};
+                        // what reaches the highest of the CTAs' bounds (at least kk logits of the CTA it comes from do) goes to the
+                        // first CTA, which selects
+                        const int pcap = PUSH / g.C;
+                        Cand* to = g.at(push, 0) + g.rank * pcap;
+                        for (int j = w.start; j < w.n; j += 32) {
+                            const Cand c = w.p[j];
+                            if (c.l >= lo) { const int at = atomicAdd(&sc->nsel, 1); if (at < pcap) to[at] = c; }
                         }
-                        float plo = SM_POS_INF;                  // the value down to which they are complete
-                        if (bstar == BINS - 1) plo = fmaxf(tw, lcut);
-                        else for (int i = lane; i < n; i += 32) plo = fminf(plo, fin_area()->fc_l[i]);
-#pragma unroll
-                        for (int o = 16; o; o >>= 1) plo = fminf(plo, __shfl_xor_sync(0xffffffffu, plo, o));
-                        for (int i = tid; i < BINS_PAD; i += NT) fbins[i] = 0u;
-                        __syncthreads();
-                        if (tid == 0) { sc->npush = n; sc->push_lo = plo; sc->nsel = 0; }
                         g.sync();
                         if (g.rank == 0) {
-                            lo = lcut;
                             bool good = true;
-                            for (int q = 0; q < g.C; ++q) { const Sc* ps = g.at(sc, q); good = good && ps->npush >= 0; lo = fmaxf(lo, ps->push_lo); }
-                            n = -1;
-                            if (good) {
-                                const int wpr = NW / g.C, q = warp / wpr;
-                                const View w2{push + q * FCAP, (warp % wpr) * 32 + lane, g.at(sc, q)->npush, 32 * wpr};
-                                n = select_top(w2, lo, lcut, L, kq, lo <= lcut, fbins, sc, scale, bstar);
-                            }
+                            for (int q = 0; q < g.C; ++q) good = good && g.at(sc, q)->nsel <= pcap;
+                            const int wpr = NW / g.C, q = warp / wpr, mine = g.at(sc, q)->nsel;
+                            __syncthreads();
+                            if (tid == 0) sc->nsel = 0;
+                            __syncthreads();
+                            const View w2{push + q * pcap, (warp % wpr) * 32 + lane, mine, 32 * wpr};
+                            if (good) n = select_top(w2, lo_all, lcut, L, kq, fbins, sc, scale, bstar);
                         }
+                    } else {
+                        n = select_top(w, lo_all, lcut, L, kq, fbins, sc, scale, bstar);
                     }
                     if (g.rank == 0) {
                         if (n > 0) {
@@ -1664,9 +1709,24 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 // the histogram counts every logit; buckets wholly below the cut are left out
                 const int b_cut = bucket(lcut);
                 const float dL = (rw.L - href) / rw.tc;
-                auto mass_est = [&](int i) {                     // (the last bucket holds everything beyond)
-                    return i == NB1 - 1 ? 0ull : (u64)__float2uint_rn(exp2f(fminf(0.0f, -(((float)(i - hoff) + 0.5f) * (RANGE / (float)NB1) + dL) * CI_LOG2E)) * CI_MASS_SCALE);
+                // the estimated mass of a logit of bucket i (the last one holds everything beyond; of the cut's bucket, the part above)
+                const float cut_part = fminf(fmaxf((href - (float)(b_cut - hoff) / scw - lcut) * scw, 0.0f), 1.0f);
+                auto mass_est = [&](int i) {
+                    const float e = exp2f(fminf(0.0f, -(((float)(i - hoff) + 0.5f) * (RANGE / (float)NB1) + dL) * CI_LOG2E)) * CI_MASS_SCALE;
+                    return i == NB1 - 1 ? 0ull : (u64)__float2uint_rn(i == b_cut ? e * cut_part : e);
                 };
+                // What the estimates are off by on the listed logits -- the largest, which make up most of a peaked row's mass.
+                long long off = 0;
+                if (ready && !sc->in_klist) {
+                    const Cand* list = wlist + warp * WCAP;
+                    const MassFn mass = rw.mass;
+                    for (int j = lane; j < min(sc->wn[warp], WCAP); j += 32) {
+                        const float l = list[j].l;
+                        if (l >= lcut) off += (long long)mass(l) - (long long)mass_est(bucket(l));
+                    }
+                }
+                off = (long long)warp_sum_u64((u64)off);
+                if (lane == 0) add64(&sc->sum_off, (u64)off);
                 // 500: how far down the lists reach in a small nucleus (they hold ~ 750)
                 const FineDecision fd = fine_decide<CL>(g, hist, mass_est, b_cut, need_topk() ? (u64)rw.kk : 0ull, 500ull, rw.topp, rw.topp < 1.0f, sc);
                 if (tid == 0) {
@@ -1714,7 +1774,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             auto keep_listed = [&](const Cand* list, int cap, float cut, const MassFn& mass) {
                 for (int j = lane; j < min(sc->wn[warp], cap); j += 32) {
                     const Cand c = list[j];
-                    if (c.l >= cut) { const uint32_t q = mass(c.l); if (q) atomicAdd(&csum[(c.idx + rw.a) / CHUNK], (u64)q); }
+                    if (c.l >= cut) { const uint32_t q = mass(c.l); if (q) add64(&csum[(c.idx + rw.a) / CHUNK], (u64)q); }
                 }
             };
             // the warps' view of the listed logits of all CTAs; over: a list overflowed
@@ -1839,6 +1899,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 Cand* blist = CL ? wlist + warp * WCAP : klist + warp * KCAP;
                 constexpr int bcap = CL ? WCAP : KCAP;
                 if (lane == 0) sc->wn[warp] = 0;
+                if (attempt) {                                   // (they start a row at zero)
+                    if (tid == 0) sc->sum_all = sc->sum_keep = 0;
+                    __syncthreads();
+                }
                 __syncwarp();
                 {
                     const float lk3 = fmaxf(rw.lcut, -SM_FLT_MAX), tl = fmaxf(rw.t_lo, lk3), t_hi = rw.t_hi;
@@ -1848,7 +1912,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     if (rw.path == PATH_BAND) {
                         if (!mp) ms = pass_mass<CL, ELT, MASK, true, false>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
                         else ms = pass_mass<CL, ELT, MASK, true, true>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
-                        if (lane == 0) { sc->g_all[warp] = ms.all; sc->g_keep[warp] = ms.keep; }
+                        if (lane == 0) { add64(&sc->sum_all, ms.all); add64(&sc->sum_keep, ms.keep); }
                     } else if (!mp) pass_mass<CL, ELT, MASK, false, false>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
                     else pass_mass<CL, ELT, MASK, false, true>(rw, nx, THEN_NEXT_ROW, mass, lk3, t_hi, tl, blist, csum);
                 }
@@ -1856,8 +1920,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 if (rw.path != PATH_BAND) break;
                 g.sync();
                 u64 s1 = 0, s_above = 0;
-                for (int i = lane; i < GW; i += 32) { const Sc* ps = g.at(sc, i / NW); s1 += ps->g_all[i % NW]; s_above += ps->g_keep[i % NW]; }
-                s1 = warp_sum_u64(s1); s_above = warp_sum_u64(s_above);
+                for (int q = 0; q < (CL ? g.C : 1); ++q) { const Sc* ps = g.at(sc, q); s1 += ps->sum_all; s_above += ps->sum_keep; }
                 bool over;
                 const View w = view_all(blist, bcap, over);
                 const u64 target = ceil_target(rw.topp, s1);
@@ -1995,7 +2058,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         derive_next();
         // (nobody reads these of this row any more)
         if (tid < NW) { sc->wn[tid] = 0; sc->swf[tid] = CI_NEG_INF; }
-        if (tid == 0) { sc->flags = 0; sc->nsel = 0; }
+        if (tid == 0) { sc->flags = 0; sc->nsel = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0; }
         if (CL) g.sync(); else __syncthreads();
         if (tid == 0 && g.rank == 0) {
             int status = rw.status;
@@ -2018,4 +2081,4 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     p.expect(-1);                                                // nothing is on its way when the CTA ends
 }
 
-}  // namespace smp
+}  // namespace SMP_NAME
