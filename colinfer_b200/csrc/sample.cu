@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "sample_host.h"
 #include "../../include/colinfer_b200.h"
 
 #define CI_THREADS 256
@@ -1461,6 +1462,104 @@ extern "C" int colinfer_max_active_clusters(int V, int dtype) {
     return active_clusters(g);
 }
 
+// ---- the chunk kernel (sample_rows.cu: a CTA per row, sample_few.cu: a cluster per row)
+namespace {
+constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024, kMaxDev = 64;
+
+int chunk_index(bool few, int dtype, bool mask) { return (few ? 4 : 0) + (dtype == COLINFER_F32 ? 0 : 2) + (mask ? 1 : 0); }
+const void* chunk_kernel(int ki) { return ki >= 4 ? colinfer_few_kernel(ki - 4) : colinfer_rows_kernel(ki); }
+
+// The device's number of SMs, and once per device and kernel the opt-in to large shared memory.
+int chunk_device(int ki, int* dev_out, int* sms_out) {
+    static bool opted[kMaxDev][8] = {};
+    static int sms[kMaxDev] = {};
+    static std::mutex guard;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= kMaxDev) return (int)cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(guard);
+    if (!opted[dev][ki]) {
+        e = cudaFuncSetAttribute(chunk_kernel(ki), cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkMaxSmem);
+        if (e == cudaSuccess && !sms[dev]) e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return (int)e;
+        opted[dev][ki] = true;
+    }
+    *dev_out = dev; *sms_out = sms[dev];
+    return 0;
+}
+
+void chunk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool few, int cluster, long long groups, int smem, cudaStream_t st) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3((unsigned)(groups * cluster), 1, 1);
+    cfg.blockDim = dim3((unsigned)(few ? colinfer_few_threads() : colinfer_rows_threads()), 1, 1);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = few ? 1 : 0;
+}
+
+// Clusters of `cluster` CTAs that the device holds at once (cached).
+int chunk_clusters(int dev, int ki, int cluster, int smem) {
+    struct Entry { int dev, ki, cs, smem, n; };
+    static Entry cache[64];
+    static int used = 0;
+    static std::mutex guard;
+    std::lock_guard<std::mutex> lock(guard);
+    for (int i = 0; i < used; ++i)
+        if (cache[i].dev == dev && cache[i].ki == ki && cache[i].cs == cluster && cache[i].smem == smem) return cache[i].n;
+    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+    chunk_config(cfg, attr, true, cluster, 1024, smem, nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, chunk_kernel(ki), &cfg) != cudaSuccess || n <= 0) return 0;
+    if (used < 64) cache[used++] = Entry{dev, ki, cluster, smem, n};
+    return n;
+}
+
+// Launches the chunk kernel where it is the faster one; returns -1 where it is not (nothing launched), else a CUDA error code.
+int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_rows, int W, const colinfer_sampler_params* params, const void* pos,
+                 int pos_is_i64, const float* u, int64_t* out_ids, colinfer_row_stats* stats, int32_t* status, int B, int R, int V, int flags, cudaStream_t stream) {
+    const long long rows = (long long)B * R;
+    if (V > kChunkMaxV || rows > 0x7ffffffeLL) return -1;
+    const bool pen = params->history != nullptr;
+    bool few = false;
+    int C = 1, dev = 0, sms = 0;
+    {
+        const int rc = chunk_device(chunk_index(false, dtype, mask != nullptr), &dev, &sms);
+        if (rc) return rc;
+    }
+    if (rows <= sms) {
+        // fewer rows than SMs: a cluster of two or four CTAs per row, where that fills the device
+        const int ki = chunk_index(true, dtype, mask != nullptr), smem = colinfer_few_smem(V, pen);
+        if (smem > kChunkMaxSmem) return -1;
+        const int rc = chunk_device(ki, &dev, &sms);
+        if (rc) return rc;
+        for (C = 4; C >= 2 && !few; C /= 2) {
+            few = V >= 16384 * C && rows <= chunk_clusters(dev, ki, C, smem);
+            if (few) break;
+        }
+        if (!few) return -1;
+    }
+    const int smem = few ? colinfer_few_smem(V, pen) : colinfer_rows_smem(V, pen);
+    if (smem > kChunkMaxSmem) return -1;
+    colinfer_sample_args a;
+    a.logits = logits;
+    a.mask = mask; a.mask_rows = mask_rows; a.W = W;
+    a.p = *params;
+    a.pos = pos; a.pos_i64 = pos_is_i64; a.u = u;
+    a.out = out_ids; a.stats = stats; a.status = status;
+    a.B = B; a.R = R; a.V = V; a.flags = flags; a.cluster = C;
+    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+    chunk_config(cfg, attr, few, C, rows, smem, stream);
+    void* args[] = {&a};
+    return (int)cudaLaunchKernelExC(&cfg, chunk_kernel(chunk_index(few, dtype, mask != nullptr)), args);
+}
+}  // namespace
+
 extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mask, int mask_rows, int W,
                                const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u,
                                int64_t* out_ids, colinfer_row_stats* stats, int32_t* status,
@@ -1489,6 +1588,11 @@ extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mas
                 const int res0 = active_clusters(g0);
                 if (res0 > 0 && (long long)B * R <= res0) use_stream = false;
             }
+        }
+        if (use_stream && choice == 0) {
+            const int rc = launch_chunk(logits, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status,
+                                        B, R, V, flags, (cudaStream_t)stream);
+            if (rc >= 0) return rc;
         }
         if (use_stream) {
             const int rc = colinfer_launch_stream(logits, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status,

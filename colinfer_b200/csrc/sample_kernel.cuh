@@ -25,6 +25,8 @@
 // the order of arrival nor on how many CTAs share a row.  Where a list overflows, a bound does not hold or the estimated
 // band misses the pivot, an exact select over the 32-bit keys runs (slower, same result).
 #pragma once
+#include <stddef.h>
+
 #include "common.cuh"
 #include "sample_host.h"
 
@@ -48,9 +50,9 @@ constexpr int NB1 = 4096;            // histogram buckets
 constexpr int HOFF = 1024;           // of these, above the sample's maximum
 constexpr float RANGE = 25.0f;       // they span RANGE temperatures
 constexpr int FASTK = 100;           // largest top_k finished from the sample's bound
-constexpr int BINS = 512;            // bins of the sample and of the selections on lists
-constexpr int BINS_PAD = BINS + BINS / 16;   // one spare word per sixteen: a lane reading its sixteen bins hits a bank of its own
-constexpr float FAST_SCALE = 32.0f;  // sample bins per unit logit (16 units)
+constexpr int BINS = 256;            // bins of the sample and of the selections on lists
+constexpr float FAST_SCALE = 16.0f;  // sample bins per unit logit (16 units)
+constexpr int BINS_BYTES = 4096;     // two sets of counts (or one of weights, a chunk in fp32, the candidates)
 constexpr int U_BYTES = SMP_LISTS;   // lists, or histogram and lists
 constexpr int FCAP = 128;            // candidates of the one-warp finish
 constexpr int KCAP = U_BYTES / 8 / NW;                       // list entries per warp: rows without a histogram,
@@ -73,11 +75,6 @@ using Args = colinfer_sample_args;
 
 template <bool B> struct BoolTag { static constexpr bool value = B; };
 struct Cand { uint32_t idx; float l; };
-
-// A row's parameters, fetched asynchronously while the CTA works on the row before.
-struct RowP {
-    float T; int kk; float topp, lmp; long long seed; float rp, pp, fp; int hlen; long long pos; float u; int pad;
-};
 
 // A row at hand.  What the phases of a row hand on lives here, not in registers: at 64 registers per thread anything that
 // stays alive across a pass is spilled, and with 226 KB of an SM's 256 in shared memory a spill is a round trip to L2.
@@ -112,7 +109,6 @@ struct WarpRing { int cons, out, key; };
 struct NextRow { const char* base; uint32_t end; int key, Nc; };
 
 struct Sc {
-    RowP rp[2];
     RowS rows[2];                      // the row at hand and the one after it, by the parity of the row's number in the CTA
     NextRow next[2];
     WarpRing ring[NW];
@@ -132,7 +128,7 @@ struct Sc {
     u64 g_all[NW], g_keep[NW];
     u64 t_cnt, t_est, sum_off;         // totals of the CTA's share of the histogram; what the estimates are off by
     u64 sum_all, sum_keep;             // masses of the CTA's chunks
-    int nsel;                          // candidates selected
+    int nsel, npush;                   // candidates selected, candidates sent to the group's first CTA
     int ok; float fin_cut; u64 fin_total; int fin_token;
     int fb[3]; u64 fe[3];              // finds of fine_decide
     // CTA-local
@@ -151,7 +147,7 @@ struct Fin {
     uint32_t so_idx[FCAP]; float so_l[FCAP]; uint32_t so_q[FCAP];
     int ties[FCAP];
 };
-static_assert(sizeof(Fin) <= 2 * BINS_PAD * 4 && 2 * FCAP * 4 <= BINS_PAD * 4, "candidates over the bins");
+static_assert(sizeof(Fin) <= BINS_BYTES && 2 * FCAP * 4 <= BINS * 4, "candidates over the bins");
 
 // Shared memory: rings, scratch, lists (or histogram and lists), bins, barriers, chunk sums, penalty tables (launches with
 // histories).  The history bitmap, a bit per position, lies over lists, bins and chunk sums while the tables are built.
@@ -159,12 +155,12 @@ constexpr int OFF_SC = NW * RING;
 constexpr int OFF_BARS = (OFF_SC + (int)sizeof(Sc) + 15) & ~15;
 constexpr int OFF_U = (OFF_BARS + NW * 8 * NST + 127) & ~127;
 constexpr int OFF_BINS = OFF_U + U_BYTES;
-constexpr int OFF_CSUM = OFF_BINS + 2 * BINS_PAD * 4;
-static_assert(2 * BINS_PAD * 4 >= BINS * 8 && BINS_PAD * 4 >= CHUNK * 4, "what lies over the bins");
+constexpr int OFF_CSUM = OFF_BINS + BINS_BYTES;
+static_assert(BINS_BYTES >= 2 * BINS * 4 && BINS_BYTES >= BINS * 8 && BINS_BYTES >= FB_NB * 8 && BINS_BYTES >= CHUNK * 4, "what lies over the bins");
 __host__ __device__ inline int max_chunks(int V) { return (V + 7 + CHUNK - 1) / CHUNK; }   // a row may start seven logits into its first chunk
 __host__ __device__ inline int pen_offset(int V, bool pen) {
     const int nc = max_chunks(V);
-    const int over = pen ? nc * 64 - U_BYTES - 2 * BINS_PAD * 4 : 0;      // what of the bitmap reaches into the chunk sums
+    const int over = pen ? nc * 64 - U_BYTES - BINS_BYTES : 0;      // what of the bitmap reaches into the chunk sums
     return (OFF_CSUM + (nc * 8 > over ? nc * 8 : over) + 15) & ~15;
 }
 __host__ __device__ inline int smem_bytes(int V, bool pen) { return pen_offset(V, pen) + (pen ? 4 * PEN_TABLE + (max_chunks(V) + 1) * 4 : 0); }
@@ -175,7 +171,6 @@ __device__ __forceinline__ Fin* fin_area() { return reinterpret_cast<Fin*>(smem 
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
-__host__ __device__ __forceinline__ int padbin(int i) { return i + (i >> 4); }
 __device__ __forceinline__ float fmax3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 __device__ __forceinline__ float max16(const float (&v)[16]) {
     const float a = fmax3(v[0], v[1], v[2]), b = fmax3(v[3], v[4], v[5]), c = fmax3(v[6], v[7], v[8]);
@@ -266,31 +261,25 @@ __device__ __forceinline__ int fine_bucket(float x, float href, float scale, flo
     return __float_as_int(t + 8388608.0f) - 0x4B000000;
 }
 
-// Bin of a BINS-bin count histogram in which the running count reaches kk, or -1; computed by the calling warp alone.
-// run_out: count down to and including that bin (all of them for -1).
-__device__ __forceinline__ int warp_count_bin(const uint32_t* hist, uint32_t kk, int lane, uint32_t& run_out) {
-    constexpr int PERB = BINS / 32;
-    static_assert(PERB == 16, "padbin() pads after every sixteenth bin");
-    uint32_t s = 0;
-#pragma unroll
-    for (int t = 0; t < PERB; ++t) s += hist[lane * (PERB + 1) + t];
+// Bin of a BINS-bin count histogram in which the running count reaches kk, or -1; computed by the calling warp alone, eight
+// bins per lane.  run_out: count down to and including that bin (all of them for -1).
+static __device__ __noinline__ int warp_count_bin(const uint32_t* hist, uint32_t kk, uint32_t& run_out) {
+    static_assert(BINS == 256, "eight bins per lane");
+    const int lane = lane_id();
+    const uint4 a = reinterpret_cast<const uint4*>(hist)[2 * lane], b = reinterpret_cast<const uint4*>(hist)[2 * lane + 1];
+    const uint32_t p1 = a.x + a.y, p3 = p1 + a.z + a.w, p5 = p3 + b.x + b.y, s = p5 + b.z + b.w;
     uint32_t incl = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
-    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
-    if (all < kk) { run_out = all; return -1; }
     const unsigned hit = __ballot_sync(0xffffffffu, incl >= kk);
+    if (!hit) { run_out = __shfl_sync(0xffffffffu, incl, 31); return -1; }
+    const uint32_t e = incl - s, need = kk - min(kk, e);             // (of the crossing lane: how far into its bins)
+    int t; uint32_t r;
+    if (need <= p3) { if (need <= p1) { t = need <= a.x ? 0 : 1; r = t ? p1 : a.x; } else { t = need <= p1 + a.z ? 2 : 3; r = t == 2 ? p1 + a.z : p3; } }
+    else { if (need <= p5) { t = need <= p3 + b.x ? 4 : 5; r = t == 4 ? p3 + b.x : p5; } else { t = need <= p5 + b.z ? 6 : 7; r = t == 6 ? p5 + b.z : s; } }
     const int hl = __ffs(hit) - 1;
-    // the crossing lane's sixteen bins, one per lane
-    const uint32_t h = lane < PERB ? hist[hl * (PERB + 1) + lane] : 0u;
-    uint32_t in2 = h;
-#pragma unroll
-    for (int o = 1; o < PERB; o <<= 1) { const uint32_t x = __shfl_up_sync(0xffffffffu, in2, o); if (lane >= o) in2 += x; }
-    in2 += __shfl_sync(0xffffffffu, incl - s, hl);
-    const unsigned h2 = __ballot_sync(0xffffffffu, in2 >= kk);
-    const int bl = __ffs(h2) - 1;
-    run_out = __shfl_sync(0xffffffffu, in2, bl);
-    return hl * PERB + bl;
+    run_out = __shfl_sync(0xffffffffu, e + r, hl);
+    return __shfl_sync(0xffffffffu, 8 * lane + t, hl);
 }
 
 // ------------------------------------------------------------------------------------------------ packed fp32 pairs
@@ -901,10 +890,10 @@ __device__ __forceinline__ int select_top(const View& w, float bound, float cut,
     const float lo = fmaxf(bound, cut);
     scale = L > lo ? (float)(BINS - 2) / (L - lo) : 0.0f;
     auto bin_of = [&](float l) { return max(0, min(BINS - 1, __float2int_rz((L - l) * scale))); };
-    for (int j = w.start; j < w.n; j += w.step) { const float l = w.p[j].l; if (l >= lo) atomicAdd(&bins[padbin(bin_of(l))], 1u); }
+    for (int j = w.start; j < w.n; j += w.step) { const float l = w.p[j].l; if (l >= lo) atomicAdd(&bins[(bin_of(l))], 1u); }
     __syncthreads();
     uint32_t run_b;
-    bstar = warp_count_bin(bins, (uint32_t)kk, lane, run_b);         // every warp scans the bins itself
+    bstar = warp_count_bin(bins, (uint32_t)kk, run_b);         // every warp scans the bins itself
     int n = (int)run_b;
     if (bstar < 0) {
         // fewer than kk listed logits reach lo: if lo is the cut, fewer than kk logits survive it and top-k removes nothing
@@ -1071,18 +1060,30 @@ __device__ bool list_select(const View& w, W wt, float base, float scale, u64 ta
 
 // One pass over the histogram, summed over the CTAs of the cluster, for everything the path decision needs: the bucket of the
 // kk-th largest count, the bucket where the running count reaches cap, and the bucket where the running estimated mass
-// reaches topp of its total.  CTA r sums the buckets [r, r + 1) * NB1 / C.  Buckets beyond `last` count nothing.
+// reaches topp of its total.  CTA r sums the buckets [r, r + 1) * NB1 / C.  Buckets beyond `last` count nothing.  The estimated
+// mass of a logit of bucket b is 2^(min(0, e0 - b * e1)) (of the last bucket, which holds everything beyond, 0; of bucket
+// `last`, last_part of it), in units of 2^-30.
+struct Estimate {
+    float e0, e1, last_part; int last;
+    __device__ __forceinline__ uint32_t operator()(int b) const {
+        float e;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fminf(0.0f, fmaf(-(float)b, e1, e0))));
+        e *= CI_MASS_SCALE;
+        return b == NB1 - 1 ? 0u : __float2uint_rn(b == last ? e * last_part : e);
+    }
+};
 struct FineDecision { int b_k; u64 n_upto; u64 total_cnt; int b_cap; int b_p; u64 est_total; };
-template <bool CL, class W>
-__device__ FineDecision fine_decide(const Grp<CL>& g, uint32_t* hist, W west, int last, u64 kk_target, u64 cap_target, float topp, bool want_p, Sc* sc) {
+template <bool CL>
+__device__ __forceinline__ FineDecision fine_decide(const Grp<CL>& g, uint32_t* hist, const Estimate& west, u64 kk_target, u64 cap_target, float topp, Sc* sc) {
     constexpr int PER = NB1 / NT;
     const int lane = lane_id(), warp = warp_id();
     const int per = CL ? PER / g.C : PER;
     const int lo = (CL ? g.rank * (NB1 / g.C) : 0) + (int)threadIdx.x * per;
     uint32_t c[PER];
-#pragma unroll
-    for (int t = 0; t < PER; ++t) c[t] = 0;
     if constexpr (CL) {
+#pragma unroll
+        for (int t = 0; t < PER; ++t) c[t] = 0;
+#pragma unroll 1
         for (int r = 0; r < g.C; ++r) {
             const uint32_t* h = g.at(hist, r);
 #pragma unroll
@@ -1095,99 +1096,95 @@ __device__ FineDecision fine_decide(const Grp<CL>& g, uint32_t* hist, W west, in
             c[t] = x.x; c[t + 1] = x.y; c[t + 2] = x.z; c[t + 3] = x.w;
         }
     }
-    u64 sc_c = 0, sc_e = 0;
+    uint32_t sc_c = 0; u64 sc_e = 0;
 #pragma unroll
     for (int t = 0; t < PER; ++t) {
-        if (lo + t <= last && c[t]) { sc_c += c[t]; if (want_p) sc_e += (u64)c[t] * west(lo + t); } else c[t] = 0;
+        if (t >= per || lo + t > west.last) c[t] = 0;
+        sc_c += c[t]; sc_e += (u64)c[t] * west(lo + t);
     }
-    const u64 in_c = warp_incl_scan_u64(sc_c, lane), in_e = warp_incl_scan_u64(sc_e, lane);
+    // two prefix scans share the barriers
+    uint32_t in_c = sc_c; u64 in_e = sc_e;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, in_c, o); const u64 y = __shfl_up_sync(0xffffffffu, in_e, o);
+        if (lane >= o) { in_c += x; in_e += y; }
+    }
     if (lane == 31) { sc->wsum[warp] = in_c; sc->wsum2[warp] = in_e; }
+    if (threadIdx.x < 3) { sc->fb[threadIdx.x] = -1; sc->fe[threadIdx.x] = 0; }
     __syncthreads();
-    if (warp == 0) {
+    u64 off_c = 0, off_e = 0, tot_c = 0, tot_e = 0;                  // every warp adds the others up
+    {
         const u64 w1 = lane < NW ? sc->wsum[lane] : 0ull, w2 = lane < NW ? sc->wsum2[lane] : 0ull;
-        const u64 i1 = warp_incl_scan_u64(w1, lane), i2 = warp_incl_scan_u64(w2, lane);
-        if (lane < NW) { sc->woff[lane] = i1 - w1; sc->woff2[lane] = i2 - w2; }
-        if (lane == NW - 1) { sc->t_cnt = i1; sc->t_est = i2; }
-        if (lane < 3) { sc->fb[lane] = -1; sc->fe[lane] = 0; }
+        off_c = warp_sum_u64(lane < warp ? w1 : 0ull); off_e = warp_sum_u64(lane < warp ? w2 : 0ull);
+        tot_c = warp_sum_u64(w1); tot_e = warp_sum_u64(w2);
     }
-    g.sync();
     FineDecision o;
-    u64 off_c = 0, off_e = 0;
-    long long off = 0;                                               // what the estimates are off by on the largest logits
-    o.total_cnt = 0; o.est_total = 0;
-    for (int r = 0; r < (CL ? g.C : 1); ++r) {
-        const Sc* ps = g.at(sc, r);
-        const u64 tc = ps->t_cnt, te = ps->t_est;
-        if (r < g.rank) { off_c += tc; off_e += te; }
-        o.total_cnt += tc; o.est_total += te;
-        off += (long long)ps->sum_off;
+    long long off = (long long)sc->sum_off;                          // what the estimates are off by on the largest logits
+    o.total_cnt = tot_c; o.est_total = tot_e;
+    if constexpr (CL) {
+        if (threadIdx.x == 0) { sc->t_cnt = tot_c; sc->t_est = tot_e; }
+        g.sync();
+        o.total_cnt = o.est_total = 0; off = 0;
+#pragma unroll 1
+        for (int r = 0; r < g.C; ++r) {
+            const Sc* ps = g.at(sc, r);
+            const u64 tc = ps->t_cnt, te = ps->t_est;
+            if (r < g.rank) { off_c += tc; off_e += te; }
+            o.total_cnt += tc; o.est_total += te;
+            off += (long long)ps->sum_off;
+        }
     }
-    const u64 ex_c = off_c + sc->woff[warp] + in_c - sc_c, ex_e = off_e + sc->woff2[warp] + in_e - sc_e;
+    const u64 ex_c = off_c + in_c - sc_c, ex_e = off_e + in_e - sc_e;
     u64 t_p = 0;
-    if (want_p && o.est_total > 0 && (long long)o.est_total + off > 0) {
+    if (topp < 1.0f && (long long)o.est_total + off > 0) {
         const long long t = (long long)ceil_target(topp, (u64)((long long)o.est_total + off)) - off;
         t_p = t < 1 ? 1ull : min((u64)t, o.est_total);
     }
-    auto tell = [&](int k, int b, u64 v) { for (int r = 0; r < (CL ? g.C : 1); ++r) { Sc* ps = g.at(sc, r); ps->fb[k] = b; ps->fe[k] = v; } };
-    if (kk_target && ex_c < kk_target && kk_target <= ex_c + sc_c) {
-        u64 run = ex_c;
+    // the three finds: at most one thread of the group each
+    const bool f0 = kk_target && ex_c < kk_target && kk_target <= ex_c + sc_c, f1 = ex_c < cap_target && cap_target <= ex_c + sc_c;
+    const bool f2 = t_p && ex_e < t_p && t_p <= ex_e + sc_e;
+    if (f0 || f1 || f2) {
+        u64 run_c = ex_c, run_e = ex_e;
+        int b0 = -1, b1 = -1, b2 = -1; u64 n0 = 0;
 #pragma unroll
-        for (int t = 0; t < PER; ++t) { run += c[t]; if (run >= kk_target) { tell(0, lo + t, run); break; } }
-    }
-    if (cap_target && ex_c < cap_target && cap_target <= ex_c + sc_c) {
-        u64 run = ex_c;
-#pragma unroll
-        for (int t = 0; t < PER; ++t) { run += c[t]; if (run >= cap_target) { tell(1, lo + t, 0); break; } }
-    }
-    if (t_p && ex_e < t_p && t_p <= ex_e + sc_e) {
-        u64 run = ex_e;
-#pragma unroll
-        for (int t = 0; t < PER; ++t) { run += c[t] ? (u64)c[t] * west(lo + t) : 0ull; if (run >= t_p) { tell(2, lo + t, 0); break; } }
+        for (int t = 0; t < PER; ++t) {
+            run_c += c[t]; run_e += (u64)c[t] * west(lo + t);
+            if (f0 && b0 < 0 && run_c >= kk_target) { b0 = lo + t; n0 = run_c; }
+            if (f1 && b1 < 0 && run_c >= cap_target) b1 = lo + t;
+            if (f2 && b2 < 0 && run_e >= t_p) b2 = lo + t;
+        }
+#pragma unroll 1
+        for (int r = 0; r < (CL ? g.C : 1); ++r) {
+            Sc* ps = g.at(sc, r);
+            if (f0) { ps->fb[0] = b0; ps->fe[0] = n0; }
+            if (f1) ps->fb[1] = b1;
+            if (f2) ps->fb[2] = b2;
+        }
     }
     g.sync();
     o.b_k = sc->fb[0]; o.n_upto = sc->fe[0]; o.b_cap = sc->fb[1]; o.b_p = sc->fb[2];
     return o;
 }
 
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
-// Fetches a row's parameters into `rp` (asynchronously; cp.async.wait_all before use).  One warp, a lane per parameter.
-__device__ __forceinline__ void fetch_params(const Args& a, long long row, RowP* rp, int lane) {
-    const int b = (int)(row / a.R);
-    auto get = [&](float* dst, const float* src, float dflt) { if (src) cp_async4(dst, src + b); else *dst = dflt; };
-    switch (lane) {
-        case 0: cp_async4(&rp->T, a.p.temperature + b); break;
-        case 1: cp_async4(&rp->kk, a.p.top_k + b); break;
-        case 2: cp_async4(&rp->topp, a.p.top_p + b); break;
-        case 3: cp_async4(&rp->lmp, a.p.log_min_p + b); break;
-        case 4: get(&rp->rp, a.p.repetition_penalty, 1.0f); break;
-        case 5: get(&rp->pp, a.p.presence_penalty, 0.0f); break;
-        case 6: get(&rp->fp, a.p.frequency_penalty, 0.0f); break;
-        case 7: if (a.p.history && a.p.hist_len) cp_async4(&rp->hlen, a.p.hist_len + b); else rp->hlen = a.p.history ? a.p.hist_stride : 0; break;
-        case 8: if (a.u == nullptr && a.p.seed) cp_async8(&rp->seed, a.p.seed + b); break;
-        case 9:
-            if (a.u == nullptr && a.pos) {
-                if (a.pos_i64) cp_async8(&rp->pos, reinterpret_cast<const long long*>(a.pos) + b);
-                else cp_async4(&rp->pos, reinterpret_cast<const int*>(a.pos) + b);
-            }
-            break;
-        case 10: if (a.u) cp_async4(&rp->u, a.u + row); break;
-        default: break;
+// A row's parameters, one 32-bit word per lane: temperature, top_k, top_p, log_min_p, seed (low), the three penalties, seed (high),
+// hist_len, position (low, high), explicit uniform.
+__device__ __forceinline__ uint32_t load_params(const Args& a, int row, int lane) {
+    const int b = a.R == 1 ? row : row / a.R;
+    const uint32_t* src = nullptr;
+    size_t at = b;
+    if (lane < 10) {
+        src = reinterpret_cast<const uint32_t*>(reinterpret_cast<const void* const*>(&a.p)[lane == 8 ? 4 : lane]);
+        if (lane == 4 || lane == 8) at = 2 * (size_t)b + (lane == 8);
+    } else if (lane < 12) {
+        if (a.u == nullptr && (a.pos_i64 || lane == 10)) src = reinterpret_cast<const uint32_t*>(a.pos);
+        if (a.pos_i64) at = 2 * (size_t)b + (lane - 10);
+    } else if (lane == 12) {
+        src = reinterpret_cast<const uint32_t*>(a.u); at = row;
     }
+    return src ? __ldg(src + at) : lane == 5 ? 0x3F800000u : lane == 9 ? (uint32_t)a.p.hist_stride : 0u;
 }
-__device__ __forceinline__ float row_uniform(const Args& a, const RowP* rp, int r) {
-    if (a.u != nullptr) return rp->u;
-    if (a.pos != nullptr && a.p.seed != nullptr) {
-        const long long p0 = a.pos_i64 ? rp->pos : (long long)*reinterpret_cast<const int*>(&rp->pos);
-        return u32_to_uniform(philox_word(philox_key(rp->seed), (u64)p0 + (u64)r));
-    }
-    return 1.0f;
-}
+static_assert(offsetof(colinfer_sampler_params, hist_len) == 9 * sizeof(void*) && offsetof(colinfer_sampler_params, seed) == 4 * sizeof(void*) &&
+              offsetof(colinfer_sampler_params, frequency_penalty) == 7 * sizeof(void*), "load_params indexes the pointers");
 
 // Where a row lies.
 template <int ELT>
@@ -1198,30 +1195,40 @@ __device__ __forceinline__ const char* place_row(const Args& a, int row, int& al
     nc = (a.V + al + CHUNK - 1) / CHUNK;
     return reinterpret_cast<const char*>(addr & ~15ull);
 }
-// Fills in row number `it` of the CTA from its parameters.  One thread.
+// Fills in a row from its parameters (load_params' words).  One warp.
 template <int ELT>
-static __device__ __noinline__ void derive_row(const Args& a, int it, int row) {
-    Sc* sc = scratch();
-    const RowP* rp = &sc->rp[it & 1];
-    RowS& rw = sc->rows[it & 1];
+static __device__ __noinline__ void derive_row(const Args& a, RowS& rw, int row, uint32_t words) {
+    auto word = [&](int l) { return __shfl_sync(0xffffffffu, words, l); };
+    auto num = [&](int l) { return __uint_as_float(word(l)); };
     const int b = a.R == 1 ? row : row / a.R, r = row - b * a.R;
-    rw.base = place_row<ELT>(a, row, rw.a, rw.end, rw.Nc);
-    rw.row = row; rw.key = row + 1;
-    rw.mrow = a.mask ? a.mask + ((size_t)b * a.mask_rows + r) * a.W : nullptr;
-    const int hlen = max(0, min(rp->hlen, a.p.hist_stride));
-    rw.hist = a.p.history ? a.p.history + (size_t)b * a.p.hist_stride : nullptr;
-    rw.hlen = hlen; rw.rp = rp->rp; rw.pp = rp->pp; rw.fp = rp->fp;
-    rw.pen_on = a.p.history != nullptr && hlen > 0 && !(rp->rp == 1.0f && rp->pp == 0.0f && rp->fp == 0.0f);
-    rw.pen_cap = hlen <= 65535 ? PEN_TABLE : 0;                  // (the counts are 16 bits)
-    const int kk = rp->kk;
-    const bool sampled = (rp->T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION);
-    const bool fastk = sampled && kk > 0 && kk <= FASTK && kk < a.V;
-    const bool wide = sampled && !fastk && ((kk > 0 && kk < a.V) || rp->topp < 1.0f);
-    rw.cls = (sampled ? ROW_SAMPLED : 0) | (fastk ? ROW_FASTK : 0) | (wide ? ROW_WIDE : 0);
-    rw.tc = fmaxf(rp->T, 1e-6f); rw.kk = kk; rw.topp = rp->topp; rw.lmp = rp->lmp;
-    rw.scw = (float)NB1 / (RANGE * rw.tc);
-    rw.u = row_uniform(a, rp, r);
-    rw.hist_slow = 0;
+    const float T = num(0), topp = num(2), rp = num(5), pp = num(6), fp = num(7);
+    const int kk = (int)word(1);
+    float u = num(12);
+    if (a.u == nullptr) {
+        const u64 seed = ((u64)word(8) << 32) | word(4);
+        long long pos = (int)word(10);
+        if (a.pos_i64) pos = (long long)(((u64)word(11) << 32) | word(10));
+        u = a.pos != nullptr && a.p.seed != nullptr ? u32_to_uniform(philox_word(philox_key((int64_t)seed), (u64)pos + (u64)r)) : 1.0f;
+    }
+    const float lmp = num(3);
+    const int hlen = a.p.history ? max(0, min((int)word(9), a.p.hist_stride)) : 0;
+    if (lane_id() == 0) {
+        rw.base = place_row<ELT>(a, row, rw.a, rw.end, rw.Nc);
+        rw.row = row; rw.key = row + 1;
+        rw.mrow = a.mask ? a.mask + ((size_t)b * a.mask_rows + r) * a.W : nullptr;
+        rw.hist = a.p.history ? a.p.history + (size_t)b * a.p.hist_stride : nullptr;
+        rw.hlen = hlen; rw.rp = rp; rw.pp = pp; rw.fp = fp;
+        rw.pen_on = hlen > 0 && !(rp == 1.0f && pp == 0.0f && fp == 0.0f);
+        rw.pen_cap = hlen <= 65535 ? PEN_TABLE : 0;              // (the counts are 16 bits)
+        const bool sampled = (T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION);
+        const bool fastk = sampled && kk > 0 && kk <= FASTK && kk < a.V;
+        const bool wide = sampled && !fastk && ((kk > 0 && kk < a.V) || topp < 1.0f);
+        rw.cls = (sampled ? ROW_SAMPLED : 0) | (fastk ? ROW_FASTK : 0) | (wide ? ROW_WIDE : 0);
+        rw.tc = fmaxf(T, 1e-6f); rw.kk = kk; rw.topp = topp; rw.lmp = lmp;
+        rw.scw = (float)NB1 / (RANGE * rw.tc);
+        rw.u = u;
+        rw.hist_slow = 0;
+    }
 }
 
 // The hardware's queue of the grid's CTAs that have not started: a running CTA asks for the index of one of them, which then
@@ -1261,8 +1268,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     Cand* push = reinterpret_cast<Cand*>(smem + OFF_U);          // [C][PUSH / C] candidates of all CTAs, over the histogram
     Cand* gath = reinterpret_cast<Cand*>(smem + OFF_U);          // [NW][GCAP] lists of all CTAs, over the histogram
     uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem + OFF_U);        // history bitmap while the tables are built (may reach over bins and csum)
-    uint32_t* sbins = reinterpret_cast<uint32_t*>(smem + OFF_BINS);      // [BINS_PAD] sample
-    uint32_t* fbins = sbins + BINS_PAD;                          // [BINS_PAD] selection
+    uint32_t* sbins = reinterpret_cast<uint32_t*>(smem + OFF_BINS);      // [BINS] sample
+    uint32_t* fbins = sbins + BINS;                          // [BINS] selection
     u64* bins = reinterpret_cast<u64*>(sbins);                   // [BINS] weighted selections, radix levels
     float* xbuf = reinterpret_cast<float*>(sbins);               // [CHUNK] the chunk the draw falls into
     u64* csum = reinterpret_cast<u64*>(smem + OFF_CSUM);         // [chunks] kept mass per chunk (the CTA's own)
@@ -1271,7 +1278,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         sc->V = V; sc->W = a.W; sc->GW = GW; sc->rank = g.rank;
         sc->drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0; sc->dead = 0;
         sc->pen_off = pen_offset(V, a.p.history != nullptr);
-        sc->flags = 0; sc->nsel = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0;
+        sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0;
     }
     if (lane == 0) {
         const uint32_t bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
@@ -1335,8 +1342,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     // The last warp looks after the row that comes next: takes it off the queue early in the first pass of the row at hand, notes
     // where it lies, fetches its parameters, and derives the rest before the row at hand ends.
     constexpr int PW = NW - 1;
-    int next_row = -1;                                           // (the last warp's)
-    auto fetch_row = [&](int it) { fetch_params(a, next_row, &sc->rp[it & 1], lane); asm volatile("cp.async.commit_group;" ::: "memory"); };
+    int next_row = -1; uint32_t next_words = 0;                  // (the last warp's)
     auto find_next = [&](int it) {                               // number it + 1
         if (CL) { const int row = grp + (it + 1) * n_grp; next_row = row < n_rows ? row : -1; }
         else {
@@ -1346,7 +1352,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             next_row = pos >= 0 ? row_of(pos) : -1;
         }
         if (next_row >= 0) {
-            fetch_row(it + 1);
+            next_words = load_params(a, next_row, lane);
             if (a.p.history) {                                   // the history's lines into L2
                 const char* h = reinterpret_cast<const char*>(a.p.history + (size_t)(a.R == 1 ? next_row : next_row / a.R) * a.p.hist_stride);
                 for (int i = lane * 128; i < min(a.p.hist_stride, 4096) * 4; i += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(h + i));
@@ -1361,19 +1367,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         }
         __syncwarp();
     };
-    auto derive = [&](int it) {
-        if (next_row >= 0) {
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) derive_row<ELT>(a, it, next_row);
-        }
-    };
+    auto derive = [&](int it) { if (next_row >= 0) derive_row<ELT>(a, sc->rows[it & 1], next_row, next_words); };
 #ifdef COLINFER_PROFILE
     long long prof_last = clock64();
 #endif
     if (warp == PW) {
         next_row = row_of(grp);
-        fetch_row(0);
+        next_words = load_params(a, next_row, lane);
         if (lane == 0) {
             RowS& rw = sc->rows[0];
             rw.base = place_row<ELT>(a, next_row, rw.a, rw.end, rw.Nc);
@@ -1429,10 +1429,24 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 for (int k = 0; k < 4; ++k) { const uint4 x = reinterpret_cast<const uint4*>(bitmap)[c * 4 + k]; s += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w); }
                 return s;
             };
+            // (where there is room behind the bitmap: every word's rank in its chunk)
+            unsigned short* wpre = reinterpret_cast<unsigned short*>(smem + OFF_U) + Nc * 32;
+            const bool ranked = Nc * 96 <= sc->pen_off - OFF_U;
             u64 local = 0, total_bits;
             for (int c = lo; c < hi; ++c) local += chunk_pop(c);
             uint32_t run = (uint32_t)block_excl_scan(local, sc, total_bits);
-            for (int c = lo; c < hi; ++c) { pt.pre[c] = run; if (c + 1 < hi) run += chunk_pop(c); }
+            for (int c = lo; c < hi; ++c) {
+                pt.pre[c] = run;
+                uint32_t in = 0;
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) {
+                    const uint4 x = reinterpret_cast<const uint4*>(bitmap)[c * 4 + k];
+                    const uint32_t n1 = in + __popc(x.x), n2 = n1 + __popc(x.y), n3 = n2 + __popc(x.z);
+                    if (ranked) reinterpret_cast<uint2*>(wpre)[c * 4 + k] = make_uint2(in | (n1 << 16), n2 | (n3 << 16));
+                    in = n3 + __popc(x.w);
+                }
+                run += in;
+            }
             if (tid == 0) pt.pre[Nc] = (uint32_t)total_bits;
             __syncthreads();
             const int cap = rw.pen_cap;
@@ -1440,12 +1454,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 int p;
                 if (!mine(v, p)) return;
                 const int c = p >> 9;
-                uint32_t rk = pt.pre[c];
-                for (int i = c * 16; i < (p >> 5); ++i) rk += __popc(bitmap[i]);   // the chunk's bits before the token's
-                rk += __popc(bitmap[p >> 5] & ((1u << (p & 31)) - 1u));
-                if ((int)rk < cap) {                             // the first to come brings the position along
-                    if (atomicAdd(&pt.ent[rk], 65536u) < 65536u) atomicAdd(&pt.ent[rk], (uint32_t)(p & (CHUNK - 1)));
-                }
+                uint32_t rk = pt.pre[c] + __popc(bitmap[p >> 5] & ((1u << (p & 31)) - 1u));
+                if (ranked) rk += wpre[p >> 5];
+                else for (int i = c * 16; i < (p >> 5); ++i) rk += __popc(bitmap[i]);
+                if ((int)rk < cap) { atomicOr(&pt.ent[rk], (uint32_t)(p & (CHUNK - 1))); atomicAdd(&pt.ent[rk], 65536u); }
             };
 #pragma unroll
             for (int j = 0; j < HP; ++j) enter(ht[j]);
@@ -1468,7 +1480,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             bool in_klist = fastk;
             if (lists) {
                 // The sample, the first two chunks of every warp: list bound, histogram layout.
-                for (int i = tid; i < 2 * BINS_PAD; i += NT) sbins[i] = 0u;
+                for (int i = tid; i < 2 * BINS; i += NT) sbins[i] = 0u;
                 if (wide) for (int i = tid; i < NB1 / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
                 float gm[8], sm = CI_NEG_INF;
 #pragma unroll
@@ -1513,11 +1525,11 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                     if (gm[k] > CI_NEG_INF && top < SM_POS_INF)
-                        atomicAdd(&sbins[padbin(max(0, min(BINS - 1, __float2int_rz((top - gm[k]) * FAST_SCALE))))], 1u);
+                        atomicAdd(&sbins[(max(0, min(BINS - 1, __float2int_rz((top - gm[k]) * FAST_SCALE))))], 1u);
                 __syncthreads();
                 auto bound = [&](int k) {                        // what at least k logits of the CTA's share reach (-FLT_MAX: unknown)
                     uint32_t have;
-                    const int bk = warp_count_bin(sbins, (uint32_t)k, lane, have);
+                    const int bk = warp_count_bin(sbins, (uint32_t)k, have);
                     return bk >= 0 && bk < BINS - 1 ? top - ((float)(bk + 1) + 0.01f) / FAST_SCALE - fabsf(top) * 1e-6f : -SM_FLT_MAX;
                 };
                 tw = bound(fastk ? rw.kk : 8);
@@ -1651,16 +1663,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         Cand* to = g.at(push, 0) + g.rank * pcap;
                         for (int j = w.start; j < w.n; j += 32) {
                             const Cand c = w.p[j];
-                            if (c.l >= lo) { const int at = atomicAdd(&sc->nsel, 1); if (at < pcap) to[at] = c; }
+                            if (c.l >= lo) { const int at = atomicAdd(&sc->npush, 1); if (at < pcap) to[at] = c; }
                         }
                         g.sync();
                         if (g.rank == 0) {
                             bool good = true;
-                            for (int q = 0; q < g.C; ++q) good = good && g.at(sc, q)->nsel <= pcap;
-                            const int wpr = NW / g.C, q = warp / wpr, mine = g.at(sc, q)->nsel;
-                            __syncthreads();
-                            if (tid == 0) sc->nsel = 0;
-                            __syncthreads();
+                            for (int q = 0; q < g.C; ++q) good = good && g.at(sc, q)->npush <= pcap;
+                            const int wpr = NW / g.C, q = warp / wpr, mine = g.at(sc, q)->npush;
                             const View w2{push + q * pcap, (warp % wpr) * 32 + lane, mine, 32 * wpr};
                             if (good) n = select_top(w2, lo_all, lcut, L, kq, fbins, sc, scale, bstar);
                         }
@@ -1709,12 +1718,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 // the histogram counts every logit; buckets wholly below the cut are left out
                 const int b_cut = bucket(lcut);
                 const float dL = (rw.L - href) / rw.tc;
-                // the estimated mass of a logit of bucket i (the last one holds everything beyond; of the cut's bucket, the part above)
-                const float cut_part = fminf(fmaxf((href - (float)(b_cut - hoff) / scw - lcut) * scw, 0.0f), 1.0f);
-                auto mass_est = [&](int i) {
-                    const float e = exp2f(fminf(0.0f, -(((float)(i - hoff) + 0.5f) * (RANGE / (float)NB1) + dL) * CI_LOG2E)) * CI_MASS_SCALE;
-                    return i == NB1 - 1 ? 0ull : (u64)__float2uint_rn(i == b_cut ? e * cut_part : e);
-                };
+                // bucket b's centre lies (b - hoff + 1/2) * RANGE / NB1 + dL temperatures below the row's maximum; of the cut's
+                // bucket only the part above the cut is kept
+                Estimate mass_est;
+                mass_est.e1 = RANGE / (float)NB1 * CI_LOG2E;
+                mass_est.e0 = ((float)hoff - 0.5f) * mass_est.e1 - dL * CI_LOG2E;
+                mass_est.last = b_cut;
+                mass_est.last_part = fminf(fmaxf((href - (float)(b_cut - hoff) / scw - lcut) * scw, 0.0f), 1.0f);
                 // What the estimates are off by on the listed logits -- the largest, which make up most of a peaked row's mass.
                 long long off = 0;
                 if (ready && !sc->in_klist) {
@@ -1728,7 +1738,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 off = (long long)warp_sum_u64((u64)off);
                 if (lane == 0) add64(&sc->sum_off, (u64)off);
                 // 500: how far down the lists reach in a small nucleus (they hold ~ 750)
-                const FineDecision fd = fine_decide<CL>(g, hist, mass_est, b_cut, need_topk() ? (u64)rw.kk : 0ull, 500ull, rw.topp, rw.topp < 1.0f, sc);
+                const FineDecision fd = fine_decide<CL>(g, hist, mass_est, need_topk() ? (u64)rw.kk : 0ull, 500ull, rw.topp, sc);
                 if (tid == 0) {
                     auto edge = [&](int bb) { return href - (float)(bb - hoff) / scw; };
                     int path = PATH_PURE;
@@ -2058,7 +2068,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         derive_next();
         // (nobody reads these of this row any more)
         if (tid < NW) { sc->wn[tid] = 0; sc->swf[tid] = CI_NEG_INF; }
-        if (tid == 0) { sc->flags = 0; sc->nsel = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0; }
+        if (tid == 0) { sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0; }
         if (CL) g.sync(); else __syncthreads();
         if (tid == 0 && g.rank == 0) {
             int status = rw.status;
