@@ -120,6 +120,15 @@ __device__ __forceinline__ u64 warp_incl_scan_u64(u64 v, int lane) {
     return v;
 }
 
+// 64-bit addition in shared memory as a 32-bit one with a carry: the hardware has no 64-bit one there, it would be a
+// compare-and-swap loop.  (The sum is complete once every adder is through.)
+__device__ __forceinline__ void add64(u64* p, u64 v) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(p);
+    const uint32_t lo = (uint32_t)v, old = atomicAdd(w, lo);
+    const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(w + 1, hi);
+}
+
 // ------------------------------------------------------------------------------------------------ bulk copy (TMA)
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

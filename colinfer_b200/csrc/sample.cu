@@ -30,7 +30,7 @@
 #include "sample_host.h"
 #include "../../include/colinfer_b200.h"
 
-#define CI_THREADS 256
+#define CI_THREADS 512
 #define CI_WARPS (CI_THREADS / 32)
 #define CI_CHUNK 4096            // elements per bulk copy
 #define CI_MAX_CHUNKS 16
@@ -42,10 +42,10 @@
 #define CI_FIN_MAX 1024          // candidates of one row at the CTA that finishes it (8 x CI_PCAP)
 #define CI_FAST_SCALE 32.0f      // its bins per unit logit (covers 16 units below the slice maximum)
 #define CI_PCAP 128              // candidates one CTA may push to the CTA that finishes the row
-#define CI_FIN_SCALE 64.0f       // bins per unit logit of the exact selection on the pushed candidates (8 units)
+#define CI_FIN_KEEP 128          // candidates that may be left after top-k
 #define CI_FIN_CAND 64           // candidates of one bin examined pairwise
 #define CI_RETRY 8               // rows a CTA may set aside for the generic path before the fast path is switched off
-#define CI_WLIST 48              // list entries per warp
+#define CI_WLIST 24              // list entries per warp
 #define CI_GLIST 1365            // gathered list entries (16 KB)
 #define CI_SEL_BINS 512          // coarse bins of the exact selection on a gathered list
 #define CI_FB_NB 256             // radix buckets per level of the fallback select (8 bits)
@@ -67,18 +67,22 @@ struct SampleArgs {
 // Profiling hook: thread 0 adds the cycles since its previous marker to the slot's total (summed over the CTA's rows).
 #define CI_PROF(slot) do { if (a.prof && tid == 0) { const long long t_ = clock64(); sc->prof[slot] += t_ - prof_last; prof_last = t_; } } while (0)
 
+#define CI_PROF_END() do { if (a.prof && tid == 0 && (int)blockIdx.x < a.prof_slots) { \
+    unsigned long long gt; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt)); \
+    a.prof[(size_t)blockIdx.x * 16 + 13] = (long long)gt; a.prof[(size_t)blockIdx.x * 16 + 12] = clock64() - prof_t0; \
+    for (int i = 0; i < 12; ++i) a.prof[(size_t)blockIdx.x * 16 + i] = sc->prof[i]; } } while (0)
+
 struct ListEntry { uint32_t idx; float l; uint32_t q; };   // gathered list: token, logit, mass
 struct Cand { uint32_t idx; float l; };                      // a warp's list / pushed candidates: token, logit
 
 // A row whose candidates have been pushed to this CTA and that waits for its exact finish.
-struct Pending { int row; float L; int aidx; int status; int count[8]; };
+struct Pending { int row; float L; int aidx; int status; int kk; float tc, topp, lmp, u; int count[8]; };
 
 // What every CTA writes into each peer's shared memory before the first cluster barrier.
 struct Hello { float lmax; int lidx; int flags; int pad; };   // flags: 1 = a bounded wait gave up, 4 = slow history path, 8 = stop using the fast path; pad: candidates pushed
 
 // Values one CTA publishes in its own shared memory for its peers to read after a later barrier.
 struct Xch {
-    u64 seg_cnt, seg_est;          // totals of this CTA's reduced bucket segment: counts, estimated mass
     u64 fb_segtot;                 // the same for the fallback radix select
     u64 s_all, s_above;            // band pass: kept mass of the slice, and of its part above the band
     u64 cta_mass;                  // kept mass of the slice under the final threshold
@@ -101,9 +105,10 @@ struct Scratch {
     int found_tid; u64 found_excl;
     float cand_l[CI_FIN_CAND]; u64 cand_w[CI_FIN_CAND]; float res_f;
     Pending pend;
-    int n_retry_common, n_retry_mine, want_fast_off;
+    int n_retry_common, n_retry_mine, any_retry, want_fast_off;   // any_retry: a CTA of the cluster has set a row aside
     int retry_common[CI_RETRY], retry_mine[CI_RETRY], retry_all[CI_RETRY * 9];
     long long prof[12];            // profiling hook: cycles per phase, summed over the CTA's rows
+    u64 seg_cnt[8], seg_est[8];    // totals of every CTA's reduced bucket segment, written by the peers: counts, estimated mass
     int bcast_i[2];                // written by the cluster's first CTA, per row parity
     u64 mass_in[2][8];             // kept mass of every CTA's slice, written by the peers, per row parity
 };
@@ -197,7 +202,7 @@ __device__ bool list_select(const ListEntry* gl, int n, W wt, u64 target, u64* b
     const int sh = max(0, 32 - __clz(span) - 9);
     for (int i = tid; i < n; i += CI_THREADS) {
         const u64 w = wt(i);
-        if (w > 0) atomicAdd(&bins[(kmax - f2key(gl[i].l)) >> sh], w);
+        if (w > 0) add64(&bins[(kmax - f2key(gl[i].l)) >> sh], w);
     }
     __syncthreads();
     int b_star; u64 before;
@@ -256,7 +261,7 @@ __device__ bool radix_select(cg::cluster_group& cluster, const RadixCtx& c, cons
                 if (l >= lk) {
                     const uint32_t key = f2key(l);
                     if (lvl == 0 || (key >> (shift + 8)) == prefix)
-                        atomicAdd(&c.fb_hist[CI_FB_NB - 1 - (int)((key >> shift) & 0xFFu)], by_mass ? (u64)mass(l) : 1ull);
+                        add64(&c.fb_hist[CI_FB_NB - 1 - (int)((key >> shift) & 0xFFu)], by_mass ? (u64)mass(l) : 1ull);
                 }
             }
         }
@@ -462,141 +467,165 @@ __device__ void bins_find(const T* bins, u64 target, Scratch* sc, int& bin, u64&
     before = sc->found_excl;
 }
 
-// Exact weighted selection among n entries (logits fl[0..n) in shared memory, weight wt(i)): the value v such that
-// W(l > v) < target <= W(l >= v).  CI_FAST_BINS bins over the distance from the row maximum, then the pivot bin's
-// entries pairwise.  Returns false when the pivot falls outside the binned range or its bin is too crowded.
-// All threads call with the same arguments.
-template <class W>
-__device__ bool lean_select(const float* fl, int n, W wt, float L, u64 target, u64* bins, Scratch* sc, float& value) {
-    const int tid = threadIdx.x;
-    for (int i = tid; i < CI_FAST_BINS; i += CI_THREADS) bins[i] = 0;
-    if (tid == 0) { sc->ncand = 0; sc->sel_ok = 0; }
-    __syncthreads();
-    for (int i = tid; i < n; i += CI_THREADS) {
-        const u64 w = wt(i);
-        if (w) atomicAdd(&bins[min(CI_FAST_BINS - 1, __float2int_rz((L - fl[i]) * CI_FIN_SCALE))], w);
-    }
-    __syncthreads();
-    int b_star; u64 before, total;
-    bins_find(bins, target, sc, b_star, before, total);
-    if (b_star < 0 || b_star >= CI_FAST_BINS - 1) return false;
-    for (int i = tid; i < n; i += CI_THREADS) {
-        const u64 w = wt(i);
-        if (w && min(CI_FAST_BINS - 1, __float2int_rz((L - fl[i]) * CI_FIN_SCALE)) == b_star) {
-            const int slot = atomicAdd(&sc->ncand, 1);
-            if (slot < CI_FIN_CAND) { sc->cand_l[slot] = fl[i]; sc->cand_w[slot] = w; }
-        }
-    }
-    __syncthreads();
-    const int nc = sc->ncand;
-    if (nc > CI_FIN_CAND) return false;
-    if (tid < nc) {
-        const float mine = sc->cand_l[tid];
-        u64 gt = 0, eq = 0;
-        for (int i = 0; i < nc; ++i) {
-            const float o = sc->cand_l[i];
-            if (o > mine) gt += sc->cand_w[i]; else if (o == mine) eq += sc->cand_w[i];
-        }
-        if (before + gt < target && target <= before + gt + eq) { sc->res_f = mine; sc->sel_ok = 1; }
-    }
-    __syncthreads();
-    value = sc->res_f;
-    return sc->sel_ok != 0;
-}
-
 // Exact finish of a row from the candidates its CTAs pushed into this CTA's shared memory: min-p, top-k, top-p and
 // the draw, all inside this CTA (no cluster traffic).  The candidates contain the row's top k logits (and possibly
-// more), in token order: CTA by CTA, each CTA's in token order.  Writes the row's outputs and returns true, or returns
-// false when the row has to take the generic path.  `work` is CI_FAST_BINS * 8 + CI_FIN_MAX * 8 bytes of scratch.
-// All threads of the CTA call.
-__device__ bool finish_pending(const SampleArgs& a, const Pending& pd, const Cand* plist, int CS, unsigned char* work, Scratch* sc) {
-    const int tid = threadIdx.x;
-    u64* bins = reinterpret_cast<u64*>(work);
-    float* fl = reinterpret_cast<float*>(work + CI_FAST_BINS * 8);
-    uint32_t* fi = reinterpret_cast<uint32_t*>(fl + CI_FIN_MAX);
-    const int row = pd.row, b = row / a.R, r = row % a.R;
-    const float tc = fmaxf(a.p.temperature[b], 1e-6f);
-    const int kk = a.p.top_k[b];
-    const float topp = a.p.top_p[b];
-    const float L = pd.L;
+// more), in token order: CTA by CTA, each CTA's in token order; a thread holds two of them.  Writes the row's outputs and
+// returns true, or returns false when the row has to take the generic path.  `work` is scratch.  All threads of the CTA call.
+// Latency is all there is to it: five block barriers, the searches repeated by every warp instead of published, the draw
+// by one warp.
+__device__ __noinline__ bool finish_pending(const SampleArgs& a, const Pending& pd, const Cand* plist, int CS, unsigned char* work, Scratch* sc) {
+    static_assert(CI_FIN_MAX == 2 * CI_THREADS && CI_WARPS == 16 && CI_FAST_BINS == 512 && CI_FIN_KEEP * 4 == CI_THREADS, "two candidates a thread");
+    const int tid = threadIdx.x, lane = lane_id(), warp = warp_id();
+    uint32_t* bins = reinterpret_cast<uint32_t*>(work);
+    float* kl = reinterpret_cast<float*>(work + CI_FAST_BINS * 4);
+    uint32_t* kq = reinterpret_cast<uint32_t*>(kl + CI_FIN_KEEP), *ki = kq + CI_FIN_KEEP;
+    const float tc = pd.tc, L = pd.L, topp = pd.topp;
+    const int kk = pd.kk;
     const float m = scale_logit(L, tc);
     MassFn mass;
     mass.init(tc, m);
-    const float thr = __fadd_rn(m, a.p.log_min_p[b]);
+    const float thr = __fadd_rn(m, pd.lmp);
     float cut = lower_logit_for(thr, tc, __fmul_rn(thr, tc));
     cut = fmaxf(cut, L - 22.0f * tc - fabsf(L) * 1e-6f);           // the mass horizon (see the generic path)
-    const float u = row_uniform(a, row, b, r);
     int pre[9];
     pre[0] = 0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) pre[q + 1] = pre[q] + (q < CS ? pd.count[q] : 0);
     const int n = pre[8];
     if (n > CI_FIN_MAX || n <= 0) return false;
-    // the concatenated lists, contiguous and in token order
-    for (int e = tid; e < n; e += CI_THREADS) {
+    // ---- this thread's candidates; how many survive min-p, and their range of keys
+    Cand c[2]; bool in[2]; uint32_t key[2];
+    uint32_t kmin = 0xFFFFFFFFu, kmax = 0u;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int e = 2 * tid + j;
         int q = 0;
 #pragma unroll
         for (int t = 1; t < 8; ++t) q += (pre[t] <= e) ? 1 : 0;
-        const Cand c = plist[q * CI_PCAP + (e - pre[q])];
-        fl[e] = c.l; fi[e] = c.idx;
+        c[j].l = CI_NEG_INF; c[j].idx = 0;
+        if (e < n) c[j] = plist[q * CI_PCAP + (e - pre[q])];
+        in[j] = c[j].l >= cut && c[j].l > CI_NEG_INF;
+        key[j] = f2key(c[j].l);
+        if (in[j]) { kmin = min(kmin, key[j]); kmax = max(kmax, key[j]); }
     }
+    kmin = __reduce_min_sync(0xffffffffu, kmin); kmax = __reduce_max_sync(0xffffffffu, kmax);
+    const int wcnt = __popc(__ballot_sync(0xffffffffu, in[0])) + __popc(__ballot_sync(0xffffffffu, in[1]));
+    if (lane == 0) { sc->warp_u[warp] = kmin; sc->warp_v[warp] = kmax; sc->warp_i[warp] = wcnt; }
+    bins[tid] = 0u;
+    if (tid == 0) { sc->ncand = 0; sc->sel_ok = 0; }
     __syncthreads();
-    // ---- top-k: the k-th largest of the candidates that survive min-p
-    u64 cnt = 0;
-    for (int i = tid; i < n; i += CI_THREADS) cnt += (fl[i] >= cut && fl[i] > CI_NEG_INF) ? 1 : 0;
-    u64 survivors;
-    block_excl_scan(cnt, sc, survivors);
+    kmin = __reduce_min_sync(0xffffffffu, sc->warp_u[lane & 15]); kmax = __reduce_max_sync(0xffffffffu, sc->warp_v[lane & 15]);
+    const int survivors = __reduce_add_sync(0xffffffffu, lane < 16 ? sc->warp_i[lane] : 0);
     if (survivors == 0) return false;
-    if ((u64)kk <= survivors) {                               // else fewer than k survive min-p: top-k removes nothing
-        float lk;
-        const float c0 = cut;
-        if (!lean_select(fl, n, [&](int i) { return (u64)((fl[i] >= c0 && fl[i] > CI_NEG_INF) ? 1 : 0); }, L, (u64)kk, bins, sc, lk))
-            return false;
+    // ---- top-k: the kk-th largest of them
+    if (kk <= survivors) {                                    // else fewer than k survive min-p: top-k removes nothing
+        const int sh = max(0, 32 - __clz(kmax - kmin) - 9);   // the bins cover [0, kmax - kmin] >> sh, at most 512
+#pragma unroll
+        for (int j = 0; j < 2; ++j) if (in[j]) atomicAdd(&bins[(kmax - key[j]) >> sh], 1u);
+        __syncthreads();
+        int b_star, before;
+        {
+            const uint4* b4 = reinterpret_cast<const uint4*>(bins) + lane * 4;   // a lane's sixteen bins
+            int s = 0, loc[16];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) { const uint4 x = b4[t]; loc[4 * t] = x.x; loc[4 * t + 1] = x.y; loc[4 * t + 2] = x.z; loc[4 * t + 3] = x.w; }
+#pragma unroll
+            for (int t = 0; t < 16; ++t) s += loc[t];
+            int incl = s;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
+            const int src = __ffs(__ballot_sync(0xffffffffu, incl >= kk)) - 1;
+            int run = incl - s, at = 15, run_at = run;
+            bool found = false;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) { if (!found && run + loc[t] >= kk) { found = true; at = t; run_at = run; } run += loc[t]; }
+            b_star = src * 16 + __shfl_sync(0xffffffffu, at, src);
+            before = __shfl_sync(0xffffffffu, run_at, src);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (in[j] && (int)((kmax - key[j]) >> sh) == b_star) {
+                const int slot = atomicAdd(&sc->ncand, 1);
+                if (slot < CI_FIN_CAND) sc->cand_l[slot] = c[j].l;
+            }
+        __syncthreads();
+        const int nc = sc->ncand, want = kk - before;
+        if (nc > CI_FIN_CAND) return false;
+        float lk = CI_NEG_INF;
+        for (int b0 = 0; b0 < nc; b0 += 32) {                 // (every warp, pairwise)
+            const float mine = b0 + lane < nc ? sc->cand_l[b0 + lane] : CI_NEG_INF;
+            int gt = 0, ge = 0;
+            for (int i = 0; i < nc; ++i) { const float o = sc->cand_l[i]; gt += o > mine ? 1 : 0; ge += o >= mine ? 1 : 0; }
+            const unsigned hit = __ballot_sync(0xffffffffu, b0 + lane < nc && gt < want && want <= ge);
+            if (hit) { lk = __shfl_sync(0xffffffffu, mine, __ffs(hit) - 1); break; }
+        }
         cut = fmaxf(cut, lower_logit_for(scale_logit(lk, tc), tc, lk));
     }
-    // ---- top-p over the kept candidates
+    // ---- what is left, in token order, with its masses
+    const bool k0 = in[0] && c[0].l >= cut, k1 = in[1] && c[1].l >= cut;
+    const unsigned lt = (1u << lane) - 1u, m0 = __ballot_sync(0xffffffffu, k0), m1 = __ballot_sync(0xffffffffu, k1);
+    if (lane == 0) sc->pcount[warp] = (unsigned short)(__popc(m0) + __popc(m1));
+    __syncthreads();
+    const int others = lane < 16 ? sc->pcount[lane] : 0;
+    const int nk = __reduce_add_sync(0xffffffffu, others);
+    if (nk == 0 || nk > CI_FIN_KEEP) return false;
+    {
+        int at = __reduce_add_sync(0xffffffffu, lane < warp ? others : 0) + __popc(m0 & lt) + __popc(m1 & lt);
+        if (k0) { kl[at] = c[0].l; kq[at] = mass(c[0].l); ki[at] = c[0].idx; ++at; }
+        if (k1) { kl[at] = c[1].l; kq[at] = mass(c[1].l); ki[at] = c[1].idx; }
+    }
+    __syncthreads();
+    // ---- top-p: the logit where the descending running mass reaches its share, four threads an entry
+    u64 s1 = 0;
+#pragma unroll
+    for (int t = 0; t < CI_FIN_KEEP / 32; ++t) s1 += t * 32 + lane < nk ? kq[t * 32 + lane] : 0u;
+    s1 = warp_sum_u64(s1);
+    if (s1 == 0) return false;
+    u64 total = s1;
     if (topp < 1.0f) {
-        const float c0 = cut;
-        u64 part = 0;
-        for (int i = tid; i < n; i += CI_THREADS) part += (fl[i] >= c0 && fl[i] > CI_NEG_INF) ? (u64)mass(fl[i]) : 0ull;
-        u64 s1;
-        block_excl_scan(part, sc, s1);
-        if (s1 == 0) return false;
-        float lp;
-        if (!lean_select(fl, n, [&](int i) { return (fl[i] >= c0 && fl[i] > CI_NEG_INF) ? (u64)mass(fl[i]) : 0ull; }, L,
-                         ceil_target(topp, s1), bins, sc, lp))
-            return false;
+        const u64 target = ceil_target(topp, s1);
+        const int e = tid >> 2;
+        const float mine = e < nk ? kl[e] : CI_NEG_INF;
+        u64 gt = 0, ge = 0;
+        for (int i = tid & 3; i < nk; i += 4) {
+            const float o = kl[i]; const u64 q = kq[i];
+            gt += o > mine ? q : 0ull; ge += o >= mine ? q : 0ull;
+        }
+        gt += __shfl_xor_sync(0xffffffffu, gt, 1); ge += __shfl_xor_sync(0xffffffffu, ge, 1);
+        gt += __shfl_xor_sync(0xffffffffu, gt, 2); ge += __shfl_xor_sync(0xffffffffu, ge, 2);
+        if (e < nk && gt < target && target <= ge) { sc->res_f = mine; sc->sel_ok = 1; }
+        __syncthreads();
+        if (!sc->sel_ok) return false;
+        const float lp = sc->res_f;
         cut = fmaxf(cut, lower_logit_for(scale_logit(lp, tc), tc, lp));
     }
     // ---- the draw: first candidate (token order) whose running kept mass reaches u * total
-    const int ept = (n + CI_THREADS - 1) / CI_THREADS;
-    const int e_lo = tid * ept, e_hi = min(e_lo + ept, n);
-    u64 mine = 0;
-    for (int i = e_lo; i < e_hi; ++i) mine += (fl[i] >= cut && fl[i] > CI_NEG_INF) ? (u64)mass(fl[i]) : 0ull;
-    u64 total;
-    const u64 excl = block_excl_scan(mine, sc, total);
-    if (total == 0) return false;
-    const u64 target = ceil_target(u, total);
-    if (excl < target && target <= excl + mine) {
-        u64 run = excl;
-        long long token = -1;
-        for (int i = e_lo; i < e_hi; ++i) {
-            run += (fl[i] >= cut && fl[i] > CI_NEG_INF) ? (u64)mass(fl[i]) : 0ull;
-            if (run >= target) { token = (long long)fi[i]; break; }
+    if (warp == 0) {
+        u64 q[4], mine = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { const int e = 4 * lane + j; q[j] = e < nk && kl[e] >= cut ? kq[e] : 0u; mine += q[j]; }
+        const u64 incl = warp_incl_scan_u64(mine, lane);
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        const u64 target = ceil_target(pd.u, total);
+        u64 run = incl - mine;
+        if (run < target && target <= incl) {
+            int j = 0;
+            for (; j < 3; ++j) { run += q[j]; if (run >= target) break; }
+            const int row = pd.row;
+            if (a.out) a.out[row] = (long long)ki[4 * lane + j];
+            if (a.status) a.status[row] = pd.status;
+            if (a.stats) {
+                colinfer_row_stats st;
+                st.lmax = L; st.lcut = cut; st.tc = tc; st.status = pd.status; st.argmax = pd.aidx; st.mass_q = total;
+                a.stats[row] = st;
+            }
         }
-        if (a.out) a.out[row] = token;
-        if (a.status) a.status[row] = pd.status;
-        if (a.stats) {
-            colinfer_row_stats st;
-            st.lmax = L; st.lcut = cut; st.tc = tc; st.status = pd.status; st.argmax = pd.aidx; st.mass_q = total;
-            a.stats[row] = st;
-        }
+        __syncwarp();                                         // (the caller takes the row off)
     }
-    __syncthreads();
     return true;
 }
 
-extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __grid_constant__ SampleArgs a) {
+extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __grid_constant__ SampleArgs a) {
     cg::cluster_group cluster = cg::this_cluster();
     // Every CTA announces that it runs; the matching wait comes just before the first write into a peer's shared memory.
     cluster.barrier_arrive();
@@ -659,7 +688,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
     bool fast_enabled = true;         // small top-k rows may take the deferred path (identical in every CTA)
     int fast_seq = 0;                 // deferred rows so far: row j is finished by CTA j % CS
     int n_set_aside = 0;              // rows set aside for the generic path by every CTA alike
-    if (tid == 0) { sc->pend.row = -1; sc->n_retry_common = 0; sc->n_retry_mine = 0; sc->want_fast_off = 0; }
+    if (tid == 0) { sc->pend.row = -1; sc->n_retry_common = 0; sc->n_retry_mine = 0; sc->any_retry = 0; sc->want_fast_off = 0; }
 
     // Every CTA that holds a deferred row finishes it; then the cluster meets so that candidates may be pushed again.
     auto flush = [&]() {
@@ -668,6 +697,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
             const bool ok = finish_pending(a, sc->pend, plist, CS, hreg, sc);
             if (tid == 0) {
                 if (!ok) {
+                    for (int q = 0; q < CS; ++q) *cluster.map_shared_rank(&sc->any_retry, q) = 1;
                     if (sc->n_retry_mine < CI_RETRY) sc->retry_mine[sc->n_retry_mine++] = sc->pend.row;
                     if (sc->n_retry_mine >= CI_RETRY - 1) sc->want_fast_off = 1;
                 }
@@ -706,6 +736,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
     const int kk = a.p.top_k[b];
     const float topp = a.p.top_p[b];
     const float log_min_p = a.p.log_min_p[b];
+    const float u = row_uniform(a, row, b, r);
     const bool fastk = allow_fast && fast_enabled && sampled && kk >= 1 && kk <= CI_FASTK && kk < V &&
                        !(a.flags & COLINFER_FORCE_DISTRIBUTION);         // identical in every CTA of the cluster
 
@@ -768,6 +799,18 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
     float tg[CI_TGROUPS];                                       // maxima of this thread's interleaved element groups
 #pragma unroll
     for (int j = 0; j < CI_TGROUPS; ++j) tg[j] = CI_NEG_INF;
+    // the mask words of this thread's first groups, on their way while the slice lands
+    constexpr int MPRE = 3;
+    uint32_t mw[MPRE][CI_TGROUPS];
+    if (mrow != nullptr) {
+#pragma unroll
+        for (int o = 0; o < MPRE; ++o)
+#pragma unroll
+            for (int k = 0; k < CI_TGROUPS; ++k) {
+                const int g = slice_lo + (tid + (o * CI_TGROUPS + k) * CI_THREADS) * 4;
+                mw[o][k] = g < min(slice_lo + n_pad, V) ? (uint32_t)__ldg(mrow + (g >> 5)) : 0xFFFFFFFFu;
+            }
+    }
     // (1) the slice lands: wait for the bulk copies, or load it with plain loads (unaligned fp32 rows, bf16)
     if (a.use_bulk) {
         const bool drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0;
@@ -832,7 +875,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
     {
         float4* row4 = reinterpret_cast<float4*>(rowbuf);
         const int n4 = n_pad >> 2;
-        for (int i0 = tid; i0 < n4; i0 += CI_TGROUPS * CI_THREADS) {
+        auto step = [&](int i0, auto word) {
             float4 v[CI_TGROUPS];
 #pragma unroll
             for (int k = 0; k < CI_TGROUPS; ++k) {
@@ -845,7 +888,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
                     const int i = i0 + k * CI_THREADS;
                     const int g = slice_lo + i * 4;             // global token index of v[k].x
                     if (i < n4 && g < V) {
-                        const uint32_t bits = ((uint32_t)__ldg(mrow + (g >> 5)) >> (g & 31)) & 0xFu;
+                        const uint32_t bits = (word(k, g) >> (g & 31)) & 0xFu;
                         if (bits != 0xFu) {
                             if (!(bits & 1u)) v[k].x = CI_NEG_INF;
                             if (!(bits & 2u)) v[k].y = CI_NEG_INF;
@@ -864,7 +907,14 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
                 lmax = up ? m4 : lmax;
                 lpos = up ? i0 + k * CI_THREADS : lpos;
             }
+        };
+#pragma unroll
+        for (int o = 0; o < MPRE; ++o) {
+            const int i0 = tid + o * CI_TGROUPS * CI_THREADS;
+            if (i0 < n4) step(i0, [&](int k, int) { return mw[o][k]; });
         }
+        for (int i0 = tid + MPRE * CI_TGROUPS * CI_THREADS; i0 < n4; i0 += CI_TGROUPS * CI_THREADS)
+            step(i0, [&](int, int g) { return (uint32_t)__ldg(mrow + (g >> 5)); });
     }
     CI_PROF(2);
     if (lpos >= 0) {
@@ -999,13 +1049,14 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
             if (rank == fast_seq % CS && tid == 0) {
                 Pending pd;
                 pd.row = row; pd.L = L; pd.aidx = aidx; pd.status = status;
+                pd.kk = kk; pd.tc = tc; pd.topp = topp; pd.lmp = log_min_p; pd.u = u;
                 for (int q = 0; q < 8; ++q) pd.count[q] = q < CS ? sc->hello[par][q].pad : 0;
                 sc->pend = pd;
             }
             ++fast_seq;
             if (fast_seq % CS == 0) flush();                    // every CTA holds a row now
         } else {
-            if (tid == 0 && sc->n_retry_common < CI_RETRY) sc->retry_common[sc->n_retry_common++] = row;
+            if (tid == 0) { sc->any_retry = 1; if (sc->n_retry_common < CI_RETRY) sc->retry_common[sc->n_retry_common++] = row; }
             if (++n_set_aside >= CI_RETRY) fast_enabled = false;
         }
         return;
@@ -1022,7 +1073,6 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
     lcut = fmaxf(lcut, L - 22.0f * tc - fabsf(L) * 1e-6f);
     bool need_topk = kk > 0 && kk < V;
     const bool need_topp = topp < 1.0f;
-    const float u = row_uniform(a, row, b, r);
 
     // (generic path from here on: the whole cluster works on the row until its token is out)
     enum { PATH_PURE = 0, PATH_LIST = 1, PATH_BAND = 2, PATH_FALLBACK = 3 };
@@ -1058,7 +1108,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
         CI_PROF(10);
         cluster.sync();                                                                // (A) local histograms complete
         CI_PROF(11);
-        // each CTA reduces its segment of the buckets over the cluster
+        // each CTA reduces its segment of the buckets over the cluster, and sends the segment's totals to its peers
         const int G = CI_NB1 / CS;
         uint32_t* myseg = (CS == 1) ? hist1 : segcnt;
         u64 pc = 0, pe = 0;
@@ -1066,30 +1116,40 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
             uint32_t sum = 0;
             if (CS == 1) sum = hist1[g];
             else {
-                for (int q = 0; q < CS; ++q) sum += cluster.map_shared_rank(hist1, q)[rank * G + g];
+                uint32_t x[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) x[q] = q < CS ? cluster.map_shared_rank(hist1, q)[rank * G + g] : 0u;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) sum += x[q];
                 segcnt[g] = sum;
             }
             pc += sum;
             pe += (u64)sum * bucket_mass_est(rank * G + g);
         }
-        const u64 totc = block_sum_u64(pc, sc);
-        const u64 tote = block_sum_u64(pe, sc);
-        if (tid == 0) { xch->seg_cnt = totc; xch->seg_est = tote; }
+        pc = warp_sum_u64(pc); pe = warp_sum_u64(pe);
+        if (lane == 0) { sc->warp_tot[warp] = pc; sc->warp_aux[warp] = pe; }
         __syncthreads();
+        if (warp == 0) {
+            pc = warp_sum_u64(lane < CI_WARPS ? sc->warp_tot[lane] : 0ull); pe = warp_sum_u64(lane < CI_WARPS ? sc->warp_aux[lane] : 0ull);
+            if (lane < CS) { Scratch* ps = cluster.map_shared_rank(sc, lane); ps->seg_cnt[rank] = pc; ps->seg_est[rank] = pe; }
+        }
         cluster.sync();                                                                // (B) reduced segments published
         u64 segc[8], sege[8], survivors = 0, est_total = 0;
-        for (int q = 0; q < CS; ++q) {
-            const Xch* px = cluster.map_shared_rank(xch, q);
-            segc[q] = px->seg_cnt; sege[q] = px->seg_est;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            segc[q] = q < CS ? sc->seg_cnt[q] : 0ull; sege[q] = q < CS ? sc->seg_est[q] : 0ull;
             survivors += segc[q]; est_total += sege[q];
         }
         if (need_topk && (u64)kk >= survivors) need_topk = false;   // fewer survivors than k: top-k removes nothing
         if (need_topk) {
             // bucket of the k-th largest logit, exactly
             int s_star = CS - 1; u64 before_seg = 0, run = 0;
-            for (int q = 0; q < CS; ++q) {
-                if (run + segc[q] >= (u64)kk) { s_star = q; before_seg = run; break; }
-                run += segc[q];
+#pragma unroll
+            for (int q = 7; q >= 0; --q) if (q < CS) {          // (from the last one down: the first that reaches it stays)
+                run = 0;
+#pragma unroll
+                for (int t = 0; t < 8; ++t) if (t < q) run += segc[t];
+                if (run + segc[q] >= (u64)kk) { s_star = q; before_seg = run; }
             }
             const uint32_t* pseg = cluster.map_shared_rank(myseg, s_star);
             int g_star; u64 before;
@@ -1108,9 +1168,12 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
             else {
                 const u64 target = ceil_target(topp, est_total);
                 int s_star = CS - 1; u64 before_seg = 0, run = 0;
-                for (int q = 0; q < CS; ++q) {
-                    if (run + sege[q] >= target) { s_star = q; before_seg = run; break; }
-                    run += sege[q];
+#pragma unroll
+                for (int q = 7; q >= 0; --q) if (q < CS) {
+                    run = 0;
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) if (t < q) run += sege[t];
+                    if (run + sege[q] >= target) { s_star = q; before_seg = run; }
                 }
                 const uint32_t* pseg = cluster.map_shared_rank(myseg, s_star);
                 int g_star; u64 before;
@@ -1343,8 +1406,10 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
     }
     // Deferred rows still waiting; then the rows that were set aside take the generic path.
     if (it == 0) cluster.barrier_wait();                       // (a cluster without rows still completes the opening barrier)
+    // (A cluster that has deferred no row and set none aside is done: nobody reads a peer's memory any more.)
+    if (fast_seq == 0 && n_set_aside == 0) { CI_PROF_END(); return; }
     flush();
-    {
+    if (sc->any_retry) {
         int n_all = 0;
         if (tid == 0) {
             for (int i = 0; i < sc->n_retry_common; ++i) sc->retry_all[n_all++] = sc->retry_common[i];
@@ -1362,12 +1427,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 2) k_sample(const __gri
             process_row(sc->retry_all[i], it, false, -1);
         }
     }
-    if (a.prof && tid == 0 && (int)blockIdx.x < a.prof_slots) {
-        unsigned long long gt; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
-        a.prof[(size_t)blockIdx.x * 16 + 13] = (long long)gt;
-        a.prof[(size_t)blockIdx.x * 16 + 12] = clock64() - prof_t0;
-        for (int i = 0; i < 12; ++i) a.prof[(size_t)blockIdx.x * 16 + i] = sc->prof[i];
-    }
+    CI_PROF_END();
 }
 
 // ------------------------------------------------------------------------------------------------ host side

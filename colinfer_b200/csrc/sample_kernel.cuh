@@ -178,15 +178,6 @@ __device__ __forceinline__ float max16(const float (&v)[16]) {
     return fmax3(fmax3(a, b, c), fmax3(d, e, v[15]), CI_NEG_INF);
 }
 
-// 64-bit addition in shared memory as a 32-bit one with a carry: the hardware has no 64-bit one there, it would be a
-// compare-and-swap loop.  (The sum is complete once every adder is through.)
-__device__ __forceinline__ void add64(u64* p, u64 v) {
-    uint32_t* w = reinterpret_cast<uint32_t*>(p);
-    const uint32_t lo = (uint32_t)v, old = atomicAdd(w, lo);
-    const uint32_t hi = (uint32_t)(v >> 32) + (old + lo < old ? 1u : 0u);
-    if (hi) atomicAdd(w + 1, hi);
-}
-
 // ------------------------------------------------------------------------------------------------ the CTAs that share a row
 template <bool CL> struct Grp {
     int C, rank;
