@@ -47,7 +47,7 @@
 #define CI_RETRY 8               // rows a CTA may set aside for the generic path before the fast path is switched off
 #define CI_WLIST 24              // list entries per warp
 #define CI_GLIST 1365            // gathered list entries (16 KB)
-#define CI_SEL_BINS 512          // coarse bins of the exact selection on a gathered list
+#define CI_SEL_BINS 256          // coarse bins of the exact selection on a gathered list
 #define CI_FB_NB 256             // radix buckets per level of the fallback select (8 bits)
 #define CI_MAX_CAND 128          // tied / neighbouring candidates examined one by one in the final list step
 #define CI_PEN_TABLE 2048        // distinct history ids per slice with an O(1) count
@@ -84,7 +84,6 @@ struct Hello { float lmax; int lidx; int flags; int pad; };   // flags: 1 = a bo
 // Values one CTA publishes in its own shared memory for its peers to read after a later barrier.
 struct Xch {
     u64 fb_segtot;                 // the same for the fallback radix select
-    u64 s_all, s_above;            // band pass: kept mass of the slice, and of its part above the band
     u64 cta_mass;                  // kept mass of the slice under the final threshold
     unsigned short wcount[CI_WARPS];   // entries in each warp's list
     int list_overflow;
@@ -109,12 +108,20 @@ struct Scratch {
     int retry_common[CI_RETRY], retry_mine[CI_RETRY], retry_all[CI_RETRY * 9];
     long long prof[12];            // profiling hook: cycles per phase, summed over the CTA's rows
     u64 seg_cnt[8], seg_est[8];    // totals of every CTA's reduced bucket segment, written by the peers: counts, estimated mass
+    u64 all_in[8], above_in[8];    // band pass: kept mass of every CTA's slice, and of its part above the band, written by the peers
     int bcast_i[2];                // written by the cluster's first CTA, per row parity
     u64 mass_in[2][8];             // kept mass of every CTA's slice, written by the peers, per row parity
 };
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
+
+// Maximum over a warp; NaN counts as less than everything else.
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
 
 // Block-wide: index of the first entry (ascending) at which the running sum of get(0..n-1) reaches `target`
 // (1 <= target <= total), and the sum before it.  All threads call; all threads get the result.
@@ -177,36 +184,75 @@ __device__ __forceinline__ float row_uniform(const SampleArgs& a, int row, int b
     return 1.0f;
 }
 
+// Bin of 32 * PER bins (ascending index) in which the running sum reaches `target` (1 <= target), and the sum before it;
+// bin = 32 * PER when the total falls short.  Every warp searches for itself: cheaper than publishing one warp's result.
+template <int PER, class T, class S>
+__device__ __forceinline__ void warp_find(const T* bins, S target, int& bin, S& before) {
+    const int lane = lane_id();
+    S loc[PER], sum = 0;
+    constexpr int STEP = 16 / sizeof(T);
+#pragma unroll
+    for (int t = 0; t < PER; t += STEP) {
+        const uint4 x = *reinterpret_cast<const uint4*>(bins + lane * PER + t);
+        if constexpr (sizeof(T) == 4) { loc[t] = x.x; loc[t + 1] = x.y; loc[t + 2] = x.z; loc[t + 3] = x.w; }
+        else { loc[t] = ((u64)x.y << 32) | x.x; loc[t + 1] = ((u64)x.w << 32) | x.z; }
+    }
+#pragma unroll
+    for (int t = 0; t < PER; ++t) sum += loc[t];
+    S incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const S x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
+    const unsigned reached = __ballot_sync(0xffffffffu, incl >= target);
+    if (!reached) { bin = 32 * PER; before = 0; return; }
+    const int src = __ffs(reached) - 1;
+    S run = incl - sum, run_at = run;
+    int at = PER - 1;
+    bool found = false;
+#pragma unroll
+    for (int t = 0; t < PER; ++t) { if (!found && run + loc[t] >= target) { found = true; at = t; run_at = run; } run += loc[t]; }
+    bin = src * PER + __shfl_sync(0xffffffffu, at, src);
+    before = __shfl_sync(0xffffffffu, run_at, src);
+}
+
+// Block-wide, one value per thread: the first thread at which the running sum reaches `target` (1 <= target <= total), and the
+// sum before it.  Two block barriers.
+__device__ __forceinline__ void thread_find(u64 v, u64 target, Scratch* s, int& idx, u64& before) {
+    const int lane = lane_id(), warp = warp_id();
+    const u64 incl = warp_incl_scan_u64(v, lane);
+    if (lane == 31) s->wsum[warp] = incl;
+    if (threadIdx.x == 0) { s->found_idx = CI_THREADS - 1; s->found_before = 0; }
+    __syncthreads();
+    const u64 excl = warp_sum_u64(lane < warp ? s->wsum[lane] : 0ull) + incl - v;
+    if (excl < target && target <= excl + v) { s->found_idx = threadIdx.x; s->found_before = excl; }
+    __syncthreads();
+    idx = s->found_idx; before = s->found_before;
+}
+
 // Exact weighted selection on a gathered list: the value v among the entries with wt > 0 such that
-// W(l > v) < target <= W(l >= v).  Up to 512 coarse bins over the entries' key range (a shift, so monotone), then the
-// entries of the pivot bin one by one (a warp each).  Returns false when the pivot bin holds more than CI_MAX_CAND
-// entries.  All threads of the CTA call; 1 <= target <= total weight.
+// W(l > v) < target <= W(l >= v).  Coarse bins over the entries' key range (a shift, so monotone), then the entries of the
+// pivot bin pairwise (by every warp).  Returns false when the pivot bin holds more than CI_MAX_CAND entries.  All threads of
+// the CTA call; 1 <= target <= total weight.
 template <class W>
-__device__ bool list_select(const ListEntry* gl, int n, W wt, u64 target, u64* bins, uint32_t* cand, Scratch* sc, float& value) {
+__device__ __noinline__ bool list_select(const ListEntry* gl, int n, W wt, u64 target, u64* bins, uint32_t* cand, Scratch* sc, float& value) {
     const int tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     uint32_t kmin = 0xFFFFFFFFu, kmax = 0u;
     for (int i = tid; i < n; i += CI_THREADS) {
         if (wt(i) > 0) { const uint32_t k = f2key(gl[i].l); kmin = min(kmin, k); kmax = max(kmax, k); }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        kmin = min(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
-        kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin); kmax = __reduce_max_sync(0xffffffffu, kmax);
     if (lane == 0) { sc->warp_u[warp] = kmin; sc->warp_v[warp] = kmax; }
     for (int i = tid; i < CI_SEL_BINS; i += CI_THREADS) bins[i] = 0;
-    if (tid == 0) { sc->ncand = 0; sc->sel_ok = 0; sc->sel_value = 0.0f; }
+    if (tid == 0) sc->ncand = 0;
     __syncthreads();
-    for (int w = 0; w < CI_WARPS; ++w) { kmin = min(kmin, sc->warp_u[w]); kmax = max(kmax, sc->warp_v[w]); }
-    const uint32_t span = kmax - kmin;                                   // bins cover [0, span] >> sh, at most 512
-    const int sh = max(0, 32 - __clz(span) - 9);
+    kmin = __reduce_min_sync(0xffffffffu, sc->warp_u[lane % CI_WARPS]); kmax = __reduce_max_sync(0xffffffffu, sc->warp_v[lane % CI_WARPS]);
+    const int sh = max(0, 32 - __clz(kmax - kmin) - 8);                  // the bins cover [0, kmax - kmin] >> sh
     for (int i = tid; i < n; i += CI_THREADS) {
         const u64 w = wt(i);
         if (w > 0) add64(&bins[(kmax - f2key(gl[i].l)) >> sh], w);
     }
     __syncthreads();
     int b_star; u64 before;
-    block_find([&](int i) { return bins[i]; }, CI_SEL_BINS, target, sc, b_star, before);
+    warp_find<CI_SEL_BINS / 32>(bins, target, b_star, before);
     for (int i = tid; i < n; i += CI_THREADS) {
         if (wt(i) > 0 && (int)((kmax - f2key(gl[i].l)) >> sh) == b_star) {
             const int slot = atomicAdd(&sc->ncand, 1);
@@ -215,21 +261,20 @@ __device__ bool list_select(const ListEntry* gl, int n, W wt, u64 target, u64* b
     }
     __syncthreads();
     const int nc = sc->ncand;
-    if (nc > CI_MAX_CAND) { __syncthreads(); return false; }
-    for (int c = warp; c < nc; c += CI_WARPS) {
-        const uint32_t kc = f2key(gl[cand[c]].l);
-        u64 gt = 0, eq = 0;
-        for (int j = lane; j < nc; j += 32) {                            // only the pivot bin's entries matter
-            const uint32_t k = f2key(gl[cand[j]].l);
-            const u64 w = wt((int)cand[j]);
-            if (k > kc) gt += w; else if (k == kc) eq += w;
+    bool ok = false;
+    if (nc <= CI_MAX_CAND) {
+        for (int c0 = 0; c0 < nc && !ok; c0 += 32) {
+            const float mine = c0 + lane < nc ? gl[cand[c0 + lane]].l : CI_NEG_INF;
+            u64 gt = before, ge = before;
+            for (int j = 0; j < nc; ++j) {                               // only the pivot bin's entries matter
+                const int e = (int)cand[j];
+                const float o = gl[e].l; const u64 w = wt(e);
+                gt += o > mine ? w : 0ull; ge += o >= mine ? w : 0ull;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, c0 + lane < nc && gt < target && target <= ge);
+            if (hit) { ok = true; value = __shfl_sync(0xffffffffu, mine, __ffs(hit) - 1); }
         }
-        gt = warp_sum_u64(gt); eq = warp_sum_u64(eq);
-        if (lane == 0 && before + gt < target && target <= before + gt + eq) { sc->sel_value = gl[cand[c]].l; sc->sel_ok = 1; }
     }
-    __syncthreads();
-    value = sc->sel_value;
-    const bool ok = sc->sel_ok != 0;
     __syncthreads();
     return ok;
 }
@@ -386,11 +431,18 @@ __device__ bool finish_on_list(const ListEntry* glist, int n, float tl, float lc
 // (lane, then component).  Positions come from four ballots, no scan.  wn is the warp's running count (uniform over
 // the warp); entries beyond CI_WLIST are dropped and counted.
 __device__ __forceinline__ void warp_append(Cand* mylist, int& wn, unsigned mk, const float* e4, uint32_t idx0, int lane) {
-    const unsigned b0 = __ballot_sync(0xffffffffu, mk & 1u), b1 = __ballot_sync(0xffffffffu, mk & 2u);
-    const unsigned b2 = __ballot_sync(0xffffffffu, mk & 4u), b3 = __ballot_sync(0xffffffffu, mk & 8u);
-    if (!(b0 | b1 | b2 | b3)) return;
+    const unsigned any = __ballot_sync(0xffffffffu, mk != 0u);
+    if (!any) return;
     const unsigned lt = (1u << lane) - 1u;
-    int at = wn + __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt);
+    int at, add;
+    if (!__ballot_sync(0xffffffffu, (mk & (mk - 1u)) != 0u)) {              // no lane has two
+        at = wn + __popc(any & lt); add = __popc(any);
+    } else {
+        const unsigned b0 = __ballot_sync(0xffffffffu, mk & 1u), b1 = __ballot_sync(0xffffffffu, mk & 2u);
+        const unsigned b2 = __ballot_sync(0xffffffffu, mk & 4u), b3 = __ballot_sync(0xffffffffu, mk & 8u);
+        at = wn + __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt);
+        add = __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (mk & (1u << j)) {
@@ -398,7 +450,7 @@ __device__ __forceinline__ void warp_append(Cand* mylist, int& wn, unsigned mk, 
             ++at;
         }
     }
-    wn += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
+    wn += add;
 }
 
 // Collects, in token order, the logits >= tl of one warp's region [r_lo, r_hi) of the slice into the warp's list.
@@ -442,29 +494,6 @@ __device__ __forceinline__ u64 block_excl_scan(u64 v, Scratch* sc, u64& total) {
     __syncthreads();
     total = sc->wtotal;
     return sc->woff[warp] + incl - v;
-}
-
-// Where the running sum of CI_FAST_BINS bins (ascending index) first reaches `target`: the bin, the sum before it, and
-// the total.  bin = -1 when target exceeds the total (or is 0).  Three __syncthreads.  All threads call.
-template <class T>
-__device__ void bins_find(const T* bins, u64 target, Scratch* sc, int& bin, u64& before, u64& total) {
-    constexpr int PER = CI_FAST_BINS / CI_THREADS;
-    const int tid = threadIdx.x;
-    u64 loc[PER], s = 0;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) { loc[j] = (u64)bins[tid * PER + j]; s += loc[j]; }
-    const u64 excl = block_excl_scan(s, sc, total);
-    if (excl < target && target <= excl + s) {
-        u64 run = excl;
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            if (run + loc[j] >= target) { sc->found_tid = tid * PER + j; sc->found_excl = run; break; }
-            run += loc[j];
-        }
-    }
-    __syncthreads();
-    bin = sc->found_tid;
-    before = sc->found_excl;
 }
 
 // Exact finish of a row from the candidates its CTAs pushed into this CTA's shared memory: min-p, top-k, top-p and
@@ -524,24 +553,7 @@ __device__ __noinline__ bool finish_pending(const SampleArgs& a, const Pending& 
         for (int j = 0; j < 2; ++j) if (in[j]) atomicAdd(&bins[(kmax - key[j]) >> sh], 1u);
         __syncthreads();
         int b_star, before;
-        {
-            const uint4* b4 = reinterpret_cast<const uint4*>(bins) + lane * 4;   // a lane's sixteen bins
-            int s = 0, loc[16];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) { const uint4 x = b4[t]; loc[4 * t] = x.x; loc[4 * t + 1] = x.y; loc[4 * t + 2] = x.z; loc[4 * t + 3] = x.w; }
-#pragma unroll
-            for (int t = 0; t < 16; ++t) s += loc[t];
-            int incl = s;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
-            const int src = __ffs(__ballot_sync(0xffffffffu, incl >= kk)) - 1;
-            int run = incl - s, at = 15, run_at = run;
-            bool found = false;
-#pragma unroll
-            for (int t = 0; t < 16; ++t) { if (!found && run + loc[t] >= kk) { found = true; at = t; run_at = run; } run += loc[t]; }
-            b_star = src * 16 + __shfl_sync(0xffffffffu, at, src);
-            before = __shfl_sync(0xffffffffu, run_at, src);
-        }
+        warp_find<CI_FAST_BINS / 32>(bins, kk, b_star, before);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
             if (in[j] && (int)((kmax - key[j]) >> sh) == b_star) {
@@ -665,7 +677,6 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     if (tid == 0 && a.use_bulk) {
         for (int c = 0; c < nchunks; ++c) mbar_init(&mbar[c], 1);
         fence_mbar_init();
-        fence_proxy_async();
     }
     const int n_clusters = (int)gridDim.x / CS;
     const long long n_rows = (long long)a.B * a.R;
@@ -674,8 +685,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     if (a.prof && tid == 0) for (int i = 0; i < 12; ++i) sc->prof[i] = 0;
 
     // Starts the bulk copies of one row's slice (thread 0 only; every thread must be done reading the buffer).
-    auto issue_row = [&](const long long rw) {
-        fence_proxy_async();                                   // earlier reads of the buffer precede these writes
+    auto issue_row = [&](const long long rw, bool first) {
+        if (!first) fence_proxy_async();                       // earlier reads of the buffer precede these writes
         const float* src = reinterpret_cast<const float*>(a.logits) + (size_t)rw * V + slice_lo;
         if (a.flags & COLINFER_TEST_DROP_COPY) return;        // test flag: nothing is armed, nothing is in flight; the waits run out
         for (int c = 0; c < nchunks; ++c) {
@@ -716,7 +727,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     // started this row's copies because it no longer needed the buffer).
     if (tid == 0) {
         sc->fail = 0; sc->hist_slow = 0; xch->list_overflow = 0;
-        if (a.use_bulk && !prefetched) issue_row(row);
+        if (a.use_bulk && !prefetched) issue_row(row, it == 0);
     }
     prefetched = false;
     CI_PROF(0);
@@ -922,23 +933,17 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         lidx = slice_lo + lpos * 4 + (v.x == lmax ? 0 : v.y == lmax ? 1 : v.z == lmax ? 2 : 3);
     }
     // block reduce (largest value, lowest index among equals)
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const float om = __shfl_xor_sync(0xffffffffu, lmax, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, lidx, o);
-        if (om > lmax || (om == lmax && oi < lidx)) { lmax = om; lidx = oi; }
+    {
+        const float wm = warp_max(lmax);
+        lidx = __reduce_min_sync(0xffffffffu, lmax == wm ? lidx : 0x7fffffff);
+        if (lane == 0) { sc->warp_f[warp] = wm; sc->warp_i[warp] = lidx; }
     }
-    if (lane == 0) { sc->warp_f[warp] = lmax; sc->warp_i[warp] = lidx; }
     if (fastk) for (int i = tid; i < CI_FAST_BINS; i += CI_THREADS) hist1[i] = 0u;   // (the penalty tables are done with)
     __syncthreads();
     {
-        float bm = sc->warp_f[0]; int bi = sc->warp_i[0];
-#pragma unroll
-        for (int w = 1; w < CI_WARPS; ++w) {
-            const float om = sc->warp_f[w]; const int oi = sc->warp_i[w];
-            if (om > bm || (om == bm && oi < bi)) { bm = om; bi = oi; }
-        }
-        lmax = bm; lidx = bi;                                   // the slice maximum, in every thread
+        const float om = sc->warp_f[lane % CI_WARPS]; const int oi = sc->warp_i[lane % CI_WARPS];
+        lmax = warp_max(om);                                    // the slice maximum, in every thread
+        lidx = __reduce_min_sync(0xffffffffu, om == lmax ? oi : 0x7fffffff);
     }
 
     // warp w owns the contiguous region [r_lo, r_hi) of the slice; lanes interleave float4 groups, so the token
@@ -958,9 +963,9 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         for (int j = 0; j < CI_TGROUPS; ++j)
             if (tg[j] > CI_NEG_INF) atomicAdd(&hist1[min(CI_FAST_BINS - 1, __float2int_rz((lmax - tg[j]) * CI_FAST_SCALE))], 1u);
         __syncthreads();
-        int bk; u64 before, have;
-        bins_find(hist1, (u64)kk, sc, bk, before, have);
-        if (have >= (u64)kk && bk >= 0 && bk < CI_FAST_BINS - 1)
+        int bk, before;
+        warp_find<CI_FAST_BINS / 32>(hist1, kk, bk, before);    // (512 without k maxima)
+        if (bk < CI_FAST_BINS - 1)
             tl_fast = lmax - ((float)(bk + 1) + 0.01f) / CI_FAST_SCALE - fabsf(lmax) * 1e-6f;
         else tl_fast = -CI_FLT_MAX;                             // fewer than k threads saw a finite logit: take them all
         CI_PROF(10);
@@ -986,12 +991,12 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         }
         // the row buffer is free: start the next row's copies now
         if (a.use_bulk && next_row >= 0) {
-            if (tid == 0) issue_row(next_row);
+            if (tid == 0) issue_row(next_row, false);
             prefetched = true;
         }
     } else if (!sampled && a.use_bulk && next_row >= 0) {
         // greedy row: only the maximum is needed from here on
-        if (tid == 0) issue_row(next_row);
+        if (tid == 0) issue_row(next_row, false);
         prefetched = true;
     }
 
@@ -1099,7 +1104,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 }
                 int bkt[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) bkt[j] = min(CI_NB1 - 1, __float2int_rz((L - e[j]) * SC));
+                for (int j = 0; j < 16; ++j)                  // (the integer part, by an addition rounded towards zero: conversions have a quarter of its rate)
+                    bkt[j] = min(CI_NB1 - 1, __float_as_int(__fadd_rz((L - e[j]) * SC, 8388608.0f)) - 0x4B000000);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) if (e[j] >= lk) atomicAdd(&hist1[bkt[j]], 1u);
             }
@@ -1153,7 +1159,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
             }
             const uint32_t* pseg = cluster.map_shared_rank(myseg, s_star);
             int g_star; u64 before;
-            block_find([&](int i) { return (u64)pseg[i]; }, G, (u64)kk - before_seg, sc, g_star, before);
+            if (G <= CI_THREADS) thread_find(tid < G ? (u64)pseg[tid] : 0ull, (u64)kk - before_seg, sc, g_star, before);
+            else block_find([&](int i) { return (u64)pseg[i]; }, G, (u64)kk - before_seg, sc, g_star, before);
             const int bk = s_star * G + g_star;
             const u64 n_upto = before_seg + before + pseg[g_star];
             if (bk >= CI_NB1 - 3 || n_upto > CI_GLIST - 64) path = PATH_FALLBACK;
@@ -1177,7 +1184,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 }
                 const uint32_t* pseg = cluster.map_shared_rank(myseg, s_star);
                 int g_star; u64 before;
-                block_find([&](int i) { return (u64)pseg[i] * bucket_mass_est(s_star * G + i); }, G, target - before_seg, sc, g_star, before);
+                if (G <= CI_THREADS) thread_find(tid < G ? (u64)pseg[tid] * bucket_mass_est(s_star * G + tid) : 0ull, target - before_seg, sc, g_star, before);
+                else block_find([&](int i) { return (u64)pseg[i] * bucket_mass_est(s_star * G + i); }, G, target - before_seg, sc, g_star, before);
                 const int bp = s_star * G + g_star;
                 const int up = a.dtype == COLINFER_BF16 ? 3 : 1, dn = a.dtype == COLINFER_BF16 ? 4 : 2;
                 if (bp + dn + 2 >= CI_NB1) path = PATH_FALLBACK;
@@ -1230,6 +1238,10 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         const float lk = fmaxf(lcut, -CI_FLT_MAX);
         u64 acc_all = 0, acc_above = 0;
         int wn = 0;
+        Mass2 mass2;
+        mass2.init(mass);
+        const float t_low = fmaxf(t_lo, lk);
+#pragma unroll 1
         for (int i0 = r_lo; i0 < r_hi; i0 += 512) {
             float e[16];
 #pragma unroll
@@ -1238,29 +1250,28 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 const float4 v = i < r_hi ? *reinterpret_cast<const float4*>(rowbuf + i) : make_float4(CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF);
                 e[4 * k] = v.x; e[4 * k + 1] = v.y; e[4 * k + 2] = v.z; e[4 * k + 3] = v.w;
             }
-            uint32_t q[16];
+            unsigned mk = 0;                                    // the band's logits among the sixteen
 #pragma unroll
-            for (int j = 0; j < 16; ++j) q[j] = e[j] >= lk ? mass(e[j]) : 0u;
-#pragma unroll
-            for (int j = 0; j < 16; j += 2) acc_all += (u64)q[j] + q[j + 1];
-            if (band) {
-                unsigned mk[4], anym = 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    mk[k] = 0;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float x = e[4 * k + j];
-                        if (x > t_hi) acc_above += q[4 * k + j];
-                        else if (x >= t_lo && x >= lk) mk[k] |= 1u << j;
-                    }
-                    anym |= mk[k];
+            for (int j = 0; j < 16; j += 2) {
+                uint32_t q0, q1;
+                mass2.whole(e[j], e[j + 1], lk, q0, q1);
+                acc_all += q0 + q1;                             // (at most 2^31)
+                if (band) {
+                    const bool a0 = e[j] > t_hi, a1 = e[j + 1] > t_hi;
+                    acc_above += (a0 ? q0 : 0u) + (a1 ? q1 : 0u);
+                    if (!a0 && e[j] >= t_low) mk |= 1u << j;
+                    if (!a1 && e[j + 1] >= t_low) mk |= 2u << j;
                 }
-                if (__ballot_sync(0xffffffffu, anym != 0u)) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        warp_append(mylist, wn, mk[k], &e[4 * k], (uint32_t)(slice_lo + i0 + k * 128 + lane * 4), lane);
+            }
+            // the band's logits are appended in no particular order: only their values and masses are looked at
+            for (unsigned any = __ballot_sync(0xffffffffu, mk != 0u); any; any = __ballot_sync(0xffffffffu, mk != 0u)) {
+                const int at = wn + __popc(any & ((1u << lane) - 1u));
+                if (mk && at < CI_WLIST) {
+                    const int t = __ffs(mk) - 1, i = i0 + (t >> 2) * 128 + lane * 4 + (t & 3);
+                    mylist[at].idx = (uint32_t)(slice_lo + i); mylist[at].l = rowbuf[i];
                 }
+                mk &= mk - 1;
+                wn += __popc(any);
             }
         }
         u64 wkeep = warp_sum_u64(band ? acc_above : acc_all);   // kept mass of the region known so far
@@ -1272,19 +1283,15 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 if (wn > CI_WLIST) xch->list_overflow = 1;
             }
             __syncthreads();
-            if (tid == 0) {
-                u64 ta = 0, tb = 0;
-                for (int w = 0; w < CI_WARPS; ++w) { ta += sc->warp_aux[w]; tb += sc->warp_tot[w]; }
-                xch->s_all = ta; xch->s_above = tb;
+            if (warp == 0) {
+                const u64 ta = warp_sum_u64(lane < CI_WARPS ? sc->warp_aux[lane] : 0ull), tb = warp_sum_u64(lane < CI_WARPS ? sc->warp_tot[lane] : 0ull);
+                if (lane < CS) { Scratch* ps = cluster.map_shared_rank(sc, lane); ps->all_in[rank] = ta; ps->above_in[rank] = tb; }
             }
-            __syncthreads();
             CI_PROF(11);
             cluster.sync();                                                            // (L) band lists and sums published
             u64 s1 = 0, s_above = 0;
-            for (int q = 0; q < CS; ++q) {
-                const Xch* px = cluster.map_shared_rank(xch, q);
-                s1 += px->s_all; s_above += px->s_above;
-            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) if (q < CS) { s1 += sc->all_in[q]; s_above += sc->above_in[q]; }
             const int n = gather_lists(cluster, CS, xch, ownlist, glist, sc, mass);
             bool ok = n >= 0 && s1 > 0;
             float cut2 = lcut;
