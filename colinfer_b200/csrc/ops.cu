@@ -3,6 +3,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "sample_host.h"
 #include "../../include/colinfer_b200.h"
 
 // ------------------------------------------------------------------------------------------------ philox_uniform
@@ -77,23 +78,31 @@ extern "C" int colinfer_apply_mask(const float* logits, const int32_t* mask, flo
 
 // ------------------------------------------------------------------------------------------------ processed_probs
 // P(t) = exp(z_t - m) / S on the kept set of the row (described by the row statistics of the fused kernel), else 0.
-__global__ void k_write_probs(const float* __restrict__ logits, const colinfer_row_stats* __restrict__ stats,
-                              float* __restrict__ out, int V) {
+// Four tokens a thread; a division and an exponential only for the kept ones.
+__global__ void __launch_bounds__(256) k_write_probs(const float* __restrict__ logits, const colinfer_row_stats* __restrict__ stats,
+                                                     float* __restrict__ out, int V, int vec) {
     const int row = blockIdx.y;
-    const colinfer_row_stats st = stats[row];
     const float* src = logits + (size_t)row * V;
     float* dst = out + (size_t)row * V;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i >= V) return;
+    float x[4];
+    const int n = min(4, V - i);
+    if (vec) { const float4 v = __ldg(reinterpret_cast<const float4*>(src + i)); x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
+    else for (int e = 0; e < 4; ++e) x[e] = e < n ? __ldg(src + i + e) : CI_NEG_INF;
+    const colinfer_row_stats st = stats[row];
     const bool bad = (st.status & (COLINFER_ROW_DEGENERATE | COLINFER_ROW_TIMEOUT)) != 0 || st.mass_q == 0;
     const float m = scale_logit(st.lmax, st.tc);
     const float S = (float)((double)st.mass_q * CI_MASS_INV);
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V; g += gridDim.x * blockDim.x) {
-        const float l = __ldg(src + g);
-        float p;
-        if (bad) p = __int_as_float(0x7fc00000);               // NaN, as a softmax without a finite maximum gives
-        else if (l >= st.lcut && l > CI_NEG_INF) p = __fdiv_rn(expf(scale_logit(l, st.tc) - m), S);
-        else p = 0.0f;
-        dst[g] = p;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float l = x[e];
+        if (bad) x[e] = __int_as_float(0x7fc00000);            // NaN, as a softmax without a finite maximum gives
+        else if (l >= st.lcut && l > CI_NEG_INF) x[e] = __fdiv_rn(expf(scale_logit(l, st.tc) - m), S);
+        else x[e] = 0.0f;
     }
+    if (vec) *reinterpret_cast<float4*>(dst + i) = make_float4(x[0], x[1], x[2], x[3]);
+    else for (int e = 0; e < n; ++e) dst[i + e] = x[e];
 }
 
 extern "C" int colinfer_processed_probs(const float* logits, const float* temperature, const int32_t* top_k,
@@ -108,12 +117,12 @@ extern "C" int colinfer_processed_probs(const float* logits, const float* temper
                             1, R, V, COLINFER_FORCE_DISTRIBUTION, stream);
     if (e) return e;
     const int threads = 256;
-    int bx = (V + threads - 1) / threads;
-    if (bx > 296) bx = 296;
+    const int bx = (V + 4 * threads - 1) / (4 * threads);
+    const int vec = (V % 4) == 0 && ((((uintptr_t)logits) | ((uintptr_t)out)) & 15) == 0 ? 1 : 0;
     for (int r0 = 0; r0 < R; r0 += 65535) {
         const int nr = R - r0 < 65535 ? R - r0 : 65535;
         k_write_probs<<<dim3(bx, nr), threads, 0, (cudaStream_t)stream>>>(logits + (size_t)r0 * V, scratch + r0,
-                                                                           out + (size_t)r0 * V, V);
+                                                                           out + (size_t)r0 * V, V, vec);
     }
     return (int)cudaGetLastError();
 }
@@ -161,9 +170,13 @@ extern "C" int colinfer_processed_probs_noalloc(const float* logits, const float
 extern "C" int colinfer_noalloc_max_rows(void) { return COLINFER_NOALLOC_MAX_ROWS; }
 
 // ------------------------------------------------------------------------------------------------ inverse_cdf
-// One CTA per row.  Sums are float64 (the reference's fp32 scan order is device dependent; float64 is what its CPU
-// cumsum accumulates in).  Warp w owns a contiguous region, lanes interleave, so the index order is (warp, step, lane).
-#define ICDF_THREADS 1024
+// A cluster of 8 CTAs per row.  Sums are float64 (the reference's fp32 scan order is device dependent; float64 is what its CPU
+// cumsum accumulates in).  A warp owns a region of consecutive tokens, a lane four of them at a time; the warp in whose region
+// the running sum reaches u * total walks over it again.  A few rows are a matter of latency: with one CTA per row nine rows
+// of 151,936 took as long as one SM needs to fetch a row twice.
+#define ICDF_THREADS 512
+#define ICDF_WARPS (ICDF_THREADS / 32)
+#define ICDF_CTAS 8
 __device__ __forceinline__ double warp_sum_f64(double v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -178,48 +191,73 @@ __device__ __forceinline__ double warp_incl_scan_f64(double v, int lane) {
     return v;
 }
 
-__global__ void __launch_bounds__(ICDF_THREADS) k_inverse_cdf(const float* __restrict__ P, const float* __restrict__ u,
-                                                              int64_t* __restrict__ out, int V) {
-    __shared__ double wtot[ICDF_THREADS / 32];
-    __shared__ long long result;
-    const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__global__ void __cluster_dims__(ICDF_CTAS, 1, 1) __launch_bounds__(ICDF_THREADS)
+k_inverse_cdf(const float* __restrict__ P, const float* __restrict__ u, int64_t* __restrict__ out, int V, int reg, int vec) {
+    __shared__ double wtot[ICDF_WARPS], ctot[ICDF_CTAS];
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();                                        // (waited for before the first write into a peer)
+    const int row = blockIdx.x / ICDF_CTAS, rank = blockIdx.x % ICDF_CTAS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* src = P + (size_t)row * V;
-    const int nwarps = ICDF_THREADS / 32;
-    const int reg = (((V + 31) / 32 + nwarps - 1) / nwarps) * 32;
-    const int lo = min(warp * reg, V), hi = min(lo + reg, V);
+    const int lo = min((rank * ICDF_WARPS + warp) * reg, V), hi = min(lo + reg, V);
+    auto four = [&](int i) {
+        if (i >= hi) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (vec) return __ldg(reinterpret_cast<const float4*>(src + i));
+        return make_float4(__ldg(src + i), i + 1 < hi ? __ldg(src + i + 1) : 0.0f, i + 2 < hi ? __ldg(src + i + 2) : 0.0f, i + 3 < hi ? __ldg(src + i + 3) : 0.0f);
+    };
     double acc = 0.0;
-    for (int i = lo + lane; i < hi; i += 32) acc += (double)__ldg(src + i);
+#pragma unroll 4
+    for (int i = lo + lane * 4; i < hi; i += 128) { const float4 v = four(i); acc += ((double)v.x + (double)v.y) + ((double)v.z + (double)v.w); }
     const double wt = warp_sum_f64(acc);
     if (lane == 0) wtot[warp] = wt;
-    if (threadIdx.x == 0) result = V - 1;
     __syncthreads();
-    double total = 0.0, woff = 0.0;
-    for (int w = 0; w < nwarps; ++w) { if (w < warp) woff += wtot[w]; total += wtot[w]; }
-    if (threadIdx.x == 0 && !(total > 0.0)) result = 0;          // a row without mass: no prefix lies below u * 0 (the reference counts none)
+    double cta = 0.0, before = 0.0;                                  // (in one order everywhere: the warps' bounds meet exactly)
+    for (int w = 0; w < ICDF_WARPS; ++w) { if (w == warp) before = cta; cta += wtot[w]; }
+    double after = before + wt;
+    cluster.barrier_wait();
+    if (threadIdx.x < ICDF_CTAS) *cluster.map_shared_rank(&ctot[rank], threadIdx.x) = cta;
+    cluster.sync();
+    double total = 0.0, off = 0.0;
+    for (int q = 0; q < ICDF_CTAS; ++q) { if (q == rank) off = total; total += ctot[q]; }
+    before += off;
+    after = warp == ICDF_WARPS - 1 ? off + cta : after + off;
     const double t = (double)u[row] * total;
-    // first index whose inclusive prefix reaches t; the owning warp is the first whose inclusive total reaches it
-    if (woff < t && woff + wt >= t) {
-        double run = woff;
-        for (int i0 = lo; i0 < hi; i0 += 32) {
-            const int i = i0 + lane;
-            const double v = i < hi ? (double)__ldg(src + i) : 0.0;
-            const double incl = warp_incl_scan_f64(v, lane);
-            const unsigned hit = __ballot_sync(0xffffffffu, run + incl >= t);
-            if (hit) {
-                if (lane == __ffs(hit) - 1) result = i;
-                break;
-            }
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
+    if (rank == 0 && threadIdx.x == 0) {
+        if (!(total > 0.0)) out[row] = 0;                            // a row without mass: no prefix lies below u * 0 (the reference counts none)
+        else if (!(t > 0.0 && t <= total)) out[row] = V - 1;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) out[row] = result;
+    // first index whose inclusive prefix reaches t; the owning warp is the first whose inclusive total reaches it
+    if (!(total > 0.0) || !(before < t && t <= after)) return;
+    int last = lo;                                                   // (of the region's non-zero ones, where rounding lets none reach t)
+    for (int i0 = lo; i0 < hi; i0 += 128) {
+        const int i = i0 + lane * 4;
+        const float4 v = four(i);
+        const double p1 = (double)v.x, p2 = p1 + (double)v.y, p3 = p2 + (double)v.z, p4 = p3 + (double)v.w;
+        const double incl = warp_incl_scan_f64(p4, lane), excl = before + (incl - p4);
+        const unsigned hit = __ballot_sync(0xffffffffu, before + incl >= t && p4 > 0.0);
+        if (hit) {
+            if (lane == __ffs(hit) - 1) {
+                const int e = excl + p1 >= t && v.x > 0.0f ? 0 : excl + p2 >= t && v.y > 0.0f ? 1 : excl + p3 >= t && v.z > 0.0f ? 2
+                            : v.w > 0.0f ? 3 : v.z > 0.0f ? 2 : v.y > 0.0f ? 1 : 0;
+                out[row] = i + e;
+            }
+            return;
+        }
+        const unsigned some = __ballot_sync(0xffffffffu, p4 > 0.0);
+        if (some) last = __shfl_sync(0xffffffffu, i + (v.w > 0.0f ? 3 : v.z > 0.0f ? 2 : v.y > 0.0f ? 1 : 0), 31 - __clz(some));
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) out[row] = last;
 }
 
 extern "C" int colinfer_inverse_cdf(const float* P, const float* u, int64_t* out, int R, int V, void* stream) {
     if (!P || !u || !out || R < 0 || V <= 0) return (int)cudaErrorInvalidValue;
     if (R == 0) return 0;
-    k_inverse_cdf<<<R, ICDF_THREADS, 0, (cudaStream_t)stream>>>(P, u, out, V);
+    const int reg = ((V + ICDF_CTAS * ICDF_WARPS - 1) / (ICDF_CTAS * ICDF_WARPS) + 127) / 128 * 128;
+    const int vec = (V % 4) == 0 && (((uintptr_t)P) & 15) == 0 ? 1 : 0;
+    for (int r0 = 0; r0 < R; r0 += 1 << 24) {
+        const int nr = R - r0 < 1 << 24 ? R - r0 : 1 << 24;
+        k_inverse_cdf<<<nr * ICDF_CTAS, ICDF_THREADS, 0, (cudaStream_t)stream>>>(P + (size_t)r0 * V, u + r0, out + r0, V, reg, vec);
+    }
     return (int)cudaGetLastError();
 }
 
@@ -319,10 +357,12 @@ extern "C" int colinfer_spec_advance(const int64_t* out_tok, const int32_t* n, i
 }
 
 // ------------------------------------------------------------------------------------------------ spec_verify (rejection)
-// Finish step: per slot, decide the accepted prefix from the row statistics of the target and draft rows, then, at a
+// Finish: per slot, decide the accepted prefix from the row statistics of the target and draft rows, then, at a
 // rejection, stream the two rows of that position once to draw from the residual max(p - q, 0).
-#define VF_THREADS 256
-#define VF_NSEG 32                     // segments a slot's rejected position is summed in (one CTA each)
+#define VF_THREADS 512
+#define VF_WARPS (VF_THREADS / 32)
+#define VF_CTAS 8                      // CTAs (a cluster) per slot
+#define VF_MAX_V 524288
 struct VerifyArgs {
     const void* tl; const void* dl; int dtype;
     const int32_t* mask; int W;
@@ -330,10 +370,8 @@ struct VerifyArgs {
     const int64_t* draft_ids; const float* ua; const float* us;
     const colinfer_row_stats* st_t; const colinfer_row_stats* st_d; const int64_t* samp_t;
     int64_t* out_tok; int32_t* n;
-    int2* slot;                        // [B] (first rejected position j, mode: 0 = token known, 1 = residual draw)
-    u64* seg_sums;                     // [B, VF_NSEG] residual mass per segment of the rejected position
-    int seg;                           // elements per segment (a multiple of 128)
-    int vec;                           // fp32 rows that take 128-bit loads
+    int reg;                           // tokens per warp's region of the rejected position (a multiple of 128)
+    int vec;                           // rows that take loads of four logits
     int B, k, V;
     const int32_t* history; const int32_t* hist_len; int hist_stride;   // the slots' penalties (NULL: none)
     const float* rp; const float* pp; const float* fp;
@@ -341,7 +379,7 @@ struct VerifyArgs {
 
 // A slot's penalties as the verify's kernels see them: every row of the slot, target and draft, is penalised with the
 // slot's history before mask and temperature, as the two sampler launches did when they took the rows' statistics.
-#define VF_BM_WORDS 512                // bitmap of one segment's tokens that occur in the history (segments up to 16,384 logits)
+#define VF_BM_WORDS (VF_MAX_V / VF_CTAS / 32)   // bitmap of a CTA's tokens that occur in the history
 struct PenSlot {
     const int32_t* h; int len; float rp, pp, fp; bool on;
     __device__ void init(const VerifyArgs& a, int b) {
@@ -413,19 +451,43 @@ struct Residual {
     }
 };
 
-// Step 1, one warp per slot: the accepted prefix from the row statistics of the target and draft rows (the lanes share
-// the count of a draft token in the slot's history; everything else every lane does alike).
-__global__ void k_verify_decide(const __grid_constant__ VerifyArgs a) {
-    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (b >= a.B) return;
-    const int k = a.k, V = a.V;
+// Four logits of a row from token i on (a multiple of 4), -inf beyond the vocabulary.
+__device__ __forceinline__ float4 load_four(const VerifyArgs& a, const void* base, size_t at, int i) {
+    float4 v = make_float4(CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF);
+    if (i >= a.V) return v;
+    if (a.vec && a.dtype == COLINFER_F32) return __ldcg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + at + i));
+    if (a.vec) {
+        const uint2 q = __ldcg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(base) + at + i));
+        return make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u), __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
+    }
+    v.x = load_logit(base, a.dtype, at + i);
+    if (i + 1 < a.V) v.y = load_logit(base, a.dtype, at + i + 1);
+    if (i + 2 < a.V) v.z = load_logit(base, a.dtype, at + i + 2);
+    if (i + 3 < a.V) v.w = load_logit(base, a.dtype, at + i + 3);
+    return v;
+}
+
+// A cluster of 8 CTAs per slot.  The accepted prefix (every CTA decides it for itself, a warp per position); the residual mass
+// of the rejected position, a region of consecutive tokens per warp; then the one warp in whose region the running mass reaches
+// us * total walks over that region again, a lane's four tokens at a time.  Launches and latency are all there is to it: decide,
+// sum and pick were three launches, the pick serial in one thread per slot.
+__global__ void __cluster_dims__(VF_CTAS, 1, 1) __launch_bounds__(VF_THREADS) k_verify_finish(const __grid_constant__ VerifyArgs a) {
+    __shared__ u64 wsum[VF_WARPS], csum[VF_CTAS];
+    __shared__ uint32_t bm[VF_BM_WORDS];
+    __shared__ int s_first;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int b = blockIdx.x / VF_CTAS, rank = blockIdx.x % VF_CTAS;
+    const int k = a.k, V = a.V, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const colinfer_row_stats* st_t = a.st_t + (size_t)b * (k + 1);
     const colinfer_row_stats* st_d = a.st_d + (size_t)b * k;
     const bool greedy = !(a.temperature[b] > 0.0f);
+    cluster.barrier_arrive();                                        // (waited for before the first write into a peer)
     PenSlot pen;
     pen.init(a, b);
-    int j = 0;
-    for (; j < k; ++j) {
+    if (tid == 0) s_first = k;
+    __syncthreads();
+    // ---- the first position whose draft token is not accepted
+    for (int j = warp; j < k; j += VF_WARPS) {
         const long long d = a.draft_ids[(size_t)b * k + j];
         bool ok;
         if (greedy) ok = (d == st_t[j].argmax);
@@ -444,149 +506,82 @@ __global__ void k_verify_decide(const __grid_constant__ VerifyArgs a) {
             // whatever the draft thought of it: 0 <= 0 must not pass)
             ok = p > 0.0 && (double)a.ua[(size_t)b * k + j] * q <= p;
         }
-        if (!ok) break;
+        if (!ok) { if (lane == 0) atomicMin(&s_first, j); break; }   // (the warp's later positions do not matter any more)
     }
-    int mode = 1;
-    if (greedy || j == k) mode = 0;
-    else if ((st_t[j].status | st_d[j].status) & (COLINFER_ROW_DEGENERATE | COLINFER_ROW_TIMEOUT)) mode = 0;
-    if (lane == 0) a.slot[b] = make_int2(j, mode);
-}
+    __syncthreads();
+    const int j = s_first;
+    const bool known = greedy || j == k || ((st_t[j].status | st_d[j].status) & (COLINFER_ROW_DEGENERATE | COLINFER_ROW_TIMEOUT)) != 0;
+    if (rank == 0) {
+        int64_t* o = a.out_tok + (size_t)b * (k + 1);
+        for (int i = tid; i <= k; i += VF_THREADS) if (i != j) o[i] = i < j ? a.draft_ids[(size_t)b * k + i] : -1;
+        if (tid == 0) {
+            if (known) o[j] = greedy ? st_t[j].argmax : a.samp_t[(size_t)b * (k + 1) + j];
+            a.n[b] = j + 1;
+        }
+    }
+    cluster.barrier_wait();
+    if (known) return;                                               // (alike in every CTA of the cluster)
 
-// Step 2, VF_NSEG CTAs per slot: the residual mass max(p - q, 0) of one segment of the rejected position's two rows,
-// streamed once with 128-bit loads where the rows allow it.
-__global__ void __launch_bounds__(VF_THREADS) k_verify_residual(const __grid_constant__ VerifyArgs a) {
-    __shared__ u64 wsum[VF_THREADS / 32];
-    __shared__ uint32_t bm[VF_BM_WORDS];
-    const int b = blockIdx.x / VF_NSEG, sgi = blockIdx.x % VF_NSEG;
-    const int2 sl = a.slot[b];
-    if (sl.y != 1) return;
-    const int j = sl.x, k = a.k, V = a.V, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // ---- the residual mass of the position's two rows
     Residual res;
-    res.init(a.st_t[(size_t)b * (k + 1) + j], a.st_d[(size_t)b * k + j]);
+    res.init(st_t[j], st_d[j]);
     const int32_t* mrow = a.mask ? a.mask + ((size_t)b * (k + 1) + j) * a.W : nullptr;
     const size_t bt = ((size_t)b * (k + 1) + j) * V, bd = ((size_t)b * k + j) * V;
-    const int lo = min(sgi * a.seg, V), hi = min(lo + a.seg, V);
-    PenSlot pen;
-    pen.init(a, b);
-    if (pen.on) pen.mark(bm, lo, hi);                                // (the same for every thread of the CTA)
-    u64 acc = 0;
-    if (a.vec) {
-        const float* pt = reinterpret_cast<const float*>(a.tl) + bt;
-        const float* pd = reinterpret_cast<const float*>(a.dl) + bd;
-        for (int i0 = lo + threadIdx.x * 4; i0 < hi; i0 += 2 * VF_THREADS * 4) {
-            const int i1 = i0 + VF_THREADS * 4;
-            const float4 t0 = __ldcg(reinterpret_cast<const float4*>(pt + i0)), d0 = __ldcg(reinterpret_cast<const float4*>(pd + i0));
-            float4 t1 = make_float4(CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF), d1 = t1;
-            if (i1 < hi) { t1 = __ldcg(reinterpret_cast<const float4*>(pt + i1)); d1 = __ldcg(reinterpret_cast<const float4*>(pd + i1)); }
-            const float tt[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w}, dd[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+    const int c_lo = min(rank * VF_WARPS * a.reg, V), lo = min(c_lo + warp * a.reg, V), hi = min(lo + a.reg, V);
+    if (pen.on) pen.mark(bm, c_lo, min(c_lo + VF_WARPS * a.reg, V));
+    auto four = [&](int i, u64 (&m)[4]) {
+        const float4 t = load_four(a, a.tl, bt, i), d = load_four(a, a.dl, bd, i);
+        const float tt[4] = {t.x, t.y, t.z, t.w}, dd[4] = {d.x, d.y, d.z, d.w};
+        const uint32_t bits = mrow != nullptr && i < V ? (uint32_t)__ldg(mrow + (i >> 5)) >> (i & 31) : 0xFu;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int i = (e < 4 ? i0 : i1 - 4) + e;
-                if (i < hi && mask_allows(mrow, i)) { float lt = tt[e], ld = dd[e]; pen.fix(bm, lo, i, lt, ld); acc += res(lt, ld); }
-            }
+        for (int e = 0; e < 4; ++e) {
+            float lt = tt[e], ld = dd[e];
+            m[e] = 0;
+            if (i + e < hi && ((bits >> e) & 1u)) { pen.fix(bm, c_lo, i + e, lt, ld); m[e] = res(lt, ld); }
         }
-    } else {
-        for (int i = lo + threadIdx.x; i < hi; i += VF_THREADS)
-            if (mask_allows(mrow, i)) {
-                float lt = load_logit(a.tl, a.dtype, bt + i), ld = load_logit(a.dl, a.dtype, bd + i);
-                pen.fix(bm, lo, i, lt, ld);
-                acc += res(lt, ld);
-            }
-    }
-    const u64 wt = warp_sum_u64(acc);
-    if (lane == 0) wsum[warp] = wt;
+        return m[0] + m[1] + m[2] + m[3];
+    };
+    u64 acc = 0;
+#pragma unroll 2
+    for (int i = lo + lane * 4; i < hi; i += 128) { u64 m[4]; acc += four(i, m); }
+    const u64 mine = warp_sum_u64(acc);
+    if (lane == 0) wsum[warp] = mine;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        u64 t = 0;
-        for (int w = 0; w < VF_THREADS / 32; ++w) t += wsum[w];
-        a.seg_sums[(size_t)b * VF_NSEG + sgi] = t;
+    const u64 others = lane < VF_WARPS ? wsum[lane] : 0ull, cta = warp_sum_u64(others);
+    if (tid < VF_CTAS) *cluster.map_shared_rank(&csum[rank], tid) = cta;
+    cluster.sync();
+    u64 total = 0, run = 0;
+    for (int q = 0; q < VF_CTAS; ++q) { const u64 c = csum[q]; total += c; run += q < rank ? c : 0ull; }
+    if (total == 0) {                                                // no residual mass: draw from p_j
+        if (rank == 0 && tid == 0) a.out_tok[(size_t)b * (k + 1) + j] = a.samp_t[(size_t)b * (k + 1) + j];
+        return;
+    }
+    const double t = ceil((double)a.us[(size_t)b * (k + 1) + j] * (double)total);
+    u64 target = t <= 1.0 ? 1ull : (u64)t;
+    if (target > total) target = total;
+    run += warp_sum_u64(lane < warp ? others : 0ull);
+    if (!(run < target && target <= run + mine)) return;
+    for (int i0 = lo; i0 < hi; i0 += 128) {
+        const int i = i0 + lane * 4;
+        u64 m[4];
+        const u64 sum = four(i, m), incl = warp_incl_scan_u64(sum, lane);
+        const unsigned hit = __ballot_sync(0xffffffffu, run + incl >= target);
+        if (hit) {
+            if (lane == __ffs(hit) - 1) {
+                u64 c = run + incl - sum;
+                int e = 0;
+                for (; e < 3; ++e) { c += m[e]; if (c >= target) break; }
+                a.out_tok[(size_t)b * (k + 1) + j] = i + e;
+            }
+            return;
+        }
+        run += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
-// Step 3, one CTA per slot: the segment in which the running residual mass reaches us * total, then the token inside it
-// (threads own consecutive chunks of the segment: token order); and the slot's outputs.
-__global__ void __launch_bounds__(VF_THREADS) k_verify_pick(const __grid_constant__ VerifyArgs a) {
-    __shared__ u64 tsum[VF_THREADS];
-    __shared__ uint32_t bm[VF_BM_WORDS];
-    __shared__ long long s_token;
-    const int b = blockIdx.x, k = a.k, V = a.V, tid = threadIdx.x;
-    const int2 sl = a.slot[b];
-    const int j = sl.x;
-    if (tid == 0) {
-        if (sl.y == 0) {
-            const bool greedy = !(a.temperature[b] > 0.0f);
-            s_token = greedy ? a.st_t[(size_t)b * (k + 1) + j].argmax : a.samp_t[(size_t)b * (k + 1) + j];
-        } else s_token = -1;
-    }
-    __syncthreads();
-    if (sl.y == 1) {
-        u64 total = 0;
-        for (int s = 0; s < VF_NSEG; ++s) total += a.seg_sums[(size_t)b * VF_NSEG + s];
-        if (total == 0) {
-            if (tid == 0) s_token = a.samp_t[(size_t)b * (k + 1) + j];   // no residual mass: draw from p_j
-        } else {
-            double t = ceil((double)a.us[(size_t)b * (k + 1) + j] * (double)total);
-            u64 target = t <= 1.0 ? 1ull : (u64)t;
-            if (target > total) target = total;
-            int sx = 0; u64 before = 0;
-            for (; sx < VF_NSEG - 1; ++sx) {
-                const u64 v = a.seg_sums[(size_t)b * VF_NSEG + sx];
-                if (before + v >= target) break;
-                before += v;
-            }
-            Residual res;
-            res.init(a.st_t[(size_t)b * (k + 1) + j], a.st_d[(size_t)b * k + j]);
-            const int32_t* mrow = a.mask ? a.mask + ((size_t)b * (k + 1) + j) * a.W : nullptr;
-            const size_t bt = ((size_t)b * (k + 1) + j) * V, bd = ((size_t)b * k + j) * V;
-            const int lo = min(sx * a.seg, V), hi = min(lo + a.seg, V);
-            const int per = (hi - lo + VF_THREADS - 1) / VF_THREADS;
-            const int c_lo = min(lo + tid * per, hi), c_hi = min(c_lo + per, hi);
-            PenSlot pen;
-            pen.init(a, b);
-            if (pen.on) pen.mark(bm, lo, hi);                        // (sx, and so this branch, is the same for every thread)
-            u64 mine = 0;
-            for (int i = c_lo; i < c_hi; ++i)
-                if (mask_allows(mrow, i)) {
-                    float lt = load_logit(a.tl, a.dtype, bt + i), ld = load_logit(a.dl, a.dtype, bd + i);
-                    pen.fix(bm, lo, i, lt, ld);
-                    mine += res(lt, ld);
-                }
-            tsum[tid] = mine;
-            __syncthreads();
-            if (tid == 0) {
-                u64 run = before;
-                int tx = VF_THREADS - 1;
-                for (int t2 = 0; t2 < VF_THREADS; ++t2) { if (run + tsum[t2] >= target) { tx = t2; break; } run += tsum[t2]; }
-                tsum[0] = run; s_token = -2 - tx;                 // (thread tx walks its chunk from the running sum `run`)
-            }
-            __syncthreads();
-            if (s_token == -2 - tid) {
-                u64 run = tsum[0];
-                long long tok = c_hi > c_lo ? c_hi - 1 : lo;
-                for (int i = c_lo; i < c_hi; ++i) {
-                    if (mask_allows(mrow, i)) {
-                        float lt = load_logit(a.tl, a.dtype, bt + i), ld = load_logit(a.dl, a.dtype, bd + i);
-                        pen.fix(bm, lo, i, lt, ld);
-                        run += res(lt, ld);
-                    }
-                    if (run >= target) { tok = i; break; }
-                }
-                s_token = tok;
-            }
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        int64_t* o = a.out_tok + (size_t)b * (k + 1);
-        for (int i = 0; i <= k; ++i) o[i] = i < j ? a.draft_ids[(size_t)b * k + i] : -1;
-        o[j] = s_token;
-        a.n[b] = j + 1;
-    }
-}
-
-// scratch_stats holds, after the 2k + 1 row statistics of every slot, the per-slot decision and the segment sums
+// scratch_stats holds the 2k + 1 row statistics of every slot: the target rows', then the draft rows'
 extern "C" int64_t colinfer_spec_verify_stats_bytes(int B, int k) {
-    return (int64_t)B * (2 * k + 1) * (int64_t)sizeof(colinfer_row_stats) + (int64_t)B * 8 + (int64_t)B * VF_NSEG * 8;
+    return (int64_t)B * (2 * k + 1) * (int64_t)sizeof(colinfer_row_stats);
 }
 extern "C" int64_t colinfer_spec_verify_ids_bytes(int B, int k) { return (int64_t)B * (k + 1) * 8; }
 
@@ -599,31 +594,23 @@ extern "C" int colinfer_spec_verify(const void* target_logits, const void* draft
         !scratch_ids || B < 0 || k < 1 || V <= 0)
         return (int)cudaErrorInvalidValue;
     if (B == 0) return 0;
-    if ((((V + VF_NSEG - 1) / VF_NSEG + 127) / 128) * 128 > VF_BM_WORDS * 32) return (int)cudaErrorInvalidValue;
+    if (V > VF_MAX_V) return (int)cudaErrorInvalidValue;
     colinfer_row_stats* st_t = scratch_stats;
     colinfer_row_stats* st_d = scratch_stats + (size_t)B * (k + 1);
-    // target rows: statistics and the plain draw of every row with its sampling uniform
-    int e = colinfer_sample(target_logits, dtype, mask, k + 1, W, params, nullptr, 0, us, scratch_ids, st_t, nullptr,
-                            B, k + 1, V, 0, stream);
-    if (e) return e;
-    // draft rows: statistics only (the first k mask rows of each slot apply)
-    e = colinfer_sample(draft_logits, dtype, mask, k + 1, W, params, nullptr, 0, nullptr, nullptr, st_d, nullptr,
-                        B, k, V, 0, stream);
+    // the target rows' statistics and the plain draw of every one of them with its sampling uniform; the draft rows' statistics
+    // (the first k mask rows of each slot apply): one launch where one kernel takes them all
+    const int e = colinfer_sample_two(target_logits, draft_logits, dtype, mask, k + 1, W, params, nullptr, 0, us, scratch_ids, st_t, nullptr,
+                                      B, k + 1, k, V, 0, stream);
     if (e) return e;
     VerifyArgs a;
     a.tl = target_logits; a.dl = draft_logits; a.dtype = dtype; a.mask = mask; a.W = W;
     a.temperature = params->temperature; a.draft_ids = draft_ids; a.ua = ua; a.us = us;
     a.st_t = st_t; a.st_d = st_d; a.samp_t = scratch_ids; a.out_tok = out_tok; a.n = n; a.B = B; a.k = k; a.V = V;
-    a.slot = reinterpret_cast<int2*>(st_d + (size_t)B * k);
-    a.seg_sums = reinterpret_cast<u64*>(a.slot + B);
-    a.seg = (((V + VF_NSEG - 1) / VF_NSEG + 127) / 128) * 128;
+    a.reg = ((V + VF_CTAS * VF_WARPS - 1) / (VF_CTAS * VF_WARPS) + 127) / 128 * 128;
     a.history = params->history; a.hist_len = params->hist_len; a.hist_stride = params->history ? params->hist_stride : 0;
     a.rp = params->repetition_penalty; a.pp = params->presence_penalty; a.fp = params->frequency_penalty;
-    a.vec = (dtype == COLINFER_F32 && (V % 4) == 0 && (((uintptr_t)target_logits) & 15) == 0 && (((uintptr_t)draft_logits) & 15) == 0) ? 1 : 0;
-    cudaStream_t st = (cudaStream_t)stream;
-    k_verify_decide<<<(B + 3) / 4, 128, 0, st>>>(a);
-    k_verify_residual<<<B * VF_NSEG, VF_THREADS, 0, st>>>(a);
-    k_verify_pick<<<B, VF_THREADS, 0, st>>>(a);
+    a.vec = (V % 4) == 0 && ((((uintptr_t)target_logits) | ((uintptr_t)draft_logits)) & (dtype == COLINFER_F32 ? 15 : 7)) == 0 ? 1 : 0;
+    k_verify_finish<<<B * VF_CTAS, VF_THREADS, 0, (cudaStream_t)stream>>>(a);
     return (int)cudaGetLastError();
 }
 

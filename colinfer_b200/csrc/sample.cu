@@ -62,6 +62,7 @@ struct SampleArgs {
     const void* pos; int pos_i64; const float* u;
     int64_t* out; colinfer_row_stats* stats; int32_t* status;
     int B, R, V; int slice_elems; int flags;
+    colinfer_second_rows second;
     long long* prof; int prof_slots;   // optional per-CTA phase timestamps (profiling hook)
 };
 // Profiling hook: thread 0 adds the cycles since its previous marker to the slot's total (summed over the CTA's rows).
@@ -175,6 +176,7 @@ __device__ __forceinline__ u64 ceil_target(float frac, u64 total) {
 
 // The row's uniform in (0, 1]: explicit, or Philox keyed by (seed, position + row of the slot), or 1 when no draw is asked.
 __device__ __forceinline__ float row_uniform(const SampleArgs& a, int row, int b, int r) {
+    if (row >= a.second.rows1) return 1.0f;
     if (a.u != nullptr) return a.u[row];
     if (a.pos != nullptr && a.p.seed != nullptr) {
         const long long p0 = a.pos_i64 ? reinterpret_cast<const long long*>(a.pos)[b]
@@ -624,7 +626,7 @@ __device__ __noinline__ bool finish_pending(const SampleArgs& a, const Pending& 
             int j = 0;
             for (; j < 3; ++j) { run += q[j]; if (run >= target) break; }
             const int row = pd.row;
-            if (a.out) a.out[row] = (long long)ki[4 * lane + j];
+            if (draws(a, row)) a.out[row] = (long long)ki[4 * lane + j];
             if (a.status) a.status[row] = pd.status;
             if (a.stats) {
                 colinfer_row_stats st;
@@ -679,7 +681,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         fence_mbar_init();
     }
     const int n_clusters = (int)gridDim.x / CS;
-    const long long n_rows = (long long)a.B * a.R;
+    const long long n_rows = a.second.rows;
     long long prof_last = clock64();
     const long long prof_t0 = prof_last;
     if (a.prof && tid == 0) for (int i = 0; i < 12; ++i) sc->prof[i] = 0;
@@ -687,7 +689,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     // Starts the bulk copies of one row's slice (thread 0 only; every thread must be done reading the buffer).
     auto issue_row = [&](const long long rw, bool first) {
         if (!first) fence_proxy_async();                       // earlier reads of the buffer precede these writes
-        const float* src = reinterpret_cast<const float*>(a.logits) + (size_t)rw * V + slice_lo;
+        const float* src = reinterpret_cast<const float*>(logits_of(a, (int)rw)) + (size_t)rw * V + slice_lo;
         if (a.flags & COLINFER_TEST_DROP_COPY) return;        // test flag: nothing is armed, nothing is in flight; the waits run out
         for (int c = 0; c < nchunks; ++c) {
             const int len = min(CI_CHUNK, slice_len - c * CI_CHUNK);
@@ -721,7 +723,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     // One row of the batch.  `it` counts this cluster's rows: its parity selects the mbarrier phase and the exchange slots.
     auto process_row = [&](const int row, const int it, const bool allow_fast, const long long next_row) {
     const int par = it & 1;
-    const int b = row / a.R, r = row % a.R;
+    int r;
+    const int b = slot_of(a, row, r);
     // ---------------------------------------------------------------------------------------- start the HBM read
     // One thread issues every bulk copy of the slice at once, before anything else (unless the previous row already
     // started this row's copies because it no longer needed the buffer).
@@ -831,7 +834,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     } else {
         const size_t g0 = (size_t)row * V + slice_lo;
         if (a.dtype == COLINFER_BF16) {
-            const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(a.logits) + g0;
+            const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(logits_of(a, row)) + g0;
             if ((((uintptr_t)src) & 15) == 0) {
                 const uint4* s4 = reinterpret_cast<const uint4*>(src);
                 for (int i = tid; i * 8 < slice_len; i += CI_THREADS) {
@@ -852,7 +855,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 for (int i = tid; i < slice_len; i += CI_THREADS) rowbuf[i] = __bfloat162float(src[i]);
             }
         } else {
-            const float* src = reinterpret_cast<const float*>(a.logits) + g0;
+            const float* src = reinterpret_cast<const float*>(logits_of(a, row)) + g0;
             for (int i = tid; i < slice_len; i += CI_THREADS) rowbuf[i] = __ldg(src + i);
         }
         __syncthreads();
@@ -1034,7 +1037,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     if (!do_dist) {
         // greedy, degenerate or failed row: the argmax.  Nobody reads a peer's memory after the barrier: leave at once.
         if (rank == 0 && tid == 0) {
-            if (a.out) a.out[row] = token;
+            if (draws(a, row)) a.out[row] = token;
             if (a.status) a.status[row] = status;
             if (a.stats) {
                 colinfer_row_stats st;
@@ -1374,7 +1377,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                             u64 c = run + incl - s4;
                             int j = 0;
                             for (; j < 3; ++j) { c += q4[j]; if (c >= target) break; }
-                            if (a.out) a.out[row] = (long long)(slice_lo + i + j);
+                            if (draws(a, row)) a.out[row] = (long long)(slice_lo + i + j);
                         }
                         break;
                     }
@@ -1386,7 +1389,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     }
 
     if (rank == 0 && tid == 0) {
-        if (token >= 0 && a.out) a.out[row] = token;           // list-path or degenerate rows (else the crossing lane stored it)
+        if (token >= 0 && draws(a, row)) a.out[row] = token;           // list-path or degenerate rows (else the crossing lane stored it)
         if (a.status) a.status[row] = status;
         if (a.stats) {
             colinfer_row_stats st;
@@ -1589,8 +1592,9 @@ int chunk_clusters(int dev, int ki, int cluster, int smem) {
 
 // Launches the chunk kernel where it is the faster one; returns -1 where it is not (nothing launched), else a CUDA error code.
 int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_rows, int W, const colinfer_sampler_params* params, const void* pos,
-                 int pos_is_i64, const float* u, int64_t* out_ids, colinfer_row_stats* stats, int32_t* status, int B, int R, int V, int flags, cudaStream_t stream) {
-    const long long rows = (long long)B * R;
+                 int pos_is_i64, const float* u, int64_t* out_ids, colinfer_row_stats* stats, int32_t* status, int B, int R, int V, int flags,
+                 const colinfer_second_rows& second, cudaStream_t stream) {
+    const long long rows = second.rows;
     if (V > kChunkMaxV || rows > 0x7ffffffeLL) return -1;
     const bool pen = params->history != nullptr;
     bool few = false;
@@ -1619,7 +1623,7 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
     a.p = *params;
     a.pos = pos; a.pos_i64 = pos_is_i64; a.u = u;
     a.out = out_ids; a.stats = stats; a.status = status;
-    a.B = B; a.R = R; a.V = V; a.flags = flags; a.cluster = C;
+    a.B = B; a.R = R; a.V = V; a.flags = flags; a.cluster = C; a.second = second;
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
     chunk_config(cfg, attr, few, C, rows, smem, stream);
     void* args[] = {&a};
@@ -1627,10 +1631,11 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
 }
 }  // namespace
 
-extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mask, int mask_rows, int W,
-                               const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u,
-                               int64_t* out_ids, colinfer_row_stats* stats, int32_t* status,
-                               int B, int R, int V, int flags, void* stream) {
+// Both sets of rows (colinfer_second_rows), or -1 where only separate launches take them (nothing is launched then).
+static int sample_rows(const void* logits, const void* logits2, int dtype, const int32_t* mask, int mask_rows, int W,
+                       const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u,
+                       int64_t* out_ids, colinfer_row_stats* stats, int32_t* status,
+                       int B, int R, int R2, int V, int flags, void* stream) {
     if (B < 0 || R < 0 || V <= 0) return (int)cudaErrorInvalidValue;
     if ((long long)B * R == 0) return 0;
     if (!logits || !params || (!out_ids && !stats)) return (int)cudaErrorInvalidValue;
@@ -1639,6 +1644,11 @@ extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mas
     if (out_ids && u == nullptr && (pos == nullptr || params->seed == nullptr)) return (int)cudaErrorInvalidValue;
     if (mask && (W < (V + 31) / 32 || mask_rows < R)) return (int)cudaErrorInvalidValue;
     if ((long long)B * R > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+    const long long rows = (long long)B * R + (long long)B * R2;
+    if (rows > 0x7fffffffLL) return -1;
+    colinfer_second_rows second;
+    second.R = R2 > 0 ? R2 : 1; second.rows1 = R2 > 0 ? B * R : 0x7fffffff; second.rows = (int)rows;
+    second.logits = R2 > 0 ? reinterpret_cast<const void*>((uintptr_t)logits2 - (uintptr_t)second.rows1 * V * (dtype == COLINFER_F32 ? 4 : 2)) : nullptr;
     // Which kernel: the caller's choice (bits COLINFER_KERNEL_* of flags), else automatic.  Few rows -- at most as many
     // as the device holds clusters at once -- are a latency problem: one CTA per row would leave most SMs idle, so each
     // row gets a whole 8-CTA cluster of the cluster-resident kernel.  More rows are a throughput problem: the streaming
@@ -1653,14 +1663,15 @@ extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mas
             colinfer_geometry g0;
             if (!pick_geometry(V, dtype, logits, 0, &g0)) {
                 const int res0 = active_clusters(g0);
-                if (res0 > 0 && (long long)B * R <= res0) use_stream = false;
+                if (res0 > 0 && rows <= res0) use_stream = false;
             }
         }
         if (use_stream && choice == 0) {
             const int rc = launch_chunk(logits, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status,
-                                        B, R, V, flags, (cudaStream_t)stream);
+                                        B, R, V, flags, second, (cudaStream_t)stream);
             if (rc >= 0) return rc;
         }
+        if (use_stream && R2 > 0) return -1;
         if (use_stream) {
             const int rc = colinfer_launch_stream(logits, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status,
                                                   B, R, V, flags, (cudaStream_t)stream);
@@ -1671,15 +1682,15 @@ extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mas
     if (pick_geometry(V, dtype, logits, forced, &g)) return (int)cudaErrorInvalidValue;
     const int resident = active_clusters(g);
     if (resident <= 0) return (int)cudaErrorInvalidConfiguration;
-    const long long clusters = (long long)B * R < resident ? (long long)B * R : resident;
+    const long long clusters = rows < resident ? rows : resident;
 
     SampleArgs a;
-    a.logits = logits; a.dtype = dtype; a.use_bulk = g.bulk_copy;
+    a.logits = logits; a.dtype = dtype; a.use_bulk = g.bulk_copy && (R2 == 0 || ((uintptr_t)logits2 & 15) == 0);
     a.mask = mask; a.mask_rows = mask_rows; a.W = W;
     a.p = *params;
     a.pos = pos; a.pos_i64 = pos_is_i64; a.u = u;
     a.out = out_ids; a.stats = stats; a.status = status;
-    a.B = B; a.R = R; a.V = V; a.slice_elems = g.slice_elems; a.flags = flags;
+    a.B = B; a.R = R; a.V = V; a.slice_elems = g.slice_elems; a.flags = flags; a.second = second;
     colinfer_profile_buffer(&a.prof, &a.prof_slots);
 
     cudaError_t e = cudaFuncSetAttribute(k_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem_bytes);
@@ -1689,4 +1700,21 @@ extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mas
     e = cudaLaunchKernelEx(&cfg, k_sample, a);
     if (e != cudaSuccess) return (int)e;
     return (int)cudaGetLastError();
+}
+
+extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mask, int mask_rows, int W,
+                               const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u,
+                               int64_t* out_ids, colinfer_row_stats* stats, int32_t* status,
+                               int B, int R, int V, int flags, void* stream) {
+    return sample_rows(logits, nullptr, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status, B, R, 0, V, flags, stream);
+}
+
+int colinfer_sample_two(const void* logits, const void* logits2, int dtype, const int32_t* mask, int mask_rows, int W,
+                        const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u, int64_t* out_ids,
+                        colinfer_row_stats* stats, int32_t* status, int B, int R, int R2, int V, int flags, void* stream) {
+    const int rc = sample_rows(logits, logits2, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status, B, R, R2, V, flags, stream);
+    if (rc >= 0) return rc;
+    const int e = sample_rows(logits, nullptr, dtype, mask, mask_rows, W, params, pos, pos_is_i64, u, out_ids, stats, status, B, R, 0, V, flags, stream);
+    if (e) return e;
+    return sample_rows(logits2, nullptr, dtype, mask, mask_rows, W, params, nullptr, 0, nullptr, nullptr, stats + (size_t)B * R, nullptr, B, R2, 0, V, flags, stream);
 }

@@ -1131,7 +1131,8 @@ __device__ __forceinline__ FineDecision fine_decide(const Grp<CL>& g, uint32_t* 
 // A row's parameters, one 32-bit word per lane: temperature, top_k, top_p, log_min_p, seed (low), the three penalties, seed (high),
 // hist_len, position (low, high), explicit uniform.
 __device__ __forceinline__ uint32_t load_params(const Args& a, int row, int lane) {
-    const int b = a.R == 1 ? row : row / a.R;
+    int r;
+    const int b = slot_of(a, row, r);
     const uint32_t* src = nullptr;
     size_t at = b;
     if (lane < 10) {
@@ -1141,9 +1142,10 @@ __device__ __forceinline__ uint32_t load_params(const Args& a, int row, int lane
         if (a.u == nullptr && (a.pos_i64 || lane == 10)) src = reinterpret_cast<const uint32_t*>(a.pos);
         if (a.pos_i64) at = 2 * (size_t)b + (lane - 10);
     } else if (lane == 12) {
-        src = reinterpret_cast<const uint32_t*>(a.u); at = row;
+        if (row < a.second.rows1) src = reinterpret_cast<const uint32_t*>(a.u);
+        at = row;
     }
-    return src ? __ldg(src + at) : lane == 5 ? 0x3F800000u : lane == 9 ? (uint32_t)a.p.hist_stride : 0u;
+    return src ? __ldg(src + at) : lane == 5 || lane == 12 ? 0x3F800000u : lane == 9 ? (uint32_t)a.p.hist_stride : 0u;
 }
 static_assert(offsetof(colinfer_sampler_params, hist_len) == 9 * sizeof(void*) && offsetof(colinfer_sampler_params, seed) == 4 * sizeof(void*) &&
               offsetof(colinfer_sampler_params, frequency_penalty) == 7 * sizeof(void*), "load_params indexes the pointers");
@@ -1151,7 +1153,7 @@ static_assert(offsetof(colinfer_sampler_params, hist_len) == 9 * sizeof(void*) &
 // Where a row lies.
 template <int ELT>
 __device__ __forceinline__ const char* place_row(const Args& a, int row, int& al, uint32_t& end, int& nc) {
-    const u64 addr = reinterpret_cast<u64>(a.logits) + (u64)row * (u64)a.V * ELT;
+    const u64 addr = reinterpret_cast<u64>(logits_of(a, row)) + (u64)row * (u64)a.V * ELT;
     al = (int)((addr & 15) / ELT);
     end = (uint32_t)((addr + (u64)a.V * ELT + 15) & ~15ull);
     nc = (a.V + al + CHUNK - 1) / CHUNK;
@@ -1162,7 +1164,8 @@ template <int ELT>
 static __device__ __noinline__ void derive_row(const Args& a, RowS& rw, int row, uint32_t words) {
     auto word = [&](int l) { return __shfl_sync(0xffffffffu, words, l); };
     auto num = [&](int l) { return __uint_as_float(word(l)); };
-    const int b = a.R == 1 ? row : row / a.R, r = row - b * a.R;
+    int r;
+    const int b = slot_of(a, row, r);
     const float T = num(0), topp = num(2), rp = num(5), pp = num(6), fp = num(7);
     const int kk = (int)word(1);
     float u = num(12);
@@ -1252,14 +1255,15 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     __syncthreads();
 
     // ---------------------------------------------------------------------------------------- which rows are this group's
-    const int n_rows = a.B * a.R;
+    const int n_rows = a.second.rows;
     const int grp = CL ? blockIdx.x / a.cluster : blockIdx.x, n_grp = CL ? gridDim.x / a.cluster : gridDim.x;
     // Without clusters the grid has a CTA per row, of which as many start as fit; a CTA that is through with its row takes the
     // next one off the hardware's queue.  Rows differ in cost (a wide row takes two or three passes, any other one): the CTAs'
     // indices are positions in an order of the rows by cost class, dearest first, which every CTA works out for itself.
     const bool dealt = !CL && n_rows > 2 * NUM_SM && n_rows <= BAL_ROWS;
     auto row_class = [&](int row) {
-        const int b = a.R == 1 ? row : row / a.R;
+        int r;
+        const int b = slot_of(a, row, r);
         const float T = a.p.temperature[b];
         const int k = a.p.top_k[b];
         if (!((T > 0.0f) || (a.flags & COLINFER_FORCE_DISTRIBUTION))) return 2;
@@ -1316,7 +1320,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         if (next_row >= 0) {
             next_words = load_params(a, next_row, lane);
             if (a.p.history) {                                   // the history's lines into L2
-                const char* h = reinterpret_cast<const char*>(a.p.history + (size_t)(a.R == 1 ? next_row : next_row / a.R) * a.p.hist_stride);
+                int r;
+                const char* h = reinterpret_cast<const char*>(a.p.history + (size_t)slot_of(a, next_row, r) * a.p.hist_stride);
                 for (int i = lane * 128; i < min(a.p.hist_stride, 4096) * 4; i += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(h + i));
             }
             if (lane == 0) {
@@ -2020,7 +2025,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                             u64 cum = incl; int e = 0;
 #pragma unroll
                             for (int j = 15; j >= 0; --j) { if (cum >= target) e = j; cum -= q[j]; }   // the first whose running mass reaches the target
-                            if (a.out) a.out[rw.row] = (long long)(c * CHUNK + lane * 16 + e - al);
+                            if (draws(a, rw.row)) a.out[rw.row] = (long long)(c * CHUNK + lane * 16 + e - al);
                         }
                     }
                 }
@@ -2038,7 +2043,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 if (g.at(&rw, q)->hist_slow) status |= COLINFER_ROW_HIST_SLOW;
                 if (g.at(sc, q)->dead) status |= COLINFER_ROW_TIMEOUT;
             }
-            if (!rw.drawn && a.out) a.out[rw.row] = rw.token;
+            if (!rw.drawn && draws(a, rw.row)) a.out[rw.row] = rw.token;
             if (a.status) a.status[rw.row] = status;
             if (a.stats) {
                 colinfer_row_stats st;
