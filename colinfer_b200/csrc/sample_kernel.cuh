@@ -1260,7 +1260,9 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     // Without clusters the grid has a CTA per row, of which as many start as fit; a CTA that is through with its row takes the
     // next one off the hardware's queue.  Rows differ in cost (a wide row takes two or three passes, any other one): the CTAs'
     // indices are positions in an order of the rows by cost class, dearest first, which every CTA works out for itself.
-    const bool dealt = !CL && n_rows > 2 * NUM_SM && n_rows <= BAL_ROWS;
+    // With at most two rows per SM they all start at once, CTA j + NUM_SM beside CTA j: the dearest rows get an SM of their own,
+    // of the others the dearest goes with the cheapest.
+    const bool dealt = !CL && n_rows > NUM_SM && n_rows <= BAL_ROWS;
     auto row_class = [&](int row) {
         int r;
         const int b = slot_of(a, row, r);
@@ -1285,6 +1287,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     // The row at a position of that order.  One warp.
     auto row_of = [&](int pos) {
         if (!dealt) return pos;
+        if (n_rows <= 2 * NUM_SM) {
+            const int pairs = n_rows - NUM_SM;
+            pos = pos >= NUM_SM ? n_rows - 1 - (pos - NUM_SM) : pos < pairs ? NUM_SM - pairs + pos : pos - pairs;
+        }
         int j = 0;
         while (j < 2 && pos >= sc->cls_tot[j]) { pos -= sc->cls_tot[j]; ++j; }
         int t = 0;                                               // the last thread with at most pos rows of class j before its own
@@ -1359,8 +1365,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         RowS& rw = sc->rows[it & 1];
         const NextRow& nx = sc->next[it & 1];
         ring_start<ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW);
-        bool found = false, derived = false;                     // (the last warp's)
-        auto look_ahead = [&]() { if (warp == PW && !found) { find_next(it); found = true; } };
+        bool asked = false, found = false, derived = false;      // (the last warp's)
+        // (A row of several passes asks when its first one is through: the CTAs that ask before it have less left to do.)
+        auto ask = [&]() { if (!CL && warp == PW && !asked) { if (lane == 0) queue_ask(sc); asked = true; } };
+        auto look_ahead = [&]() { if (warp == PW && !found) { ask(); __syncwarp(); find_next(it); found = true; } };
         auto derive_next = [&]() { if (warp == PW && !derived) { look_ahead(); derive(it + 1); derived = true; if (lane == 0) sc->next[(it + 1) & 1].key = 0; } };
         SM_PROF(0);
 
@@ -1517,10 +1525,9 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 if (tid == 0) { rw.lref = lref; rw.count_hist = count_hist; }
             }
             SM_PROF(2);
-            if (!CL && tid == PW * 32) queue_ask(sc);
-            look_ahead();
             if (tid == 0) sc->tw = tw;
             const bool one_pass = !(cls & ROW_SAMPLED) || in_klist;
+            if (one_pass) look_ahead();
             const int then = one_pass ? THEN_NEXT_ROW : THEN_AGAIN;
             const float t = tw > -SM_FLT_MAX ? tw : SM_POS_INF;  // no bound: nothing is listed
             const int bad = (lists && !(tw > -SM_FLT_MAX) ? 1 : 0) | (wide && !count_hist ? 4 : 0);
@@ -1529,6 +1536,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             else if (count_hist) top1.l = pass_hist<CL, ELT, MASK>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF, from);
             else top1.l = pass_list<CL, ELT, MASK>(rw, nx, !one_pass, seen, then, t, list, lcap);
             SM_PROF(3);
+            ask();
             if (lists) top1.l = warp_max(top1.l);
             if (lane == 0) {
                 sc->wf[warp] = top1.l; sc->wi[warp] = top1.idx;
@@ -1871,6 +1879,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             SM_PROF(7);
 
             // -------------------------------------------------------------------------------- mass pass: kept mass per chunk
+            look_ahead();
             for (int attempt = 0; rw.path != PATH_LIST && attempt < 3; ++attempt) {
                 // (with one CTA per row the band's list takes the histogram's place: the path is decided)
                 Cand* blist = CL ? wlist + warp * WCAP : klist + warp * KCAP;
