@@ -165,13 +165,23 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
         // ------------------------------------------------------------------------------------ the pass
         float m = CI_NEG_INF, s = 0.0f;
         int wn = 0;
-        for (int i0 = r_lo; i0 < r_hi; i0 += 512) {
-            float4 v[4];
+        // (the next batch is under way while this one is worked on: with one batch in flight a warp's nineteen round trips to
+        // HBM are most of the row's time)
+        float4 nv[4];
+        auto fetch = [&](int i0) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int i = i0 + k * 128 + lane * 4;
-                v[k] = i < r_hi ? rw.load4(i) : make_float4(CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF);
+                nv[k] = i < r_hi ? rw.load4(i) : make_float4(CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF);
             }
+        };
+        fetch(r_lo);
+#pragma unroll 1
+        for (int i0 = r_lo; i0 < r_hi; i0 += 512) {
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = nv[k];
+            fetch(i0 + 512);
             float bm = CI_NEG_INF;
 #pragma unroll
             for (int k = 0; k < 4; ++k) bm = fmaxf(bm, fmaxf(fmaxf(v[k].x, v[k].y), fmaxf(v[k].z, v[k].w)));
