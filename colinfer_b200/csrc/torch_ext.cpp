@@ -196,6 +196,83 @@ std::vector<at::Tensor> lowrank_draft(const at::Tensor& ap, const at::Tensor& g2
     return res;
 }
 
+// logprobs(rows [r, V], toks [r], n_top) -> chosen [r], top_ids [r, n_top], top_lp [r, n_top]
+// (engine/runtime/scheduler.py:714-722)
+std::vector<at::Tensor> logprobs(const at::Tensor& rows, const at::Tensor& toks, int64_t n_top) {
+    TORCH_CHECK(rows.dim() == 2, "rows [r, V]");
+    TORCH_CHECK(rows.is_cuda() && rows.is_contiguous(), "rows must be a contiguous CUDA tensor");
+    check(toks, at::kLong, "toks");
+    const int64_t r = rows.size(0), V = rows.size(1);
+    TORCH_CHECK(toks.numel() == r, "one token per row");
+    TORCH_CHECK(n_top >= 0 && n_top <= std::min<int64_t>(32, V), "n_top in [0, ", std::min<int64_t>(32, V), "]");
+    const int dt = dtype_code(rows);
+    c10::cuda::CUDAGuard guard(rows.device());
+    at::Tensor chosen = at::empty({r}, rows.options().dtype(at::kFloat));
+    at::Tensor ids = at::empty({r, n_top}, rows.options().dtype(at::kLong)), lp = at::empty({r, n_top}, rows.options().dtype(at::kFloat));
+    if (r) cuda_ok(colinfer_logprobs(rows.data_ptr(), dt, toks.data_ptr<int64_t>(), (int)n_top, chosen.data_ptr<float>(),
+                                     n_top ? ids.data_ptr<int64_t>() : nullptr, n_top ? lp.data_ptr<float>() : nullptr, (int)r, (int)V, stream()), "logprobs");
+    return {chosen, ids, lp};
+}
+
+// processed_probs(logits [R, V], temperature [1], top_k [1], top_p [1], log_min_p [1]) -> [R, V] (engine/spec/accept.py:23-33)
+at::Tensor processed_probs(const at::Tensor& logits, const at::Tensor& temperature, const at::Tensor& top_k, const at::Tensor& top_p,
+                           const at::Tensor& log_min_p) {
+    check(logits, at::kFloat, "logits");
+    TORCH_CHECK(logits.dim() == 2, "logits [R, V]");
+    const colinfer_sampler_params p = params_of(1, temperature, top_k, top_p, log_min_p, {}, {}, {}, {}, {}, {});
+    const int64_t R = logits.size(0), V = logits.size(1);
+    c10::cuda::CUDAGuard guard(logits.device());
+    at::Tensor out = at::empty_like(logits);
+    at::Tensor scratch = at::empty({std::max<int64_t>(R, 1) * (int64_t)sizeof(colinfer_row_stats)}, logits.options().dtype(at::kByte));
+    cuda_ok(colinfer_processed_probs(logits.data_ptr<float>(), p.temperature, p.top_k, p.top_p, p.log_min_p, out.data_ptr<float>(),
+                                     reinterpret_cast<colinfer_row_stats*>(scratch.data_ptr()), (int)R, (int)V, stream()), "processed_probs");
+    return out;
+}
+
+// inverse_cdf(P [R, V], u [R]) -> [R] (engine/spec/accept.py:36-40)
+at::Tensor inverse_cdf(const at::Tensor& P, const at::Tensor& u_in) {
+    check(P, at::kFloat, "P");
+    TORCH_CHECK(P.dim() == 2, "P [R, V]");
+    const at::Tensor u = u_in.contiguous();
+    check(u, at::kFloat, "u");
+    TORCH_CHECK(u.numel() == P.size(0), "u [R]");
+    c10::cuda::CUDAGuard guard(P.device());
+    at::Tensor out = at::empty({P.size(0)}, P.options().dtype(at::kLong));
+    cuda_ok(colinfer_inverse_cdf(P.data_ptr<float>(), u.data_ptr<float>(), out.data_ptr<int64_t>(), (int)P.size(0), (int)P.size(1), stream()), "inverse_cdf");
+    return out;
+}
+
+// spec_verify(target [B, k + 1, V], draft [B, k, V], draft_ids [B, k], the slot parameters, ua [B, k], us [B, k + 1], mask?) ->
+// out_tok [B, k + 1], n [B]
+std::vector<at::Tensor> spec_verify(const at::Tensor& target, const at::Tensor& draft, const at::Tensor& draft_ids, const at::Tensor& temperature,
+                                    const at::Tensor& top_k, const at::Tensor& top_p, const at::Tensor& log_min_p, const Opt& seed, const Opt& rep,
+                                    const Opt& pres, const Opt& freq, const Opt& history, const Opt& hist_len, const at::Tensor& ua,
+                                    const at::Tensor& us, const Opt& mask) {
+    TORCH_CHECK(target.is_cuda() && target.is_contiguous(), "target_logits must be a contiguous CUDA tensor");
+    check(draft, target.scalar_type(), "draft_logits");
+    const int dt = dtype_code(target);
+    TORCH_CHECK(target.dim() == 3 && draft.dim() == 3, "target_logits [B, k+1, V], draft_logits [B, k, V]");
+    const int64_t B = target.size(0), k1 = target.size(1), k = k1 - 1, V = target.size(2);
+    TORCH_CHECK(k >= 1 && draft.size(0) == B && draft.size(1) == k && draft.size(2) == V, "draft_logits must be [B, k, V] with k >= 1");
+    check(draft_ids, at::kLong, "draft_ids"); check(ua, at::kFloat, "ua"); check(us, at::kFloat, "us");
+    TORCH_CHECK(draft_ids.numel() == B * k && ua.numel() == B * k && us.numel() == B * k1, "draft_ids, ua [B, k]; us [B, k+1]");
+    const colinfer_sampler_params p = params_of(B, temperature, top_k, top_p, log_min_p, seed, rep, pres, freq, history, hist_len);
+    int W = 0;
+    if (mask) {
+        check(*mask, at::kInt, "mask");
+        TORCH_CHECK(mask->dim() == 3 && mask->size(0) == B && mask->size(1) == k1 && mask->size(2) >= (V + 31) / 32, "mask [B, k+1, W]");
+        W = (int)mask->size(2);
+    }
+    c10::cuda::CUDAGuard guard(target.device());
+    at::Tensor stats = at::empty({colinfer_spec_verify_stats_bytes((int)B, (int)k)}, target.options().dtype(at::kByte));
+    at::Tensor ids = at::empty({B, k1}, draft_ids.options()), out_tok = at::empty({B, k1}, draft_ids.options());
+    at::Tensor n = at::empty({B}, draft_ids.options().dtype(at::kInt));
+    cuda_ok(colinfer_spec_verify(target.data_ptr(), draft.data_ptr(), dt, W ? mask->data_ptr<int32_t>() : nullptr, W, &p, draft_ids.data_ptr<int64_t>(),
+                                 ua.data_ptr<float>(), us.data_ptr<float>(), out_tok.data_ptr<int64_t>(), n.data_ptr<int32_t>(),
+                                 reinterpret_cast<colinfer_row_stats*>(stats.data_ptr()), ids.data_ptr<int64_t>(), (int)B, (int)k, (int)V, stream()), "spec_verify");
+    return {out_tok, n};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -205,5 +282,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("draw", &draw, "fused penalties + mask + temperature + min-p / top-k / top-p + argmax or seeded draw: one launch");
     m.def("spec_accept", &spec_accept, "exact-match accept, bonus token and stop cut of the speculative cycle");
     m.def("spec_advance", &spec_advance, "the bookkeeping after a cycle, in place on the device");
+    m.def("logprobs", &logprobs, "log-probability of the emitted tokens and of the n_top most likely ones: one launch");
+    m.def("processed_probs", &processed_probs, "renormalised probabilities of one request's rows after the filters");
+    m.def("inverse_cdf", &inverse_cdf, "first token whose cumulative probability reaches u");
+    m.def("spec_verify", &spec_verify, "rejection verify: accepted prefix, then a draw from the residual of target and draft");
     m.def("lowrank_draft", &lowrank_draft, "the greedy draft of the low-rank heads: top candidates, exact rescoring, argmax, probability: one launch");
 }

@@ -15,6 +15,12 @@ MAX_TOP = 32
 def logprobs_tensors(rows: torch.Tensor, toks: torch.Tensor, n_top: int):
     """rows [r, V] fp32 / bf16 raw logits (CUDA, contiguous), toks [r] int64 -> (chosen fp32 [r], top_ids int64
     [r, n_top], top_lp fp32 [r, n_top]) on the device; nothing is synchronised."""
+    ext = _lib.ext()
+    if ext is not None and hasattr(ext, "logprobs"):
+        try:
+            return tuple(ext.logprobs(rows, toks, n_top))
+        except TypeError:                                      # (not tensors: the checks below say which)
+            pass
     if rows.dim() != 2:
         raise RuntimeError("rows [r, V]")
     check_tensor(rows, None, "rows")

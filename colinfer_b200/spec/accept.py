@@ -67,6 +67,12 @@ def processed_probs(logits: torch.Tensor, temperature: torch.Tensor, top_k: torc
     """logits [R, V] fp32 (rows of one request) -> renormalised probabilities [R, V] after the filters.
     temperature / top_k / top_p / log_min_p: 1-element device tensors (the slot's parameters).
     (engine/spec/accept.py:23-33)"""
+    ext = _lib.ext()
+    if ext is not None and hasattr(ext, "processed_probs"):
+        try:
+            return ext.processed_probs(logits, temperature, top_k, top_p, log_min_p)
+        except TypeError:                                      # (not tensors: the checks below say which)
+            pass
     check_tensor(logits, torch.float32, "logits")
     if logits.dim() != 2:
         raise RuntimeError("logits [R, V]")
@@ -87,6 +93,12 @@ def processed_probs(logits: torch.Tensor, temperature: torch.Tensor, top_k: torc
 def inverse_cdf(P: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
     """P [R, V] probabilities, u [R] uniforms in (0, 1] -> [R] int64: the first index whose CDF reaches u
     (never a zero-probability token).  (engine/spec/accept.py:36-40)"""
+    ext = _lib.ext()
+    if ext is not None and hasattr(ext, "inverse_cdf"):
+        try:
+            return ext.inverse_cdf(P, u)
+        except TypeError:                                      # (not tensors: the checks below say which)
+            pass
     check_tensor(P, torch.float32, "P")
     if P.dim() != 2:
         raise RuntimeError("P [R, V]")

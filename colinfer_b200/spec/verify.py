@@ -87,6 +87,15 @@ def spec_verify(target_logits: torch.Tensor, draft_logits: torch.Tensor, draft_i
     uniforms, us [B, k+1] sampling uniforms, mask [B, k+1, W] int32 applied to both models' rows.  Accept draft i iff ua_i * q_i(d_i) <= p_i(d_i); at the first
     rejection emit a draw from normalize(max(p - q, 0)); with no rejection emit a draw from p_k.  temperature <= 0:
     accept while the draft equals the target's argmax.  Returns (out_tok [B, k+1] int64 padded with -1, n [B] int32)."""
+    ext = _lib.ext()
+    if ext is not None and hasattr(ext, "spec_verify"):
+        g = lambda name: getattr(p, name, None)  # noqa: E731
+        try:
+            return tuple(ext.spec_verify(target_logits, draft_logits, draft_ids, p.temperature, p.top_k, p.top_p, p.log_min_p, g("seed"),
+                                         g("repetition_penalty"), g("presence_penalty"), g("frequency_penalty"), g("history"),
+                                         g("hist_len"), ua, us, mask))
+        except TypeError:                                      # (not tensors: the checks below say which)
+            pass
     check_tensor(target_logits, None, "target_logits")
     check_tensor(draft_logits, target_logits.dtype, "draft_logits")
     dt = _dtype_code(target_logits)
