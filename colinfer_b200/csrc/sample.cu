@@ -1535,13 +1535,22 @@ extern "C" int colinfer_max_active_clusters(int V, int dtype) {
 // ---- the chunk kernel (sample_rows.cu: a CTA per row, sample_few.cu: a cluster per row)
 namespace {
 constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024, kMaxDev = 64;
+// More rows than SMs: two CTAs of 512 threads per SM, one of which reads while the other one is in its block-wide steps; or one of
+// 1,024 where two do not fit (penalty tables of large vocabularies: 512 bf16 rows of 262,144 logits with histories 222 -> 174 us),
+// and for bf16 vocabularies beyond 229,376, whose rows have so many equal logits that the lists of 512 threads overflow (512 flat
+// rows of 262,144 with mixed filters 276 -> 249 us; of 201,792 it is 173 against 213).
+constexpr int kTwoPerSm = 113 * 1024, kRowV = 229376;
 
-int chunk_index(bool few, int dtype, bool mask) { return (few ? 4 : 0) + (dtype == COLINFER_F32 ? 0 : 2) + (mask ? 1 : 0); }
-const void* chunk_kernel(int ki) { return ki >= 4 ? colinfer_few_kernel(ki - 4) : colinfer_rows_kernel(ki); }
+// The sets of instantiations: a CTA of 512 threads per row, two per SM (ROWS); a CTA of 1,024 threads per row (ROW); a cluster of
+// CTAs per row (FEW).
+enum { ROWS = 0, FEW = 1, ROW = 2 };
+int chunk_index(int set, int dtype, bool mask) { return 4 * set + (dtype == COLINFER_F32 ? 0 : 2) + (mask ? 1 : 0); }
+const void* chunk_kernel(int ki) { return ki >= 8 ? colinfer_row_kernel(ki - 8) : ki >= 4 ? colinfer_few_kernel(ki - 4) : colinfer_rows_kernel(ki); }
+int chunk_smem(int set, int V, bool pen) { return set == FEW ? colinfer_few_smem(V, pen) : set == ROW ? colinfer_row_smem(V, pen) : colinfer_rows_smem(V, pen); }
 
 // The device's number of SMs, and once per device and kernel the opt-in to large shared memory.
 int chunk_device(int ki, int* dev_out, int* sms_out) {
-    static bool opted[kMaxDev][8] = {};
+    static bool opted[kMaxDev][12] = {};
     static int sms[kMaxDev] = {};
     static std::mutex guard;
     int dev = 0;
@@ -1559,10 +1568,10 @@ int chunk_device(int ki, int* dev_out, int* sms_out) {
     return 0;
 }
 
-void chunk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool few, int cluster, long long groups, int smem, cudaStream_t st) {
+void chunk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int set, int cluster, long long groups, int smem, cudaStream_t st) {
     cfg = cudaLaunchConfig_t{};
     cfg.gridDim = dim3((unsigned)(groups * cluster), 1, 1);
-    cfg.blockDim = dim3((unsigned)(few ? colinfer_few_threads() : colinfer_rows_threads()), 1, 1);
+    cfg.blockDim = dim3((unsigned)(set == FEW ? colinfer_few_threads() : set == ROW ? colinfer_row_threads() : colinfer_rows_threads()), 1, 1);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1570,7 +1579,7 @@ void chunk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool few, 
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = few ? 1 : 0;
+    cfg.numAttrs = set == FEW ? 1 : 0;
 }
 
 // Clusters of `cluster` CTAs that the device holds at once (cached).
@@ -1583,7 +1592,7 @@ int chunk_clusters(int dev, int ki, int cluster, int smem) {
     for (int i = 0; i < used; ++i)
         if (cache[i].dev == dev && cache[i].ki == ki && cache[i].cs == cluster && cache[i].smem == smem) return cache[i].n;
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
-    chunk_config(cfg, attr, true, cluster, 1024, smem, nullptr);
+    chunk_config(cfg, attr, FEW, cluster, 1024, smem, nullptr);
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, chunk_kernel(ki), &cfg) != cudaSuccess || n <= 0) return 0;
     if (used < 64) cache[used++] = Entry{dev, ki, cluster, smem, n};
@@ -1597,26 +1606,31 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
     const long long rows = second.rows;
     if (V > kChunkMaxV || rows > 0x7ffffffeLL) return -1;
     const bool pen = params->history != nullptr;
-    bool few = false;
-    int C = 1, dev = 0, sms = 0;
+    int set = ROWS, C = 1, dev = 0, sms = 0;
     {
-        const int rc = chunk_device(chunk_index(false, dtype, mask != nullptr), &dev, &sms);
+        const int rc = chunk_device(chunk_index(ROWS, dtype, mask != nullptr), &dev, &sms);
         if (rc) return rc;
     }
     if (rows <= sms) {
-        // fewer rows than SMs: a cluster of two or four CTAs per row, where that fills the device
-        const int ki = chunk_index(true, dtype, mask != nullptr), smem = colinfer_few_smem(V, pen);
+        // At most a row per SM, more than the cluster-resident kernel holds at once: a cluster of two or four CTAs per row, where
+        // they all run at once.  64 fp32 rows of 151,936 logits with mixed filters and histories: 62 us, 73 us with the streaming
+        // kernel (a CTA per row, half of the SMs idle).  From 75 rows on there is one CTA per row either way, and the streaming
+        // kernel's 1,024 threads get a row through sooner.
+        const int ki = chunk_index(FEW, dtype, mask != nullptr), smem = colinfer_few_smem(V, pen);
         if (smem > kChunkMaxSmem) return -1;
         const int rc = chunk_device(ki, &dev, &sms);
         if (rc) return rc;
-        for (C = 4; C >= 2 && !few; C /= 2) {
-            few = V >= 16384 * C && rows <= chunk_clusters(dev, ki, C, smem);
-            if (few) break;
+        for (C = 4; C >= 2; C /= 2) {
+            if (V >= 16384 * C && rows <= chunk_clusters(dev, ki, C, smem)) { set = FEW; break; }
         }
-        if (!few) return -1;
-    }
-    const int smem = few ? colinfer_few_smem(V, pen) : colinfer_rows_smem(V, pen);
+        if (set != FEW) return -1;
+    } else if ((dtype == COLINFER_BF16 && V > kRowV) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
+    const int smem = chunk_smem(set, V, pen), ki = chunk_index(set, dtype, mask != nullptr);
     if (smem > kChunkMaxSmem) return -1;
+    {
+        const int rc = chunk_device(ki, &dev, &sms);
+        if (rc) return rc;
+    }
     colinfer_sample_args a;
     a.logits = logits;
     a.mask = mask; a.mask_rows = mask_rows; a.W = W;
@@ -1625,9 +1639,9 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
     a.out = out_ids; a.stats = stats; a.status = status;
     a.B = B; a.R = R; a.V = V; a.flags = flags; a.cluster = C; a.second = second;
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
-    chunk_config(cfg, attr, few, C, rows, smem, stream);
+    chunk_config(cfg, attr, set, C, rows, smem, stream);
     void* args[] = {&a};
-    return (int)cudaLaunchKernelExC(&cfg, chunk_kernel(chunk_index(few, dtype, mask != nullptr)), args);
+    return (int)cudaLaunchKernelExC(&cfg, chunk_kernel(ki), args);
 }
 }  // namespace
 

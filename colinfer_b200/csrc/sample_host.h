@@ -35,6 +35,9 @@ struct colinfer_sample_args {
 const void* colinfer_rows_kernel(int index);   // a CTA per row (sample_rows.cu)
 int colinfer_rows_smem(int V, bool pen);
 int colinfer_rows_threads();
+const void* colinfer_row_kernel(int index);    // a CTA of twice the threads per row (sample_row.cu)
+int colinfer_row_smem(int V, bool pen);
+int colinfer_row_threads();
 const void* colinfer_few_kernel(int index);    // a cluster of CTAs per row (sample_few.cu)
 int colinfer_few_smem(int V, bool pen);
 int colinfer_few_threads();

@@ -822,6 +822,23 @@ static __device__ __noinline__ u64 pass_window(RowS& rw, const NextRow& nx, Mass
     return warp_sum_u64(hi);
 }
 
+// Exact masses of the keys [klo, khi], 2^sh of them a bin, from the largest down.
+template <bool CL, int ELT, bool MASK>
+static __device__ __noinline__ void pass_bracket(RowS& rw, const NextRow& nx, MassFn mass, uint32_t klo, uint32_t khi, int sh, u64* bins) {
+    run_pass<CL, ELT, MASK>(rw, nx, false, 0, THEN_NOTHING, [&](const auto& k) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = k.group(j, CI_NEG_INF);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t f = f2key(x[e]);
+                if (f >= klo && f <= khi) add64(&bins[(khi - f) >> sh], (u64)mass(x[e]));
+            }
+        }
+    });
+}
+
 // The rarer uses of the passes, as functions of their own.
 // The lowest token of the warp's chunks whose logit is L.
 template <bool CL, int ELT, bool MASK>
@@ -1287,7 +1304,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     // The row at a position of that order.  One warp.
     auto row_of = [&](int pos) {
         if (!dealt) return pos;
-        if (n_rows <= 2 * NUM_SM) {
+        if (CTAS_PER_SM == 2 && n_rows <= 2 * NUM_SM) {
             const int pairs = n_rows - NUM_SM;
             pos = pos >= NUM_SM ? n_rows - 1 - (pos - NUM_SM) : pos < pairs ? NUM_SM - pairs + pos : pos - pairs;
         }
@@ -1813,6 +1830,36 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 pivot = key2f(prefix);
                 return true;
             };
+            // The pivot by mass among the logits of [lo, hi], `above` being the mass beyond them: a pass per 256-fold narrowing of
+            // the bracket.  A band of bf16 logits, which may hold thousands of equal ones, has at most 256 values: one pass.
+            // False when the pivot lies elsewhere.
+            auto bracket_select = [&](float lo, float hi, u64 target, u64 above, float& pivot) {
+                uint32_t klo = f2key(lo), khi = f2key(hi);
+                const bool coarse = ELT == 2 && !rw.pen_on;      // every logit is a bf16: one value among any 2^16 neighbouring keys
+                for (int step = 0; step < 5; ++step) {
+                    const uint32_t span = khi - klo;
+                    if (span < (coarse ? 65536u : 1u)) {
+                        uint32_t k = khi;
+                        if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
+                        pivot = key2f(k);
+                        return true;
+                    }
+                    const int sh = max(coarse ? 16 : 0, 24 - __clz(span));       // at most BINS bins
+                    g.sync();
+                    for (int i = tid; i < BINS; i += NT) bins[i] = 0;
+                    __syncthreads();
+                    pass_bracket<CL, ELT, MASK>(rw, nx, rw.mass, klo, khi, sh, bins);
+                    g.sync();
+                    int b; u64 before, tot;
+                    bins_find([&](int i) { u64 t = 0; for (int q = 0; q < (CL ? g.C : 1); ++q) t += g.at(bins, q)[i]; return t; }, BINS, target - above, sc, b, before, tot);
+                    __syncthreads();
+                    if (b < 0) return false;
+                    above += before;
+                    khi -= (uint32_t)b << sh;
+                    klo = max(klo, khi - ((1u << sh) - 1u));
+                }
+                return false;
+            };
             // raises the cut to a pivot (ties at the pivot are kept)
             auto raise_cut = [&](float pivot) {
                 const float cut = fmaxf(rw.lcut, lower_logit_for(scale_logit(pivot, rw.tc), rw.tc, pivot));
@@ -1931,7 +1978,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 }
                 if (ok) break;
                 bool found_band = false;
-                if (attempt == 0 && !over && s1 > 0) {
+                float lpiv;
+                if (s1 > 0 && s_above < target && bracket_select(fmaxf(rw.t_lo, fmaxf(rw.lcut, -SM_FLT_MAX)), fminf(rw.t_hi, rw.L), target, s_above, lpiv)) {
+                    // the band holds the pivot, but more logits than the lists
+                    raise_cut(lpiv);
+                    if (tid == 0) rw.path = PATH_PURE;
+                    found_band = true;
+                } else if (attempt == 0 && s1 > 0) {
                     // The estimated band missed the pivot.  Exact masses of the BINS buckets next to the band, on the side
                     // the pivot lies, give its bucket; the mass pass then runs again around it.
                     const int w0 = target <= s_above ? max(0, rw.band_top - BINS + 1) : max(0, rw.band_bot);
@@ -1958,8 +2011,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     }
                 }
                 if (!found_band) {
-                    // a list overflowed, or the pivot lies far from the estimate: exact radix select by mass
-                    float lpiv;
+                    // the pivot lies far from the estimate: exact radix select by mass
                     if (radix_select(true, lpiv)) raise_cut(lpiv);
                     __syncthreads();
                     if (tid == 0) rw.path = PATH_PURE;
