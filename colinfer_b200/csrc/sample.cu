@@ -48,7 +48,7 @@
 #define CI_WLIST 24              // list entries per warp
 #define CI_GLIST 1365            // gathered list entries (16 KB)
 #define CI_SEL_BINS 256          // coarse bins of the exact selection on a gathered list
-#define CI_FB_NB 256             // radix buckets per level of the fallback select (8 bits)
+#define CI_FB_NB 1024             // radix buckets per level of the fallback select (8 bits)
 #define CI_MAX_CAND 128          // tied / neighbouring candidates examined one by one in the final list step
 #define CI_PEN_TABLE 2048        // distinct history ids per slice with an O(1) count
 #define CI_WAIT_CYCLES 400000000LL
@@ -281,21 +281,27 @@ __device__ __noinline__ bool list_select(const ListEntry* gl, int n, W wt, u64 t
     return ok;
 }
 
-// Exact radix select over the order-preserving 32-bit keys of the logits >= lcut, four levels of 8 bits, across the
-// cluster.  by_mass: the pivot where the descending cumulative mass first reaches top_p of the total; else the kk-th
-// largest.  Returns false when the filter removes nothing (fewer survivors than kk); else pivot holds the pivot logit.
-// Every CTA of the cluster calls it with identical arguments and takes identical decisions.
+// Exact select among the keys [klo, khi] of the row, across the cluster: a pass over the slices per 1,024-fold narrowing of the
+// bracket.  by_mass: where the descending cumulative mass reaches `target` (0: top_p of the bracket's mass); else the target-th
+// largest.  coarse: every logit is a bf16, of which any 2^16 neighbouring keys hold one.  Returns false when the bracket falls
+// short of the target (a top-k that removes nothing); else pivot holds the pivot logit.  Every CTA of the cluster calls it with
+// identical arguments and takes identical decisions.
 struct RadixCtx {
     const float* rowbuf; int n_pad; u64* fb_hist; u64* fb_seg; Xch* xch; Scratch* sc; int rank, CS;
 };
-__device__ bool radix_select(cg::cluster_group& cluster, const RadixCtx& c, const MassFn& mass, float lcut, bool by_mass,
-                             u64 kk, float topp, float& pivot) {
+__device__ __noinline__ bool radix_select(cg::cluster_group& cluster, const RadixCtx& c, const MassFn& mass, uint32_t klo, uint32_t khi,
+                                          bool coarse, bool by_mass, u64 target, float topp, float& pivot) {
     const int tid = threadIdx.x;
-    const float lk = fmaxf(lcut, -CI_FLT_MAX);
-    uint32_t prefix = 0;
-    u64 target = by_mass ? 0 : kk;
-    for (int lvl = 0; lvl < 4; ++lvl) {
-        const int shift = 24 - 8 * lvl;
+    for (int lvl = 0; lvl < 5; ++lvl) {
+        const uint32_t span = khi - klo;
+        if (lvl && span < (coarse ? 65536u : 1u)) {
+            uint32_t k = khi;
+            if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
+            pivot = key2f(k);
+            return true;
+        }
+        const int sh = max(coarse ? 16 : 0, 22 - __clz(span));            // at most CI_FB_NB bins
+        __syncthreads();
         for (int i = tid; i < CI_FB_NB; i += CI_THREADS) c.fb_hist[i] = 0;
         __syncthreads();
         const float4* row4 = reinterpret_cast<const float4*>(c.rowbuf);
@@ -304,12 +310,8 @@ __device__ bool radix_select(cg::cluster_group& cluster, const RadixCtx& c, cons
             const float e4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float l = e4[j];
-                if (l >= lk) {
-                    const uint32_t key = f2key(l);
-                    if (lvl == 0 || (key >> (shift + 8)) == prefix)
-                        add64(&c.fb_hist[CI_FB_NB - 1 - (int)((key >> shift) & 0xFFu)], by_mass ? (u64)mass(l) : 1ull);
-                }
+                const uint32_t key = f2key(e4[j]);
+                if (key >= klo && key <= khi) add64(&c.fb_hist[(khi - key) >> sh], by_mass ? (u64)mass(e4[j]) : 1ull);
             }
         }
         __syncthreads();
@@ -328,11 +330,8 @@ __device__ bool radix_select(cg::cluster_group& cluster, const RadixCtx& c, cons
         cluster.sync();                                                    // reduced segments published
         u64 grand = 0, segtots[8];
         for (int q = 0; q < c.CS; ++q) { segtots[q] = cluster.map_shared_rank(c.xch, q)->fb_segtot; grand += segtots[q]; }
-        if (lvl == 0) {
-            if (by_mass) target = ceil_target(topp, grand);
-            else if (target >= grand) return false;
-        }
-        if (grand == 0) return false;
+        if (lvl == 0 && target == 0) target = ceil_target(topp, grand);
+        if (grand == 0 || target > grand || (!by_mass && lvl == 0 && target >= grand)) { cluster.sync(); return false; }
         int s_star = c.CS - 1; u64 before_seg = 0, run = 0;
         for (int q = 0; q < c.CS; ++q) {
             if (run + segtots[q] >= target) { s_star = q; before_seg = run; break; }
@@ -342,10 +341,11 @@ __device__ bool radix_select(cg::cluster_group& cluster, const RadixCtx& c, cons
         int g_star; u64 before;
         block_find([&](int i) { return pseg[i]; }, G, target - before_seg, c.sc, g_star, before);
         target -= before_seg + before;
-        prefix = (prefix << 8) | (uint32_t)(CI_FB_NB - 1 - (s_star * G + g_star));
+        khi -= (uint32_t)(s_star * G + g_star) << sh;
+        klo = max(klo, khi - ((1u << sh) - 1u));
+        cluster.sync();                                                    // (the segments have been read)
     }
-    pivot = key2f(prefix);
-    return true;
+    return false;
 }
 
 // Gathers the per-warp lists of every CTA of the cluster into glist, in token order (CTA rank, warp, position).
@@ -1083,6 +1083,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     const bool need_topp = topp < 1.0f;
 
     // (generic path from here on: the whole cluster works on the row until its token is out)
+    const bool coarse = a.dtype == COLINFER_BF16 && !has_pen;   // every logit is a bf16
     enum { PATH_PURE = 0, PATH_LIST = 1, PATH_BAND = 2, PATH_FALLBACK = 3 };
     int path = PATH_PURE;
     float t_hi = CI_NEG_INF, t_lo = CI_POS_INF;                 // band thresholds (PATH_BAND), list threshold (PATH_LIST: t_lo)
@@ -1227,9 +1228,9 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         // reads precede the peers' next cluster barrier, and the first write below follows this CTA's next barrier)
         const RadixCtx rc = {rowbuf, n_pad, fb_hist, fb_seg, xch, sc, rank, CS};
         float lpiv;
-        if (kk > 0 && kk < V && radix_select(cluster, rc, mass, lcut, false, (u64)kk, topp, lpiv))
+        if (kk > 0 && kk < V && radix_select(cluster, rc, mass, f2key(fmaxf(lcut, -CI_FLT_MAX)), f2key(L), coarse, false, (u64)kk, topp, lpiv))
             lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
-        if (need_topp && radix_select(cluster, rc, mass, lcut, true, 0, topp, lpiv))
+        if (need_topp && radix_select(cluster, rc, mass, f2key(fmaxf(lcut, -CI_FLT_MAX)), f2key(L), coarse, true, 0, topp, lpiv))
             lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
         path = PATH_PURE;
         t_hi = CI_NEG_INF; t_lo = CI_POS_INF;
@@ -1325,7 +1326,14 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 // by mass, then recomputes its regions' kept mass.  Rare; same result, more time.
                 const RadixCtx rc = {rowbuf, n_pad, fb_hist, fb_seg, xch, sc, rank, CS};
                 float lpiv;
-                if (radix_select(cluster, rc, mass, lcut, true, 0, topp, lpiv))
+                uint32_t klo = f2key(fmaxf(lcut, -CI_FLT_MAX)), khi = f2key(L);
+                u64 want = 0;
+                if (s1 > 0) {                                                  // on which side of the band's upper edge it lies is known
+                    want = ceil_target(topp, s1);
+                    if (want <= s_above) klo = f2key(t_hi) + 1u;
+                    else { khi = min(khi, f2key(t_hi)); want -= s_above; }
+                }
+                if (radix_select(cluster, rc, mass, klo, khi, coarse, true, want, topp, lpiv))
                     lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
                 const float lk3 = fmaxf(lcut, -CI_FLT_MAX);
                 u64 acc = 0;
@@ -1646,6 +1654,7 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
 }  // namespace
 
 // Both sets of rows (colinfer_second_rows), or -1 where only separate launches take them (nothing is launched then).
+static const int kMinSlice = 4096;
 static int sample_rows(const void* logits, const void* logits2, int dtype, const int32_t* mask, int mask_rows, int W,
                        const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u,
                        int64_t* out_ids, colinfer_row_stats* stats, int32_t* status,
@@ -1670,14 +1679,17 @@ static int sample_rows(const void* logits, const void* logits2, int dtype, const
     // fit the streaming kernel.
     const int choice = (flags >> 8) & 7;                   // 0 auto, 1 streaming, 2 .. 5: clusters of 1, 2, 4, 8
     if (choice > 5) return (int)cudaErrorInvalidValue;
-    const int forced = choice >= 2 ? (1 << (choice - 2)) : 0;
+    int forced = choice >= 2 ? (1 << (choice - 2)) : 0;
     if (choice <= 1) {
         bool use_stream = true;
         if (choice == 0) {
-            colinfer_geometry g0;
-            if (!pick_geometry(V, dtype, logits, 0, &g0)) {
+            // the widest cluster of which the device holds as many as there are rows, and whose CTAs have a few thousand logits
+            // each (17 fp32 rows of 151,936 logits with mixed filters: clusters of four 36 us, of eight, in two turns, 46 us)
+            for (int c = 8; c >= 1 && use_stream; c /= 2) {
+                colinfer_geometry g0;
+                if ((c > 1 ? V < kMinSlice * c : V >= 4 * kMinSlice) || pick_geometry(V, dtype, logits, c, &g0)) continue;
                 const int res0 = active_clusters(g0);
-                if (res0 > 0 && rows <= res0) use_stream = false;
+                if (res0 > 0 && rows <= res0) { use_stream = false; forced = c; }
             }
         }
         if (use_stream && choice == 0) {
