@@ -38,6 +38,8 @@ struct Sc {
     int overflow;
     uint32_t fc_idx[FCAP]; float fc_l[FCAP];
     float sel_l; int sel_i;          // slow path: the previous pick
+    float cm[8], cs[8];              // a cluster's first CTA: every CTA's (maximum, sum),
+    uint32_t ct_idx[8 * MAX_TOP]; float ct_l[8 * MAX_TOP];   // and its slice's top n_top, in order
 };
 
 struct Row {
@@ -104,21 +106,27 @@ struct Args {
 
 // LOADER: 1 = fp32 rows that take 128-bit loads, 2 = bf16 rows that take 64-bit loads of four logits, 0 = the general
 // loader (unaligned rows, vocabularies that are not a multiple of 4).
-template <int LOADER>
+// CL: a cluster shares a row, a slice each; every CTA takes its slice's log-sum-exp and top n_top, the first one merges them.
+template <int LOADER, bool CL>
 __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_constant__ Args a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int V = a.V, n_top = a.n_top;
     __shared__ __align__(16) uint32_t hist[BINS];
     __shared__ Cand ownlist[NW * WLIST];
     __shared__ Sc sc;
-    const int reg = (((V + 127) / 128 + NW - 1) / NW) * 128;
-    const int r_lo = min(warp * reg, V), r_hi = min(r_lo + reg, V);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = CL ? (int)cluster.num_blocks() : 1, crank = CL ? (int)cluster.block_rank() : 0;
+    if (CL) cluster.barrier_arrive();                               // (waited for before the first write into a peer)
+    bool running = false;
+    // the row's groups of 128 logits, dealt evenly: a warp has a run of consecutive ones
+    const int groups = (V + 127) / 128, part = crank * NW + warp;
+    const int r_lo = min((int)((long long)groups * part / (C * NW)) * 128, V), r_hi = min((int)((long long)groups * (part + 1) / (C * NW)) * 128, V);
     Cand* mylist = ownlist + warp * WLIST;
     if (tid >= NW && tid < 32) {                                    // neutral entries for the warps this CTA does not have
         sc.wm[tid] = CI_NEG_INF; sc.ws[tid] = 0.0f; sc.wf[tid] = CI_NEG_INF; sc.wcount[tid] = -1;
     }
 
-    for (int row = blockIdx.x; row < a.rows; row += gridDim.x) {
+    for (int row = blockIdx.x / C; row < a.rows; row += gridDim.x / C) {
         __syncthreads();
         Row rw;
         rw.V = V; rw.vec = LOADER == 1; rw.vec16 = LOADER == 2;
@@ -234,6 +242,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
         }
         if (lane == 0) { sc.wm[warp] = m; sc.ws[warp] = s; }
         for (int i = tid; i < BINS; i += NT) hist[i] = 0u;
+        if (lane == 0) sc.wcount[warp] = wn;
         const int over = __syncthreads_or(wn > WLIST);
         float M = sc.wm[lane], S = sc.ws[lane];
 #pragma unroll
@@ -241,16 +250,42 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
             const float m2 = __shfl_xor_sync(0xffffffffu, M, o), s2 = __shfl_xor_sync(0xffffffffu, S, o);
             lse_merge(M, S, m2, s2);
         }
-        const float lse = M + logf(S);                              // -inf + log(0) = NaN for a row without finite logits
-        if (tid == 0 && a.chosen) {
+        // (of a slice with nothing in it 0: only the merged value counts)
+        const float lse = CL ? 0.0f : M + logf(S);                              // -inf + log(0) = NaN for a row without finite logits
+        auto put = [&](int rank, uint32_t idx, float l) {           // the slice's alternative of that rank
+            if (CL) { Sc* first = cluster.map_shared_rank(&sc, 0); first->ct_idx[crank * MAX_TOP + rank] = idx; first->ct_l[crank * MAX_TOP + rank] = l; }
+            else { a.top_ids[(size_t)row * n_top + rank] = idx == 0xFFFFFFFFu ? -1ll : (long long)idx; a.top_lp[(size_t)row * n_top + rank] = l - lse; }
+        };
+        if (CL) {
+            if (!running) { cluster.barrier_wait(); running = true; }
+            if (tid == 0) { Sc* first = cluster.map_shared_rank(&sc, 0); first->cm[crank] = M; first->cs[crank] = S; }
+        } else if (tid == 0 && a.chosen) {
             const long long t = a.toks ? a.toks[row] : -1;
             a.chosen[row] = (t >= 0 && t < V) ? rw.at((int)t) - lse : __int_as_float(0x7fc00000);
         }
-        if (n_top <= 0) continue;
+        if (!CL && n_top <= 0) continue;
 
         // ------------------------------------------------------------------------------------ the top n_top
-        bool done = false;
-        if (!over && tw > -LP_FLT_MAX && tw <= M) {
+        bool done = n_top <= 0;
+        const bool usable = !done && !over && tw > -LP_FLT_MAX && tw <= M;
+        const int listed = __reduce_add_sync(0xffffffffu, lane < NW ? sc.wcount[lane] : 0);
+        if (usable && listed >= n_top && listed <= FCAP) {
+            // few enough to be ranked as they are: every one against all others, four threads each
+            const int off = __reduce_add_sync(0xffffffffu, lane < warp ? sc.wcount[lane] : 0);
+            for (int j = lane; j < wn; j += 32) { sc.fc_idx[off + j] = mylist[j].idx; sc.fc_l[off + j] = mylist[j].l; }
+            __syncthreads();
+            const int c = tid / 4;
+            int rank = 0;
+            if (c < listed) {
+                const float lc = sc.fc_l[c]; const uint32_t ic = sc.fc_idx[c];
+                for (int o = tid & 3; o < listed; o += 4) rank += before(sc.fc_l[o], sc.fc_idx[o], lc, ic) ? 1 : 0;
+            }
+            rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+            rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+            if (c < listed && (tid & 3) == 0 && rank < n_top) put(rank, sc.fc_idx[c], sc.fc_l[c]);
+            done = true;
+        } else if (usable) {
+            __syncthreads();                                        // (the counts have been read)
             const float scale = M > tw ? (float)(BINS - 2) / (M - tw) : 0.0f;
             auto bin_of = [&](float l) { return min(BINS - 1, __float2int_rz((M - l) * scale)); };
             for (int j = lane; j < wn; j += 32) atomicAdd(&hist[bin_of(mylist[j].l)], 1u);
@@ -295,8 +330,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
                     rank += __shfl_xor_sync(0xffffffffu, rank, 2);
                     if (TPC == 8) rank += __shfl_xor_sync(0xffffffffu, rank, 4);
                     if (part == 0 && c < (int)nc && rank < n_top) {
-                        a.top_ids[(size_t)row * n_top + rank] = (long long)sc.fc_idx[c];
-                        a.top_lp[(size_t)row * n_top + rank] = sc.fc_l[c] - lse;
+                        put(rank, sc.fc_idx[c], sc.fc_l[c]);
                     }
                 }
                 done = true;
@@ -309,7 +343,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
             __syncthreads();
             for (int r = 0; r < n_top; ++r) {
                 const float pl = sc.sel_l; const uint32_t pi = (uint32_t)sc.sel_i;
-                const bool first = sc.sel_i < 0;
+                const bool first = sc.sel_i == -1, none = sc.sel_i == -2;   // none: the slice has no further logits
                 float bl = CI_NEG_INF; uint32_t bi = 0xFFFFFFFFu;
                 for (int i0 = r_lo; i0 < r_hi; i0 += 128) {
                     const int i = i0 + lane * 4;
@@ -318,7 +352,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const uint32_t id = (uint32_t)(i + j);
-                        if (i + j < V && (first || before(pl, pi, e4[j], id)) && (bi == 0xFFFFFFFFu || before(e4[j], id, bl, bi))) { bl = e4[j]; bi = id; }
+                        if (i + j < V && !none && (first || before(pl, pi, e4[j], id)) && (bi == 0xFFFFFFFFu || before(e4[j], id, bl, bi))) { bl = e4[j]; bi = id; }
                     }
                 }
 #pragma unroll
@@ -339,15 +373,46 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_logprobs(const __grid_const
                         if (oi != 0xFFFFFFFFu && (ci == 0xFFFFFFFFu || before(ol, oi, cl, ci))) { cl = ol; ci = oi; }
                     }
                     if (lane == 0) {
-                        sc.sel_l = cl; sc.sel_i = (int)ci;
-                        a.top_ids[(size_t)row * n_top + r] = ci == 0xFFFFFFFFu ? -1ll : (long long)ci;
-                        a.top_lp[(size_t)row * n_top + r] = cl - lse;
+                        sc.sel_l = cl; sc.sel_i = ci == 0xFFFFFFFFu ? -2 : (int)ci;
+                        put(r, ci, cl);
                     }
                 }
                 __syncthreads();
             }
         }
+        if (CL) {
+            // ------------------------------------------------------------------------------------ the first CTA merges
+            cluster.sync();
+            if (crank == 0) {
+                M = sc.cm[0]; S = sc.cs[0];
+                for (int q = 1; q < C; ++q) lse_merge(M, S, sc.cm[q], sc.cs[q]);
+                const float all = M + logf(S);
+                if (tid == 0 && a.chosen) {
+                    const long long t = a.toks ? a.toks[row] : -1;
+                    a.chosen[row] = (t >= 0 && t < V) ? rw.at((int)t) - all : __int_as_float(0x7fc00000);
+                }
+                // two threads per candidate count those before it
+                const int e = tid >> 1, q = e / MAX_TOP, j = e % MAX_TOP;
+                int rank = 0;
+                const bool is = q < C && j < n_top;
+                if (is) {
+                    const float l = sc.ct_l[e]; const uint32_t x = sc.ct_idx[e];
+                    for (int o = tid & 1; o < C * n_top; o += 2) {
+                        const int f = (o / n_top) * MAX_TOP + o % n_top;
+                        if (f != e && (before(sc.ct_l[f], sc.ct_idx[f], l, x) || (f < e && sc.ct_l[f] == l && sc.ct_idx[f] == x))) ++rank;
+                    }
+                }
+                rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+                if (is && !(tid & 1) && rank < n_top) {
+                    const uint32_t x = sc.ct_idx[e];
+                    a.top_ids[(size_t)row * n_top + rank] = x == 0xFFFFFFFFu ? -1ll : (long long)x;
+                    a.top_lp[(size_t)row * n_top + rank] = sc.ct_l[e] - all;
+                }
+            }
+            cluster.sync();
+        }
     }
+    if (CL && !running) cluster.barrier_wait();
 }
 
 }  // namespace lpk
@@ -380,10 +445,31 @@ extern "C" int colinfer_logprobs(const void* logits, int dtype, const int64_t* t
     a.toks = toks; a.n_top = n_top; a.chosen = chosen; a.top_ids = top_ids; a.top_lp = top_lp;
     a.rows = rows; a.V = V;
     const int slots = sm_count[dev] * lpk::CTAS_PER_SM;
-    const int grid = rows < slots ? rows : slots;
     const bool vec16 = dtype == COLINFER_BF16 && (V % 4) == 0 && (((uintptr_t)logits) & 7) == 0;
-    if (a.vec) lpk::k_logprobs<1><<<grid, lpk::NT, 0, (cudaStream_t)stream>>>(a);
-    else if (vec16) lpk::k_logprobs<2><<<grid, lpk::NT, 0, (cudaStream_t)stream>>>(a);
-    else lpk::k_logprobs<0><<<grid, lpk::NT, 0, (cudaStream_t)stream>>>(a);
+    const int loader = a.vec ? 1 : vec16 ? 2 : 0;
+    // Fewer rows than half the CTAs the device holds (three quarters of them, as clusters): a cluster of 8, 4 or 2 shares a row, as far as its slices have a batch for
+    // every warp or so (one row of 151,936 logits took 29 us in one CTA).
+    int C = 8;
+    while (C > 1 && ((long long)rows * C > slots * 3 / 4 || V < 4096 * C)) C /= 2;
+    if (C > 1) {
+        const void* const kernels[3] = {(const void*)lpk::k_logprobs<0, true>, (const void*)lpk::k_logprobs<1, true>, (const void*)lpk::k_logprobs<2, true>};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(rows * C), 1, 1);
+        cfg.blockDim = dim3(lpk::NT, 1, 1);
+        cfg.stream = (cudaStream_t)stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)C;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        void* args[] = {&a};
+        return (int)cudaLaunchKernelExC(&cfg, kernels[loader], args);
+    }
+    const int grid = rows < slots ? rows : slots;
+    if (loader == 1) lpk::k_logprobs<1, false><<<grid, lpk::NT, 0, (cudaStream_t)stream>>>(a);
+    else if (loader == 2) lpk::k_logprobs<2, false><<<grid, lpk::NT, 0, (cudaStream_t)stream>>>(a);
+    else lpk::k_logprobs<0, false><<<grid, lpk::NT, 0, (cudaStream_t)stream>>>(a);
     return (int)cudaGetLastError();
 }

@@ -359,7 +359,7 @@ extern "C" int colinfer_spec_advance(const int64_t* out_tok, const int32_t* n, i
 // ------------------------------------------------------------------------------------------------ spec_verify (rejection)
 // Finish: per slot, decide the accepted prefix from the row statistics of the target and draft rows, then, at a
 // rejection, stream the two rows of that position once to draw from the residual max(p - q, 0).
-#define VF_THREADS 512
+#define VF_THREADS 1024
 #define VF_WARPS (VF_THREADS / 32)
 #define VF_CTAS 8                      // CTAs (a cluster) per slot
 #define VF_MAX_V 524288
@@ -436,16 +436,25 @@ __device__ double token_prob(const colinfer_row_stats& st, float l, long long to
 }
 // residual mass of one token in units of 2^-40 (fp32 arithmetic, integer result: order-independent sums)
 struct Residual {
-    colinfer_row_stats st, sd; float mt, md, inv_t, inv_d;
+    colinfer_row_stats st, sd; float mt, md, inv_t, inv_d, rt, rd; bool fast;
     __device__ void init(const colinfer_row_stats& st_, const colinfer_row_stats& sd_) {
         st = st_; sd = sd_;
         mt = scale_logit(st.lmax, st.tc); md = scale_logit(sd.lmax, sd.tc);
+        // (the two-step division of MassFn: the IEEE quotient unless the divisor's significand is all ones)
+        rt = __frcp_rn(st.tc); rd = __frcp_rn(sd.tc);
+        fast = (__float_as_uint(st.tc) & 0x7FFFFFu) != 0x7FFFFFu && (__float_as_uint(sd.tc) & 0x7FFFFFu) != 0x7FFFFFu;
         inv_t = (float)(1.0 / ((double)st.mass_q * CI_MASS_INV)); inv_d = (float)(1.0 / ((double)sd.mass_q * CI_MASS_INV));
     }
+    __device__ __forceinline__ float div(float l, float tc, float r) const {
+        if (!fast || !(fabsf(l) < 1e30f) || fabsf(l) < 1e-30f) return scale_logit(l, tc);
+        const float q0 = l * r;
+        return fmaf(fmaf(-q0, tc, l), r, q0);
+    }
     __device__ __forceinline__ u64 operator()(float lt, float ld) const {
-        float p = 0.0f, q = 0.0f;
-        if (lt >= st.lcut && lt > CI_NEG_INF) p = exp2f((scale_logit(lt, st.tc) - mt) * CI_LOG2E) * inv_t;
-        if (ld >= sd.lcut && ld > CI_NEG_INF) q = exp2f((scale_logit(ld, sd.tc) - md) * CI_LOG2E) * inv_d;
+        if (!(lt >= st.lcut && lt > CI_NEG_INF)) return 0ull;          // no target probability: no residual
+        float q = 0.0f;
+        const float p = exp2f((div(lt, st.tc, rt) - mt) * CI_LOG2E) * inv_t;
+        if (ld >= sd.lcut && ld > CI_NEG_INF) q = exp2f((div(ld, sd.tc, rd) - md) * CI_LOG2E) * inv_d;
         const float rres = p - q;
         return rres > 0.0f ? __float2ull_rn(rres * 1099511627776.0f) : 0ull;   // units of 2^-40
     }

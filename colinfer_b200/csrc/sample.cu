@@ -35,6 +35,7 @@
 #define CI_CHUNK 4096            // elements per bulk copy
 #define CI_MAX_CHUNKS 16
 #define CI_NB1 4096              // fine buckets over the distance from the row maximum
+#define CI_TOP 2.0f              // logits up to CI_TOP * temperature below the maximum correct a row's estimated mass
 #define CI_RANGE 25.0f           // the buckets cover distances up to CI_RANGE * temperature
 #define CI_FASTK 100             // largest top_k handled by the per-slice candidate lists
 #define CI_FAST_BINS 512         // bins of the thread-maxima histogram and of the exact finish
@@ -45,7 +46,7 @@
 #define CI_FIN_KEEP 128          // candidates that may be left after top-k
 #define CI_FIN_CAND 64           // candidates of one bin examined pairwise
 #define CI_RETRY 8               // rows a CTA may set aside for the generic path before the fast path is switched off
-#define CI_WLIST 24              // list entries per warp
+#define CI_WLIST 48              // list entries per warp
 #define CI_GLIST 1365            // gathered list entries (16 KB)
 #define CI_SEL_BINS 256          // coarse bins of the exact selection on a gathered list
 #define CI_FB_NB 1024             // radix buckets per level of the fallback select (8 bits)
@@ -108,6 +109,7 @@ struct Scratch {
     int n_retry_common, n_retry_mine, any_retry, want_fast_off;   // any_retry: a CTA of the cluster has set a row aside
     int retry_common[CI_RETRY], retry_mine[CI_RETRY], retry_all[CI_RETRY * 9];
     long long prof[12];            // profiling hook: cycles per phase, summed over the CTA's rows
+    u64 seg_off[8];                // ... and what the estimates are off by on the largest logits
     u64 seg_cnt[8], seg_est[8];    // totals of every CTA's reduced bucket segment, written by the peers: counts, estimated mass
     u64 all_in[8], above_in[8];    // band pass: kept mass of every CTA's slice, and of its part above the band, written by the peers
     int bcast_i[2];                // written by the cluster's first CTA, per row parity
@@ -1094,6 +1096,10 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         const float lk = fmaxf(lcut, -CI_FLT_MAX);             // excludes -inf (masked / padding) as well
         for (int i = tid; i < CI_NB1; i += CI_THREADS) hist1[i] = 0u;
         if (tid == 0) xch->list_overflow = 0;
+        const bool exact_top = need_topp && !need_topk;
+        float* toplist = reinterpret_cast<float*>(ownlist);
+        const float t_top = fmaxf(L - CI_TOP * tc, lk);
+        if (tid == 0) sc->ncand = 0;
         __syncthreads();
         {
             const float4* row4 = reinterpret_cast<const float4*>(rowbuf);
@@ -1112,6 +1118,18 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                     bkt[j] = min(CI_NB1 - 1, __float_as_int(__fadd_rz((L - e[j]) * SC, 8388608.0f)) - 0x4B000000);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) if (e[j] >= lk) atomicAdd(&hist1[bkt[j]], 1u);
+                // The largest logits are noted: what their buckets' estimates are off by is worked out below.  (They make up most
+                // of a peaked row's mass, and a band that misses the pivot costs two more passes and a select.)
+                if (exact_top) {
+                    float top = e[0];
+#pragma unroll
+                    for (int j = 1; j < 16; ++j) top = fmaxf(top, e[j]);
+                    if (top >= t_top) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (e[j] >= t_top) { const int at = atomicAdd(&sc->ncand, 1); if (at < CI_THREADS) toplist[at] = e[j]; }
+                    }
+                }
             }
         }
         __syncthreads();
@@ -1138,17 +1156,29 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         }
         pc = warp_sum_u64(pc); pe = warp_sum_u64(pe);
         if (lane == 0) { sc->warp_tot[warp] = pc; sc->warp_aux[warp] = pe; }
+        if (exact_top) {
+            long long off = 0;
+            if (tid < sc->ncand) {
+                const float x = toplist[tid];
+                off = (long long)mass(x) - (long long)bucket_mass_est(min(CI_NB1 - 1, __float_as_int(__fadd_rz((L - x) * SC, 8388608.0f)) - 0x4B000000));
+            }
+            const u64 o = warp_sum_u64((u64)off);
+            if (lane == 0) sc->wsum[warp] = o;
+        }
         __syncthreads();
         if (warp == 0) {
             pc = warp_sum_u64(lane < CI_WARPS ? sc->warp_tot[lane] : 0ull); pe = warp_sum_u64(lane < CI_WARPS ? sc->warp_aux[lane] : 0ull);
-            if (lane < CS) { Scratch* ps = cluster.map_shared_rank(sc, lane); ps->seg_cnt[rank] = pc; ps->seg_est[rank] = pe; }
+            const u64 po = exact_top ? warp_sum_u64(lane < CI_WARPS ? sc->wsum[lane] : 0ull) : 0ull;
+            if (lane < CS) { Scratch* ps = cluster.map_shared_rank(sc, lane); ps->seg_cnt[rank] = pc; ps->seg_est[rank] = pe; ps->seg_off[rank] = po; }
         }
         cluster.sync();                                                                // (B) reduced segments published
         u64 segc[8], sege[8], survivors = 0, est_total = 0;
+        long long off_total = 0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             segc[q] = q < CS ? sc->seg_cnt[q] : 0ull; sege[q] = q < CS ? sc->seg_est[q] : 0ull;
             survivors += segc[q]; est_total += sege[q];
+            off_total += q < CS ? (long long)sc->seg_off[q] : 0ll;
         }
         if (need_topk && (u64)kk >= survivors) need_topk = false;   // fewer survivors than k: top-k removes nothing
         if (need_topk) {
@@ -1177,7 +1207,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
             // bucket where the descending cumulative estimated mass reaches top_p of the estimated total
             if (est_total == 0) path = PATH_FALLBACK;
             else {
-                const u64 target = ceil_target(topp, est_total);
+                const long long t_off = (long long)est_total + off_total > 0 ? (long long)ceil_target(topp, (u64)((long long)est_total + off_total)) - off_total : 1;
+                const u64 target = t_off < 1 ? 1ull : min((u64)t_off, est_total);
                 int s_star = CS - 1; u64 before_seg = 0, run = 0;
 #pragma unroll
                 for (int q = 7; q >= 0; --q) if (q < CS) {
