@@ -601,6 +601,34 @@ static cudaError_t opt_in() {
     return e;
 }
 
+static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int G, int N, size_t smem, cudaStream_t st) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(G, N); cfg.blockDim = dim3(NT); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = G; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+}
+
+// Clusters of G CTAs that the current device holds at once (cached).
+static int active_clusters(bool fp4, int G, size_t smem) {
+    struct Entry { int dev, fp4, G; size_t smem; int n; };
+    static Entry cache[64];
+    static int used = 0;
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < used; ++i)
+        if (cache[i].dev == dev && cache[i].fp4 == (int)fp4 && cache[i].G == G && cache[i].smem == smem) return cache[i].n;
+    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+    cluster_config(cfg, attr, G, 256, smem, nullptr);
+    int n = 0;
+    const cudaError_t e = fp4 ? cudaOccupancyMaxActiveClusters(&n, k_draft_pick<true, true>, &cfg) : cudaOccupancyMaxActiveClusters(&n, k_draft_pick<false, true>, &cfg);
+    if (e != cudaSuccess) return 0;
+    if (used < 64) cache[used++] = Entry{dev, (int)fp4, G, smem, n};
+    return n;
+}
+
 }  // namespace dpk
 
 extern "C" int64_t colinfer_draft_pick_scratch_bytes(int N) {
@@ -621,28 +649,33 @@ extern "C" int colinfer_draft_pick(const float* ap, const void* x, const void* w
     if (!ap || !x || !w || !out_ids || !scratch || (fp4 && !sf) || N > 65535 || (((uintptr_t)x) & 15) || (((uintptr_t)w) & 15) ||
         (((uintptr_t)scratch) & 15) || scratch_bytes < colinfer_draft_pick_scratch_bytes(N))
         return (int)cudaErrorInvalidValue;
-    // CTAs per slot: as many as fill the part once when slots are few.  4 or 8 of them share the reading of the row as a
-    // cluster when the row allows it (128-bit loads, a share that fits the registers); otherwise every CTA reads all of it.
-    const int G = ctas_per_slot ? ctas_per_slot : N <= 9 ? 8 : N <= 37 ? 4 : N <= 74 ? 2 : 1;
-    const bool split = (G == 4 || G == 8) && (Vd & 3) == 0 && (((uintptr_t)ap) & 15) == 0 &&
-                       ((Vd >> 2) + G * dpk::NT - 1) / (G * dpk::NT) <= dpk::RMAX;
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e = dpk::opt_in();
+    if (e != cudaSuccess) return (int)e;
+    const size_t smem = dpk::SMEM_FIXED + (size_t)K * 2;
+    // 4 or 8 CTAs of a slot share the reading of the row as a cluster when the row allows it (128-bit loads, a share that fits the
+    // registers); otherwise every CTA reads all of it.
+    auto splits = [&](int g) {
+        return (g == 4 || g == 8) && (Vd & 3) == 0 && (((uintptr_t)ap) & 15) == 0 && ((Vd >> 2) + g * dpk::NT - 1) / (g * dpk::NT) <= dpk::RMAX;
+    };
+    // CTAs per slot: the most with which all slots run at once.  (12 slots of 69,632: clusters of eight 27 us, of four 31 us; 37
+    // slots: clusters of four, a second turn of which is needed, 55 us, two CTAs each 52 us.)
+    int G = ctas_per_slot;
+    if (!G) {
+        G = N <= 9 ? 8 : N <= 37 ? 4 : N <= 74 ? 2 : 1;
+        if (splits(8) && N <= dpk::active_clusters(fp4, 8, smem)) G = 8;
+        else if (splits(4)) G = N <= dpk::active_clusters(fp4, 4, smem) ? 4 : N <= 74 ? 2 : 1;
+    }
+    const bool split = splits(G);
     dpk::Args a;
     a.ap = ap; a.x = (const __nv_bfloat16*)x; a.w = w; a.sf = (const uint8_t*)sf; a.gs = gs; a.vocab_ids = vocab_ids;
     a.out_ids = out_ids; a.out_p = out_p; a.out_idx = out_idx; a.out_ex = out_ex;
     a.partials = reinterpret_cast<dpk::Partial*>(scratch);
     a.counters = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(scratch) + (size_t)N * 16 * sizeof(dpk::Partial));
     a.Vd = Vd; a.K = K; a.NC = NC; a.G = G; a.rows_w = (long long)rows_w;
-    cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = dpk::opt_in();
-    if (e != cudaSuccess) return (int)e;
-    const size_t smem = dpk::SMEM_FIXED + (size_t)K * 2;
     if (split) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(G, N); cfg.blockDim = dim3(dpk::NT); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = G; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr; cfg.numAttrs = 1;
+        cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+        dpk::cluster_config(cfg, attr, G, N, smem, st);
         e = fp4 ? cudaLaunchKernelEx(&cfg, dpk::k_draft_pick<true, true>, a) : cudaLaunchKernelEx(&cfg, dpk::k_draft_pick<false, true>, a);
         return (int)(e != cudaSuccess ? e : cudaGetLastError());
     }

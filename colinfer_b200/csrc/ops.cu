@@ -263,40 +263,49 @@ extern "C" int colinfer_inverse_cdf(const float* P, const float* u, int64_t* out
 
 // ------------------------------------------------------------------------------------------------ spec_accept
 // The accept / bonus / stop-cut lines of the reference's speculative cycle (engine/spec/mtp.py:406-415, 422-423),
-// one thread per slot instead of ~20 tiny launches.
+// a warp per slot instead of ~20 tiny launches: the lanes take a position each, so that the comparisons of a slot cost one round
+// trip to memory and not one after the other.
 __global__ void k_spec_accept(const int64_t* __restrict__ pred, const int64_t* __restrict__ tok,
                               const int64_t* __restrict__ stop_ids, const int32_t* __restrict__ active,
                               int64_t* __restrict__ out_tok, int32_t* __restrict__ n_out, int B, int k1, int S) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b >= B) return;
     const int k = k1 - 1;
     const int64_t* pr = pred + (size_t)b * k1;
     const int64_t* d = tok + (size_t)b * k1 + 1;
-    int n = 1;
-    while (n - 1 < k && pr[n - 1] == d[n - 1]) ++n;
-    int64_t bonus = pr[n - 1];
-    if (stop_ids != nullptr) {
-        const int64_t* st = stop_ids + (size_t)b * S;
-        bool cut = false;
-        for (int i = 0; i < n - 1 && i < k && !cut; ++i) {
-            for (int s = 0; s < S; ++s) {
-                if (d[i] == st[s]) { n = i + 1; bonus = d[i]; cut = true; break; }
-            }
-        }
-    }
-    if (active != nullptr) n *= active[b];
+    const int64_t* st = stop_ids != nullptr ? stop_ids + (size_t)b * S : nullptr;
     int64_t* o = out_tok + (size_t)b * k1;
-    for (int i = 0; i < k; ++i) o[i] = d[i];
-    o[k] = bonus;
-    if (n >= 1) o[n - 1] = bonus;
-    n_out[b] = n;
+    const int act = active != nullptr ? active[b] : 1;
+    // the drafts that match, up to the first that does not; the first of them that is a stop token
+    int n = k + 1, cut = -1;
+    for (int i0 = 0; i0 < k; i0 += 32) {
+        const int i = i0 + lane;
+        const int64_t di = i < k ? d[i] : 0;
+        const unsigned miss = __ballot_sync(0xffffffffu, i < k && pr[i] != di);
+        bool stops = false;
+        if (st != nullptr && i < k) for (int s = 0; s < S; ++s) stops |= di == st[s];
+        const int m = miss ? __ffs(miss) - 1 : 32;
+        const unsigned hit = __ballot_sync(0xffffffffu, stops) & (m < 32 ? (1u << m) - 1u : 0xFFFFFFFFu);
+        if (hit) { cut = i0 + __ffs(hit) - 1; break; }
+        if (miss) { n = i0 + m + 1; break; }
+    }
+    if (cut >= 0) n = cut + 1;
+    const int64_t bonus = cut >= 0 ? d[cut] : pr[n - 1];
+    for (int i = lane; i < k; i += 32) o[i] = d[i];
+    __syncwarp();
+    n *= act;
+    if (lane == 0) {
+        o[k] = bonus;
+        if (n >= 1) o[n - 1] = bonus;
+        n_out[b] = n;
+    }
 }
 
 extern "C" int colinfer_spec_accept(const int64_t* pred, const int64_t* tok, const int64_t* stop_ids,
                                     const int32_t* active, int64_t* out_tok, int32_t* n, int B, int k1, int S, void* stream) {
     if (!pred || !tok || !out_tok || !n || B < 0 || k1 < 1 || S < 0) return (int)cudaErrorInvalidValue;
     if (B == 0) return 0;
-    k_spec_accept<<<(B + 127) / 128, 128, 0, (cudaStream_t)stream>>>(pred, tok, S > 0 ? stop_ids : nullptr, active, out_tok, n, B, k1, S);
+    k_spec_accept<<<(B + 3) / 4, 128, 0, (cudaStream_t)stream>>>(pred, tok, S > 0 ? stop_ids : nullptr, active, out_tok, n, B, k1, S);
     return (int)cudaGetLastError();
 }
 
