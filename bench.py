@@ -42,7 +42,8 @@ if ROOT not in sys.path:
 V = 151_936
 HIST = 2048
 CPU_SAMPLE_ROWS = 256
-TRAFFIC_RECORD = os.path.join(ROOT, "profiles", "k_sample_stream_config3_traffic.json")
+TRAFFIC_RECORD = os.path.join(ROOT, "profiles", "k_sample_rows_config3_traffic.json")
+SMS = 148               # a B200's: more rows than these take the chunk kernel with a CTA per row
 
 
 def measured_peak():
@@ -51,6 +52,11 @@ def measured_peak():
             return float(json.load(f)["hbm_gbs"]), "measured"
     except Exception:
         return 6650.0, "fallback"
+
+
+def kernel_of(rows: int, few: int) -> str:
+    """The kernel that colinfer_sample picks for fp32 rows of the usual vocabulary (few: clusters of 8 the device holds)."""
+    return "k_sample (cluster-resident)" if rows <= few else "k_sample (a CTA per row)" if rows > SMS else "k_sample (a cluster per row) or k_sample_stream"
 
 
 def recorded_traffic(kernel_name: str, rows: int):
@@ -465,7 +471,7 @@ def run_sweep(torch, dev, lib, peak, reps: int):
         sp = wl.sampler_params(w["params"], V, dev)
         logits, pos = w["logits"].to(dev), w["pos"].to(dev)
         med, best = per_launch_us(torch, lambda: draw(logits, sp, pos), flush, reps)
-        c3[str(B)] = entry(med, best, B, wl.bytes_per_row(V, 4, False, HIST), "k_sample" if B <= few else "k_sample_stream", "row")
+        c3[str(B)] = entry(med, best, B, wl.bytes_per_row(V, 4, False, HIST), kernel_of(B, few), "row")
         del logits, sp
     out["config3_rows"] = c3
     # bf16 large-vocabulary stress: [512, 262144], 30 % grammar mask, top_k 1000, top_p 0.98, min_p 0.01
@@ -474,7 +480,7 @@ def run_sweep(torch, dev, lib, peak, reps: int):
     sp = wl.sampler_params(w["params"], VL, dev)
     logits, pos, mask = w["logits"].to(dev), w["pos"].to(dev), w["mask"].to(dev)
     med, best = per_launch_us(torch, lambda: draw(logits, sp, pos, mask=mask), flush, reps)
-    out["config4_bf16_512x262144"] = entry(med, best, 512, wl.bytes_per_row(VL, 2, True, 0), "k_sample_stream", "row")
+    out["config4_bf16_512x262144"] = entry(med, best, 512, wl.bytes_per_row(VL, 2, True, 0), "k_sample (1,024 threads per row)", "row")
     del logits, mask, sp
     # speculative verify: k = 8 drafts per slot, temperature 0.8, top_p 0.95; one slot (latency) and 64 slots
     ver = {}
@@ -485,7 +491,7 @@ def run_sweep(torch, dev, lib, peak, reps: int):
         d_ids = draw(draft, sp, None, u=c2["ud"].to(dev))
         ua, us = c2["ua"].to(dev), c2["us"].to(dev)
         med, best = per_launch_us(torch, lambda: spec_verify(target, draft, d_ids, sp, ua, us), flush, max(5, reps // 2))
-        e = entry(med, best, B, 17 * V * 4, "k_sample / k_sample_stream x2 + k_verify_finish", "verify")
+        e = entry(med, best, B, 17 * V * 4, "k_sample over both models' rows + k_verify_finish", "verify")
         ver[str(B)] = e
         del target, draft
     out["config2_verify_slots"] = ver
@@ -695,7 +701,7 @@ def main():
         # which kernel colinfer_sample ran: few rows (at most the clusters the device holds at once) take the
         # cluster-resident kernel, more rows the streaming kernel; --cluster forces one of them
         few = B <= lib.colinfer_max_active_clusters(V, _lib.F32)
-        kernel_name = "k_sample" if args.cluster > 0 or (args.cluster == 0 and few) else "k_sample_stream"
+        kernel_name = "k_sample (cluster-resident)" if args.cluster > 0 or (args.cluster == 0 and few) else "k_sample_stream" if args.cluster < 0 else kernel_of(B, 0)
         peak, peak_kind = measured_peak()
         achieved = bytes_row * B / (kernel_ms * 1e-3) / 1e9
         traffic, traffic_src = recorded_traffic(kernel_name, B)

@@ -63,7 +63,8 @@ enum { COLINFER_F32 = 0, COLINFER_BF16 = 1 };
 enum {
     COLINFER_FORCE_DISTRIBUTION = 1, /* build the distribution even for temperature <= 0 (processed_probs does) */
     /* which kernel runs (tests and benchmarks; results are the same): default automatic -- few rows take the
-       cluster-resident kernel, one 8-CTA cluster per row, more rows the streaming kernel */
+       cluster-resident kernel (the widest cluster of 8, 4 or 2 CTAs per row with which all rows run at once), then the chunk
+       kernel with a cluster per row, then the streaming kernel, and more rows than SMs the chunk kernel with a CTA per row */
     COLINFER_KERNEL_STREAM   = 0x100, /* the streaming kernel */
     COLINFER_KERNEL_CLUSTER1 = 0x200, /* the cluster-resident kernel with clusters of 1, */
     COLINFER_KERNEL_CLUSTER2 = 0x300, /* 2, */
