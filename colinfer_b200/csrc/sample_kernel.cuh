@@ -48,7 +48,8 @@ constexpr int CHUNK = 512;           // logits per chunk: 16 per lane
 constexpr int RING = NST * 2048;     // bytes of ring per warp: a stage is 2 KB of fp32, or 1 KB of bf16 (and an fp32 copy of one chunk behind them)
 constexpr int NB1 = 4096;            // histogram buckets
 constexpr int HOFF = 1024;           // of these, above the sample's maximum
-constexpr float RANGE = 25.0f;       // they span RANGE temperatures
+constexpr float RANGE = 29.0f;       // they span RANGE temperatures: three quarters of that reach from the sample's maximum to the mass horizon
+                                     // (what falls short of it is missing from the estimates: at 25, a row of T = 0.53 and top_p = 0.996 missed its band)
 constexpr int FASTK = 100;           // largest top_k finished from the sample's bound
 constexpr int BINS = 256;            // bins of the sample and of the selections on lists
 constexpr float FAST_SCALE = 16.0f;  // sample bins per unit logit (16 units)
@@ -1958,13 +1959,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 const View w = view_all(blist, bcap, over);
                 const u64 target = ceil_target(rw.topp, s1);
                 bool ok = !over && s1 > 0 && s_above < target;
+                u64 s_band = 0;
                 if (ok) {
                     const float t_hi = rw.t_hi, t_lo = rw.t_lo, lcut = rw.lcut;
                     const MassFn mass = rw.mass;
                     const float bs = t_hi < SM_POS_INF ? t_hi : rw.L;
                     // (a small nucleus lists everything above the cut: the bins span [cut, base], not [-max, base])
                     const float scale = (float)(BINS - 2) / fmaxf(bs - fmaxf(t_lo, lcut), 1e-30f);
-                    float lp; u64 s_band;
+                    float lp;
                     ok = list_select(w, [&](float l) { return (u64)mass(l); }, bs, scale, target - s_above, bins, sc, lp, s_band);
                     if (ok) {
                         const float cut2 = fmaxf(lcut, lower_logit_for(scale_logit(lp, mass.tc), mass.tc, lp));
@@ -1979,7 +1981,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 if (ok) break;
                 bool found_band = false;
                 float lpiv;
-                if (s1 > 0 && s_above < target && bracket_select(fmaxf(rw.t_lo, fmaxf(rw.lcut, -SM_FLT_MAX)), fminf(rw.t_hi, rw.L), target, s_above, lpiv)) {
+                if (s1 > 0 && s_above < target && (over || target <= s_above + s_band) && bracket_select(fmaxf(rw.t_lo, fmaxf(rw.lcut, -SM_FLT_MAX)), fminf(rw.t_hi, rw.L), target, s_above, lpiv)) {
                     // the band holds the pivot, but more logits than the lists
                     raise_cut(lpiv);
                     if (tid == 0) rw.path = PATH_PURE;
