@@ -46,7 +46,7 @@
 #define CI_FIN_KEEP 128          // candidates that may be left after top-k
 #define CI_FIN_CAND 64           // candidates of one bin examined pairwise
 #define CI_RETRY 8               // rows a CTA may set aside for the generic path before the fast path is switched off
-#define CI_WLIST 48              // list entries per warp
+#define CI_WLIST 24              // list entries per warp
 #define CI_GLIST 1365            // gathered list entries (16 KB)
 #define CI_SEL_BINS 256          // coarse bins of the exact selection on a gathered list
 #define CI_FB_NB 1024             // radix buckets per level of the fallback select (8 bits)
@@ -104,7 +104,7 @@ struct Scratch {
     int hist_slow;
     u64 wsum[CI_WARPS], woff[CI_WARPS], wtotal;   // block scan
     int found_tid; u64 found_excl;
-    float cand_l[CI_FIN_CAND]; u64 cand_w[CI_FIN_CAND]; float res_f;
+    float cand_l[CI_FIN_CAND]; float res_f;
     Pending pend;
     int n_retry_common, n_retry_mine, any_retry, want_fast_off;   // any_retry: a CTA of the cluster has set a row aside
     int retry_common[CI_RETRY], retry_mine[CI_RETRY], retry_all[CI_RETRY * 9];
