@@ -3,7 +3,7 @@
 `python -m colinfer_b200.build` (or build() from the graft entry) runs nvcc on the sources in csrc/.  nvcc cross-compiles,
 so no GPU is needed to build.  The library has a plain C ABI (include/colinfer_b200.h) and does not link against torch.
 
-The streaming kernel is compiled once per instantiation (csrc/stream_part.cu with -DCOLINFER_STREAM_PART=0..8), side by
+The streaming kernel (around as many rows as SMs) is compiled once per instantiation (csrc/stream_part.cu with -DCOLINFER_STREAM_PART=0..8), side by
 side, which keeps a full build to about a minute.  Objects are kept under colinfer_b200/build/obj and reused while they
 are newer than every source and header.
 """

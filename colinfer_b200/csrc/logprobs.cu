@@ -6,8 +6,9 @@
 // while one CTA is in its short block-wide steps (the sample's bound, the selection of the alternatives) the other one
 // streams.  Warp w owns a contiguous region of the row; lanes read 128-bit groups, four in flight per thread.  Each thread keeps an online (maximum, sum of exp) pair; the first batch
 // of every warp (a tenth of the row at 151,936 logits) bounds the n_top-th largest logit from below, and the pass lists
-// what reaches the bound (a few hundred logits), from which one warp takes the exact top n_top in descending order
-// (equal logits: lower token first).  A row whose lists overflow (long runs of equal logits) takes n_top extra passes.
+// what reaches the bound (a few hundred logits), from which the exact top n_top are taken by rank, in descending order
+// (equal logits: lower token first).  Up to 111 rows are shared by the CTAs of a cluster, whose first one merges the slices' maxima,
+// sums and alternatives.  256 rows of 151,936 fp32 logits: 50.8 -> 47.7 us, 74 rows 35 -> 26 us.  A row whose lists overflow (long runs of equal logits) takes n_top extra passes.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>

@@ -173,7 +173,7 @@ extern "C" int colinfer_noalloc_max_rows(void) { return COLINFER_NOALLOC_MAX_ROW
 // A cluster of 8 CTAs per row.  Sums are float64 (the reference's fp32 scan order is device dependent; float64 is what its CPU
 // cumsum accumulates in).  A warp owns a region of consecutive tokens, a lane four of them at a time; the warp in whose region
 // the running sum reaches u * total walks over it again.  A few rows are a matter of latency: with one CTA per row nine rows
-// of 151,936 took as long as one SM needs to fetch a row twice.
+// of 151,936 took as long as one SM needs to fetch a row twice: processed_probs() and this, of 9 rows, 92 -> 45 us.
 #define ICDF_THREADS 512
 #define ICDF_WARPS (ICDF_THREADS / 32)
 #define ICDF_CTAS 8
@@ -488,7 +488,8 @@ __device__ __forceinline__ float4 load_four(const VerifyArgs& a, const void* bas
 // A cluster of 8 CTAs per slot.  The accepted prefix (every CTA decides it for itself, a warp per position); the residual mass
 // of the rejected position, a region of consecutive tokens per warp; then the one warp in whose region the running mass reaches
 // us * total walks over that region again, a lane's four tokens at a time.  Launches and latency are all there is to it: decide,
-// sum and pick were three launches, the pick serial in one thread per slot.
+// sum and pick were three launches, the pick serial in one thread per slot.  Verify of 1 x 8 drafts over 151,936 logits, with
+// both models' rows in one sampler launch: 118 -> 59 us.
 __global__ void __cluster_dims__(VF_CTAS, 1, 1) __launch_bounds__(VF_THREADS) k_verify_finish(const __grid_constant__ VerifyArgs a) {
     __shared__ u64 wsum[VF_WARPS], csum[VF_CTAS];
     __shared__ uint32_t bm[VF_BM_WORDS];

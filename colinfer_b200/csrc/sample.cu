@@ -10,7 +10,7 @@
 // units of 2^-30 and summed as integers, so every sum, every cumulative-mass crossing and the CDF crossing are
 // independent of thread, CTA and cluster geometry and of the other rows in the launch (the reference's row-invariance
 // property).  How the threshold is found depends on the row's parameters:
-//   top_k <= 128   each CTA bounds its slice's k-th largest logit from below with a histogram of its threads' maxima,
+//   top_k <= 100   each CTA bounds its slice's k-th largest logit from below with a histogram of its threads' maxima,
 //                  collects the few logits above that bound in token order, and the cluster's first CTA finishes
 //                  top-k, top-p and the draw exactly on the gathered list (two cluster barriers in all);
 //   larger top_k   a fine count histogram over the distance from the row maximum (4096 buckets, reduced across the
@@ -19,8 +19,15 @@
 //                  one pass sums the exact mass above a narrow band around it and gathers the band, the pivot is found
 //                  exactly on the list, and the draw walks the row once more only inside one warp's region;
 //   neither        one mass pass and the draw.
-// If a list would overflow, or the estimated band misses the true pivot, an exact 4-level radix select over the
-// order-preserving 32-bit keys runs instead (slower, same result).
+// If a list would overflow, or the estimated band misses the true pivot, an exact select over the order-preserving 32-bit keys
+// runs instead: a pass over the resident slices per 1,024-fold narrowing (slower, same result).
+//
+// What bounds it is latency: one row's chain of block-wide steps, and code that every step executes for the first time (a third of
+// the stalls are instruction fetches), not bytes.  So: one CTA of 512 threads per SM (with 256 the passes over a slice took
+// twice as long, at 1,024 there are too few registers), searches repeated by every warp instead of published by one, sums pushed to the peers before a
+// barrier instead of fetched after it, masses two logits per instruction, 64-bit shared-memory additions as 32-bit ones with a
+// carry.  One fp32 row of 151,936 logits on a B200, device time: top_k 100 23.1 -> 16.5 us, top-p alone 33.5 -> 26 us, no filter
+// 14.5 -> 12 us; four rows with a grammar mask 21.5 -> 13.8 us.
 //
 // What the reference does in ~25 torch / FlashInfer launches per slot (engine/spec/accept.py:23-52 after
 // engine/runtime/sampler.py:50-56) is one launch here.

@@ -1,11 +1,11 @@
 // sample_kernel.cuh -- the fused logits -> token kernel (sm_100a).
 //
-// A row of logits is cut into chunks of 512 and read by the 16 warps of a CTA, chunk c by warp c mod 16; with few rows
-// in a launch the CTAs of a thread-block cluster (2, 4 or 8) share a row, chunk c going to warp c mod 16 C of the cluster.
-// Every warp pulls its own chunks into a private two-stage ring in shared memory with bulk copies (TMA, one mbarrier per
+// A row of logits is cut into chunks of 512 and read by the NW warps of a CTA, chunk c by warp c mod NW; with few rows
+// in a launch the CTAs of a thread-block cluster share a row, chunk c going to warp c mod NW * C of the cluster.
+// Every warp pulls its own chunks into a private ring of NST stages in shared memory with bulk copies (TMA, one mbarrier per
 // stage, every wait bounded), so that loads are in flight while the warps compute, meet at barriers or finish a row, and
 // the first chunks of the row's next pass, or of the CTA's next row, are on their way before the current pass ends.
-// Two CTAs of 512 threads per SM: one streams while the other one is in its short block-wide steps.
+// sample_rows.cu, sample_row.cu and sample_few.cu say how many threads and CTAs per SM, and why.
 //
 // Rows start at any alignment: chunks are counted from the 16-byte boundary at or below the row's first logit ("position"
 // p = token + a), what lies outside the row reads as -inf.  History penalties are applied to a chunk in shared memory before
@@ -24,6 +24,12 @@
 // Masses are exp(z - max) in integer units of 2^-30 and all sums are integer: results depend neither on the batch nor on
 // the order of arrival nor on how many CTAs share a row.  Where a list overflows, a bound does not hold or the estimated
 // band misses the pivot, an exact select over the 32-bit keys runs (slower, same result).
+//
+// What bounds it is instructions: 592 rows of 151,936 fp32 logits with mixed filters and histories issue in 61 % of the cycles, at
+// 30 % of DRAM's rate; the exact masses of a wide row take 16 instructions per logit, its histogram 10.  Hence masses two logits per
+// instruction with rounding additions instead of conversions, one histogram instead of a walk over radix levels, the draw from per-chunk sums.
+// 1,024 such rows: 342 us with one CTA of 1,024 threads per SM walking over the rows, 264 us here; 512 bf16 rows of 262,144 with a mask
+// 335 -> 242 us; 201 rows of 100,003 (no row but the first 16-byte aligned) 79 -> 62 us.
 #pragma once
 #include <stddef.h>
 
