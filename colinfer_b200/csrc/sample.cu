@@ -34,6 +34,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "host_util.h"
 #include "sample_host.h"
 #include "../../include/colinfer_b200.h"
 
@@ -1497,11 +1498,17 @@ static int g_prof_slots = 0;
 static const int kFixedSmem = 24 * 1024 + (CI_WARPS * CI_WLIST + 8 * CI_PCAP) * (int)sizeof(Cand) + CI_MAX_CHUNKS * 8 +
                               (int)sizeof(Xch) + (int)sizeof(Scratch) + 64;
 
+static const int kMaxSmem = 226 * 1024;                    // of any geometry
+static cudaError_t sample_opt_in() {
+    static SmemOptIn opt_in;
+    return opt_in((const void*)k_sample, kMaxSmem);
+}
+
 // forced: 0 = the smallest cluster that holds the row; 1, 2, 4, 8 = that cluster size
 static int pick_geometry(int V, int dtype, const void* logits, int forced, colinfer_geometry* g) {
     if (V <= 0) return 1;
     const int cap2 = (113 * 1024 - kFixedSmem) / 4;           // slice elements that allow two CTAs per SM
-    const int cap1 = (226 * 1024 - kFixedSmem) / 4;           // one CTA per SM
+    const int cap1 = (kMaxSmem - kFixedSmem) / 4;           // one CTA per SM
     const int max_slice = CI_CHUNK * CI_MAX_CHUNKS;
     int cs = 0, slice = 0;
     auto slice_for = [&](int c) { return (((V + c - 1) / c) + 127) & ~127; };
@@ -1563,7 +1570,7 @@ static int active_clusters(const colinfer_geometry& g) {
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     for (int i = 0; i < used; ++i)
         if (cache[i].dev == dev && cache[i].smem == g.smem_bytes && cache[i].cs == g.cluster) return cache[i].n;
-    if (cudaFuncSetAttribute(k_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem_bytes) != cudaSuccess) return -2;
+    if (sample_opt_in() != cudaSuccess) return -2;
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
     fill_launch(cfg, attr, g, 1024, nullptr);
     int n = 0;
@@ -1757,7 +1764,7 @@ static int sample_rows(const void* logits, const void* logits2, int dtype, const
     a.B = B; a.R = R; a.V = V; a.slice_elems = g.slice_elems; a.flags = flags; a.second = second;
     colinfer_profile_buffer(&a.prof, &a.prof_slots);
 
-    cudaError_t e = cudaFuncSetAttribute(k_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem_bytes);
+    cudaError_t e = sample_opt_in();
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
     fill_launch(cfg, attr, g, clusters, (cudaStream_t)stream);
