@@ -50,3 +50,28 @@ def test_threads_with_different_row_counts_do_not_disturb_each_other():
 
     assert _hammer([call(0, 3), call(1, 20), call(2, 3), call(3, 20)], 1000) == []
     assert torch.equal(outs[0][:3], outs[1][:3]) and torch.equal(outs[1], outs[3])
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "nvfp4"])
+def test_threads_with_different_hidden_sizes_do_not_disturb_each_other(fmt):
+    """Rescoring of hidden sizes whose activations take more than the default 48 KB of shared memory, 50 and 96 KB."""
+    L = _lib.lib()
+    sizes, rows_w = (25_600, 49_152), 8
+    cand = torch.arange(rows_w, device="cuda")[None].contiguous()
+    xs = [torch.randn(1, K, device="cuda").bfloat16() for K in sizes]
+    ws = [torch.randn(rows_w, K, device="cuda").bfloat16() for K in sizes]
+    sf = torch.full((rows_w, sizes[1] // 16), 0x38, dtype=torch.uint8, device="cuda")          # E4M3 1.0
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    outs = [torch.zeros(1, rows_w, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+
+    def call(i):
+        x, w, K = xs[i % 2], ws[i % 2], sizes[i % 2]
+        if fmt == "bf16":
+            return lambda: L.colinfer_rescore_bf16(x.data_ptr(), w.data_ptr(), cand.data_ptr(), outs[i].data_ptr(), 1, K, rows_w, rows_w,
+                                                   streams[i].cuda_stream)
+        return lambda: L.colinfer_rescore_nvfp4(x.data_ptr(), w.data_ptr(), sf.data_ptr(), 1.0, cand.data_ptr(), outs[i].data_ptr(), 1, K, rows_w, rows_w,
+                                                streams[i].cuda_stream)
+
+    assert _hammer([call(i) for i in range(4)], 1000) == []
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3])
