@@ -31,6 +31,7 @@
 #include <mutex>
 
 #include "../../include/colinfer_b200.h"
+#include "host_util.h"
 #include "rescore_row.cuh"
 
 namespace cg = cooperative_groups;
@@ -609,24 +610,18 @@ static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, i
     cfg.attrs = attr; cfg.numAttrs = 1;
 }
 
-// Clusters of G CTAs that the current device holds at once (cached).
+// Clusters of G CTAs that the current device holds at once (remembered).
 static int active_clusters(bool fp4, int G, size_t smem) {
-    struct Entry { int dev, fp4, G; size_t smem; int n; };
-    static Entry cache[64];
-    static int used = 0;
-    static std::mutex mu;
+    static Remembered known;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    std::lock_guard<std::mutex> lock(mu);
-    for (int i = 0; i < used; ++i)
-        if (cache[i].dev == dev && cache[i].fp4 == (int)fp4 && cache[i].G == G && cache[i].smem == smem) return cache[i].n;
-    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
-    cluster_config(cfg, attr, G, 256, smem, nullptr);
-    int n = 0;
-    const cudaError_t e = fp4 ? cudaOccupancyMaxActiveClusters(&n, k_draft_pick<true, true>, &cfg) : cudaOccupancyMaxActiveClusters(&n, k_draft_pick<false, true>, &cfg);
-    if (e != cudaSuccess) return 0;
-    if (used < 64) cache[used++] = Entry{dev, (int)fp4, G, smem, n};
-    return n;
+    return known(((uint64_t)dev << 40) | ((uint64_t)fp4 << 32) | ((uint64_t)G << 24) | (uint64_t)smem, [&]() {
+        cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+        cluster_config(cfg, attr, G, 256, smem, nullptr);
+        int n = 0;
+        const cudaError_t e = fp4 ? cudaOccupancyMaxActiveClusters(&n, k_draft_pick<true, true>, &cfg) : cudaOccupancyMaxActiveClusters(&n, k_draft_pick<false, true>, &cfg);
+        return e == cudaSuccess ? n : -1;
+    });
 }
 
 }  // namespace dpk

@@ -1558,25 +1558,19 @@ static void fill_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, cons
     cfg.numAttrs = 1;
 }
 
-// Clusters of this geometry that the current device holds at once (cached per device and geometry): the kernel is
+// Clusters of this geometry that the current device holds at once (remembered per device and geometry): the kernel is
 // persistent, each cluster walks over rows, so the grid never exceeds this.
 static int active_clusters(const colinfer_geometry& g) {
-    struct Entry { int dev, smem, cs, n; };
-    static Entry cache[16];
-    static int used = 0;
-    static std::mutex guard;
-    std::lock_guard<std::mutex> lock(guard);
+    static Remembered known;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-    for (int i = 0; i < used; ++i)
-        if (cache[i].dev == dev && cache[i].smem == g.smem_bytes && cache[i].cs == g.cluster) return cache[i].n;
-    if (sample_opt_in() != cudaSuccess) return -2;
-    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
-    fill_launch(cfg, attr, g, 1024, nullptr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_sample, &cfg) != cudaSuccess || n <= 0) return -3;
-    if (used < 16) cache[used++] = Entry{dev, g.smem_bytes, g.cluster, n};
-    return n;
+    return known(((uint64_t)dev << 32) | ((uint64_t)g.cluster << 24) | (uint64_t)g.smem_bytes, [&]() {
+        if (sample_opt_in() != cudaSuccess) return -2;
+        cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+        fill_launch(cfg, attr, g, 1024, nullptr);
+        int n = 0;
+        return cudaOccupancyMaxActiveClusters(&n, k_sample, &cfg) == cudaSuccess && n > 0 ? n : -3;
+    });
 }
 
 extern "C" int colinfer_max_active_clusters(int V, int dtype) {
@@ -1587,7 +1581,7 @@ extern "C" int colinfer_max_active_clusters(int V, int dtype) {
 
 // ---- the chunk kernel (sample_rows.cu: a CTA per row, sample_few.cu: a cluster per row)
 namespace {
-constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024, kMaxDev = 64;
+constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024;
 // More rows than SMs: two CTAs of 512 threads per SM, one of which reads while the other one is in its block-wide steps; or one of
 // 1,024 where two do not fit (penalty tables of large vocabularies: 512 bf16 rows of 262,144 logits with histories 222 -> 174 us),
 // and for bf16 vocabularies beyond 229,376, whose rows have so many equal logits that the lists of 512 threads overflow (512 flat
@@ -1603,13 +1597,13 @@ int chunk_smem(int set, int V, bool pen) { return set == FEW ? colinfer_few_smem
 
 // The device's number of SMs, and once per device and kernel the opt-in to large shared memory.
 int chunk_device(int ki, int* dev_out, int* sms_out) {
-    static bool opted[kMaxDev][12] = {};
-    static int sms[kMaxDev] = {};
+    static bool opted[kMaxDevices][12] = {};
+    static int sms[kMaxDevices] = {};
     static std::mutex guard;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    if (dev < 0 || dev >= kMaxDev) return (int)cudaErrorInvalidDevice;
+    if (dev < 0 || dev >= kMaxDevices) return (int)cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(guard);
     if (!opted[dev][ki]) {
         e = cudaFuncSetAttribute(chunk_kernel(ki), cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkMaxSmem);
@@ -1635,21 +1629,15 @@ void chunk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int set, i
     cfg.numAttrs = set == FEW ? 1 : 0;
 }
 
-// Clusters of `cluster` CTAs that the device holds at once (cached).
+// Clusters of `cluster` CTAs that the device holds at once (remembered).
 int chunk_clusters(int dev, int ki, int cluster, int smem) {
-    struct Entry { int dev, ki, cs, smem, n; };
-    static Entry cache[64];
-    static int used = 0;
-    static std::mutex guard;
-    std::lock_guard<std::mutex> lock(guard);
-    for (int i = 0; i < used; ++i)
-        if (cache[i].dev == dev && cache[i].ki == ki && cache[i].cs == cluster && cache[i].smem == smem) return cache[i].n;
-    cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
-    chunk_config(cfg, attr, FEW, cluster, 1024, smem, nullptr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, chunk_kernel(ki), &cfg) != cudaSuccess || n <= 0) return 0;
-    if (used < 64) cache[used++] = Entry{dev, ki, cluster, smem, n};
-    return n;
+    static Remembered known;
+    return known(((uint64_t)dev << 40) | ((uint64_t)ki << 32) | ((uint64_t)cluster << 24) | (uint64_t)smem, [&]() {
+        cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
+        chunk_config(cfg, attr, FEW, cluster, 1024, smem, nullptr);
+        int n = 0;
+        return cudaOccupancyMaxActiveClusters(&n, chunk_kernel(ki), &cfg) == cudaSuccess ? n : -1;
+    });
 }
 
 // Launches the chunk kernel where it is the faster one; returns -1 where it is not (nothing launched), else a CUDA error code.
