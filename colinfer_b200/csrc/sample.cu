@@ -1229,8 +1229,10 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 int g_star; u64 before;
                 if (G <= CI_THREADS) thread_find(tid < G ? (u64)pseg[tid] * bucket_mass_est(s_star * G + tid) : 0ull, target - before_seg, sc, g_star, before);
                 else block_find([&](int i) { return (u64)pseg[i] * bucket_mass_est(s_star * G + i); }, G, target - before_seg, sc, g_star, before);
-                const int bp = s_star * G + g_star;
+                int bp = s_star * G + g_star;
                 const int up = a.dtype == COLINFER_BF16 ? 3 : 1, dn = a.dtype == COLINFER_BF16 ? 4 : 2;
+                const int s8 = (a.flags & COLINFER_TEST_MISS_BAND) ? (row & 1 ? 8 : -8) : 0;   // test hook: a band eight buckets off
+                bp = max(0, min(bp + s8, CI_NB1 - 1));
                 if (bp + dn + 2 >= CI_NB1) path = PATH_FALLBACK;
                 else {
                     path = PATH_BAND;
@@ -1267,6 +1269,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         // reads precede the peers' next cluster barrier, and the first write below follows this CTA's next barrier)
         const RadixCtx rc = {rowbuf, n_pad, fb_hist, fb_seg, xch, sc, rank, CS};
         float lpiv;
+        status |= COLINFER_ROW_SELECT_SLOW;
         if (kk > 0 && kk < V && radix_select(cluster, rc, mass, f2key(fmaxf(lcut, -CI_FLT_MAX)), f2key(L), coarse, false, (u64)kk, topp, lpiv))
             lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
         if (need_topp && radix_select(cluster, rc, mass, f2key(fmaxf(lcut, -CI_FLT_MAX)), f2key(L), coarse, true, 0, topp, lpiv))
@@ -1367,6 +1370,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 float lpiv;
                 uint32_t klo = f2key(fmaxf(lcut, -CI_FLT_MAX)), khi = f2key(L);
                 u64 want = 0;
+                status |= COLINFER_ROW_SELECT_SLOW;
                 if (s1 > 0) {                                                  // on which side of the band's upper edge it lies is known
                     want = ceil_target(topp, s1);
                     if (want <= s_above) klo = f2key(t_hi) + 1u;
