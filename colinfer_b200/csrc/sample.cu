@@ -54,7 +54,7 @@
 #define CI_FIN_KEEP 128          // candidates that may be left after top-k
 #define CI_FIN_CAND 64           // candidates of one bin examined pairwise
 #define CI_RETRY 8               // rows a CTA may set aside for the generic path before the fast path is switched off
-#define CI_WLIST 24              // list entries per warp
+#define CI_WLIST 24              // list entries per warp of a cluster of eight (in smaller ones as many more as there are fewer warps: SampleArgs::list_cap)
 #define CI_GLIST 1365            // gathered list entries (16 KB)
 #define CI_SEL_BINS 256          // coarse bins of the exact selection on a gathered list
 #define CI_FB_NB 1024             // radix buckets per level of the fallback select (8 bits)
@@ -70,7 +70,7 @@ struct SampleArgs {
     colinfer_sampler_params p;
     const void* pos; int pos_i64; const float* u;
     int64_t* out; colinfer_row_stats* stats; int32_t* status;
-    int B, R, V; int slice_elems; int flags;
+    int B, R, V; int slice_elems; int list_cap; int flags;
     colinfer_second_rows second;
     long long* prof; int prof_slots;   // optional per-CTA phase timestamps (profiling hook)
 };
@@ -362,7 +362,7 @@ __device__ __noinline__ bool radix_select(cg::cluster_group& cluster, const Radi
 // Returns the number of entries, or -1 when a list overflowed or the total exceeds the capacity.  The entries' masses
 // are computed here (the warps' lists hold token and logit only).  All threads call.
 __device__ int gather_lists(cg::cluster_group& cluster, int CS, Xch* xch, Cand* ownlist, ListEntry* glist, Scratch* sc,
-                            const MassFn& mass) {
+                            const MassFn& mass, int list_cap) {
     const int tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     const int np = CS * CI_WARPS;                                          // (CTA, warp) pairs, at most 128
     int overflow = 0;
@@ -387,7 +387,7 @@ __device__ int gather_lists(cg::cluster_group& cluster, int CS, Xch* xch, Cand* 
     for (int e = tid; e < n; e += CI_THREADS) {
         int lo = 0, hi = np - 1;                                           // last pair p with poff[p] <= e
         while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (sc->poff[mid] <= e) lo = mid; else hi = mid - 1; }
-        const Cand c = *(cluster.map_shared_rank(ownlist, lo / CI_WARPS) + (lo % CI_WARPS) * CI_WLIST + (e - sc->poff[lo]));
+        const Cand c = *(cluster.map_shared_rank(ownlist, lo / CI_WARPS) + (lo % CI_WARPS) * list_cap + (e - sc->poff[lo]));
         ListEntry en;
         en.idx = c.idx; en.l = c.l; en.q = mass(c.l);
         glist[e] = en;
@@ -441,8 +441,8 @@ __device__ bool finish_on_list(const ListEntry* glist, int n, float tl, float lc
 
 // Appends the components of one float4 group selected by the 4-bit mask mk to the warp's list, in token order
 // (lane, then component).  Positions come from four ballots, no scan.  wn is the warp's running count (uniform over
-// the warp); entries beyond CI_WLIST are dropped and counted.
-__device__ __forceinline__ void warp_append(Cand* mylist, int& wn, unsigned mk, const float* e4, uint32_t idx0, int lane) {
+// the warp); entries beyond list_cap are dropped and counted.
+__device__ __forceinline__ void warp_append(Cand* mylist, int list_cap, int& wn, unsigned mk, const float* e4, uint32_t idx0, int lane) {
     const unsigned any = __ballot_sync(0xffffffffu, mk != 0u);
     if (!any) return;
     const unsigned lt = (1u << lane) - 1u;
@@ -458,7 +458,7 @@ __device__ __forceinline__ void warp_append(Cand* mylist, int& wn, unsigned mk, 
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (mk & (1u << j)) {
-            if (at < CI_WLIST) { mylist[at].idx = idx0 + j; mylist[at].l = e4[j]; }
+            if (at < list_cap) { mylist[at].idx = idx0 + j; mylist[at].l = e4[j]; }
             ++at;
         }
     }
@@ -467,7 +467,7 @@ __device__ __forceinline__ void warp_append(Cand* mylist, int& wn, unsigned mk, 
 
 // Collects, in token order, the logits >= tl of one warp's region [r_lo, r_hi) of the slice into the warp's list.
 // Four float4 groups per lane and step are loaded together (their latencies overlap); appends are rare.
-__device__ __forceinline__ void collect_region(const float* rowbuf, int r_lo, int r_hi, float tl, Cand* mylist, int& wn,
+__device__ __forceinline__ void collect_region(const float* rowbuf, int r_lo, int r_hi, float tl, Cand* mylist, int list_cap, int& wn,
                                                uint32_t slice_lo, int lane) {
     for (int i0 = r_lo; i0 < r_hi; i0 += 512) {
         float4 v[4];
@@ -483,7 +483,7 @@ __device__ __forceinline__ void collect_region(const float* rowbuf, int r_lo, in
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float e4[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
-                warp_append(mylist, wn, mk[k], e4, slice_lo + (uint32_t)(i0 + k * 128 + lane * 4), lane);
+                warp_append(mylist, list_cap, wn, mk[k], e4, slice_lo + (uint32_t)(i0 + k * 128 + lane * 4), lane);
             }
         }
     }
@@ -674,8 +674,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     uint32_t* cand = reinterpret_cast<uint32_t*>(hreg + CI_NB1 * 4 + CI_SEL_BINS * 8);
     u64* fb_hist = reinterpret_cast<u64*>(hreg);                              // fallback radix, over hist1
     u64* fb_seg = fb_hist + CI_FB_NB;
-    Cand* ownlist = reinterpret_cast<Cand*>(hreg + 24 * 1024);                // [CI_WARPS][CI_WLIST] this CTA's lists
-    Cand* plist = ownlist + CI_WARPS * CI_WLIST;                              // [8][CI_PCAP] candidates pushed by the cluster
+    Cand* ownlist = reinterpret_cast<Cand*>(hreg + 24 * 1024);                // [CI_WARPS][list_cap] this CTA's lists
+    Cand* plist = ownlist + CI_WARPS * a.list_cap;                              // [8][CI_PCAP] candidates pushed by the cluster
     u64* mbar = reinterpret_cast<u64*>(plist + 8 * CI_PCAP);
     Xch* xch = reinterpret_cast<Xch*>(mbar + CI_MAX_CHUNKS);
     Scratch* sc = reinterpret_cast<Scratch*>(xch + 1);
@@ -963,7 +963,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     // order inside a region is (step, lane, component).
     const int reg = ((n_pad / 128 + CI_WARPS - 1) / CI_WARPS) * 128;
     const int r_lo = min(warp * reg, n_pad), r_hi = min(r_lo + reg, n_pad);
-    Cand* mylist = ownlist + warp * CI_WLIST;
+    const int list_cap = a.list_cap;
+    Cand* mylist = ownlist + warp * list_cap;
 
     // ---------------------------------------------------------------------------------------- small top-k: candidates of the slice
     // The k-th largest of the threads' group maxima (CI_TGROUPS disjoint groups per thread) bounds the slice's k-th largest logit from below, and every logit of the
@@ -983,7 +984,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
         else tl_fast = -CI_FLT_MAX;                             // fewer than k threads saw a finite logit: take them all
         CI_PROF(10);
         int wn = 0;
-        collect_region(rowbuf, r_lo, r_hi, tl_fast, mylist, wn, (uint32_t)slice_lo, lane);
+        collect_region(rowbuf, r_lo, r_hi, tl_fast, mylist, list_cap, wn, (uint32_t)slice_lo, lane);
         CI_PROF(11);
         if (lane == 0) sc->warp_i[warp] = wn;
         __syncthreads();                                        // every thread is done with the row buffer
@@ -994,7 +995,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
             const int c = sc->warp_i[w];
             if (w < warp) woff += c;
             my_count += c;
-            over |= c > CI_WLIST;
+            over |= c > list_cap;
         }
         if (over || my_count > CI_PCAP) my_count = 0xFFFF;      // overflow marker: the row takes the generic path later
         else {
@@ -1249,16 +1250,16 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     if (path == PATH_LIST) {
         const float tl = fmaxf(fmaxf(t_lo, lcut), -CI_FLT_MAX);
         int wn = 0;
-        collect_region(rowbuf, r_lo, r_hi, tl, mylist, wn, (uint32_t)slice_lo, lane);
+        collect_region(rowbuf, r_lo, r_hi, tl, mylist, list_cap, wn, (uint32_t)slice_lo, lane);
         if (lane == 0) {
-            xch->wcount[warp] = (unsigned short)min(wn, CI_WLIST);
-            if (wn > CI_WLIST) xch->list_overflow = 1;
+            xch->wcount[warp] = (unsigned short)min(wn, list_cap);
+            if (wn > list_cap) xch->list_overflow = 1;
         }
         __syncthreads();
         CI_PROF(6);
         cluster.sync();                                                                // (L) lists published
         // every CTA gathers the lists and finishes alike (identical inputs, identical decisions)
-        const int n = gather_lists(cluster, CS, xch, ownlist, glist, sc, mass);
+        const int n = gather_lists(cluster, CS, xch, ownlist, glist, sc, mass, list_cap);
         if (n > 0 && finish_on_list(glist, n, tl, lcut, tc, kk, need_topp, topp, u, bins, cand, sc, token, lcut, total_mass)) done = true;
         else path = PATH_FALLBACK;
     }
@@ -1312,7 +1313,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
             // the band's logits are appended in no particular order: only their values and masses are looked at
             for (unsigned any = __ballot_sync(0xffffffffu, mk != 0u); any; any = __ballot_sync(0xffffffffu, mk != 0u)) {
                 const int at = wn + __popc(any & ((1u << lane) - 1u));
-                if (mk && at < CI_WLIST) {
+                if (mk && at < list_cap) {
                     const int t = __ffs(mk) - 1, i = i0 + (t >> 2) * 128 + lane * 4 + (t & 3);
                     mylist[at].idx = (uint32_t)(slice_lo + i); mylist[at].l = rowbuf[i];
                 }
@@ -1325,8 +1326,8 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
             const u64 wall = warp_sum_u64(acc_all);
             if (lane == 0) {
                 sc->warp_tot[warp] = wkeep; sc->warp_aux[warp] = wall;
-                xch->wcount[warp] = (unsigned short)min(wn, CI_WLIST);
-                if (wn > CI_WLIST) xch->list_overflow = 1;
+                xch->wcount[warp] = (unsigned short)min(wn, list_cap);
+                if (wn > list_cap) xch->list_overflow = 1;
             }
             __syncthreads();
             if (warp == 0) {
@@ -1338,7 +1339,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
             u64 s1 = 0, s_above = 0;
 #pragma unroll
             for (int q = 0; q < 8; ++q) if (q < CS) { s1 += sc->all_in[q]; s_above += sc->above_in[q]; }
-            const int n = gather_lists(cluster, CS, xch, ownlist, glist, sc, mass);
+            const int n = gather_lists(cluster, CS, xch, ownlist, glist, sc, mass, list_cap);
             bool ok = n >= 0 && s1 > 0;
             float cut2 = lcut;
             if (ok) {
@@ -1360,7 +1361,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
                 lcut = cut2;
                 // add the kept band entries of this warp's own list to its region's kept mass
                 u64 add = 0;
-                const int mine = min(wn, CI_WLIST);
+                const int mine = min(wn, list_cap);
                 for (int j = lane; j < mine; j += 32) if (mylist[j].l >= lcut) add += mass(mylist[j].l);
                 wkeep += warp_sum_u64(add);
             } else {
@@ -1508,6 +1509,14 @@ static cudaError_t sample_opt_in() {
     return opt_in((const void*)k_sample, kMaxSmem);
 }
 
+// List entries per warp: what clusters of eight hold in 128 warps, spread over fewer, as far as the slice leaves room.  With 24 a
+// warp whatever the cluster, rows with a top_k of a thousand overflowed a list in clusters of four and went through the radix
+// select: 24 fp32 rows of 151,936 logits 99 us, 43 us with these.
+static int list_cap(int cluster, int slice) {
+    const int want = CI_WLIST * 8 / cluster, room = CI_WLIST + (kMaxSmem - slice * 4 - kFixedSmem) / (CI_WARPS * (int)sizeof(Cand));
+    return want < room ? want : room;
+}
+
 // forced: 0 = the smallest cluster that holds the row; 1, 2, 4, 8 = that cluster size
 static int pick_geometry(int V, int dtype, const void* logits, int forced, colinfer_geometry* g) {
     if (V <= 0) return 1;
@@ -1526,7 +1535,7 @@ static int pick_geometry(int V, int dtype, const void* logits, int forced, colin
     }
     g->cluster = cs;
     g->slice_elems = slice;
-    g->smem_bytes = slice * 4 + kFixedSmem;
+    g->smem_bytes = slice * 4 + kFixedSmem + CI_WARPS * (list_cap(cs, slice) - CI_WLIST) * (int)sizeof(Cand);
     g->bulk_copy = (dtype == COLINFER_F32 && (V % 4) == 0 && (((uintptr_t)logits) & 15) == 0) ? 1 : 0;
     return 0;
 }
@@ -1753,7 +1762,7 @@ static int sample_rows(const void* logits, const void* logits2, int dtype, const
     a.p = *params;
     a.pos = pos; a.pos_i64 = pos_is_i64; a.u = u;
     a.out = out_ids; a.stats = stats; a.status = status;
-    a.B = B; a.R = R; a.V = V; a.slice_elems = g.slice_elems; a.flags = flags; a.second = second;
+    a.B = B; a.R = R; a.V = V; a.slice_elems = g.slice_elems; a.list_cap = list_cap(g.cluster, g.slice_elems); a.flags = flags; a.second = second;
     colinfer_profile_buffer(&a.prof, &a.prof_slots);
 
     cudaError_t e = sample_opt_in();

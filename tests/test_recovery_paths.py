@@ -41,3 +41,20 @@ def test_a_band_off_the_pivot_is_found_out(form, dtype):
     few = [0, 1, len(good) - 1]
     want, info = O.draw(logits[few].float().numpy(), {n: v[few] for n, v in np_params(params).items()}, None, u=u[few].numpy())
     check_tokens(got.cpu().numpy()[few], want, info, f"band off, {form} {dtype}")
+
+
+@pytest.mark.parametrize("rows,V", [(3, 151_936), (24, 151_936), (24, 65_536), (5, 32_000)])
+def test_a_top_k_of_a_thousand_fits_the_lists_of_every_cluster(rows, V):
+    """Clusters of eight, four, two and one: a cluster's lists hold the same number of logits whatever its size, so that a top_k of
+    a thousand needs no exact select.  (In 64 warps of 24 entries each a thousand evenly spread logits overflowed one: the launch
+    of 24 rows took 99 us instead of 43.)"""
+    m = mods()
+    g = torch.Generator().manual_seed(rows + V)
+    x = (torch.randn(rows, 1, V, generator=g) * 2).cuda()
+    params = wl._params(rows, V, torch.ones(rows), torch.full((rows,), 1000), torch.full((rows,), 0.98), torch.full((rows,), 0.01))
+    sp = wl.sampler_params(params, V, "cuda")
+    u = wl.open_unit(g, rows, 1)
+    got, st = m["draw"](x, sp, None, u=u.cuda(), status=True, flags=_lib.KERNEL_AUTO)
+    assert int(st.abs().sum()) == 0
+    want, info = O.draw(x[:2].cpu().numpy(), {n: v[:2] for n, v in np_params(params).items()}, None, u=u[:2].numpy())
+    check_tokens(got.cpu().numpy()[:2], want, info, f"top_k 1000, {rows} x {V}")
