@@ -78,6 +78,7 @@ SIGNATURES = {
     "colinfer_spec_verify_stats_bytes": (C.c_int64, [C.c_int, C.c_int]),
     "colinfer_spec_verify_ids_bytes": (C.c_int64, [C.c_int, C.c_int]),
     "colinfer_sample_geometry": (C.c_int, [C.c_int, C.c_int, C.c_void_p, C.c_int, C.POINTER(Geometry)]),
+    "colinfer_sample_copy_range": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "colinfer_max_active_clusters": (C.c_int, [C.c_int, C.c_int]),
     "colinfer_gather_ids": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p,
                                       C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),

@@ -1586,6 +1586,16 @@ static int active_clusters(const colinfer_geometry& g) {
     });
 }
 
+extern "C" int colinfer_sample_copy_range(const void* logits, int dtype, int rows, int V, int row, int64_t* begin, int64_t* end) {
+    if (rows < 1 || V < 1 || row < 0 || row >= rows || !begin || !end || (dtype != COLINFER_F32 && dtype != COLINFER_BF16)) return (int)cudaErrorInvalidValue;
+    const u64 bytes = (u64)V * (dtype == COLINFER_F32 ? 4 : 2), start = (u64)(uintptr_t)logits, addr = start + (u64)row * bytes, base = addr & ~15ull;
+    const uint32_t span = row_span(addr, bytes, (u64)row, (u64)(rows - 1 - row));
+    *begin = (int64_t)(base + (span & 1u ? 16 : 0) - start);
+    *end = (int64_t)(base + ((span & ~15u) - (uint32_t)base) - start);
+    if (*end <= *begin) *begin = *end = (int64_t)(addr - start);
+    return 0;
+}
+
 extern "C" int colinfer_max_active_clusters(int V, int dtype) {
     colinfer_geometry g;
     if (pick_geometry(V, dtype, nullptr, 0, &g)) return -1;

@@ -9,6 +9,15 @@ struct colinfer_second_rows {
     const void* logits; int R; int rows1; int rows;
 };
 #ifdef __CUDACC__
+// What the chunk kernel's bulk copies fetch of a row of `bytes` bytes at `addr`: whole units of 16 bytes, of which the first and
+// the last may hold bytes of the neighbouring rows (`before` and `after` of which the buffer has).  Where a unit would reach
+// beyond the buffer the copies begin a unit later (bit 0 of the result) or end a unit earlier (the result's other bits: the low
+// word of the address at which they end); the kernel reads the logits left out by ordinary loads.
+__host__ __device__ inline uint32_t row_span(unsigned long long addr, unsigned long long bytes, unsigned long long before, unsigned long long after) {
+    const unsigned long long end = addr + bytes, up = (end + 15) & ~15ull;
+    return (uint32_t)(up - end > after * bytes ? up - 16 : up) | ((addr & 15) > before * bytes ? 1u : 0u);
+}
+
 template <class A> __device__ __forceinline__ int slot_of(const A& a, int row, int& r) {
     const bool two = row >= a.second.rows1;
     const int i = two ? row - a.second.rows1 : row, R = two ? a.second.R : a.R;

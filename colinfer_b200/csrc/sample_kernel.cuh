@@ -8,7 +8,7 @@
 // sample_rows.cu, sample_row.cu and sample_few.cu say how many threads and CTAs per SM, and why.
 //
 // Rows start at any alignment: chunks are counted from the 16-byte boundary at or below the row's first logit ("position"
-// p = token + a), what lies outside the row reads as -inf.  History penalties are applied to a chunk in shared memory before
+// p = token + a), what lies outside the row reads as -inf.  Nothing outside the buffer is read (row_span).  History penalties are applied to a chunk in shared memory before
 // the pass reads it, the grammar mask to the registers it is read into; all passes then see effective logits.
 //
 //   greedy        one pass: maximum and its lowest index
@@ -86,7 +86,7 @@ struct Cand { uint32_t idx; float l; };
 // A row at hand.  What the phases of a row hand on lives here, not in registers: at 64 registers per thread anything that
 // stays alive across a pass is spilled, and with 226 KB of an SM's 256 in shared memory a spill is a round trip to L2.
 struct RowS {
-    const char* base; uint32_t end;    // the 16-byte boundary at or below its first logit; the low word of the one at or above its end
+    const char* base; uint32_t end;    // the 16-byte boundary at or below its first logit; what of it is copied (row_span)
     int row, key;                      // its index, and that plus 1
     int a, Nc;                         // position of the first logit, chunks
     const int32_t* mrow;               // grammar mask (NULL: none)
@@ -365,12 +365,22 @@ __device__ __forceinline__ void pen_patch(RowS& rw, uint32_t at, int c, const Pe
     __syncwarp();
 }
 
-// The logits of the first and last chunk that lie outside the row read as -inf.
+// Completes the first or last chunk of a row at stage `st`: what lies outside the row reads as -inf, and the units of 16 bytes
+// that no copy may fetch whole (row_span) come by ordinary loads.
 template <int ELT>
-static __device__ __noinline__ void mend_edges(uint32_t st, int c, int a) {
-    const int lane = lane_id(), lo = c == 0 ? a : 0, hi = scratch()->V + a - c * CHUNK;
-    for (int p = lane; p < CHUNK; p += 32)
-        if (p < lo || p >= hi) { if (ELT == 4) sts32(st + 4 * p, CI_NEG_INF); else sts16(st + 2 * p, 0xFF80u); }
+static __device__ __noinline__ void mend_edges(const RowS& rw, uint32_t st, int c) {
+    constexpr int UNIT = 16 / ELT;
+    const int lane = lane_id(), lo = c == 0 ? rw.a : 0, hi = scratch()->V + rw.a - c * CHUNK;
+    auto put = [&](int p) {
+        if (ELT == 4) sts32(st + 4 * p, __ldcg(reinterpret_cast<const float*>(rw.base) + c * CHUNK + p));
+        else sts16(st + 2 * p, __ldcg(reinterpret_cast<const unsigned short*>(rw.base) + c * CHUNK + p));
+    };
+    auto none = [&](int p) { if (ELT == 4) sts32(st + 4 * p, CI_NEG_INF); else sts16(st + 2 * p, 0xFF80u); };
+    if (lane < lo) none(lane);
+    for (int p = hi + lane; p < CHUNK; p += 32) none(p);
+    if (c == 0 && (rw.end & 1u) && lane >= lo && lane < min(UNIT, hi)) put(lane);
+    const int p = (int)((rw.end & ~15u) - (uint32_t)reinterpret_cast<u64>(rw.base)) / ELT - c * CHUNK + lane;   // from where the copies end
+    if (lane < UNIT && p >= lo && p < min(hi, CHUNK)) put(p);
     __syncwarp();
 }
 
@@ -392,12 +402,13 @@ struct Pipe {
     }
     __device__ __forceinline__ uint32_t conv() const { return buf + NST * CHB; }          // bf16: an fp32 copy of one chunk
     __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) % NST) * CHB; }
-    __device__ __forceinline__ void issue(const char* p, uint32_t bytes, u64 pol) {
+    // skip: bytes at the start of the stage that are left out
+    __device__ __forceinline__ void issue(const char* p, uint32_t bytes, u64 pol, uint32_t skip = 0) {
         if (asks) {
             const uint32_t s = (uint32_t)(cons + out) % NST;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * s), "r"(bytes) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-                         ::"r"(buf + s * CHB), "l"(p), "r"(bytes), "r"(bar + 8 * s), "l"(pol) : "memory");
+            if (bytes) asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                         ::"r"(buf + s * CHB + skip), "l"(p), "r"(bytes), "r"(bar + 8 * s), "l"(pol) : "memory");
         }
         ++out;
     }
@@ -432,21 +443,22 @@ struct Pipe {
     }
 };
 
-// Bytes of chunk c of a row of Nc chunks that ends at `end` (low word, as all of it: rows are short).
+// Bytes of the chunk at p that are copied of a row whose copies end at `end` (RowS; low words, as all of it: rows are short).
 template <int ELT>
 __device__ __forceinline__ uint32_t chunk_bytes(const char* p, uint32_t end) {
-    const uint32_t left = end - (uint32_t)reinterpret_cast<u64>(p);
+    const uint32_t left = (end & ~15u) - (uint32_t)reinterpret_cast<u64>(p);
     return left < (uint32_t)(CHUNK * ELT) ? left : (uint32_t)(CHUNK * ELT);
 }
-
-// Asks for the first chunks of row `key`, as far as they are not under way.
+// Asks for the first chunks of row `key`, as far as they are not under way.  (Out of line: every pass starts and ends with it,
+// and what it needs would be spilled there.)
 template <int ELT>
-__device__ __forceinline__ void ring_start(int key, const char* base, uint32_t end, int Nc, int gw, int GW) {
+static __device__ __noinline__ void ring_start(int key, const char* base, uint32_t end, int Nc, int gw, int GW, bool keep) {
     Pipe<ELT> p;
     p.expect(key);
-    while (p.out < NST && gw + p.out * GW < Nc) {
-        const char* q = base + (size_t)(gw + p.out * GW) * Pipe<ELT>::CHB;
-        p.issue(q, chunk_bytes<ELT>(q, end), l2_policy(true));
+    for (int c = gw + p.out * GW; p.out < NST && c < Nc; c += GW) {
+        const char* q = base + (size_t)c * Pipe<ELT>::CHB;
+        const uint32_t skip = c == 0 && (end & 1u) ? 16u : 0u, bytes = chunk_bytes<ELT>(q, end);
+        p.issue(q + skip, bytes > skip ? bytes - skip : 0u, l2_policy(keep), skip);
     }
     p.save(key);
 }
@@ -531,7 +543,7 @@ __device__ __forceinline__ Chunk<ELT, MASK> open_chunk(RowS& rw, uint32_t st, ui
     Chunk<ELT, MASK> k;
     k.c = c; k.mw = mw; k.sh = (-rw.a) & 31; k.wide = ELT == 4;
     wrote = false;
-    if (fresh && (c == 0 || c == rw.Nc - 1)) { mend_edges<ELT>(st, c, rw.a); wrote = true; }
+    if (fresh && ((c == 0 && rw.a) || c == rw.Nc - 1)) { mend_edges<ELT>(rw, st, c); wrote = true; }
     k.at = st + lane * 4 * ELT;
     if (pen) {
         if (ELT == 4) { if (fresh) { pen_patch(rw, st, c, pk); wrote = true; } }
@@ -556,16 +568,15 @@ template <bool CL, int ELT, bool MASK, class F>
 __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep, int seen, int then, F f) {
     constexpr int CHB = CHUNK * ELT;
     Sc* sc = scratch();
-    Pipe<ELT> p;
-    p.expect(rw.key);
     const int GW = CL ? sc->GW : NW;
     const int gw = (CL ? sc->rank * NW : 0) + warp_id();
     const int Nc = rw.Nc;
     const bool pen_on = rw.pen_on != 0;
+    ring_start<ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, keep);
+    Pipe<ELT> p;
     const u64 pol = l2_policy(keep);
-    int cn = gw + p.out * GW;                                            // the next chunk to ask for
+    int cn = gw + p.out * GW;                                            // the next chunk to ask for (no more a row's first)
     const char* next = rw.base + (size_t)cn * CHB;
-    while (p.out < NST && cn < Nc) { p.issue(next, chunk_bytes<ELT>(next, rw.end), pol); next += GW * CHB; cn += GW; }
     uint32_t mw[MASK ? 3 : 1];                                           // mask words of this chunk and the next two
     if (MASK) {
 #pragma unroll
@@ -591,16 +602,12 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
         ++p.cons; --p.out;
         if (cn < Nc) { p.issue(next, cn == Nc - 1 ? chunk_bytes<ELT>(next, rw.end) : CHB, pol); next += GW * CHB; cn += GW; }
     }
+    p.save(rw.key);
     // the first chunks of what comes next
-    const bool other = then == THEN_NEXT_ROW;
     const int nkey = *(volatile const int*)&nx.key;
     __threadfence_block();
-    const int nnc = then == THEN_NOTHING ? 0 : !other ? Nc : nkey ? nx.Nc : 0;
-    for (int c = gw; p.out < NST && c < nnc; c += GW) {
-        const char* q = (other ? nx.base : rw.base) + (size_t)c * CHB;
-        p.issue(q, chunk_bytes<ELT>(q, other ? nx.end : rw.end), l2_policy(other));
-    }
-    p.save(other ? nkey : rw.key);
+    if (then == THEN_AGAIN) ring_start<ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, false);
+    else if (then == THEN_NEXT_ROW && nkey) ring_start<ELT>(nkey, nx.base, nx.end, nx.Nc, gw, GW, true);
 }
 
 // Appends the logits of the chunk selected by the lanes' masks mk to the warp's list (no particular order).
@@ -1177,9 +1184,10 @@ static_assert(offsetof(colinfer_sampler_params, hist_len) == 9 * sizeof(void*) &
 // Where a row lies.
 template <int ELT>
 __device__ __forceinline__ const char* place_row(const Args& a, int row, int& al, uint32_t& end, int& nc) {
-    const u64 addr = reinterpret_cast<u64>(logits_of(a, row)) + (u64)row * (u64)a.V * ELT;
+    const u64 bytes = (u64)a.V * ELT, addr = reinterpret_cast<u64>(logits_of(a, row)) + (u64)row * bytes;
+    const bool two = row >= a.second.rows1;
     al = (int)((addr & 15) / ELT);
-    end = (uint32_t)((addr + (u64)a.V * ELT + 15) & ~15ull);
+    end = row_span(addr, bytes, two ? row - a.second.rows1 : row, (two ? a.second.rows : min(a.second.rows1, a.second.rows)) - 1 - row);
     nc = (a.V + al + CHUNK - 1) / CHUNK;
     return reinterpret_cast<const char*>(addr & ~15ull);
 }
@@ -1381,14 +1389,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         }
     }
     __syncthreads();
-    ring_start<ELT>(sc->rows[0].key, sc->rows[0].base, sc->rows[0].end, sc->rows[0].Nc, gw, GW);   // the logits travel while the parameters do
+    ring_start<ELT>(sc->rows[0].key, sc->rows[0].base, sc->rows[0].end, sc->rows[0].Nc, gw, GW, true);   // the logits travel while the parameters do
     if (warp == PW) derive(0);
     __syncthreads();
 
     for (int it = 0; ; ++it) {
         RowS& rw = sc->rows[it & 1];
         const NextRow& nx = sc->next[it & 1];
-        ring_start<ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW);
+        ring_start<ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW, true);
         bool asked = false, found = false, derived = false;      // (the last warp's)
         // (A row of several passes asks when its first one is through: the CTAs that ask before it have less left to do.)
         auto ask = [&]() { if (!CL && warp == PW && !asked) { if (lane == 0) queue_ask(sc); asked = true; } };

@@ -163,6 +163,10 @@ typedef struct colinfer_geometry {
 } colinfer_geometry;
 int colinfer_sample_geometry(int V, int dtype, const void* logits, int cluster, colinfer_geometry* out);
 
+/* Which bytes of `logits` [rows, V], counted from its start, the chunk kernel's bulk copies read of one row (for tests): whole
+ * units of 16 bytes around the row, never beyond the buffer's first and last byte (begin = end: none). */
+int colinfer_sample_copy_range(const void* logits, int dtype, int rows, int V, int row, int64_t* begin, int64_t* end);
+
 /* How many clusters of the sampler's geometry for this vocabulary the current device holds at once (occupancy query). */
 int colinfer_max_active_clusters(int V, int dtype);
 
