@@ -2075,14 +2075,17 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         // the chunk in fp32, penalties applied (its CTA has the tables), then masked
                         const char* base = rw.base;
                         const int al = rw.a;
-                        for (int p = lane; p < CHUNK; p += 32) {
-                            const int t = c * CHUNK + p - al;
-                            float x = CI_NEG_INF;
+                        float x[CHUNK / 32];                     // (loaded all at once)
+#pragma unroll
+                        for (int j = 0; j < CHUNK / 32; ++j) {
+                            const int p = j * 32 + lane, t = c * CHUNK + p - al;
+                            x[j] = CI_NEG_INF;
                             if (t >= 0 && t < V)
-                                x = ELT == 4 ? __ldcg(reinterpret_cast<const float*>(base) + c * CHUNK + p)
-                                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(base)[c * CHUNK + p]);
-                            xbuf[p] = x;
+                                x[j] = ELT == 4 ? __ldcg(reinterpret_cast<const float*>(base) + c * CHUNK + p)
+                                                : __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(base) + c * CHUNK + p) << 16);
                         }
+#pragma unroll
+                        for (int j = 0; j < CHUNK / 32; ++j) xbuf[j * 32 + lane] = x[j];
                         __syncwarp();
                         if (rw.pen_on) { const PenPeek pk = pen_peek(pen_tab(sc), rw.pen_cap, c, lane); if (pk.r0 != pk.r1) pen_patch(rw, smem_u32(xbuf), c, pk); }
                         const float lkf = fmaxf(rw.lcut, -SM_FLT_MAX);
