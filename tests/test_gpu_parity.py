@@ -23,8 +23,8 @@ MARGIN = 1e-6          # fp32 exponentials differ from float64 ones by ~1e-7 rel
 
 @pytest.fixture(autouse=True, params=["auto", "stream"])
 def _kernel_choice(request):
-    """Every test runs twice: with the automatic kernel choice (few rows: cluster-resident kernel, else the streaming
-    kernel) and with the streaming kernel forced, so that small cases cover both kernels."""
+    """Every test runs twice: with the automatic kernel choice (few rows: the cluster-resident kernel, as many rows as SMs: the
+    streaming kernel, more: the chunk kernel) and with the streaming kernel forced, so that small cases cover that one too."""
     assert torch.cuda.is_available(), "the gpu tests need a CUDA device"
     _lib.lib()
     _lib.default_kernel_flags = _lib.kernel_flags(0 if request.param == "auto" else -1)
@@ -596,7 +596,7 @@ def test_missed_band_estimate_retries_exactly(_kernel_choice):
     """The top-p band is an estimate; with the test hook it is misplaced (above the pivot on odd rows, below on even
     ones): the exact window pass must find the pivot's bucket and the tokens must not change."""
     if _kernel_choice != "stream":
-        pytest.skip("the hook belongs to the streaming kernel")
+        pytest.skip("the other kernels: test_recovery_paths.py")
     m = mods()
     V = wl.V_QWEN
     w = wl.config3(32)
