@@ -72,7 +72,6 @@ constexpr int FB_NB = 256;           // radix buckets per level of the fallback 
 constexpr int PEN_TABLE = 2048;      // distinct history ids with an O(1) count
 constexpr int LIST_MAX = 1400;       // logits a list selection may hold
 constexpr int BAL_ROWS = 16384;      // launches up to this many rows deal their rows to the CTAs by cost class
-constexpr int MAX_V = 524288;
 constexpr long long WAIT_CYCLES = 400000000LL;
 #define SM_FLT_MAX 3.402823466e38f
 #define SM_POS_INF (__int_as_float(0x7f800000))
@@ -132,7 +131,7 @@ struct Sc {
     float4 pub;                        // the CTA's maximum, its lowest token, tw and flags
     float tw; int flags;               // 1 list overflow or no bound, 2 a wait ran out, 4 histogram not counted
     int wn[NW];
-    u64 g_all[NW], g_keep[NW];
+    u64 g_all[NW];
     u64 t_cnt, t_est, sum_off;         // totals of the CTA's share of the histogram; what the estimates are off by
     u64 sum_all, sum_keep;             // masses of the CTA's chunks
     int nsel, npush;                   // candidates selected, candidates sent to the group's first CTA
@@ -250,13 +249,6 @@ __device__ __forceinline__ u64 ceil_target(float frac, u64 total) {
     const double t = ceil((double)frac * (double)total);
     u64 q = t <= 1.0 ? 1ull : (u64)t;
     return q > total ? total : q;
-}
-
-// Bucket of a logit: floor((href - x) * scale) + hoff clamped to [0, NB1), as a rounding float add (no conversion
-// instruction).  A logit exactly on an edge may land in either neighbour; every user keeps a whole bucket of margin.
-__device__ __forceinline__ int fine_bucket(float x, float href, float scale, float hoff_minus_half) {
-    const float t = fminf(fmaxf(fmaf(href - x, scale, hoff_minus_half), 0.0f), (float)(NB1 - 1));
-    return __float_as_int(t + 8388608.0f) - 0x4B000000;
 }
 
 // Bin of a BINS-bin count histogram in which the running count reaches kk, or -1; computed by the calling warp alone, eight
