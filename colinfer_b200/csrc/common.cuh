@@ -52,30 +52,34 @@ __device__ __forceinline__ float lower_logit_for(float zt, float tc, float start
     return key2f(k);
 }
 
+// l / tc by two fused multiply-adds with r = 1 / tc rounded to nearest: q0 = l r, then q0 + (l - q0 tc) r.  One correction step
+// after P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990);
+// for a divisor known beforehand N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating correctly rounded floating-point division
+// when the divisor is known in advance", IEEE Trans. Comput. 53 (2004).  It gives the IEEE quotient where nothing under- or
+// overflows on the way; a divisor whose significand is all ones may leave it one unit off.
+__device__ __forceinline__ float quotient(float l, float tc, float r) {
+    const float q0 = l * r;
+    return fmaf(fmaf(-q0, tc, l), r, q0);
+}
+
 // Kept mass of one element in units of 2^-30: exp(z - m), z = l / tc.  The same function feeds every histogram and
 // every prefix sum, so all sums are exact integer sums of the same addends (order independent, reproducible).
-// The division is the two-FMA sequence q = l * r, q += fma(-q, tc, l) * r with r = 1 / tc rounded to nearest, which
-// gives the IEEE quotient for every operand in range (it can be one unit off only when tc's significand is all ones);
-// it only feeds masses -- thresholds and ties always use the exact division.  The exponential is the hardware
+// The division (quotient) only feeds masses -- thresholds and ties always use the exact one.  The exponential is the hardware
 // ex2.approx (relative error ~2^-22); results below 2^-31 round to zero mass.
 struct MassFn {
     float tc, rinv, m;
     __device__ __forceinline__ void init(float tc_, float m_) { tc = tc_; rinv = __frcp_rn(tc_); m = m_; }
     __device__ __forceinline__ uint32_t operator()(float l) const {
-        const float q0 = l * rinv;
-        const float z = fmaf(fmaf(-q0, tc, l), rinv, q0);
         float e;
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((z - m) * CI_LOG2E));
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((quotient(l, tc, rinv) - m) * CI_LOG2E));
         return __float2uint_rn(e * CI_MASS_SCALE);
     }
     // Four masses at once (0 for logits below lk); the same values as operator().
     __device__ __forceinline__ void four(const float (&l)[4], float lk, uint32_t (&q)[4]) const {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float q0 = l[j] * rinv;
-            const float z = fmaf(fmaf(-q0, tc, l[j]), rinv, q0);
             float e;
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((z - m) * CI_LOG2E));
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((quotient(l[j], tc, rinv) - m) * CI_LOG2E));
             q[j] = l[j] >= lk ? __float2uint_rn(e * CI_MASS_SCALE) : 0u;
         }
     }
@@ -88,6 +92,12 @@ __device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0,
 __device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
+// quotient() of a pair; ntc: -tc.
+__device__ __forceinline__ u64 quotient2(u64 l, u64 ntc, u64 r) {
+    const u64 q0 = mul2(l, r);
+    return fma2(fma2(q0, ntc, l), r, q0);
+}
+
 // The masses of MassFn for pairs of logits, each as two floats: mass = (hi * 2^15 + lo * 2^-15) * 2^15 with hi a multiple of
 // 2^-15 and lo an integer, |lo| <= 2^14.  The arithmetic is MassFn's, operation by operation, two logits per instruction;
 // rounding the exponential to a multiple of 2^-30 takes two rounding additions instead of a conversion, which would double
@@ -96,9 +106,7 @@ struct Mass2 {
     u64 rinv, ntc, nm;
     __device__ __forceinline__ void init(const MassFn& f) { rinv = pk2(f.rinv, f.rinv); ntc = pk2(-f.tc, -f.tc); nm = pk2(-f.m, -f.m); }
     __device__ __forceinline__ void operator()(float l0, float l1, u64& hi, u64& lo) const {
-        const u64 l = pk2(l0, l1);
-        const u64 q0 = mul2(l, rinv);
-        const u64 z = fma2(fma2(q0, ntc, l), rinv, q0);
+        const u64 z = quotient2(pk2(l0, l1), ntc, rinv);
         float y0, y1, e0, e1;
         up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));
@@ -110,9 +118,7 @@ struct Mass2 {
     }
     // The masses as whole numbers, 0 for logits below lk: the bits of the two rounding sums, put together.
     __device__ __forceinline__ void whole(float l0, float l1, float lk, uint32_t& m0, uint32_t& m1) const {
-        const u64 l = pk2(l0, l1);
-        const u64 q0 = mul2(l, rinv);
-        const u64 z = fma2(fma2(q0, ntc, l), rinv, q0);
+        const u64 z = quotient2(pk2(l0, l1), ntc, rinv);
         float y0, y1, e0, e1;
         up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));

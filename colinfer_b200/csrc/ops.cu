@@ -449,15 +449,13 @@ struct Residual {
     __device__ void init(const colinfer_row_stats& st_, const colinfer_row_stats& sd_) {
         st = st_; sd = sd_;
         mt = scale_logit(st.lmax, st.tc); md = scale_logit(sd.lmax, sd.tc);
-        // (the two-step division of MassFn: the IEEE quotient unless the divisor's significand is all ones)
         rt = __frcp_rn(st.tc); rd = __frcp_rn(sd.tc);
         fast = (__float_as_uint(st.tc) & 0x7FFFFFu) != 0x7FFFFFu && (__float_as_uint(sd.tc) & 0x7FFFFFu) != 0x7FFFFFu;
         inv_t = (float)(1.0 / ((double)st.mass_q * CI_MASS_INV)); inv_d = (float)(1.0 / ((double)sd.mass_q * CI_MASS_INV));
     }
     __device__ __forceinline__ float div(float l, float tc, float r) const {
         if (!fast || !(fabsf(l) < 1e30f) || fabsf(l) < 1e-30f) return scale_logit(l, tc);
-        const float q0 = l * r;
-        return fmaf(fmaf(-q0, tc, l), r, q0);
+        return quotient(l, tc, r);                                     // (the same value: common.cuh)
     }
     __device__ __forceinline__ u64 operator()(float lt, float ld) const {
         if (!(lt >= st.lcut && lt > CI_NEG_INF)) return 0ull;          // no target probability: no residual
