@@ -649,7 +649,9 @@ __device__ __noinline__ bool finish_pending(const SampleArgs& a, const Pending& 
     return true;
 }
 
-extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __grid_constant__ SampleArgs a) {
+// EIGHT: clusters of eight, whose lists have CI_WLIST entries a warp (a size known only at launch cost them 2 %).
+template <bool EIGHT>
+__global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __grid_constant__ SampleArgs a) {
     cg::cluster_group cluster = cg::this_cluster();
     // Every CTA announces that it runs; the matching wait comes just before the first write into a peer's shared memory.
     cluster.barrier_arrive();
@@ -674,11 +676,11 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     uint32_t* cand = reinterpret_cast<uint32_t*>(hreg + CI_NB1 * 4 + CI_SEL_BINS * 8);
     u64* fb_hist = reinterpret_cast<u64*>(hreg);                              // fallback radix, over hist1
     u64* fb_seg = fb_hist + CI_FB_NB;
-    Cand* ownlist = reinterpret_cast<Cand*>(hreg + 24 * 1024);                // [CI_WARPS][list_cap] this CTA's lists
-    Cand* plist = ownlist + CI_WARPS * a.list_cap;                              // [8][CI_PCAP] candidates pushed by the cluster
+    Cand* plist = reinterpret_cast<Cand*>(hreg + 24 * 1024);                  // [8][CI_PCAP] candidates pushed by the cluster
     u64* mbar = reinterpret_cast<u64*>(plist + 8 * CI_PCAP);
     Xch* xch = reinterpret_cast<Xch*>(mbar + CI_MAX_CHUNKS);
     Scratch* sc = reinterpret_cast<Scratch*>(xch + 1);
+    Cand* ownlist = reinterpret_cast<Cand*>(sc + 1);                          // [CI_WARPS][list_cap] this CTA's lists: last, so that the others lie at fixed offsets
     // penalty tables alias the work area (used before the first histogram)
     uint32_t* pen_bits = reinterpret_cast<uint32_t*>(hreg);
     const int nw = slice_cap >> 5;
@@ -963,7 +965,7 @@ extern "C" __global__ void __launch_bounds__(CI_THREADS, 1) k_sample(const __gri
     // order inside a region is (step, lane, component).
     const int reg = ((n_pad / 128 + CI_WARPS - 1) / CI_WARPS) * 128;
     const int r_lo = min(warp * reg, n_pad), r_hi = min(r_lo + reg, n_pad);
-    const int list_cap = a.list_cap;
+    const int list_cap = EIGHT ? CI_WLIST : a.list_cap;
     Cand* mylist = ownlist + warp * list_cap;
 
     // ---------------------------------------------------------------------------------------- small top-k: candidates of the slice
@@ -1504,9 +1506,10 @@ static const int kFixedSmem = 24 * 1024 + (CI_WARPS * CI_WLIST + 8 * CI_PCAP) * 
                               (int)sizeof(Xch) + (int)sizeof(Scratch) + 64;
 
 static const int kMaxSmem = 226 * 1024;                    // of any geometry
-static cudaError_t sample_opt_in() {
-    static SmemOptIn opt_in;
-    return opt_in((const void*)k_sample, kMaxSmem);
+static const void* sample_kernel(int cluster) { return cluster == 8 ? (const void*)k_sample<true> : (const void*)k_sample<false>; }
+static cudaError_t sample_opt_in(int cluster) {
+    static SmemOptIn opt_in[2];
+    return opt_in[cluster == 8](sample_kernel(cluster), kMaxSmem);
 }
 
 // List entries per warp: what clusters of eight hold in 128 warps, spread over fewer, as far as the slice leaves room.  With 24 a
@@ -1578,11 +1581,11 @@ static int active_clusters(const colinfer_geometry& g) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     return known(((uint64_t)dev << 32) | ((uint64_t)g.cluster << 24) | (uint64_t)g.smem_bytes, [&]() {
-        if (sample_opt_in() != cudaSuccess) return -2;
+        if (sample_opt_in(g.cluster) != cudaSuccess) return -2;
         cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
         fill_launch(cfg, attr, g, 1024, nullptr);
         int n = 0;
-        return cudaOccupancyMaxActiveClusters(&n, k_sample, &cfg) == cudaSuccess && n > 0 ? n : -3;
+        return cudaOccupancyMaxActiveClusters(&n, sample_kernel(g.cluster), &cfg) == cudaSuccess && n > 0 ? n : -3;
     });
 }
 
@@ -1775,13 +1778,12 @@ static int sample_rows(const void* logits, const void* logits2, int dtype, const
     a.B = B; a.R = R; a.V = V; a.slice_elems = g.slice_elems; a.list_cap = list_cap(g.cluster, g.slice_elems); a.flags = flags; a.second = second;
     colinfer_profile_buffer(&a.prof, &a.prof_slots);
 
-    cudaError_t e = sample_opt_in();
+    cudaError_t e = sample_opt_in(g.cluster);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[1];
     fill_launch(cfg, attr, g, clusters, (cudaStream_t)stream);
-    e = cudaLaunchKernelEx(&cfg, k_sample, a);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaGetLastError();
+    void* args[] = {&a};
+    return (int)cudaLaunchKernelExC(&cfg, sample_kernel(g.cluster), args);
 }
 
 extern "C" int colinfer_sample(const void* logits, int dtype, const int32_t* mask, int mask_rows, int W,

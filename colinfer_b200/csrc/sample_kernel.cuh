@@ -441,10 +441,11 @@ __device__ __forceinline__ uint32_t chunk_bytes(const char* p, uint32_t end) {
     const uint32_t left = (end & ~15u) - (uint32_t)reinterpret_cast<u64>(p);
     return left < (uint32_t)(CHUNK * ELT) ? left : (uint32_t)(CHUNK * ELT);
 }
-// Asks for the first chunks of row `key`, as far as they are not under way.  (Out of line: every pass starts and ends with it,
-// and what it needs would be spilled there.)
+// Asks for the first chunks of row `key`, as far as they are not under way.  Every pass starts and ends with it: out of line where
+// a thread has 64 registers and what it needs would be spilled (200 fp32 rows of 151,936 without a filter 78 us inline, 74 us so),
+// inline in the kernels of clusters (21 rows of 217,408, top_k 50: 25 us out of line, 24 us so).
 template <int ELT>
-static __device__ __noinline__ void ring_start(int key, const char* base, uint32_t end, int Nc, int gw, int GW, bool keep) {
+__device__ __forceinline__ void ring_start_here(int key, const char* base, uint32_t end, int Nc, int gw, int GW, bool keep) {
     Pipe<ELT> p;
     p.expect(key);
     for (int c = gw + p.out * GW; p.out < NST && c < Nc; c += GW) {
@@ -453,6 +454,15 @@ static __device__ __noinline__ void ring_start(int key, const char* base, uint32
         p.issue(q + skip, bytes > skip ? bytes - skip : 0u, l2_policy(keep), skip);
     }
     p.save(key);
+}
+template <int ELT>
+static __device__ __noinline__ void ring_start_call(int key, const char* base, uint32_t end, int Nc, int gw, int GW, bool keep) {
+    ring_start_here<ELT>(key, base, end, Nc, gw, GW, keep);
+}
+template <bool CL, int ELT>
+__device__ __forceinline__ void ring_start(int key, const char* base, uint32_t end, int Nc, int gw, int GW, bool keep) {
+    if constexpr (CL) ring_start_here<ELT>(key, base, end, Nc, gw, GW, keep);
+    else ring_start_call<ELT>(key, base, end, Nc, gw, GW, keep);
 }
 
 // The mask word of one lane for chunk c: words (512 c - a) / 32 + lane, lanes 0 .. 16.
@@ -564,7 +574,7 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
     const int gw = (CL ? sc->rank * NW : 0) + warp_id();
     const int Nc = rw.Nc;
     const bool pen_on = rw.pen_on != 0;
-    ring_start<ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, keep);
+    ring_start<CL, ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, keep);
     Pipe<ELT> p;
     const u64 pol = l2_policy(keep);
     int cn = gw + p.out * GW;                                            // the next chunk to ask for (no more a row's first)
@@ -598,8 +608,8 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
     // the first chunks of what comes next
     const int nkey = *(volatile const int*)&nx.key;
     __threadfence_block();
-    if (then == THEN_AGAIN) ring_start<ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, false);
-    else if (then == THEN_NEXT_ROW && nkey) ring_start<ELT>(nkey, nx.base, nx.end, nx.Nc, gw, GW, true);
+    if (then == THEN_AGAIN) ring_start<CL, ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, false);
+    else if (then == THEN_NEXT_ROW && nkey) ring_start<CL, ELT>(nkey, nx.base, nx.end, nx.Nc, gw, GW, true);
 }
 
 // Appends the logits of the chunk selected by the lanes' masks mk to the warp's list (no particular order).
@@ -1381,14 +1391,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         }
     }
     __syncthreads();
-    ring_start<ELT>(sc->rows[0].key, sc->rows[0].base, sc->rows[0].end, sc->rows[0].Nc, gw, GW, true);   // the logits travel while the parameters do
+    ring_start<CL, ELT>(sc->rows[0].key, sc->rows[0].base, sc->rows[0].end, sc->rows[0].Nc, gw, GW, true);   // the logits travel while the parameters do
     if (warp == PW) derive(0);
     __syncthreads();
 
     for (int it = 0; ; ++it) {
         RowS& rw = sc->rows[it & 1];
         const NextRow& nx = sc->next[it & 1];
-        ring_start<ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW, true);
+        ring_start<CL, ELT>(rw.key, rw.base, rw.end, rw.Nc, gw, GW, true);
         bool asked = false, found = false, derived = false;      // (the last warp's)
         // (A row of several passes asks when its first one is through: the CTAs that ask before it have less left to do.)
         auto ask = [&]() { if (!CL && warp == PW && !asked) { if (lane == 0) queue_ask(sc); asked = true; } };
