@@ -528,7 +528,7 @@ def main():
                     help="N > 1: how the sampled ids are gathered -- peer: one small kernel that stores them into every rank's "
                          "buffer over NVLink (falls back to nccl when peer memory cannot be mapped); nccl: all_gather")
     ap.add_argument("--cluster", type=int, default=0,
-                    help="0: automatic (few rows: cluster-resident kernel, else the streaming kernel); -1: streaming kernel; "
+                    help="0: automatic (few rows: cluster-resident kernel, about a row per SM: streaming kernel, else the chunk kernel); -1: streaming kernel; "
                          "1/2/4/8: the cluster-resident kernel with that cluster size")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3) if args.impl == "ours" else args.warmup
@@ -699,7 +699,7 @@ def main():
 
     if rank == 0:
         # which kernel colinfer_sample ran: few rows (at most the clusters the device holds at once) take the
-        # cluster-resident kernel, more rows the streaming kernel; --cluster forces one of them
+        # cluster-resident kernel, more rows the chunk or the streaming kernel; --cluster forces one of them
         few = B <= lib.colinfer_max_active_clusters(V, _lib.F32)
         kernel_name = "k_sample (cluster-resident)" if args.cluster > 0 or (args.cluster == 0 and few) else "k_sample_stream" if args.cluster < 0 else kernel_of(B, 0)
         peak, peak_kind = measured_peak()

@@ -22,8 +22,8 @@
 // If a list would overflow, or the estimated band misses the true pivot, an exact select over the order-preserving 32-bit keys
 // runs instead: a pass over the resident slices per 1,024-fold narrowing (slower, same result).
 //
-// What bounds it is latency: one row's chain of block-wide steps, and code that every step executes for the first time (a third of
-// the stalls are instruction fetches), not bytes.  So: one CTA of 512 threads per SM (with 256 the passes over a slice took
+// What bounds it is latency: one row's chain of block-wide steps, and code that every step executes for the first time, not bytes
+// (one row, top_k 50: of the warps' stall cycles 43 % are waits at barriers, 23 % instruction fetches).  So: one CTA of 512 threads per SM (with 256 the passes over a slice took
 // twice as long, at 1,024 there are too few registers), searches repeated by every warp instead of published by one, sums pushed to the peers before a
 // barrier instead of fetched after it, masses two logits per instruction, 64-bit shared-memory additions as 32-bit ones with a
 // carry.  One fp32 row of 151,936 logits on a B200, device time: top_k 100 23.1 -> 16.5 us, top-p alone 33.5 -> 26 us, no filter
@@ -57,7 +57,7 @@
 #define CI_WLIST 24              // list entries per warp of a cluster of eight (in smaller ones as many more as there are fewer warps: SampleArgs::list_cap)
 #define CI_GLIST 1365            // gathered list entries (16 KB)
 #define CI_SEL_BINS 256          // coarse bins of the exact selection on a gathered list
-#define CI_FB_NB 1024             // radix buckets per level of the fallback select (8 bits)
+#define CI_FB_NB 1024             // buckets per level of the fallback select
 #define CI_MAX_CAND 128          // tied / neighbouring candidates examined one by one in the final list step
 #define CI_PEN_TABLE 2048        // distinct history ids per slice with an O(1) count
 #define CI_WAIT_CYCLES 400000000LL
@@ -1610,8 +1610,11 @@ namespace {
 constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024;
 // More rows than SMs: two CTAs of 512 threads per SM, one of which reads while the other one is in its block-wide steps; or one of
 // 1,024 where two do not fit (penalty tables of large vocabularies: 512 bf16 rows of 262,144 logits with histories 222 -> 174 us),
-// and for bf16 vocabularies beyond 229,376, whose rows have so many equal logits that the lists of 512 threads overflow (512 flat
-// rows of 262,144 with mixed filters 276 -> 249 us; of 201,792 it is 173 against 213).
+// and for bf16 vocabularies beyond 229,376.  There mixed filters (a top_p close to 1 among them) overflow the lists of 512 threads
+// with equal logits.  Time of one CTA per SM over that of two, mean of 160 to 592 rows, N(0, 2^2), mixed filters and the others:
+// 151,936 0.99 and 1.02 - 1.18; 201,792 0.91 and 0.97 - 1.13; 229,376 0.64 and 0.96 - 1.10; 262,144 0.58 and 0.95 - 1.08 (a row
+// without any filter loses 8 %).  How many are equal goes by the rows' spread too, which the host does not see: at N(0, 1) mixed
+// filters have it 0.59 at 151,936 already, under a grammar mask 0.93 there and 0.85 at 262,144.
 constexpr int kTwoPerSm = 113 * 1024, kRowV = 229376;
 
 // The sets of instantiations: a CTA of 512 threads per row, two per SM (ROWS); a CTA of 1,024 threads per row (ROW); a cluster of
@@ -1680,9 +1683,11 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
     }
     if (rows <= sms) {
         // At most a row per SM, more than the cluster-resident kernel holds at once: a cluster of two or four CTAs per row, where
-        // they all run at once.  64 fp32 rows of 151,936 logits with mixed filters and histories: 62 us, 73 us with the streaming
-        // kernel (a CTA per row, half of the SMs idle).  From 75 rows on there is one CTA per row either way, and the streaming
-        // kernel's 1,024 threads get a row through sooner.
+        // they all run at once.  From 75 rows on there is one CTA per row either way, and the streaming kernel's 1,024 threads get
+        // a row through sooner.  60 fp32 rows of 151,936 logits, streaming kernel (half of the SMs idle) and here: mixed filters 62
+        // and 53 us (64 rows with histories 73 and 61), top-p 60 and 53, top_k 50 36 and 27, top_k 1000 65 and 68, no filter 29 and 32,
+        // greedy 12 and 18; bf16 mixed 609 and 82, top-p 74 and 57, no filter 29 and 32.  The host does not see the filters: over
+        // mixed (twice), top_k 50, top_k 1000, top-p and half greedy it is 0.91 of the time.
         const int ki = chunk_index(FEW, dtype, mask != nullptr), smem = colinfer_few_smem(V, pen);
         if (smem > kChunkMaxSmem) return -1;
         const int rc = chunk_device(ki, &dev, &sms);
@@ -1691,6 +1696,10 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
             if (V >= 16384 * C && rows <= chunk_clusters(dev, ki, C, smem)) { set = FEW; break; }
         }
         if (set != FEW) return -1;
+        // More rows than SMs.  149 and 200 fp32 rows of 151,936, streaming kernel and here: mixed 66, 66 and 72, 77 us; top-p 124, 125
+        // and 104, 106; top_k 50 65, 83 and 41, 42; top_k 1000 124, 129 and 102, 114; no filter 63, 64 and 65, 74; greedy 29, 31 and
+        // 27, 36: over the same six 0.91 and 0.93 of the time (a wide row alone on an SM has half the threads here).  400 rows: mixed
+        // 115 and 107, top-p 183 and 165, no filter 97 and 133; 592: 166 and 140, 242 and 201, 132 and 138.
     } else if ((dtype == COLINFER_BF16 && V > kRowV) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
     const int smem = chunk_smem(set, V, pen), ki = chunk_index(set, dtype, mask != nullptr);
     if (smem > kChunkMaxSmem) return -1;
@@ -1712,8 +1721,9 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
 }
 }  // namespace
 
+static const int kMinSlice = 4096;                         // logits per CTA of a cluster at least
+
 // Both sets of rows (colinfer_second_rows), or -1 where only separate launches take them (nothing is launched then).
-static const int kMinSlice = 4096;
 static int sample_rows(const void* logits, const void* logits2, int dtype, const int32_t* mask, int mask_rows, int W,
                        const colinfer_sampler_params* params, const void* pos, int pos_is_i64, const float* u,
                        int64_t* out_ids, colinfer_row_stats* stats, int32_t* status,
@@ -1732,10 +1742,9 @@ static int sample_rows(const void* logits, const void* logits2, int dtype, const
     second.R = R2 > 0 ? R2 : 1; second.rows1 = R2 > 0 ? B * R : 0x7fffffff; second.rows = (int)rows;
     second.logits = R2 > 0 ? reinterpret_cast<const void*>((uintptr_t)logits2 - (uintptr_t)second.rows1 * V * (dtype == COLINFER_F32 ? 4 : 2)) : nullptr;
     // Which kernel: the caller's choice (bits COLINFER_KERNEL_* of flags), else automatic.  Few rows -- at most as many
-    // as the device holds clusters at once -- are a latency problem: one CTA per row would leave most SMs idle, so each
-    // row gets a whole 8-CTA cluster of the cluster-resident kernel.  More rows are a throughput problem: the streaming
-    // kernel (one CTA per row, later passes over L2).  The cluster-resident kernel also runs when a row's tables do not
-    // fit the streaming kernel.
+    // as the device holds clusters at once -- are a latency problem: each row gets a cluster of eight, four or two CTAs of the
+    // cluster-resident kernel.  More go to the chunk kernel, or, about a row per SM, to the streaming kernel (launch_chunk).  The
+    // cluster-resident kernel also runs when a row's tables do not fit the others.
     const int choice = (flags >> 8) & 7;                   // 0 auto, 1 streaming, 2 .. 5: clusters of 1, 2, 4, 8
     if (choice > 5) return (int)cudaErrorInvalidValue;
     int forced = choice >= 2 ? (1 << (choice - 2)) : 0;

@@ -1,5 +1,5 @@
 // sample_few.cu -- the fused kernel with a cluster of two or four CTAs per row, for launches of fewer rows than SMs: one CTA of 512
-// threads per SM with four chunks under way per warp.  64 rows of 151,936 fp32 logits with mixed filters and histories 74 -> 62 us
+// threads per SM with four chunks under way per warp.  64 rows of 151,936 fp32 logits with mixed filters and histories 74 -> 61 us
 // (with a CTA per row half of the SMs had none).
 #define SMP_NAME smp_few
 #define SMP_THREADS 512

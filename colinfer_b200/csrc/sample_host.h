@@ -1,4 +1,4 @@
-// sample_host.h -- what the host side of the fused kernel and its two sets of instantiations know of each other.
+// sample_host.h -- what the host side of the fused kernel and its three sets of instantiations know of each other.
 #pragma once
 #include "../../include/colinfer_b200.h"
 

@@ -28,8 +28,9 @@
 // What bounds it is instructions: 592 rows of 151,936 fp32 logits with mixed filters and histories issue in 61 % of the cycles, at
 // 30 % of DRAM's rate; the exact masses of a wide row take 16 instructions per logit, its histogram 10.  Hence masses two logits per
 // instruction with rounding additions instead of conversions, one histogram instead of a walk over radix levels, the draw from per-chunk sums.
-// 1,024 such rows: 342 us with one CTA of 1,024 threads per SM walking over the rows, 264 us here; 512 bf16 rows of 262,144 with a mask
-// 335 -> 242 us; 201 rows of 100,003 (no row but the first 16-byte aligned) 79 -> 62 us.
+// 1,024 such rows: 342 us with one CTA of 1,024 threads per SM walking over the rows, 258 us here; 512 bf16 rows of 262,144 with a mask
+// 353 -> 234 us; 201 rows of 100,003 (no row but the first 16-byte aligned) 80 -> 62 us.  Rows without a filter, and greedy ones, are
+// slower than there by up to a third (400 fp32 rows of 151,936: 97 -> 133 us, 47 -> 57 us).
 #pragma once
 #include <stddef.h>
 
