@@ -5,7 +5,7 @@
 #define SMP_THREADS 512
 #define SMP_CTAS 1
 #define SMP_STAGES 4
-#define SMP_LISTS 45056
+#define SMP_LISTS 65536
 #include "sample_kernel.cuh"
 
 const void* colinfer_few_kernel(int index) {

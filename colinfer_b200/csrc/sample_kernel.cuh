@@ -14,10 +14,11 @@
 //   greedy        one pass: maximum and its lowest index
 //   top_k <= 100  one pass.  The first chunk of every warp (the CTA's sample) bounds the k-th largest logit from below; the
 //                 pass lists what reaches the bound, the row is finished on the list
-//   top_p, large top_k   pass 1 also counts a 4096-bucket histogram laid out from the sample's maximum; it gives the bucket
-//                 of the k-th largest (the logits down to it are listed in a second pass and selected exactly), or, by
-//                 estimated masses, of the top-p pivot: pass 2 sums the exact masses, per chunk those above a narrow band
-//                 around the estimate, and lists the band, in which the pivot is found exactly
+//   larger top_k  a full histogram gives the bucket of the k-th largest, a second pass lists what reaches it, for an exact selection
+//   top_p         pass 1 also sums the row's mass (approximately) and counts a histogram, laid out from the sample's maximum: of
+//                 a quarter of the logits with a CTA per row, where the rows of an SM share its time, of all of them in a cluster.
+//                 They say where the top-p pivot lies: pass 2 sums the exact masses, per chunk those above a band around the
+//                 estimate, and lists the band, in which the pivot is found exactly
 //   neither       pass 2 sums the masses per chunk
 // The draw: the chunk in which the running kept mass reaches its target, then one warp inside that chunk.  Rows whose
 // listed logits hold all of their mass (peaked rows, an active min-p) are finished from the list after one pass.
@@ -25,12 +26,14 @@
 // the order of arrival nor on how many CTAs share a row.  Where a list overflows, a bound does not hold or the estimated
 // band misses the pivot, an exact select over the 32-bit keys runs (slower, same result).
 //
-// What bounds it is instructions: 592 rows of 151,936 fp32 logits with mixed filters and histories issue in 61 % of the cycles, at
-// 30 % of DRAM's rate; the exact masses of a wide row take 16 instructions per logit, its histogram 10.  Hence masses two logits per
-// instruction with rounding additions instead of conversions, one histogram instead of a walk over radix levels, the draw from per-chunk sums.
-// 1,024 such rows: 342 us with one CTA of 1,024 threads per SM walking over the rows, 258 us here; 512 bf16 rows of 262,144 with a mask
-// 353 -> 234 us; 201 rows of 100,003 (no row but the first 16-byte aligned) 80 -> 62 us.  Rows without a filter, and greedy ones, are
-// slower than there by up to a third (400 fp32 rows of 151,936: 97 -> 133 us, 47 -> 57 us).
+// What bounds it.  A pass over a row that is in HBM: bytes (592 greedy rows of 151,936 fp32 logits 64 us, of which 53 at the copy
+// rate).  A wide row: the second pass's instructions, and the chains of block-wide steps between the passes, a third of its
+// time, during which the SM's other row has the pipes to itself.  Hence masses two logits per instruction with rounding additions
+// instead of conversions, a histogram of a sample, one warp that decides and one that draws while searches are repeated by every warp
+// instead of published behind barriers.  A thread has 80 registers: with 64 (512 threads) the passes kept what a row needs in local
+// memory, which beside 226 KB of shared memory is L2, and two rows on an SM were slower than one after the other.
+// Before and now, one B200, 151,936 fp32 logits, us: 592 rows greedy 69 -> 64, without a filter 138 -> 125, top_p 203 -> 191,
+// top_k 50 81 -> 78, top_k 1000 251 -> 181; 360 bf16 rows with mixed filters 159 -> 100.
 #pragma once
 #include <stddef.h>
 
@@ -53,8 +56,8 @@ constexpr int CTAS_PER_SM = SMP_CTAS;
 constexpr int NST = SMP_STAGES;      // stages of a warp's ring
 constexpr int CHUNK = 512;           // logits per chunk: 16 per lane
 constexpr int RING = NST * 2048;     // bytes of ring per warp: a stage is 2 KB of fp32, or 1 KB of bf16 (and an fp32 copy of one chunk behind them)
-constexpr int NB1 = 4096;            // histogram buckets
-constexpr int HOFF = 1024;           // of these, above the sample's maximum
+constexpr int NB1 = 1024;            // histogram buckets
+constexpr int HOFF = 256;            // of these, above the sample's maximum (what lies above them counts in the first)
 constexpr float RANGE = 29.0f;       // they span RANGE temperatures: three quarters of that reach from the sample's maximum to the mass horizon
                                      // (what falls short of it is missing from the estimates: at 25, a row of T = 0.53 and top_p = 0.996 missed its band)
 constexpr int FASTK = 100;           // largest top_k finished from the sample's bound
@@ -63,15 +66,21 @@ constexpr float FAST_SCALE = 16.0f;  // sample bins per unit logit (16 units)
 constexpr int BINS_BYTES = 4096;     // two sets of counts (or one of weights, a chunk in fp32, the candidates)
 constexpr int U_BYTES = SMP_LISTS;   // lists, or histogram and lists
 constexpr int FCAP = 128;            // candidates of the one-warp finish
+constexpr int OFF_LISTS = NB1 * 4;   // lists behind a histogram
 constexpr int KCAP = U_BYTES / 8 / NW;                       // list entries per warp: rows without a histogram,
-constexpr int PUSH = 2048;           // candidates the CTAs of a cluster send to the first one, in equal shares
-constexpr int KCAP_CL = (U_BYTES - PUSH * 8) / 8 / NW;   // the same in a CTA of a cluster (behind the candidates of all CTAs),
-constexpr int WCAP = (U_BYTES - NB1 * 4) / 8 / NW;           // rows with one
-constexpr int GCAP = NB1 * 4 / 8 / NW;                       // entries per warp gathered from all CTAs of a cluster
-constexpr int FIN_CAND = 64;         // entries of one bin compared pairwise
+constexpr int WCAP = (U_BYTES - NB1 * 4) / 8 / NW;           // rows with one;
+// in a CTA of a cluster half of that, the other half being for what the CTAs of a cluster send each other:
+constexpr int GCAP = WCAP / 2;                               // entries per warp gathered from all CTAs,
+constexpr int OFF_GATHER = OFF_LISTS + GCAP * NW * 8;        // or the candidates sent to the first one, in equal shares
+constexpr int PUSH = 2048;
+constexpr int WCAP_CL = GCAP, KCAP_CL = OFF_GATHER / 8 / NW;
+static_assert(PUSH <= GCAP * NW || SMP_CTAS == 2 || SMP_THREADS == 1024, "candidates over the gathered entries");
+// A band is to hold this many logits on either side of the estimated pivot: a third of what the lists hold.
+constexpr int BAND_SIDE = 7 * KCAP * NW / 20 < 1200 ? 7 * KCAP * NW / 20 : 1200;
+constexpr int FIN_CAND = 128;        // entries of one bin compared pairwise
 constexpr int FB_NB = 256;           // radix buckets per level of the fallback select
 constexpr int PEN_TABLE = 2048;      // distinct history ids with an O(1) count
-constexpr int LIST_MAX = 1400;       // logits a list selection may hold
+constexpr int LIST_MAX = 2200;       // logits a list selection may hold
 constexpr int BAL_ROWS = 16384;      // launches up to this many rows deal their rows to the CTAs by cost class
 constexpr long long WAIT_CYCLES = 400000000LL;
 #define SM_FLT_MAX 3.402823466e38f
@@ -95,7 +104,7 @@ struct RowS {
     int cls;                           // ROW_* below
     float tc, topp, lmp, u; int kk;
     float scw;                         // histogram buckets per unit logit
-    float lref; int count_hist;        // the sample's maximum (the group's); pass 1 counts the histogram
+    float lref; int count_hist, hist_full;   // the sample's maximum (the group's); pass 1 counts the histogram, of all logits
     float L; int aidx, status;         // the row's maximum, the lowest token that has it
     int hist_ready;
     float lcut, horizon; int minp;     // smallest kept logit; the mass horizon; the cut lies above it
@@ -130,20 +139,18 @@ struct Sc {
     float wf[NW]; int wi[NW];
     int in_klist;                      // the lists of the row at hand take the histogram's place
     float4 pub;                        // the CTA's maximum, its lowest token, tw and flags
-    float tw; int flags;               // 1 list overflow or no bound, 2 a wait ran out, 4 histogram not counted
+    float tw; int flags;               // 1 list overflow or no bound, 2 a wait ran out, 4 histogram not counted, 8 mass out of range, 16 lists behind a histogram
     int wn[NW];
     u64 g_all[NW];
-    u64 t_cnt, t_est, sum_off;         // totals of the CTA's share of the histogram; what the estimates are off by
+    float est[NW];                     // the warps' shares of the row's mass relative to the sample's maximum
     u64 sum_all, sum_keep;             // masses of the CTA's chunks
     int nsel, npush;                   // candidates selected, candidates sent to the group's first CTA
     int ok; float fin_cut; u64 fin_total; int fin_token;
-    int fb[3]; u64 fe[3];              // finds of fine_decide
     // CTA-local
-    u64 wsum[NW], woff[NW], wtotal, wsum2[NW], woff2[NW];
+    u64 wsum[NW], woff[NW], wtotal;
     int found; u64 found_excl;
-    int ncand; float res_f; int sel_ok; uint32_t cand_kmin, cand_kmax;
-    float cand_l[FIN_CAND]; u64 cand_w[FIN_CAND];
-    int x_chunk; u64 x_before;
+    int ncand; uint32_t cand_kmin, cand_kmax;
+    float cand_l[FIN_CAND]; uint32_t cand_w[FIN_CAND];
 };
 
 // Candidates: as selected (over the sample's bins); by descending logit and by ascending token, with masses (over those of the
@@ -163,6 +170,7 @@ constexpr int OFF_BARS = (OFF_SC + (int)sizeof(Sc) + 15) & ~15;
 constexpr int OFF_U = (OFF_BARS + NW * 8 * NST + 127) & ~127;
 constexpr int OFF_BINS = OFF_U + U_BYTES;
 constexpr int OFF_CSUM = OFF_BINS + BINS_BYTES;
+static_assert(NB1 == 1024, "decide_row: 32 buckets per lane");
 static_assert(BINS_BYTES >= 2 * BINS * 4 && BINS_BYTES >= BINS * 8 && BINS_BYTES >= FB_NB * 8 && BINS_BYTES >= CHUNK * 4, "what lies over the bins");
 __host__ __device__ inline int max_chunks(int V) { return (V + 7 + CHUNK - 1) / CHUNK; }   // a row may start seven logits into its first chunk
 __host__ __device__ inline int pen_offset(int V, bool pen) {
@@ -309,6 +317,9 @@ __device__ __forceinline__ PenTab pen_tab(const Sc* sc) {
 }
 // The entries of one chunk, and a lane's first one, fetched a chunk ahead.
 struct PenPeek { uint32_t r0, r1, ent; };
+// A row's penalties, and how many entries its tables hold.
+struct PenVals { float rp, pp, fp; int cap; };
+__device__ __forceinline__ PenVals pen_vals(const RowS& rw) { return PenVals{rw.rp, rw.pp, rw.fp, rw.pen_cap}; }
 __device__ __forceinline__ PenPeek pen_peek(const PenTab& t, int cap, int c, int lane) {
     PenPeek k;
     k.r0 = t.pre[c]; k.r1 = t.pre[c + 1];
@@ -348,13 +359,13 @@ static __device__ __noinline__ void pen_patch_more(RowS& rw, uint32_t at, int c,
     }
 }
 // Replaces the penalised logits of chunk c (fp32, at shared address `at`) by their penalised values.  A warp calls.
-__device__ __forceinline__ void pen_patch(RowS& rw, uint32_t at, int c, const PenPeek& k) {
+__device__ __forceinline__ void pen_patch(RowS& rw, uint32_t at, int c, const PenPeek& k, const PenVals& v) {
     if (k.ent) {                                                         // (an entry counts at least one occurrence)
         const uint32_t q = at + 4 * (k.ent & 0xFFFFu);
         const float x = lds32(q);
-        if (x > CI_NEG_INF) sts32(q, apply_penalty(x, (int)(k.ent >> 16), rw.rp, rw.pp, rw.fp));
+        if (x > CI_NEG_INF) sts32(q, apply_penalty(x, (int)(k.ent >> 16), v.rp, v.pp, v.fp));
     }
-    if (k.r1 - k.r0 > 32 || k.r1 > (uint32_t)rw.pen_cap) pen_patch_more(rw, at, c, k.r0, k.r1);
+    if (k.r1 - k.r0 > 32 || k.r1 > (uint32_t)v.cap) pen_patch_more(rw, at, c, k.r0, k.r1);
     __syncwarp();
 }
 
@@ -383,7 +394,7 @@ struct Pipe {
     static constexpr int CHB = CHUNK * ELT;
     uint32_t buf, bar;                 // shared-memory addresses of the stages and of their barriers
     int cons, out;                     // chunks consumed, chunks under way
-    bool asks;                         // the lane that asks for chunks (none once a wait ran out)
+    bool asks;                         // the lane asks for chunks (no more once a wait ran out)
 
     __device__ __forceinline__ Pipe() {
         const int warp = warp_id();
@@ -391,23 +402,27 @@ struct Pipe {
         bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
         const Sc* sc = scratch();
         cons = sc->ring[warp].cons; out = sc->ring[warp].out;
-        asks = lane_id() == 0 && !(sc->drop | sc->dead);
+        asks = !(sc->drop | sc->dead);
     }
     __device__ __forceinline__ uint32_t conv() const { return buf + NST * CHB; }          // bf16: an fp32 copy of one chunk
     __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) % NST) * CHB; }
+    // Copies `bytes` to `dst`, counted on `bar`.  The warp calls, one lane acts (unless a wait of its own ran out).
+    __device__ __forceinline__ void copy(uint32_t dst, const char* p, uint32_t bytes, uint32_t bar, u64 pol) const {
+        asm volatile("{\n\t.reg .pred e, a;\n\tsetp.ne.u32 a, %5, 0;\n\telect.sync _|e, 0xffffffff;\n\tand.pred e, e, a;\n\t"
+                     "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
+                     "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n\t}"
+                     ::"r"(dst), "l"(p), "r"(bytes), "r"(bar), "l"(pol), "r"((uint32_t)asks) : "memory");
+    }
     // skip: bytes at the start of the stage that are left out
     __device__ __forceinline__ void issue(const char* p, uint32_t bytes, u64 pol, uint32_t skip = 0) {
-        if (asks) {
-            const uint32_t s = (uint32_t)(cons + out) % NST;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * s), "r"(bytes) : "memory");
-            if (bytes) asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-                         ::"r"(buf + s * CHB + skip), "l"(p), "r"(bytes), "r"(bar + 8 * s), "l"(pol) : "memory");
-        }
+        const uint32_t s = (uint32_t)(cons + out) % NST;
+        if (bytes) copy(buf + s * CHB + skip, p, bytes, bar + 8 * s, pol);
+        else if (lane_id() == 0 && asks) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar + 8 * s) : "memory");
         ++out;
     }
     // The bytes of the chunk j places from the next one to consume are there.
-    __device__ __forceinline__ void wait(int j = 0) {
-        const uint32_t b = bar + 8 * ((uint32_t)(cons + j) % NST), par = ((uint32_t)(cons + j) / NST) & 1u;
+    __device__ __forceinline__ void wait(int j = 0) { wait_at(bar + 8 * ((uint32_t)(cons + j) % NST), ((uint32_t)(cons + j) / NST) & 1u); }
+    __device__ __forceinline__ void wait_at(uint32_t b, uint32_t par) {
         auto test = [&]() {
             uint32_t ok;
             asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -417,11 +432,10 @@ struct Pipe {
         if (!test()) {
             // (with the test flag nothing was asked for: the wait runs out, once per CTA and warp)
             Sc* sc = scratch();
-            if (*(volatile int*)&sc->dead) return;
             const long long t0 = clock64();
-            while (!test()) if (clock64() - t0 > WAIT_CYCLES) { sc->dead = 1; asks = false; break; }
-            __syncwarp();
+            while (!test()) if (*(volatile int*)&sc->dead || clock64() - t0 > WAIT_CYCLES) { sc->dead = 1; asks = false; break; }
         }
+        __syncwarp();
     }
     // Between passes: what was asked for ahead stays when it belongs to row `key`, else it is let land and dropped.
     __device__ __forceinline__ void expect(int key) {
@@ -538,35 +552,36 @@ struct Chunk {
     }
 };
 
-// Prepares the chunk at stage `st`.  fresh: it has just arrived (its edges and, for fp32, its penalties are still to be
-// applied); wrote: the stage was changed.
+// The chunk at stage `st`, its edges mended; the penalties of a row with them: fp32 chunks in place, once (fresh), bf16 ones
+// through an fp32 copy at `conv`.
 template <int ELT, bool MASK>
-__device__ __forceinline__ Chunk<ELT, MASK> open_chunk(RowS& rw, uint32_t st, uint32_t conv, int c, bool fresh, bool pen, const PenPeek& pk, uint32_t mw, bool& wrote) {
-    const int lane = lane_id();
+__device__ __forceinline__ Chunk<ELT, MASK> open_chunk(const RowS& rw, uint32_t st, int c, uint32_t mw) {
     Chunk<ELT, MASK> k;
-    k.c = c; k.mw = mw; k.sh = (-rw.a) & 31; k.wide = ELT == 4;
-    wrote = false;
-    if (fresh && ((c == 0 && rw.a) || c == rw.Nc - 1)) { mend_edges<ELT>(rw, st, c); wrote = true; }
-    k.at = st + lane * 4 * ELT;
-    if (pen) {
-        if (ELT == 4) { if (fresh) { pen_patch(rw, st, c, pk); wrote = true; } }
-        else {                                                           // penalised values are fp32: through an fp32 copy of the chunk
-#pragma unroll
-            for (int j = 0; j < 4; ++j) sts128(conv + lane * 16 + j * 512, k.stored(j));
-            __syncwarp();
-            pen_patch(rw, conv, c, pk);
-            k.at = conv + lane * 16; k.wide = true;
-        }
-    }
+    k.c = c; k.mw = mw; k.sh = MASK ? (-rw.a) & 31 : 0; k.wide = ELT == 4;
+    k.at = st + lane_id() * 4 * ELT;
     return k;
+}
+template <int ELT, bool MASK>
+__device__ __forceinline__ void penalise(RowS& rw, Chunk<ELT, MASK>& k, uint32_t st, uint32_t conv, bool fresh, const PenPeek& pk, const PenVals& v) {
+    if (ELT == 4) { if (fresh) pen_patch(rw, st, k.c, pk, v); }
+    else {
+        const int lane = lane_id();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sts128(conv + lane * 16 + j * 512, k.stored(j));
+        __syncwarp();
+        pen_patch(rw, conv, k.c, pk, v);
+        k.at = conv + lane * 16; k.wide = true;
+    }
 }
 
 // What the ring asks for when a pass has asked for all of its own chunks.
 enum { THEN_NOTHING = 0, THEN_AGAIN = 1, THEN_NEXT_ROW = 2 };
 
-// One pass of the calling warp over its chunks of the row at hand: f(chunk) on every one.  keep: the row's L2
-// policy; seen: how many of its
-// first chunks have been read before (and lie in the ring as they were left).
+// One pass of the calling warp over its chunks of the row at hand: f(chunk) on every one.  keep: the row's L2 policy; seen: how
+// many of its first chunks have been read before (and lie in the ring as they were left).
+// A chunk is refilled where it lay: as long as there is more to ask for the ring is full, so the chunk asked for next belongs in the
+// stage just read.  The state of the ring is three registers, edges are one comparison, the copy is issued by an elected lane (known
+// to be one, its operands need no loop over lanes).
 template <bool CL, int ELT, bool MASK, class F>
 __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep, int seen, int then, F f) {
     constexpr int CHB = CHUNK * ELT;
@@ -578,8 +593,11 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
     ring_start<CL, ELT>(rw.key, rw.base, rw.end, Nc, gw, GW, keep);
     Pipe<ELT> p;
     const u64 pol = l2_policy(keep);
-    int cn = gw + p.out * GW;                                            // the next chunk to ask for (no more a row's first)
-    const char* next = rw.base + (size_t)cn * CHB;
+    const int n = gw < Nc ? (Nc - 1 - gw) / GW + 1 : 0;                  // chunks of the warp
+    const char* next = rw.base + (size_t)(gw + NST * GW) * CHB;          // the next chunk to ask for, and how many there are
+    int ask = max(n - NST, 0);
+    const int last = (Nc - 1) % GW == gw ? (int)chunk_bytes<ELT>(rw.base + (size_t)(Nc - 1) * CHB, rw.end) : CHB;   // bytes of the warp's last chunk
+    int edge = gw == 0 && rw.a ? 0 : Nc - 1;                             // the next chunk whose edges want mending
     uint32_t mw[MASK ? 3 : 1];                                           // mask words of this chunk and the next two
     if (MASK) {
 #pragma unroll
@@ -587,24 +605,51 @@ __device__ __forceinline__ void run_pass(RowS& rw, const NextRow& nx, bool keep,
     }
     PenPeek pk = {0, 0, 0};
     if (pen_on && gw < Nc) pk = pen_peek(pen_tab(sc), rw.pen_cap, gw, lane_id());
+    uint32_t s = (uint32_t)p.cons % NST, par = ((uint32_t)p.cons / NST) & 1u;
+    int c = gw;
+    auto loop = [&](auto pen) {
+        constexpr bool PEN = decltype(pen)::value;
+        const PenTab pt = pen_tab(sc);
+        const PenVals pv = PEN ? pen_vals(rw) : PenVals{};
+        uint32_t after0 = 0, after1 = 0;                                     // of the chunk after the next one
+        if (PEN && n > 1) { after0 = pt.pre[c + GW]; after1 = pt.pre[c + GW + 1]; }
 #pragma unroll 1
-    for (int c = gw; c < Nc; c += GW) {
-        if (seen == 0) p.wait();
-        bool wrote = false;
-        const PenPeek pcur = pk;
-        if (pen_on && c + GW < Nc) pk = pen_peek(pen_tab(sc), rw.pen_cap, c + GW, lane_id());
-        f(open_chunk<ELT, MASK>(rw, p.stage(), p.conv(), c, seen == 0, pen_on && pcur.r0 != pcur.r1, pcur, mw[0], wrote));
-        if (MASK) {
-            mw[0] = mw[MASK ? 1 : 0]; mw[MASK ? 1 : 0] = mw[MASK ? 2 : 0];
-            if (c + 3 * GW < Nc) mw[MASK ? 2 : 0] = mask_word(rw.mrow, sc->W, rw.a, c + 3 * GW, lane_id());
+        for (int left = n; left; --left) {
+            const uint32_t st = p.buf + s * CHB, bar = p.bar + 8 * s;
+            const bool fresh = seen <= 0;
+            bool wrote = !fresh;                                             // the stage was changed by ordinary stores
+            if (fresh) {
+                p.wait_at(bar, par);
+                if (c == edge) { mend_edges<ELT>(rw, st, c); wrote = true; }
+            }
+            if (c == edge) edge = Nc - 1;
+            --seen;
+            auto k = open_chunk<ELT, MASK>(rw, st, c, mw[0]);
+            if (PEN) {
+                const PenPeek cur = pk;
+                pk.r0 = after0; pk.r1 = after1;                          // (loads of which nothing waits in this turn)
+                pk.ent = left > 1 && after0 + lane_id() < min(after1, (uint32_t)pv.cap) ? pt.ent[after0 + lane_id()] : 0u;
+                if (left > 2) { after0 = pt.pre[c + 2 * GW]; after1 = pt.pre[c + 2 * GW + 1]; }
+                if (cur.r0 != cur.r1) { penalise(rw, k, st, p.conv(), fresh, cur, pv); wrote = true; }
+            }
+            f(k);
+            if (MASK) {
+                mw[0] = mw[MASK ? 1 : 0]; mw[MASK ? 1 : 0] = mw[MASK ? 2 : 0];
+                if (c + 3 * GW < Nc) mw[MASK ? 2 : 0] = mask_word(rw.mrow, sc->W, rw.a, c + 3 * GW, lane_id());
+            }
+            // gives the stage back (what the warp changed in it with ordinary stores comes before the next copy) and asks for more
+            if (wrote) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (ask) {
+                p.copy(st, next, --ask ? CHB : last, bar, pol);
+                next += (size_t)GW * CHB;
+            }
+            c += GW;
+            if (++s == NST) { s = 0; par ^= 1u; }
         }
-        // gives the stage back (what the warp changed in it with ordinary stores comes before the next copy) and asks for more
-        if (wrote || seen) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        seen = max(seen - 1, 0);
-        __syncwarp();
-        ++p.cons; --p.out;
-        if (cn < Nc) { p.issue(next, cn == Nc - 1 ? chunk_bytes<ELT>(next, rw.end) : CHB, pol); next += GW * CHB; cn += GW; }
-    }
+    };
+    if (pen_on) loop(BoolTag<true>{}); else loop(BoolTag<false>{});
+    p.cons += n; p.out = 0;
     p.save(rw.key);
     // the first chunks of what comes next
     const int nkey = *(volatile const int*)&nx.key;
@@ -697,53 +742,87 @@ struct Buckets {
     }
 };
 
-// The same with a count of the buckets of the logits >= from (what lies below, and -inf, cannot be kept).
-template <bool CL, int ELT, bool MASK>
-__device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap, float href, float scale, int hoff, float from) {
+// The same with a count of the buckets of the logits >= from (what lies below, and -inf, cannot be kept).  FULL: of all of them.
+// Else of a quarter of those that are not listed, one group of every lane and chunk, each counting four (the listed ones are added
+// when the pass is over), and with the mass of all logits relative to href (fp32, in `mass`): with that known, the quarter only has
+// to say how much mass lies below a logit, to which the largest logits, whose share a sample would miss, do not belong.  What is
+// left to the sample moves the estimated top-p pivot by about 200 places of 30,000 (standard deviation; N(0, 2^2), T = 0.5 - 1.2), a
+// fifth of what the band around it reaches to either side.
+// Counting all of a row takes 10 instructions per logit and a shared-memory addition per logit, the mass 2.
+constexpr uint32_t SAMPLED = 4;
+template <bool CL, int ELT, bool MASK, bool FULL, bool SUM>
+__device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool keep, int seen, int then, float t, Cand* list, int cap, float href, float scale, int hoff, float from, float tc, float& mass) {
     float lmax = CI_NEG_INF;
+    const float yc = CI_LOG2E / tc;
+    const u64 yk = pk2(yc, yc), y0 = pk2(-href * yc, -href * yc);
+    u64 sum = 0;
     const Buckets bk(href, scale, hoff);
     const uint32_t h0 = smem_u32(smem) + OFF_U - (0x4B000000u << 2);
     const u64 hr = pk2(href, href), k4 = pk2((float)(NB1 - 1), (float)(NB1 - 1)), mg = pk2(8388608.0f, 8388608.0f), neg = pk2(-1.0f, -1.0f);
     run_pass<CL, ELT, MASK>(rw, nx, keep, seen, then, [&](const auto& k) {
-        float m = CI_NEG_INF;
         auto count = [&](float x, float b) {
             const uint32_t at = h0 + (__float_as_uint(b) << 2);
-            asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p red.shared.add.u32 [%0], 1;\n\t}" ::"r"(at), "f"(x), "f"(from) : "memory");
+            if (FULL) asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p red.shared.add.u32 [%0], 1;\n\t}" ::"r"(at), "f"(x), "f"(from) : "memory");
+            else asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\tsetp.lt.and.f32 p, %1, %3, p;\n\t@p red.shared.add.u32 [%0], %4;\n\t}" ::"r"(at), "f"(x), "f"(from), "f"(t), "n"(SAMPLED) : "memory");
         };
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 v = k.group(j, CI_NEG_INF);
-            m = max4(v, m);
+        auto count4 = [&](const float4 v) {
             float d0, d1, d2, d3, b0, b1, b2, b3;
             up2(fma2(pk2(v.x, v.y), neg, hr), d0, d1);
             up2(fma2(pk2(v.z, v.w), neg, hr), d2, d3);
             up2(fma2(pk2(bk.sat(d0), bk.sat(d1)), k4, mg), b0, b1);
             up2(fma2(pk2(bk.sat(d2), bk.sat(d3)), k4, mg), b2, b3);
             count(v.x, b0); count(v.y, b1); count(v.z, b2); count(v.w, b3);
+        };
+        float m = CI_NEG_INF;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = k.group(j, CI_NEG_INF);
+            m = max4(v, m);
+            if (FULL) count4(v);
+            if (SUM) {
+                float a0, a1, a2, a3;
+                up2(fma2(pk2(v.x, v.y), yk, y0), a0, a1);
+                up2(fma2(pk2(v.z, v.w), yk, y0), a2, a3);
+                asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a0)); asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a1));
+                asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a2)); asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a3));
+                sum = add2(sum, add2(pk2(a0, a1), pk2(a2, a3)));
+            }
         }
+        if (!FULL) count4(k.group(k.c & 3, CI_NEG_INF));
         lmax = fmaxf(lmax, m);
         list_above(rw.a, list, cap, t, m >= t, k);
     });
+    float s0, s1;
+    up2(sum, s0, s1);
+    mass = s0 + s1;
     return lmax;
 }
 
 // The mass pass: per chunk the mass of the logits >= lk (BAND: of those above t_hi) into csum, and, BAND, the logits of
 // [tl, t_hi] into the warp's list and the mass of all logits >= lk.  MINP: lk may lie above the mass horizon.
-// What bounds it: ~ 12 issue slots and one exponential per logit (an SM has 4 and 1/2 per cycle and 32 logits).
+// The masses are MassFn's, operation by operation: rounded to a multiple of 2^-15 (t, a float at 384) and the rest to 2^-30 (w, at
+// 12582912), whose bits are summed as integers.  What bounds it is issue and the pipes about alike: two logits take 10 packed
+// instructions of two cycles, two exponentials of eight, and, BAND, 12 compares, selects and additions.
 struct Masses { u64 all, keep; };
+// Above t_hi: the two parts of a mass to their sums; from tl on: the logit's bit to the mask.  Five instructions without a branch.
+__device__ __forceinline__ void band_add(float x, float t_hi, float tl, float hi, uint32_t lo, uint32_t bit, float& sh, uint32_t& sl, uint32_t& mk) {
+    asm("{\n\t.reg .pred p, q;\n\tsetp.gt.f32 p, %3, %4;\n\tsetp.ge.and.f32 q, %3, %5, !p;\n\t"
+        "@p add.f32 %0, %0, %6;\n\t@p add.u32 %1, %1, %7;\n\t@q or.b32 %2, %2, %8;\n\t}"
+        : "+f"(sh), "+r"(sl), "+r"(mk) : "f"(x), "f"(t_hi), "f"(tl), "f"(hi), "r"(lo), "r"(bit));
+}
 template <bool CL, int ELT, bool MASK, bool BAND, bool MINP>
 __device__ __forceinline__ Masses pass_mass(RowS& rw, const NextRow& nx, int then, MassFn mass, float lk, float t_hi, float tl, Cand* list, u64* csum) {
-    Mass2 m2;
-    m2.init(mass);
+    const u64 rinv = pk2(mass.rinv, mass.rinv), ntc = pk2(-mass.tc, -mass.tc), nm = pk2(-mass.m, -mass.m);
     u64 keep = 0;
     int all_h = 0, all_l = 0;
     run_pass<CL, ELT, MASK>(rw, nx, false, 0, then, [&](const auto& k) {
         bool mend = MINP;
-        u64 sh, sl;                                                      // sums of the chunk: exact (multiples of 2^-15 up to 16, integers up to 2^18)
-        float ah, al, s0, s1;
+        u64 sh;                                                          // sums of the chunk: exact (multiples of 2^-15 up to 16, integers up to 2^18)
+        uint32_t sl, al;
+        float ah, s0, s1;
         unsigned mk;
         while (true) {
-            sh = sl = 0; ah = al = 0.0f; mk = 0;
+            sh = 0; sl = al = 0; ah = 0.0f; mk = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 float4 v = k.group(j, SM_LOW);
@@ -751,37 +830,40 @@ __device__ __forceinline__ Masses pass_mass(RowS& rw, const NextRow& nx, int the
                     v.x = v.x >= lk ? v.x : SM_LOW; v.y = v.y >= lk ? v.y : SM_LOW;
                     v.z = v.z >= lk ? v.z : SM_LOW; v.w = v.w >= lk ? v.w : SM_LOW;
                 }
-                u64 hi, lo;
-                float h0, h1, l0, l1;
-                m2(v.x, v.y, hi, lo);
-                sh = add2(sh, hi); sl = add2(sl, lo);
-                if (BAND) {
-                    up2(hi, h0, h1); up2(lo, l0, l1);
-                    if (v.x > t_hi) { ah += h0; al += l0; } else if (v.x >= tl) mk |= 1u << (4 * j);
-                    if (v.y > t_hi) { ah += h1; al += l1; } else if (v.y >= tl) mk |= 2u << (4 * j);
-                }
-                m2(v.z, v.w, hi, lo);
-                sh = add2(sh, hi); sl = add2(sl, lo);
-                if (BAND) {
-                    up2(hi, h0, h1); up2(lo, l0, l1);
-                    if (v.z > t_hi) { ah += h0; al += l0; } else if (v.z >= tl) mk |= 4u << (4 * j);
-                    if (v.w > t_hi) { ah += h1; al += l1; } else if (v.w >= tl) mk |= 8u << (4 * j);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float x0 = h ? v.z : v.x, x1 = h ? v.w : v.y;
+                    const u64 z = quotient2(pk2(x0, x1), ntc, rinv);
+                    float y0, y1, e0, e1, h0, h1;
+                    up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(y1));
+                    const u64 e = pk2(e0, e1), hi = add2(add2(e, pk2(384.0f, 384.0f)), pk2(-384.0f, -384.0f));
+                    const u64 w = fma2(fma2(hi, pk2(-1.0f, -1.0f), e), pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f));
+                    const uint32_t w0 = (uint32_t)w, w1 = (uint32_t)(w >> 32);
+                    sh = add2(sh, hi);
+                    sl += w0 + w1;
+                    if (BAND) {
+                        up2(hi, h0, h1);
+                        band_add(x0, t_hi, tl, h0, w0, 1u << (4 * j + 2 * h), ah, al, mk);
+                        band_add(x1, t_hi, tl, h1, w1, 2u << (4 * j + 2 * h), ah, al, mk);
+                    }
                 }
             }
             up2(sh, s0, s1);
             if (MINP || mend || !__any_sync(0xffffffffu, !(s0 + s1 < 1e9f))) break;
             mend = true;                                                 // a logit of -inf: once more
         }
-        float r0, r1;
-        up2(sl, r0, r1);
-        const int ch = __float2int_rn((s0 + s1) * 32768.0f), cl = __float2int_rn(r0 + r1);
+        // (12582912's bits are a multiple of 2^22: below that stands the sum of the rests)
+        static_assert((0x4B400000u & 0x3FFFFFu) == 0, "the bits of 12582912");
+        const int ch = __float2int_rn((s0 + s1) * 32768.0f), cl = (int)(sl << 10) >> 10;
         if (BAND) { all_h += ch; all_l += cl; }
         const uint32_t wh = __reduce_add_sync(0xffffffffu, (unsigned)(BAND ? __float2int_rn(ah * 32768.0f) : ch));
-        const int wl = (int)__reduce_add_sync(0xffffffffu, (unsigned)(BAND ? __float2int_rn(al) : cl));
+        const int wl = (int)__reduce_add_sync(0xffffffffu, (unsigned)(BAND ? (int)(al << 10) >> 10 : cl));
         const u64 q = ((u64)wh << 15) + (u64)(long long)wl;
         if (lane_id() == 0) csum[k.c] = q;
         keep += q;
-        if (BAND) list_append(rw.a, list, CL ? WCAP : KCAP, mk, k);
+        if (BAND) list_append(rw.a, list, CL ? WCAP_CL : KCAP, mk, k);
     });
     Masses r;
     r.keep = keep;
@@ -866,7 +948,11 @@ static __device__ __noinline__ int argmax_pass(RowS& rw, const NextRow& nx, floa
 // The histogram counted from the row's maximum.
 template <bool CL, int ELT, bool MASK>
 static __device__ __noinline__ void recount_pass(RowS& rw, const NextRow& nx) {
-    pass_hist<CL, ELT, MASK>(rw, nx, true, 0, THEN_AGAIN, SM_POS_INF, nullptr, 0, rw.L, rw.scw, 0, rw.lcut);
+    float est;
+    pass_hist<CL, ELT, MASK, true, true>(rw, nx, true, 0, THEN_AGAIN, SM_POS_INF, nullptr, 0, rw.L, rw.scw, 0, rw.lcut, rw.tc, est);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) est += __shfl_xor_sync(0xffffffffu, est, o);
+    if (lane_id() == 0) scratch()->est[warp_id()] = est;
 }
 // The logits a large top-k can keep.
 template <bool CL, int ELT, bool MASK>
@@ -911,8 +997,9 @@ __device__ __forceinline__ int select_top(const View& w, float bound, float cut,
 // candidate, and its mass.
 static __device__ __noinline__ void order_candidates(int nc, const MassFn mass) {
     Sc* sc = scratch();
-    constexpr int TPC = NT / FCAP;                                   // threads per candidate
-    const int i = threadIdx.x / TPC, part = threadIdx.x % TPC;
+    constexpr int TPC = NT >= 1024 ? 8 : NT >= 512 ? 4 : 2;          // threads per candidate
+    static_assert(TPC * FCAP <= NT, "a few threads per candidate");
+    const int i = threadIdx.x / TPC, part = threadIdx.x % TPC;         // (none of i >= FCAP)
     if (threadIdx.x < FCAP) {
         const int t = threadIdx.x;
         if (t >= nc) { fin_area()->fc_idx[t] = 0xFFFFFFu; fin_area()->fc_l[t] = CI_NEG_INF; fin_area()->sv_l[t] = CI_NEG_INF; fin_area()->sv_q[t] = 0; fin_area()->so_l[t] = CI_NEG_INF; fin_area()->so_q[t] = 0; }
@@ -920,7 +1007,7 @@ static __device__ __noinline__ void order_candidates(int nc, const MassFn mass) 
     }
     __syncthreads();
     // (tokens: their difference saturated to 1; equal logits share a rank and are told apart by arrival)
-    const float my_l = fin_area()->fc_l[i], my_i = (float)fin_area()->fc_idx[i];
+    const float my_l = i < FCAP ? fin_area()->fc_l[i] : CI_NEG_INF, my_i = i < FCAP ? (float)fin_area()->fc_idx[i] : 0.0f;
     int rv = 0; float rif = 0.0f;
     auto sat = [](float d) { float r; asm("add.rn.sat.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(d)); return r; };
     for (int j = part * 4; j < nc; j += 4 * TPC) {
@@ -1001,33 +1088,56 @@ static __device__ __noinline__ void finish_warp(float lo, float L, float scale, 
     }
 }
 
-// Exact weighted selection among the listed logits of the warps' views: the value v with W(l > v) < target <= W(l >= v).
-// BINS linear bins over (base - l) * scale, then the pivot bin's entries pairwise.  False when the pivot leaves the binned
-// range or its bin is too crowded.  total: the weight of all entries.  All threads call with the same arguments.
-template <class W>
-__device__ bool list_select(const View& w, W wt, float base, float scale, u64 target, u64* bins, Sc* sc, float& value, u64& total) {
-    const int tid = threadIdx.x;
-    for (int i = tid; i < BINS; i += NT) bins[i] = 0;
-    if (tid == 0) { sc->ncand = 0; sc->sel_ok = 0; sc->cand_kmin = 0xFFFFFFFFu; sc->cand_kmax = 0u; }
+// Exact weighted selection among the listed logits >= c0 of the warps' views, each weighing 1 or its mass: the value v with
+// W(l > v) < target <= W(l >= v).  BINS linear bins over (base - l) * scale, then the pivot bin's entries pairwise; every warp does
+// the searches itself, so that they cost no barriers.  False when the pivot leaves the binned range or its bin is too crowded.
+// total: the weight of all entries.  All threads call with the same arguments; a barrier lies between two calls.
+static __device__ __noinline__ bool list_select(const View w, bool by_mass, const MassFn mass, float c0, float base, float scale, u64 target, float& value, u64& total) {
+    Sc* sc = scratch();
+    const int tid = threadIdx.x, lane = lane_id();
+    uint32_t* lo = reinterpret_cast<uint32_t*>(smem + OFF_BINS);         // a bin's weight: low and high 16 bits of the entries' summed apart
+    uint32_t* hi = lo + BINS;
+    for (int i = tid; i < 2 * BINS; i += NT) lo[i] = 0;
+    if (tid == 0) { sc->ncand = 0; sc->cand_kmin = 0xFFFFFFFFu; sc->cand_kmax = 0u; }
     __syncthreads();
     auto bin_of = [&](float l) { return max(0, min(BINS - 1, __float2int_rz((base - l) * scale))); };
+    auto weight = [&](float l) { return l >= c0 ? by_mass ? mass(l) : 1u : 0u; };
+#pragma unroll 2
     for (int i = w.start; i < w.n; i += w.step) {
         const float l = w.p[i].l;
-        const u64 q = wt(l);
-        if (q) add64(&bins[bin_of(l)], q);
+        const uint32_t q = weight(l);
+        if (q) { const int b = bin_of(l); atomicAdd(&lo[b], q & 0xFFFFu); if (q >> 16) atomicAdd(&hi[b], q >> 16); }
     }
     __syncthreads();
-    int b_star; u64 before;
-    bins_find([&](int i) { return bins[i]; }, BINS, target, sc, b_star, before, total);
-    if (b_star < 0 || b_star >= BINS - 1) return false;
+    static_assert(BINS == 256, "eight bins per lane");
+    u64 s = 0;
+    {
+        const uint4 a = reinterpret_cast<const uint4*>(lo)[2 * lane], b = reinterpret_cast<const uint4*>(lo)[2 * lane + 1];
+        const uint4 c = reinterpret_cast<const uint4*>(hi)[2 * lane], d = reinterpret_cast<const uint4*>(hi)[2 * lane + 1];
+        s = ((u64)a.x + a.y) + ((u64)a.z + a.w) + ((u64)b.x + b.y) + ((u64)b.z + b.w) + ((((u64)c.x + c.y) + ((u64)c.z + c.w) + ((u64)d.x + d.y) + ((u64)d.z + d.w)) << 16);
+    }
+    const u64 incl = warp_incl_scan_u64(s, lane);
+    total = __shfl_sync(0xffffffffu, incl, 31);
+    const unsigned hit = __ballot_sync(0xffffffffu, incl >= target);
+    if (!hit || target == 0) return false;
+    const int hl = __ffs(hit) - 1, bl = 8 * hl + (lane & 7);
+    const u64 one = ((u64)hi[bl] << 16) + lo[bl];                        // (lanes 0 .. 7: the bins of that lane)
+    u64 run = one;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) { const u64 t = __shfl_up_sync(0xffffffffu, run, o); if ((lane & 7) >= o) run += t; }
+    run += __shfl_sync(0xffffffffu, incl - s, hl);
+    const int first = __ffs(__ballot_sync(0xffffffffu, run >= target)) - 1;
+    const int b_star = 8 * hl + first;
+    const u64 before = __shfl_sync(0xffffffffu, run - one, first);
+    if (b_star >= BINS - 1) return false;
     for (int i = w.start; i < w.n; i += w.step) {
         const float l = w.p[i].l;
-        const u64 q = wt(l);
-        if (q && bin_of(l) == b_star) {
-            const int slot = atomicAdd(&sc->ncand, 1);
-            if (slot < FIN_CAND) { sc->cand_l[slot] = l; sc->cand_w[slot] = q; }
-            else { const uint32_t k = f2key(l); atomicMin(&sc->cand_kmin, k); atomicMax(&sc->cand_kmax, k); }
-        }
+        if (bin_of(l) != b_star) continue;
+        const uint32_t q = weight(l);
+        if (!q) continue;
+        const int slot = atomicAdd(&sc->ncand, 1);
+        if (slot < FIN_CAND) { sc->cand_l[slot] = l; sc->cand_w[slot] = q; }
+        else { const uint32_t k = f2key(l); atomicMin(&sc->cand_kmin, k); atomicMax(&sc->cand_kmax, k); }
     }
     __syncthreads();
     const int nc = sc->ncand;
@@ -1040,126 +1150,170 @@ __device__ bool list_select(const View& w, W wt, float base, float scale, u64 ta
         value = key2f(kmin);
         return true;
     }
-    if (tid < nc) {
-        const float mine = sc->cand_l[tid];
+    float mine = 0.0f;
+    bool found = false;
+#pragma unroll 1
+    for (int j = lane; j < nc && !found; j += 32) {
+        mine = sc->cand_l[j];
         u64 gt = 0, eq = 0;
         for (int i = 0; i < nc; ++i) {
             const float o = sc->cand_l[i];
             if (o > mine) gt += sc->cand_w[i]; else if (o == mine) eq += sc->cand_w[i];
         }
-        if (before + gt < target && target <= before + gt + eq) { sc->res_f = mine; sc->sel_ok = 1; }
+        found = before + gt < target && target <= before + gt + eq;
     }
-    __syncthreads();
-    value = sc->res_f;
-    return sc->sel_ok != 0;
+    __syncwarp();
+    const unsigned who = __ballot_sync(0xffffffffu, found);
+    if (!who) return false;
+    value = __shfl_sync(0xffffffffu, mine, __ffs(who) - 1);
+    return true;
 }
 
-// One pass over the histogram, summed over the CTAs of the cluster, for everything the path decision needs: the bucket of the
-// kk-th largest count, the bucket where the running count reaches cap, and the bucket where the running estimated mass
-// reaches topp of its total.  CTA r sums the buckets [r, r + 1) * NB1 / C.  Buckets beyond `last` count nothing.  The estimated
-// mass of a logit of bucket b is 2^(min(0, e0 - b * e1)) (of the last bucket, which holds everything beyond, 0; of bucket
-// `last`, last_part of it), in units of 2^-30.
-struct Estimate {
-    float e0, e1, last_part; int last;
-    __device__ __forceinline__ uint32_t operator()(int b) const {
+// How a wide row is cut, from its histogram (summed over the CTAs of the cluster): by one warp of every CTA.  A lane holds 32
+// buckets; a rank or a share of the estimated mass is found by a scan over the lanes and one over the buckets of the lane it
+// falls into.  The estimated mass of a logit of bucket b is 2^min(0, e0 - b * e1) (of the last bucket, which holds everything
+// beyond, 0; of the cut's bucket the part above the cut): float sums, they only say where to look.
+// The bucket that holds the rank-th largest logit (-1: there are fewer), and how many there are before it and with it.  inc, cnt: of
+// the lane's buckets and those before, and of the lane's alone.
+struct Ranked { int b; uint32_t before, with; };
+static __device__ __noinline__ Ranked ranked(const uint32_t* hist, int last, uint32_t inc, uint32_t cnt, uint32_t rank) {
+    const int lane = lane_id();
+    const unsigned hit = __ballot_sync(0xffffffffu, inc >= rank);
+    const int hl = hit ? __ffs(hit) - 1 : 31, b = hl * 32 + lane;
+    const uint32_t n = b > last ? 0u : hist[b];
+    uint32_t i = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t x = __shfl_up_sync(0xffffffffu, i, o); if (lane >= o) i += x; }
+    i += __shfl_sync(0xffffffffu, inc - cnt, hl);
+    const unsigned in = __ballot_sync(0xffffffffu, i >= rank);
+    const int t = in ? __ffs(in) - 1 : 31;
+    return Ranked{hit ? hl * 32 + t : -1, __shfl_sync(0xffffffffu, i - n, t), __shfl_sync(0xffffffffu, i, t)};
+}
+template <bool CL>
+static __device__ __noinline__ void decide_row(const Grp<CL> g, RowS& rw, int elt, bool miss) {
+    Sc* sc = scratch();
+    const uint32_t* hist = reinterpret_cast<const uint32_t*>(smem + (CL ? OFF_BINS : OFF_U));
+    const int lane = lane_id(), C = CL ? g.C : 1;
+    const bool ready = rw.hist_ready != 0, full = !ready || rw.hist_full;
+    const float href = ready ? rw.lref : rw.L, lcut = rw.lcut, scw = rw.scw, width = RANGE / (float)NB1 * rw.tc;
+    const int hoff = ready ? HOFF : 0;
+    const int last = Buckets(href, scw, hoff)(lcut);                     // buckets wholly below the cut are left out
+    // bucket b's centre lies (b - hoff + 1/2) * RANGE / NB1 + dL temperatures below the row's maximum
+    const float e1 = RANGE / (float)NB1 * CI_LOG2E;
+    const float e0 = ((float)hoff - 0.5f) * e1 - (rw.L - href) * __frcp_rn(rw.tc) * CI_LOG2E;
+    const float last_part = fminf(fmaxf((href - (float)(last - hoff) * width - lcut) * scw, 0.0f), 1.0f);
+    auto edge = [&](int b) { return href - (float)(b - hoff) * width; };
+    auto weight = [&](int b) {
         float e;
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fminf(0.0f, fmaf(-(float)b, e1, e0))));
-        e *= CI_MASS_SCALE;
-        return b == NB1 - 1 ? 0u : __float2uint_rn(b == last ? e * last_part : e);
-    }
-};
-struct FineDecision { int b_k; u64 n_upto; u64 total_cnt; int b_cap; int b_p; u64 est_total; };
-template <bool CL>
-__device__ __forceinline__ FineDecision fine_decide(const Grp<CL>& g, uint32_t* hist, const Estimate& west, u64 kk_target, u64 cap_target, float topp, Sc* sc) {
-    constexpr int PER = NB1 / NT;
-    const int lane = lane_id(), warp = warp_id();
-    const int per = CL ? PER / g.C : PER;
-    const int lo = (CL ? g.rank * (NB1 / g.C) : 0) + (int)threadIdx.x * per;
-    uint32_t c[PER];
-    if constexpr (CL) {
+        return b == NB1 - 1 ? 0.0f : e;
+    };
+    auto at = [&](int b) { return b > last ? 0u : hist[b]; };
+    // the lane's buckets
+    uint32_t cnt = 0; float est = 0.0f, cut_off = 0.0f;                  // (cut_off: what lies below the cut)
+#pragma unroll 2
+    for (int j = 0; j < 8; ++j) {
+        const int b = lane * 32 + 4 * ((j + lane) & 7);                  // (the lanes start at different banks)
+        const uint4 x = *reinterpret_cast<const uint4*>(hist + b);
+        const uint32_t n[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int t = 0; t < PER; ++t) c[t] = 0;
-#pragma unroll 1
-        for (int r = 0; r < g.C; ++r) {
-            const uint32_t* h = g.at(hist, r);
-#pragma unroll
-            for (int t = 0; t < PER; ++t) if (t < per) c[t] += h[lo + t];
-        }
-    } else {
-#pragma unroll
-        for (int t = 0; t < PER; t += 4) {
-            const uint4 x = *reinterpret_cast<const uint4*>(hist + lo + t);
-            c[t] = x.x; c[t + 1] = x.y; c[t + 2] = x.z; c[t + 3] = x.w;
+        for (int i = 0; i < 4; ++i) {
+            const float w = (float)n[i] * weight(b + i);
+            if (b + i <= last) { cnt += n[i]; est += b + i == last ? w * last_part : w; }
+            if (b + i >= last) cut_off += b + i == last ? w * (1.0f - last_part) : w;
         }
     }
-    uint32_t sc_c = 0; u64 sc_e = 0;
-#pragma unroll
-    for (int t = 0; t < PER; ++t) {
-        if (t >= per || lo + t > west.last) c[t] = 0;
-        sc_c += c[t]; sc_e += (u64)c[t] * west(lo + t);
-    }
-    // two prefix scans share the barriers
-    uint32_t in_c = sc_c; u64 in_e = sc_e;
+    uint32_t inc_c = cnt; float inc_e = est;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, in_c, o); const u64 y = __shfl_up_sync(0xffffffffu, in_e, o);
-        if (lane >= o) { in_c += x; in_e += y; }
+        const uint32_t x = __shfl_up_sync(0xffffffffu, inc_c, o); const float y = __shfl_up_sync(0xffffffffu, inc_e, o);
+        if (lane >= o) { inc_c += x; inc_e += y; }
     }
-    if (lane == 31) { sc->wsum[warp] = in_c; sc->wsum2[warp] = in_e; }
-    if (threadIdx.x < 3) { sc->fb[threadIdx.x] = -1; sc->fe[threadIdx.x] = 0; }
-    __syncthreads();
-    u64 off_c = 0, off_e = 0, tot_c = 0, tot_e = 0;                  // every warp adds the others up
-    {
-        const u64 w1 = lane < NW ? sc->wsum[lane] : 0ull, w2 = lane < NW ? sc->wsum2[lane] : 0ull;
-        off_c = warp_sum_u64(lane < warp ? w1 : 0ull); off_e = warp_sum_u64(lane < warp ? w2 : 0ull);
-        tot_c = warp_sum_u64(w1); tot_e = warp_sum_u64(w2);
-    }
-    FineDecision o;
-    long long off = (long long)sc->sum_off;                          // what the estimates are off by on the largest logits
-    o.total_cnt = tot_c; o.est_total = tot_e;
-    if constexpr (CL) {
-        if (threadIdx.x == 0) { sc->t_cnt = tot_c; sc->t_est = tot_e; }
-        g.sync();
-        o.total_cnt = o.est_total = 0; off = 0;
-#pragma unroll 1
-        for (int r = 0; r < g.C; ++r) {
-            const Sc* ps = g.at(sc, r);
-            const u64 tc = ps->t_cnt, te = ps->t_est;
-            if (r < g.rank) { off_c += tc; off_e += te; }
-            o.total_cnt += tc; o.est_total += te;
-            off += (long long)ps->sum_off;
-        }
-    }
-    const u64 ex_c = off_c + in_c - sc_c, ex_e = off_e + in_e - sc_e;
-    u64 t_p = 0;
-    if (topp < 1.0f && (long long)o.est_total + off > 0) {
-        const long long t = (long long)ceil_target(topp, (u64)((long long)o.est_total + off)) - off;
-        t_p = t < 1 ? 1ull : min((u64)t, o.est_total);
-    }
-    // the three finds: at most one thread of the group each
-    const bool f0 = kk_target && ex_c < kk_target && kk_target <= ex_c + sc_c, f1 = ex_c < cap_target && cap_target <= ex_c + sc_c;
-    const bool f2 = t_p && ex_e < t_p && t_p <= ex_e + sc_e;
-    if (f0 || f1 || f2) {
-        u64 run_c = ex_c, run_e = ex_e;
-        int b0 = -1, b1 = -1, b2 = -1; u64 n0 = 0;
+    const uint32_t total = __shfl_sync(0xffffffffu, inc_c, 31);
+    const float mass = __shfl_sync(0xffffffffu, inc_e, 31);
+    // the row's mass relative to its maximum, without what lies below the cut
+    float all = 0.0f;
+    for (int i = lane; i < NW * C; i += 32) all += g.at(sc, i / NW)->est[i % NW];
 #pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            run_c += c[t]; run_e += (u64)c[t] * west(lo + t);
-            if (f0 && b0 < 0 && run_c >= kk_target) { b0 = lo + t; n0 = run_c; }
-            if (f1 && b1 < 0 && run_c >= cap_target) b1 = lo + t;
-            if (f2 && b2 < 0 && run_e >= t_p) b2 = lo + t;
+    for (int o = 16; o; o >>= 1) { all += __shfl_xor_sync(0xffffffffu, all, o); cut_off += __shfl_xor_sync(0xffffffffu, cut_off, o); }
+    {
+        float e;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((href - rw.L) * __frcp_rn(rw.tc) * CI_LOG2E));
+        all = all * e - cut_off;
+    }
+    auto find_rank = [&](uint32_t rank, uint32_t& before, uint32_t& with) {
+        const Ranked r = ranked(hist, last, inc_c, cnt, rank);
+        before = r.before; with = r.with;
+        return r.b;
+    };
+    int path = PATH_PURE;
+    float t_hi = CI_NEG_INF, t_lo = SM_POS_INF;
+    int band_top = 0, band_bot = 0;
+    uint32_t before, with;
+    if (rw.kk > 0 && rw.kk < sc->V && (uint32_t)rw.kk < total) {         // (else at most k reach the cut's bucket: top-k removes nothing)
+        const int b = find_rank((uint32_t)rw.kk, before, with);
+        // (bucket 0 of a histogram laid out from the sample may hold logits from far above it)
+        if (b < (ready ? 1 : 0) || b >= NB1 - 3 || with > (uint32_t)LIST_MAX) path = PATH_FALLBACK;
+        else { path = PATH_LIST; t_lo = edge(b + 2) - 0.01f * width - fabsf(href) * 1e-6f; }
+    } else if (rw.topp < 1.0f) {
+        const float target = mass - (1.0f - rw.topp) * all;
+        const unsigned hit = __ballot_sync(0xffffffffu, inc_e >= target);
+        int bp = -1;
+        float part = 0.5f;                                               // of the pivot's bucket, what lies above it
+        if (mass > 0.0f) {
+            const int hl = hit ? __ffs(hit) - 1 : 31;
+            const float w = (float)at(hl * 32 + lane) * weight(hl * 32 + lane) * (hl * 32 + lane == last ? last_part : 1.0f);
+            float i = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const float x = __shfl_up_sync(0xffffffffu, i, o); if (lane >= o) i += x; }
+            i += __shfl_sync(0xffffffffu, inc_e - est, hl);
+            const unsigned in = __ballot_sync(0xffffffffu, i >= target);
+            bp = hl * 32 + (in ? __ffs(in) - 1 : 31);
+            bp = min(bp, last);
+            part = __saturatef(__fdividef(target - __shfl_sync(0xffffffffu, i - w, bp & 31), fmaxf(__shfl_sync(0xffffffffu, w, bp & 31), 1e-30f)));
         }
-#pragma unroll 1
-        for (int r = 0; r < (CL ? g.C : 1); ++r) {
-            Sc* ps = g.at(sc, r);
-            if (f0) { ps->fb[0] = b0; ps->fe[0] = n0; }
-            if (f1) ps->fb[1] = b1;
-            if (f2) ps->fb[2] = b2;
+        if (bp < 0) path = PATH_FALLBACK;
+        else {
+            // how many lie before the pivot's bucket and with it (at least one logit's rank apart)
+            uint32_t n = hist[(bp & ~31) + lane];
+            if ((bp & ~31) + lane > last) n = 0;
+            uint32_t i = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const uint32_t x = __shfl_up_sync(0xffffffffu, i, o); if (lane >= o) i += x; }
+            i += __shfl_sync(0xffffffffu, inc_c - cnt, bp >> 5);
+            const uint32_t n0 = __shfl_sync(0xffffffffu, i - n, bp & 31), n1 = __shfl_sync(0xffffffffu, i, bp & 31);
+            // The band: so many logits on either side of the estimated pivot, within buckets by interpolation.  After a full count a
+            // hundred (bf16: four hundred, one value's logits are many), after a sample more, the more the further down.
+            uint32_t x0 = 0, x1 = 0;
+            const uint32_t rank = n0 + (uint32_t)(part * (float)(n1 - n0)), near = elt == 2 ? 400u : 100u;
+            const uint32_t side = full ? near : min(min((uint32_t)BAND_SIDE, 300u + (uint32_t)sc->V / 256), near + rank / 4);
+            auto logit_at = [&](uint32_t r, int& bb) {                   // about the r-th largest
+                bb = find_rank(r, x0, x1);
+                return href - ((float)(bb - hoff) + __fdividef((float)(r - x0), fmaxf((float)(x1 - x0), 1.0f))) * width;
+            };
+            band_top = 0; t_hi = SM_POS_INF;
+            if (rank > side) t_hi = logit_at(rank - side, band_top);
+            t_lo = rank + side > total ? -SM_FLT_MAX : logit_at(rank + side, band_bot);
+            if (!(t_lo > -SM_FLT_MAX)) band_bot = NB1 - 1;
+            const int cap = find_rank(500u, x0, x1);
+            if (cap < 0 || cap > band_bot) {
+                band_top = 0; band_bot = cap < 0 ? NB1 - 1 : cap - 1;
+                t_hi = SM_POS_INF; t_lo = cap < 0 ? -SM_FLT_MAX : edge(cap);
+            }
+            path = PATH_BAND;
+            if (band_bot >= NB1 - 2) { t_lo = -SM_FLT_MAX; band_bot = NB1 - 1; }
+            band_top = max(band_top, 0);
+            if (!(t_lo < t_hi)) t_lo = t_hi - width;
+            if (miss && band_top > 0) {                                  // test hook: a band off by its own width and eight buckets (above or below by row parity)
+                const int by = band_bot - band_top + 8, s8 = (rw.row & 1) ? by : -by;
+                if (band_top + s8 > 0 && band_bot + s8 + 2 < NB1) {
+                    band_top += s8; band_bot += s8;
+                    t_hi = edge(band_top); t_lo = edge(band_bot + 1);
+                }
+            }
         }
     }
-    g.sync();
-    o.b_k = sc->fb[0]; o.n_upto = sc->fe[0]; o.b_cap = sc->fb[1]; o.b_p = sc->fb[2];
-    return o;
+    if (lane == 0) { rw.path = path; rw.t_hi = t_hi; rw.t_lo = t_lo; rw.band_top = band_top; rw.band_bot = band_bot; rw.href = href; rw.hoff = hoff; }
 }
 
 // A row's parameters, one 32-bit word per lane: temperature, top_k, top_p, log_min_p, seed (low), the three penalties, seed (high),
@@ -1262,11 +1416,12 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     const int GW = NW * g.C, gw = g.rank * NW + warp;            // warps of the group, this warp among them
 
     Sc* sc = scratch();
-    Cand* klist = reinterpret_cast<Cand*>(smem + OFF_U);         // [NW][KCAP]: rows without a histogram,
+    Cand* klist = reinterpret_cast<Cand*>(smem + OFF_U);         // [NW][KCAPC]: rows without a histogram,
     uint32_t* hist = reinterpret_cast<uint32_t*>(smem + OFF_U);  // or [NB1],
-    Cand* wlist = reinterpret_cast<Cand*>(smem + OFF_U + NB1 * 4);       // [NW][WCAP]
-    Cand* push = reinterpret_cast<Cand*>(smem + OFF_U);          // [C][PUSH / C] candidates of all CTAs, over the histogram
-    Cand* gath = reinterpret_cast<Cand*>(smem + OFF_U);          // [NW][GCAP] lists of all CTAs, over the histogram
+    Cand* wlist = reinterpret_cast<Cand*>(smem + OFF_U + OFF_LISTS);     // [NW][WCAPC]
+    Cand* push = reinterpret_cast<Cand*>(smem + OFF_U + OFF_GATHER);     // [C][PUSH / C] candidates of all CTAs,
+    Cand* gath = push;                                           // or [NW][GCAP] lists of all CTAs
+    constexpr int WCAPC = CL ? WCAP_CL : WCAP, KCAPC = CL ? KCAP_CL : KCAP;
     uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem + OFF_U);        // history bitmap while the tables are built (may reach over bins and csum)
     uint32_t* sbins = reinterpret_cast<uint32_t*>(smem + OFF_BINS);      // [BINS] sample
     uint32_t* fbins = sbins + BINS;                          // [BINS] selection
@@ -1274,11 +1429,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     float* xbuf = reinterpret_cast<float*>(sbins);               // [CHUNK] the chunk the draw falls into
     u64* csum = reinterpret_cast<u64*>(smem + OFF_CSUM);         // [chunks] kept mass per chunk (the CTA's own)
 
+    constexpr int PW = NW - 1;                                   // the warp that looks after the row that comes next
+    uint32_t next_words = 0;                                     // (its parameters, a word per lane)
+    if (CL && warp == PW) next_words = load_params(a, blockIdx.x / a.cluster, lane);   // (before the logits keep the memory busy)
     if (tid == 0) {
         sc->V = V; sc->W = a.W; sc->GW = GW; sc->rank = g.rank;
         sc->drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0; sc->dead = 0;
         sc->pen_off = pen_offset(V, a.p.history != nullptr);
-        sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0;
+        sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_all = sc->sum_keep = 0;
     }
     if (lane == 0) {
         const uint32_t bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
@@ -1330,7 +1488,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         while (j < 2 && pos >= sc->cls_tot[j]) { pos -= sc->cls_tot[j]; ++j; }
         int t = 0;                                               // the last thread with at most pos rows of class j before its own
 #pragma unroll
-        for (int step = NT / 2; step; step >>= 1) if (sc->cls_pre[j][t + step] <= pos) t += step;
+        for (int step = 512; step; step >>= 1) if (t + step < NT && sc->cls_pre[j][t + step] <= pos) t += step;
         int left = pos - sc->cls_pre[j][t], row = 0;
         for (int j0 = 0; j0 < per_thread; j0 += 32) {
             const int k = t * per_thread + j0 + lane;
@@ -1348,8 +1506,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     };
     // The last warp looks after the row that comes next: takes it off the queue early in the first pass of the row at hand, notes
     // where it lies, fetches its parameters, and derives the rest before the row at hand ends.
-    constexpr int PW = NW - 1;
-    int next_row = -1; uint32_t next_words = 0;                  // (the last warp's)
+    int next_row = -1;                                           // (the last warp's)
     auto find_next = [&](int it) {                               // number it + 1
         if (CL) { const int row = grp + (it + 1) * n_grp; next_row = row < n_rows ? row : -1; }
         else {
@@ -1381,7 +1538,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
 #endif
     if (warp == PW) {
         next_row = row_of(grp);
-        next_words = load_params(a, next_row, lane);
+        if (!CL) next_words = load_params(a, next_row, lane);
         if (lane == 0) {
             RowS& rw = sc->rows[0];
             rw.base = place_row<ELT>(a, next_row, rw.a, rw.end, rw.Nc);
@@ -1410,11 +1567,11 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         // ------------------------------------------------------------------------------------ penalty tables
         if (rw.pen_on) {
             // A bitmap of the history's tokens among the CTA's chunks (position order), popcounts per chunk, their prefix: a
-            // token's rank is its table entry.  The first four ids per thread stay in registers.
+            // token's rank is its table entry.  The first PEN_TABLE ids stay in registers.
             const PenTab pt = pen_tab(sc);
             const int hlen = rw.hlen, Nc = rw.Nc, al = rw.a;
             const int32_t* h = rw.hist;
-            constexpr int HP = 4;
+            constexpr int HP = (PEN_TABLE + NT - 1) / NT;
             int ht[HP];
 #pragma unroll
             for (int j = 0; j < HP; ++j) { const int i = tid + j * NT; ht[j] = i < hlen ? __ldg(h + i) : -1; }
@@ -1480,8 +1637,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
         {
             const int cls = rw.cls;
             const bool fastk = (cls & ROW_FASTK) != 0, wide = (cls & ROW_WIDE) != 0, lists = fastk || wide;
-            Cand* list = wlist + warp * WCAP;
-            int lcap = WCAP;
+            Cand* list = wlist + warp * WCAPC;
+            int lcap = WCAPC;
             float tw = -SM_FLT_MAX;                              // the CTA's list bound
             float lref = CI_NEG_INF;                             // the sample's maximum (the group's): buckets hang from it
             float from = -SM_FLT_MAX;                            // nothing below can be kept
@@ -1504,17 +1661,17 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         const uint32_t mw = MASK ? mask_word(rw.mrow, a.W, rw.a, c, lane) : 0u;
                         PenPeek pk = {0, 0, 0};
                         if (rw.pen_on) pk = pen_peek(pen_tab(sc), rw.pen_cap, c, lane);
-                        bool wrote;
                         p.wait(j);
-                        const auto k = open_chunk<ELT, MASK>(rw, p.stage(j), p.conv(), c, true, pk.r0 != pk.r1, pk, mw, wrote);
+                        if ((c == 0 && rw.a) || c == rw.Nc - 1) mend_edges<ELT>(rw, p.stage(j), c);
+                        auto k = open_chunk<ELT, MASK>(rw, p.stage(j), c, mw);
+                        if (pk.r0 != pk.r1) penalise(rw, k, p.stage(j), p.conv(), true, pk, pen_vals(rw));
                         ++seen;
 #pragma unroll
                         for (int e = 0; e < 4; ++e) { gm[4 * j + e] = max4(k.group(e, CI_NEG_INF), CI_NEG_INF); sm = fmaxf(sm, gm[4 * j + e]); }
                         __syncwarp();
                     }
                 }
-#pragma unroll
-                for (int o = 16; o; o >>= 1) sm = fmaxf(sm, __shfl_xor_sync(0xffffffffu, sm, o));
+                sm = warp_max(sm);
                 if (lane == 0) sc->swf[warp] = sm;
                 if (CL && wide) g.sync(); else __syncthreads();
                 // the bins of the bound hang from the smallest finite warp maximum plus 4: a few dominant tokens in the sample
@@ -1525,11 +1682,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     hi = fmaxf(hi, x);
                     if (x > CI_NEG_INF) lo = fminf(lo, x);
                 }
-#pragma unroll
-                for (int o = 16; o; o >>= 1) {
-                    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-                    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-                }
+                hi = warp_max(hi); lo = -warp_max(-lo);
                 lref = hi;
                 const float top = fminf(lo + 4.0f, hi);          // +inf when no warp saw a finite logit
 #pragma unroll
@@ -1550,14 +1703,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     const float tc = rw.tc;
                     const float sure = fmaxf(lref + rw.lmp * tc, lref - 22.0f * tc) - fabsf(lref) * 1e-5f - 1e-5f * tc;
                     const int share = (rw.Nc + g.C - 1) / g.C;   // chunks of the CTA
-                    const float t2 = bound(max(1, (CL ? KCAP_CL : KCAP) * NW * NW / share));
+                    const float t2 = bound(max(1, KCAPC * NW * NW / share));
                     count_hist = !(t2 > -SM_FLT_MAX && t2 < sure);
-                    from = fmaxf(from, sure);
+                    from = lref - 22.0f * tc - fabsf(lref) * 1e-5f - 1e-5f * tc;
                     if (!count_hist) { tw = sure; in_klist = true; }
                 }
-                if (in_klist) { list = CL ? push + PUSH + warp * KCAP_CL : klist + warp * KCAP; lcap = CL ? KCAP_CL : KCAP; }
+                if (in_klist) { list = klist + warp * KCAPC; lcap = KCAPC; }
                 if (tid == 0) sc->in_klist = in_klist;
-                if (tid == 0) { rw.lref = lref; rw.count_hist = count_hist; }
+                if (tid == 0) { rw.lref = lref; rw.count_hist = count_hist; rw.hist_full = CL || (rw.kk > 0 && rw.kk < V); }
             }
             SM_PROF(2);
             if (tid == 0) sc->tw = tw;
@@ -1565,17 +1718,24 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             if (one_pass) look_ahead();
             const int then = one_pass ? THEN_NEXT_ROW : THEN_AGAIN;
             const float t = tw > -SM_FLT_MAX ? tw : SM_POS_INF;  // no bound: nothing is listed
-            const int bad = (lists && !(tw > -SM_FLT_MAX) ? 1 : 0) | (wide && !count_hist ? 4 : 0);
+            const int bad = (lists && !(tw > -SM_FLT_MAX) ? 1 : 0) | (wide && !count_hist ? 4 : 0) | (lists && !in_klist ? 16 : 0);
             Top top1{CI_NEG_INF, 0x7fffffff};
+            float est = 0.0f;                                    // the lane's share of the row's mass relative to lref
             if (!lists) top1 = pass_max<CL, ELT, MASK>(rw, nx, !one_pass, then);
-            else if (count_hist) top1.l = pass_hist<CL, ELT, MASK>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF, from);
+            else if (count_hist && (CL || (rw.kk > 0 && rw.kk < V))) top1.l = pass_hist<CL, ELT, MASK, true, CL>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF, from, rw.tc, est);
+            else if (!CL && count_hist) top1.l = pass_hist<CL, ELT, MASK, CL, true>(rw, nx, true, seen, then, t, list, lcap, lref, rw.scw, HOFF, from, rw.tc, est);
             else top1.l = pass_list<CL, ELT, MASK>(rw, nx, !one_pass, seen, then, t, list, lcap);
             SM_PROF(3);
             ask();
             if (lists) top1.l = warp_max(top1.l);
+            if (count_hist) {
+#pragma unroll
+                for (int o = 16; o; o >>= 1) est += __shfl_xor_sync(0xffffffffu, est, o);
+            }
             if (lane == 0) {
+                sc->est[warp] = est;
                 sc->wf[warp] = top1.l; sc->wi[warp] = top1.idx;
-                const int f = bad | (lists && sc->wn[warp] > lcap ? 1 : 0);
+                const int f = bad | (lists && sc->wn[warp] > lcap ? 1 : 0) | (est < 1e30f ? 0 : 8);
                 if (f) atomicOr(&sc->flags, f);
             }
         }
@@ -1598,8 +1758,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             const int cls = rw.cls;
             const bool sampled = (cls & ROW_SAMPLED) != 0, fastk = (cls & ROW_FASTK) != 0, lists = (cls & (ROW_FASTK | ROW_WIDE)) != 0;
             const bool in_klist = sc->in_klist != 0;
-            Cand* list = !in_klist ? wlist + warp * WCAP : CL ? push + PUSH + warp * KCAP_CL : klist + warp * KCAP;
-            const int lcap = !in_klist ? WCAP : CL ? KCAP_CL : KCAP;
+            Cand* list = !in_klist ? wlist + warp * WCAPC : klist + warp * KCAPC;
+            const int lcap = !in_klist ? WCAPC : KCAPC;
             float L = CI_NEG_INF, lo_all = -SM_FLT_MAX;
             int aidx = 0x7fffffff, fl = 0;
             {
@@ -1611,7 +1771,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 lo_all = warp_max(e.z);
                 fl = (int)__reduce_or_sync(0xffffffffu, (unsigned)__float_as_int(e.w));
             }
-            const bool lists_ok = lists && !(fl & 1);
+            const bool lists_ok = lists && !(fl & 1), all_klist = lists && !(fl & 16);   // (of all CTAs)
             const bool finite_max = (L > CI_NEG_INF) && (L < SM_POS_INF);
             if (lists && (a.stats || !finite_max)) {
                 // the lowest index of the maximum, for rows whose pass only listed: from the lists, else from one more pass
@@ -1649,7 +1809,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             }
             if (tid == 0) {
                 rw.L = L; rw.aidx = aidx; rw.status = sampled && !finite_max ? COLINFER_ROW_DEGENERATE : 0;
-                rw.hist_ready = rw.count_hist && !(fl & 4) && !fastk && (L - rw.lref) * rw.scw < (float)(HOFF - 2);   // the maximum lies inside the buckets
+                rw.hist_ready = rw.count_hist && !(fl & 12) && !fastk && (rw.hist_full ? (L - rw.lref) * rw.scw < (float)(HOFF - 2) : !(fl & 1));   // the maximum lies inside the buckets; what was not sampled is listed
                 rw.minp = lcut > horizon;
                 rw.lcut = fmaxf(lcut, horizon); rw.horizon = horizon; rw.mass = mass;
                 rw.drawn = 0; rw.token = aidx; rw.total = 0; rw.listed = 0;
@@ -1698,9 +1858,12 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     done = ps->ok != 0;
                     if (tid == 0) {
                         if (done) { rw.token = ps->fin_token; rw.lcut = ps->fin_cut; rw.total = ps->fin_total; }
-                        if (CL) rw.hist_ready = 0;               // (candidates lie over the histogram)
                         // lists that hold all the mass, too long for the one-warp finish: selected on as they are
-                        if (!CL && !done && !fastk && in_klist) { rw.path = PATH_LIST; rw.listed = 1; rw.t_lo = lo_all; }
+                        if (!done && !fastk && all_klist) {
+                            int n = 0;
+                            if (CL) for (int q = 0; q < g.C; ++q) n += g.at(sc, q)->npush;
+                            if (n <= GCAP * NW * 3 / 4) { rw.path = PATH_LIST; rw.listed = 1; rw.t_lo = lo_all; }
+                        }
                     }
                 }
             }
@@ -1721,71 +1884,22 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     recount_pass<CL, ELT, MASK>(rw, nx);
                     g.sync();
                 }
-                const bool ready = rw.hist_ready != 0;
-                const float href = ready ? rw.lref : rw.L; const int hoff = ready ? HOFF : 0;
-                const float lcut = rw.lcut, scw = rw.scw;
-                const Buckets bucket(href, scw, hoff);
-                // the histogram counts every logit; buckets wholly below the cut are left out
-                const int b_cut = bucket(lcut);
-                const float dL = (rw.L - href) / rw.tc;
-                // bucket b's centre lies (b - hoff + 1/2) * RANGE / NB1 + dL temperatures below the row's maximum; of the cut's
-                // bucket only the part above the cut is kept
-                Estimate mass_est;
-                mass_est.e1 = RANGE / (float)NB1 * CI_LOG2E;
-                mass_est.e0 = ((float)hoff - 0.5f) * mass_est.e1 - dL * CI_LOG2E;
-                mass_est.last = b_cut;
-                mass_est.last_part = fminf(fmaxf((href - (float)(b_cut - hoff) / scw - lcut) * scw, 0.0f), 1.0f);
-                // What the estimates are off by on the listed logits -- the largest, which make up most of a peaked row's mass.
-                long long off = 0;
-                if (ready && !sc->in_klist) {
-                    const Cand* list = wlist + warp * WCAP;
-                    const MassFn mass = rw.mass;
-                    for (int j = lane; j < min(sc->wn[warp], WCAP); j += 32) {
-                        const float l = list[j].l;
-                        if (l >= lcut) off += (long long)mass(l) - (long long)mass_est(bucket(l));
-                    }
+                // a histogram that was sampled left the listed logits out
+                if (rw.hist_ready && !rw.hist_full) {
+                    const Cand* list = wlist + warp * WCAPC;
+                    const Buckets bucket(rw.lref, rw.scw, HOFF);
+                    for (int j = lane; j < min(sc->wn[warp], WCAPC); j += 32) atomicAdd(&hist[bucket(list[j].l)], 1u);
                 }
-                off = (long long)warp_sum_u64((u64)off);
-                if (lane == 0) add64(&sc->sum_off, (u64)off);
-                // 500: how far down the lists reach in a small nucleus (they hold ~ 750)
-                const FineDecision fd = fine_decide<CL>(g, hist, mass_est, need_topk() ? (u64)rw.kk : 0ull, 500ull, rw.topp, sc);
-                if (tid == 0) {
-                    auto edge = [&](int bb) { return href - (float)(bb - hoff) / scw; };
-                    int path = PATH_PURE;
-                    float t_hi = CI_NEG_INF, t_lo = SM_POS_INF;
-                    int band_top = 0, band_bot = 0;
-                    const bool topk = need_topk() && (u64)rw.kk < fd.total_cnt;  // else at most k reach the cut's bucket: top-k removes nothing
-                    if (topk) {
-                        // (bucket 0 of a histogram laid out from the sample may hold logits from far above it)
-                        if (fd.b_k < (ready ? 1 : 0) || fd.b_k >= NB1 - 3 || fd.n_upto > (u64)LIST_MAX) path = PATH_FALLBACK;
-                        else { path = PATH_LIST; t_lo = edge(fd.b_k + 2) - 0.01f / scw - fabsf(href) * 1e-6f; }
-                    } else if (rw.topp < 1.0f) {
-                        const int bp = fd.b_p, bcap = fd.b_cap;
-                        const int up = ELT == 2 ? 3 : 1, dn = ELT == 2 ? 4 : 1;
-                        if (fd.est_total == 0 || bp < (ready ? 1 : 0)) path = PATH_FALLBACK;
-                        else if (bcap < 0 || bcap > bp + dn + 1) {
-                            // small nucleus: list everything down to well below the estimated pivot; nothing is "above"
-                            path = PATH_BAND;
-                            t_hi = SM_POS_INF;
-                            t_lo = bcap < 0 ? -SM_FLT_MAX : edge(bcap);
-                            band_top = 0; band_bot = bcap < 0 ? NB1 - 1 : bcap;
-                        } else if (bp + dn + 2 >= NB1) path = PATH_FALLBACK;
-                        else {
-                            path = PATH_BAND;
-                            t_hi = bp - up <= 0 ? SM_POS_INF : edge(bp - up);
-                            t_lo = edge(bp + dn + 1);
-                            band_top = max(0, bp - up); band_bot = bp + dn;
-                            if (a.flags & COLINFER_TEST_MISS_BAND) {     // test hook: a band eight buckets off (above or below by row parity)
-                                const int s8 = (rw.row & 1) ? 8 : -8;
-                                if (bp - up + s8 > 0 && bp + dn + s8 + 2 < NB1) {
-                                    t_hi = edge(bp - up + s8); t_lo = edge(bp + dn + 1 + s8);
-                                    band_top = bp - up + s8; band_bot = bp + dn + s8;
-                                }
-                            }
-                        }
+                g.sync();
+                if constexpr (CL) {                              // the histograms of all CTAs
+                    for (int b = 2 * tid; b < NB1; b += 2 * NT) {
+                        uint2 n = make_uint2(0, 0);
+                        for (int r = 0; r < g.C; ++r) { const uint2 x = *reinterpret_cast<const uint2*>(g.at(hist, r) + b); n.x += x.x; n.y += x.y; }
+                        *reinterpret_cast<uint2*>(sbins + b) = n;
                     }
-                    rw.path = path; rw.t_hi = t_hi; rw.t_lo = t_lo; rw.band_top = band_top; rw.band_bot = band_bot; rw.href = href; rw.hoff = hoff;
+                    __syncthreads();
                 }
+                if (warp == 0) decide_row<CL>(g, rw, ELT, (a.flags & COLINFER_TEST_MISS_BAND) != 0);
             } else if (tid == 0) { rw.path = PATH_PURE; rw.t_hi = CI_NEG_INF; rw.t_lo = SM_POS_INF; }
             if (CL) g.sync(); else __syncthreads();              // (the path is known, the finds are read, the lists are free)
             SM_PROF(6);
@@ -1797,8 +1911,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     if (c.l >= cut) { const uint32_t q = mass(c.l); if (q) add64(&csum[(c.idx + rw.a) / CHUNK], (u64)q); }
                 }
             };
-            // the warps' view of the listed logits of all CTAs; over: a list overflowed
-            auto view_all = [&](Cand* list, int cap, bool& over) {
+            // the warps' view of the listed logits of all CTAs, in a cluster those >= floor; over: a list overflowed
+            auto view_all = [&](Cand* list, int cap, float floor, bool& over) {
                 View w{list, lane, 0, 32};
                 over = false;
                 if constexpr (CL) {
@@ -1807,8 +1921,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         const int c = g.at(sc, q)->wn[warp];
                         const Cand* src = g.at(list, q);
                         if (c > cap) over = true;
-                        for (int j = lane; j < min(c, cap); j += 32) if (n + j < GCAP) gath[warp * GCAP + n + j] = src[j];
-                        n += min(c, cap);
+                        for (int j = lane; j - lane < min(c, cap); j += 32) {
+                            const Cand x = src[min(j, cap - 1)];
+                            const bool is = j < min(c, cap) && x.l >= floor;
+                            const unsigned who = __ballot_sync(0xffffffffu, is);
+                            const int at = n + __popc(who & ((1u << lane) - 1u));
+                            if (is && at < GCAP) gath[warp * GCAP + at] = x;
+                            n += __popc(who);
+                        }
                     }
                     if (n > GCAP) over = true;
                     w.p = gath + warp * GCAP; w.n = min(n, GCAP);
@@ -1888,8 +2008,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
 
             // -------------------------------------------------------------------------------- large top-k (then top-p) on a list
             if (rw.path == PATH_LIST) {
-                Cand* list = CL ? wlist + warp * WCAP : klist + warp * KCAP;
-                constexpr int cap = CL ? WCAP : KCAP;
+                Cand* list = CL && !rw.listed ? wlist + warp * WCAPC : klist + warp * KCAPC;
+                const int cap = CL && !rw.listed ? WCAPC : KCAPC;
                 for (int c = tid; c < rw.Nc; c += NT) csum[c] = 0;
                 if (!rw.listed) {
                     if (lane == 0) sc->wn[warp] = 0;
@@ -1900,7 +2020,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 const MassFn mass = rw.mass;
                 const float tc = rw.tc, tl = fmaxf(fmaxf(rw.t_lo, rw.lcut), -SM_FLT_MAX);
                 bool over;
-                const View w = view_all(list, cap, over);
+                const View w = view_all(list, cap, tl, over);
                 float cut = fmaxf(rw.lcut, -SM_FLT_MAX);
                 bool ok = !over;
                 const float L = rw.L, scale = (float)(BINS - 2) / fmaxf(L - tl, 1e-30f);
@@ -1912,7 +2032,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     if (ok && need_topk() && (u64)rw.kk <= surv) {   // else fewer than k survive min-p: top-k removes nothing
                         float lkk; u64 tot;
                         const float c0 = cut;
-                        ok = list_select(w, [&](float l) { return (u64)(l >= c0 ? 1 : 0); }, L, scale, (u64)rw.kk, bins, sc, lkk, tot);
+                        ok = list_select(w, false, mass, c0, L, scale, (u64)rw.kk, lkk, tot);
                         if (ok) { cut = fmaxf(cut, lower_logit_for(scale_logit(lkk, tc), tc, lkk)); ok = cut >= tl; }   // else a tie partner could lie outside the list
                     }
                 }
@@ -1924,7 +2044,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     ok = s1 > 0;
                     if (ok) {
                         float lp; u64 tot;
-                        ok = list_select(w, [&](float l) { return l >= c0 ? (u64)mass(l) : 0ull; }, L, scale, ceil_target(rw.topp, s1), bins, sc, lp, tot);
+                        ok = list_select(w, true, mass, c0, L, scale, ceil_target(rw.topp, s1), lp, tot);
                         if (ok) { cut = fmaxf(cut, lower_logit_for(scale_logit(lp, tc), tc, lp)); ok = cut >= tl; }
                     }
                 }
@@ -1947,8 +2067,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             look_ahead();
             for (int attempt = 0; rw.path != PATH_LIST && attempt < 3; ++attempt) {
                 // (with one CTA per row the band's list takes the histogram's place: the path is decided)
-                Cand* blist = CL ? wlist + warp * WCAP : klist + warp * KCAP;
-                constexpr int bcap = CL ? WCAP : KCAP;
+                Cand* blist = CL ? wlist + warp * WCAPC : klist + warp * KCAP;
+                constexpr int bcap = CL ? WCAPC : KCAP;
                 if (lane == 0) sc->wn[warp] = 0;
                 if (attempt) {                                   // (they start a row at zero)
                     if (tid == 0) sc->sum_all = sc->sum_keep = 0;
@@ -1973,7 +2093,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                 u64 s1 = 0, s_above = 0;
                 for (int q = 0; q < (CL ? g.C : 1); ++q) { const Sc* ps = g.at(sc, q); s1 += ps->sum_all; s_above += ps->sum_keep; }
                 bool over;
-                const View w = view_all(blist, bcap, over);
+                const View w = view_all(blist, bcap, -SM_FLT_MAX, over);
                 const u64 target = ceil_target(rw.topp, s1);
                 bool ok = !over && s1 > 0 && s_above < target;
                 u64 s_band = 0;
@@ -1984,7 +2104,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     // (a small nucleus lists everything above the cut: the bins span [cut, base], not [-max, base])
                     const float scale = (float)(BINS - 2) / fmaxf(bs - fmaxf(t_lo, lcut), 1e-30f);
                     float lp;
-                    ok = list_select(w, [&](float l) { return (u64)mass(l); }, bs, scale, target - s_above, bins, sc, lp, s_band);
+                    ok = list_select(w, true, mass, -SM_FLT_MAX, bs, scale, target - s_above, lp, s_band);
                     if (ok) {
                         const float cut2 = fmaxf(lcut, lower_logit_for(scale_logit(lp, mass.tc), mass.tc, lp));
                         if (cut2 < t_lo) ok = false;             // a tie partner could lie below the band
@@ -2043,37 +2163,30 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             // -------------------------------------------------------------------------------- the draw: chunk, then logit
             g.sync();                                            // the chunks' kept masses are complete
             {
-                const int Nc = rw.Nc;
-                const int per = (Nc + NT - 1) / NT;
-                const int c_lo = min(tid * per, Nc), c_hi = min(c_lo + per, Nc);
+                // the chunk in which the running kept mass reaches its target: a stretch of chunks per warp, a run of them per lane; the
+                // warp whose stretch it is goes on
+                const int Nc = rw.Nc, stretch = (Nc + NW - 1) / NW, run = (stretch + 31) / 32;
+                const int c_lo = min(min(warp * stretch + lane * run, (warp + 1) * stretch), Nc), c_hi = min(min(c_lo + run, (warp + 1) * stretch), Nc);
                 auto kept = [&](int c) { return g.at(csum, CL ? (c / NW) % g.C : 0)[c]; };
-                u64 s = 0, total;
+                u64 s = 0;
                 for (int c = c_lo; c < c_hi; ++c) s += kept(c);
-                const u64 excl = block_excl_scan(s, sc, total);
-                const u64 target = ceil_target(rw.u, total);
-                if (total > 0 && excl < target && target <= excl + s) {
-                    u64 run = excl;
-                    for (int c = c_lo; c < c_hi; ++c) {
-                        const u64 q = kept(c);
-                        if (run + q >= target) { sc->x_chunk = c; sc->x_before = run; break; }
-                        run += q;
-                    }
-                }
-                if (tid == 0) { rw.total = total; if (total > 0) rw.drawn = 1; else rw.status |= COLINFER_ROW_DEGENERATE; }
+                u64 before = warp_incl_scan_u64(s, lane);
+                if (lane == 31) sc->wsum[warp] = before;
                 __syncthreads();
-                derive_next();
-                if (total == 0) {
-                    if ((rw.cls & ROW_WIDE) && !a.stats) {       // (a row without any kept mass emits its argmax)
-                        const int x = argmax_pass<CL, ELT, MASK>(rw, nx, rw.L);
-                        if (lane == 0) sc->wi[warp] = x;
-                        g.sync();
-                        int y = 0x7fffffff;
-                        for (int i = lane; i < GW; i += 32) y = min(y, g.at(sc, i / NW)->wi[i % NW]);
-                        y = (int)__reduce_min_sync(0xffffffffu, (unsigned)y);
-                        if (tid == 0) rw.token = y == 0x7fffffff ? 0 : y;
+                const u64 ws = lane < NW ? sc->wsum[lane] : 0ull, upto = warp_incl_scan_u64(ws, lane), total = __shfl_sync(0xffffffffu, upto, 31);
+                const u64 target = ceil_target(rw.u, total);
+                const int it_is = __ffs(__ballot_sync(0xffffffffu, upto >= target)) - 1;
+                if (tid == 0) { rw.total = total; if (total > 0) rw.drawn = 1; else rw.status |= COLINFER_ROW_DEGENERATE; }
+                if (total > 0 && warp == it_is) {
+                    before += __shfl_sync(0xffffffffu, upto - ws, warp);
+                    const int hl = __ffs(__ballot_sync(0xffffffffu, before >= target)) - 1;
+                    before -= s;
+                    int c = c_lo;
+                    if (lane == hl) {
+                        for (; c < c_hi - 1; ++c) { const u64 q = kept(c); if (before + q >= target) break; before += q; }
                     }
-                } else if (warp == 0) {
-                    const int c = sc->x_chunk;
+                    before = __shfl_sync(0xffffffffu, before, hl);
+                    c = __shfl_sync(0xffffffffu, c, hl);
                     if (!CL || ((c / NW) % g.C) == g.rank) {
                         // the chunk in fp32, penalties applied (its CTA has the tables), then masked
                         const char* base = rw.base;
@@ -2090,7 +2203,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
 #pragma unroll
                         for (int j = 0; j < CHUNK / 32; ++j) xbuf[j * 32 + lane] = x[j];
                         __syncwarp();
-                        if (rw.pen_on) { const PenPeek pk = pen_peek(pen_tab(sc), rw.pen_cap, c, lane); if (pk.r0 != pk.r1) pen_patch(rw, smem_u32(xbuf), c, pk); }
+                        if (rw.pen_on) { const PenPeek pk = pen_peek(pen_tab(sc), rw.pen_cap, c, lane); if (pk.r0 != pk.r1) pen_patch(rw, smem_u32(xbuf), c, pk, pen_vals(rw)); }
                         const float lkf = fmaxf(rw.lcut, -SM_FLT_MAX);
                         const MassFn mass = rw.mass;
                         u64 q16 = 0; uint32_t q[16];
@@ -2102,7 +2215,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                             q[e] = x >= lkf ? mass(x) : 0u;
                             q16 += q[e];
                         }
-                        const u64 incl = sc->x_before + warp_incl_scan_u64(q16, lane);
+                        const u64 incl = before + warp_incl_scan_u64(q16, lane);
                         const unsigned hit = __ballot_sync(0xffffffffu, incl >= target);
                         if (hit && lane == __ffs(hit) - 1) {
                             u64 cum = incl; int e = 0;
@@ -2112,14 +2225,24 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         }
                     }
                 }
+                derive_next();
             }
         }
         SM_PROF(10);
         derive_next();
         // (nobody reads these of this row any more)
         if (tid < NW) { sc->wn[tid] = 0; sc->swf[tid] = CI_NEG_INF; }
-        if (tid == 0) { sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_off = sc->sum_all = sc->sum_keep = 0; }
+        if (tid == 0) { sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_all = sc->sum_keep = 0; }
         if (CL) g.sync(); else __syncthreads();
+        if (!done && rw.total == 0 && (rw.cls & ROW_WIDE) && !a.stats) {         // (a row without any kept mass emits its argmax)
+            const int x = argmax_pass<CL, ELT, MASK>(rw, nx, rw.L);
+            if (lane == 0) sc->wi[warp] = x;
+            g.sync();
+            int y = 0x7fffffff;
+            for (int i = lane; i < GW; i += 32) y = min(y, g.at(sc, i / NW)->wi[i % NW]);
+            y = (int)__reduce_min_sync(0xffffffffu, (unsigned)y);
+            if (tid == 0) rw.token = y == 0x7fffffff ? 0 : y;
+        }
         if (tid == 0 && g.rank == 0) {
             int status = rw.status;
             for (int q = 0; q < g.C; ++q) {
