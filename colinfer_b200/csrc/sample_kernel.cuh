@@ -14,7 +14,8 @@
 //   greedy        one pass: maximum and its lowest index
 //   top_k <= 100  one pass.  The first chunk of every warp (the CTA's sample) bounds the k-th largest logit from below; the
 //                 pass lists what reaches the bound, the row is finished on the list
-//   larger top_k  a full histogram gives the bucket of the k-th largest, a second pass lists what reaches it, for an exact selection
+//   larger top_k  one pass as well where the sample says that the lists can hold the k largest; they are selected from there
+//                 exactly.  Else a full histogram gives the bucket of the k-th largest, and a second pass lists what reaches it
 //   top_p         pass 1 also sums the row's mass (approximately) and counts a histogram, laid out from the sample's maximum: of
 //                 a quarter of the logits with a CTA per row, where the rows of an SM share its time, of all of them in a cluster.
 //                 They say where the top-p pivot lies: pass 2 sums the exact masses, per chunk those above a band around the
@@ -33,7 +34,7 @@
 // instead of published behind barriers.  A thread has 80 registers: with 64 (512 threads) the passes kept what a row needs in local
 // memory, which beside 226 KB of shared memory is L2, and two rows on an SM were slower than one after the other.
 // Before and now, one B200, 151,936 fp32 logits, us: 592 rows greedy 69 -> 64, without a filter 138 -> 125, top_p 203 -> 191,
-// top_k 50 81 -> 78, top_k 1000 251 -> 181; 360 bf16 rows with mixed filters 159 -> 100.
+// top_k 50 81 -> 78, top_k 1000 251 -> 117; 296 rows top_k 1000 121 -> 67; 360 bf16 rows with mixed filters 159 -> 100.
 #pragma once
 #include <stddef.h>
 
@@ -1707,6 +1708,14 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     count_hist = !(t2 > -SM_FLT_MAX && t2 < sure);
                     from = lref - 22.0f * tc - fabsf(lref) * 1e-5f - 1e-5f * tc;
                     if (!count_hist) { tw = sure; in_klist = true; }
+                    else if (rw.kk > 0 && rw.kk < V) {
+                        // So does a row with a top-k, where the sample says how far down the k-th largest lies: four standard
+                        // deviations below that and no more than half of what the lists hold.
+                        const float f = (float)min(2 * NW, share) / (float)share, want = (float)rw.kk / (float)g.C * f;
+                        const int r = (int)(want + 4.0f * sqrtf(want)) + 8;
+                        const float t3 = bound(r);
+                        if ((float)r < 0.55f * f * (float)(KCAPC * NW) && t3 > -SM_FLT_MAX) { count_hist = false; tw = fmaxf(t3, sure); in_klist = true; }
+                    }
                 }
                 if (in_klist) { list = klist + warp * KCAPC; lcap = KCAPC; }
                 if (tid == 0) sc->in_klist = in_klist;
@@ -1865,6 +1874,16 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                             if (n <= GCAP * NW * 3 / 4) { rw.path = PATH_LIST; rw.listed = 1; rw.t_lo = lo_all; }
                         }
                     }
+                } else if (lists_ok && all_klist) {
+                    // a top-k's list reaches down to its bound: it does if it has k logits
+                    int n = 0;
+                    for (int j = lane; j < min(sc->wn[warp], lcap); j += 32) n += list[j].l >= lo_all ? 1 : 0;
+                    n = (int)__reduce_add_sync(0xffffffffu, (unsigned)n);
+                    if (lane == 0 && n) atomicAdd(&sc->npush, n);
+                    g.sync();
+                    n = 0;
+                    for (int q = 0; q < (CL ? g.C : 1); ++q) n += g.at(sc, q)->npush;
+                    if (tid == 0 && n >= rw.kk && (!CL || n <= GCAP * NW * 3 / 4)) { rw.path = PATH_LIST; rw.listed = 1; rw.t_lo = lo_all; }
                 }
             }
         }
