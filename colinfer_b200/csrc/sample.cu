@@ -1608,16 +1608,16 @@ extern "C" int colinfer_max_active_clusters(int V, int dtype) {
 // ---- the chunk kernel (sample_rows.cu: a CTA per row, sample_few.cu: a cluster per row)
 namespace {
 constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024;
-// More rows than SMs: two CTAs of 512 threads per SM, one of which reads while the other one is in its block-wide steps; or one of
-// 1,024 where two do not fit (penalty tables of large vocabularies: 512 bf16 rows of 262,144 logits with histories 222 -> 174 us),
-// and for bf16 vocabularies beyond 229,376.  There mixed filters (a top_p close to 1 among them) overflow the lists of 512 threads
-// with equal logits.  Time of one CTA per SM over that of two, mean of 160 to 592 rows, N(0, 2^2), mixed filters and the others:
-// 151,936 0.99 and 1.02 - 1.18; 201,792 0.91 and 0.97 - 1.13; 229,376 0.64 and 0.96 - 1.10; 262,144 0.58 and 0.95 - 1.08 (a row
-// without any filter loses 8 %).  How many are equal goes by the rows' spread too, which the host does not see: at N(0, 1) mixed
-// filters have it 0.59 at 151,936 already, under a grammar mask 0.93 there and 0.85 at 262,144.
-constexpr int kTwoPerSm = 113 * 1024, kRowV = 229376;
+// More rows than SMs: two CTAs of 384 threads per SM, one of which reads while the other one is in its block-wide steps.  One of
+// 1,024 where two do not fit (penalty tables of vocabularies beyond some 330,000), and with histories beyond 216,000 logits for bf16
+// rows (a top_p close to 1 beside penalties overflows the lists of 384 threads with equal logits) and for up to two rows per SM (a row
+// alone on an SM gets through sooner with 1,024).  262,144 logits with histories of 2,048, one CTA per SM and two, us: 512 bf16 rows
+// mixed 312 and 493; 160 fp32 rows mixed 109 and 142, no filter 76 and 98, 512 of them mixed 250 and 222, top_p 416 and 354.
+// Without histories two are the faster everywhere but at 160 to 296 half greedy bf16 rows (56 and 60, 79 and 87): 512 bf16 rows
+// greedy 87 and 61, mixed 212 and 189, top_p 360 and 312, top_k 1000 217 and 142; under a mask top_p 465 and 388, top_k 1000 187 and 171.
+constexpr int kTwoPerSm = 113 * 1024, kRowV = 216000;
 
-// The sets of instantiations: a CTA of 512 threads per row, two per SM (ROWS); a CTA of 1,024 threads per row (ROW); a cluster of
+// The sets of instantiations: a CTA of 384 threads per row, two per SM (ROWS); a CTA of 1,024 threads per row (ROW); a cluster of
 // CTAs per row (FEW).
 enum { ROWS = 0, FEW = 1, ROW = 2 };
 int chunk_index(int set, int dtype, bool mask) { return 4 * set + (dtype == COLINFER_F32 ? 0 : 2) + (mask ? 1 : 0); }
@@ -1700,7 +1700,7 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
         // and 104, 106; top_k 50 65, 83 and 41, 42; top_k 1000 124, 129 and 102, 114; no filter 63, 64 and 65, 74; greedy 29, 31 and
         // 27, 36: over the same six 0.91 and 0.93 of the time (a wide row alone on an SM has half the threads here).  400 rows: mixed
         // 115 and 107, top-p 183 and 165, no filter 97 and 133; 592: 166 and 140, 242 and 201, 132 and 138.
-    } else if ((dtype == COLINFER_BF16 && V > kRowV) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
+    } else if ((pen && V > kRowV && (dtype == COLINFER_BF16 || rows <= 2 * sms)) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
     const int smem = chunk_smem(set, V, pen), ki = chunk_index(set, dtype, mask != nullptr);
     if (smem > kChunkMaxSmem) return -1;
     {

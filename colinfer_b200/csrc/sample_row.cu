@@ -1,6 +1,5 @@
 // sample_row.cu -- the fused kernel with one CTA of 1,024 threads per row and SM, for launches of more rows than SMs whose rows
-// want more shared memory than half an SM has, and for bf16 rows of more than 229,376 logits, whose lists want more room
-// (kRowV in sample.cu).
+// want more shared memory than half an SM has, and for long rows with histories (kRowV in sample.cu).
 #define SMP_NAME smp_row
 #define SMP_THREADS 1024
 #define SMP_CTAS 1
