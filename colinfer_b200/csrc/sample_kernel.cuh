@@ -75,7 +75,7 @@ constexpr int GCAP = WCAP / 2;                               // entries per warp
 constexpr int OFF_GATHER = OFF_LISTS + GCAP * NW * 8;        // or the candidates sent to the first one, in equal shares
 constexpr int PUSH = 2048;
 constexpr int WCAP_CL = GCAP, KCAP_CL = OFF_GATHER / 8 / NW;
-static_assert(PUSH <= GCAP * NW || SMP_CTAS == 2 || SMP_THREADS == 1024, "candidates over the gathered entries");
+static_assert(PUSH <= GCAP * NW || SMP_CTAS == 2 || SMP_THREADS > 512, "candidates over the gathered entries");
 // A band is to hold this many logits on either side of the estimated pivot: a third of what the lists hold.
 constexpr int BAND_SIDE = 7 * KCAP * NW / 20 < 1200 ? 7 * KCAP * NW / 20 : 1200;
 constexpr int FIN_CAND = 128;        // entries of one bin compared pairwise
@@ -1098,11 +1098,15 @@ static __device__ __noinline__ bool list_select(const View w, bool by_mass, cons
     const int tid = threadIdx.x, lane = lane_id();
     uint32_t* lo = reinterpret_cast<uint32_t*>(smem + OFF_BINS);         // a bin's weight: low and high 16 bits of the entries' summed apart
     uint32_t* hi = lo + BINS;
+    // (again, within a bin of several values and more entries than are compared pairwise: a penalised logit beside many equal ones)
+    float top = SM_POS_INF;
+#pragma unroll 1
+    for (int level = 0; level < 3; ++level) {
     for (int i = tid; i < 2 * BINS; i += NT) lo[i] = 0;
     if (tid == 0) { sc->ncand = 0; sc->cand_kmin = 0xFFFFFFFFu; sc->cand_kmax = 0u; }
     __syncthreads();
     auto bin_of = [&](float l) { return max(0, min(BINS - 1, __float2int_rz((base - l) * scale))); };
-    auto weight = [&](float l) { return l >= c0 ? by_mass ? mass(l) : 1u : 0u; };
+    auto weight = [&](float l) { return l >= c0 && l <= top ? by_mass ? mass(l) : 1u : 0u; };
 #pragma unroll 2
     for (int i = w.start; i < w.n; i += w.step) {
         const float l = w.p[i].l;
@@ -1118,7 +1122,7 @@ static __device__ __noinline__ bool list_select(const View w, bool by_mass, cons
         s = ((u64)a.x + a.y) + ((u64)a.z + a.w) + ((u64)b.x + b.y) + ((u64)b.z + b.w) + ((((u64)c.x + c.y) + ((u64)c.z + c.w) + ((u64)d.x + d.y) + ((u64)d.z + d.w)) << 16);
     }
     const u64 incl = warp_incl_scan_u64(s, lane);
-    total = __shfl_sync(0xffffffffu, incl, 31);
+    if (level == 0) total = __shfl_sync(0xffffffffu, incl, 31);
     const unsigned hit = __ballot_sync(0xffffffffu, incl >= target);
     if (!hit || target == 0) return false;
     const int hl = __ffs(hit) - 1, bl = 8 * hl + (lane & 7);
@@ -1147,9 +1151,13 @@ static __device__ __noinline__ bool list_select(const View w, bool by_mass, cons
         // that value is the pivot: the weight above the bin is below the target, with the bin it reaches it.
         uint32_t kmin = sc->cand_kmin, kmax = sc->cand_kmax;
         for (int i = 0; i < FIN_CAND; ++i) { const uint32_t k = f2key(sc->cand_l[i]); kmin = min(kmin, k); kmax = max(kmax, k); }
-        if (kmin != kmax) return false;
         value = key2f(kmin);
-        return true;
+        if (kmin == kmax) return true;
+        c0 = value; top = base = key2f(kmax);
+        scale = (float)(BINS - 2) / (top - c0);
+        target -= before;
+        __syncthreads();                                             // (the candidates have been read)
+        continue;
     }
     float mine = 0.0f;
     bool found = false;
@@ -1168,6 +1176,8 @@ static __device__ __noinline__ bool list_select(const View w, bool by_mass, cons
     if (!who) return false;
     value = __shfl_sync(0xffffffffu, mine, __ffs(who) - 1);
     return true;
+    }
+    return false;
 }
 
 // How a wide row is cut, from its histogram (summed over the CTAs of the cluster): by one warp of every CTA.  A lane holds 32
