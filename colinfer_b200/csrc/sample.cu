@@ -1685,9 +1685,8 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
         // At most a row per SM, more than the cluster-resident kernel holds at once: a cluster of two or four CTAs per row, where
         // they all run at once.  From 75 rows on there is one CTA per row either way, and the streaming kernel's 1,024 threads get
         // a row through sooner.  60 fp32 rows of 151,936 logits, streaming kernel (half of the SMs idle) and here: mixed filters 62
-        // and 53 us (64 rows with histories 73 and 61), top-p 60 and 53, top_k 50 36 and 27, top_k 1000 65 and 68, no filter 29 and 32,
-        // greedy 12 and 18; bf16 mixed 609 and 82, top-p 74 and 57, no filter 29 and 32.  The host does not see the filters: over
-        // mixed (twice), top_k 50, top_k 1000, top-p and half greedy it is 0.91 of the time.
+        // and 54 us, top-p 61 and 54, top_k 50 36 and 27, top_k 1000 66 and 67, no filter 29 and 29 - 32, greedy 12 and 17; bf16 mixed 108
+        // and 58, top-p 77 and 56, no filter 29 and 29.  The host does not see the filters.
         const int ki = chunk_index(FEW, dtype, mask != nullptr), smem = colinfer_few_smem(V, pen);
         if (smem > kChunkMaxSmem) return -1;
         const int rc = chunk_device(ki, &dev, &sms);
@@ -1696,10 +1695,10 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
             if (V >= 16384 * C && rows <= chunk_clusters(dev, ki, C, smem)) { set = FEW; break; }
         }
         if (set != FEW) return -1;
-        // More rows than SMs.  149 and 200 fp32 rows of 151,936, streaming kernel and here: mixed 66, 66 and 72, 77 us; top-p 124, 125
-        // and 104, 106; top_k 50 65, 83 and 41, 42; top_k 1000 124, 129 and 102, 114; no filter 63, 64 and 65, 74; greedy 29, 31 and
-        // 27, 36: over the same six 0.91 and 0.93 of the time (a wide row alone on an SM has half the threads here).  400 rows: mixed
-        // 115 and 107, top-p 183 and 165, no filter 97 and 133; 592: 166 and 140, 242 and 201, 132 and 138.
+        // More rows than SMs.  149 and 200 fp32 rows of 151,936, streaming kernel and here: mixed 66, 68 and 69, 72 us; top-p 125, 125
+        // and 96, 100; top_k 50 65, 83 and 37, 38; top_k 1000 126, 130 and 55, 61; half greedy 46, 47 and 45, 50; greedy 29, 31 and
+        // 25, 29 (a wide row alone on an SM has a third of the threads here).  400 rows: mixed 117 and 104, top-p 184 and 158, no filter
+        // 97 and 105; 592: 166 and 135, 245 and 197, 133 and 130.
     } else if ((pen && V > kRowV && (dtype == COLINFER_BF16 || rows <= 2 * sms)) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
     const int smem = chunk_smem(set, V, pen), ki = chunk_index(set, dtype, mask != nullptr);
     if (smem > kChunkMaxSmem) return -1;

@@ -15,7 +15,8 @@
 //            above a narrow band, whose logits are gathered and resolved exactly); the draw rescans one warp's region
 //   neither  pass 2 sums the masses; the draw rescans one warp's region
 // Masses are exp(z - max) in integer units of 2^-30 and all sums are integer: results do not depend on the batch.
-// If a list overflows or the estimated band misses, an exact radix select over the 32-bit keys runs (4 more passes).
+// If a list overflows or the estimated band misses, the pivot is found by narrowing the keys of the band, or of the row, 256-fold per
+// pass (a top-k's by an exact radix select, 4 more passes).
 #pragma once
 #include "common.cuh"
 #include "../../include/colinfer_b200.h"
@@ -793,8 +794,8 @@ static __device__ bool radix_select(const Row& rw, int r_lo, int r_hi, const Mas
 // The pivot by mass among the effective logits of [lo, hi], `above` being the mass beyond them: a pass per 256-fold narrowing of the
 // bracket, over exact masses.  bf16 logits without penalties have at most one value among any 2^16 neighbouring keys: a band that holds
 // thousands of equal ones has a few dozen values and takes one pass.  False when the pivot lies elsewhere.
-// A pass takes a seventh of one of the radix select's (only the band's logits add anything) and there are one to three instead of
-// four: 128 bf16 rows of 151,936 with mixed filters 630 -> 102 us, 128 fp32 rows of 262,144 929 -> 155 us.
+// Only the band's logits add anything, and there are one to three passes instead of the radix select's four over all logits: 128 bf16
+// rows of 151,936 with mixed filters 630 -> 110 us, 128 fp32 rows of 262,144 929 -> 199 us.
 static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, int r_hi, const MassFn& mass, float lo, float hi, u64 target, u64 above, u64* bins, Sc* sc, float& pivot) {
     const int tid = threadIdx.x, lane = lane_id();
     uint32_t klo = f2key(lo), khi = f2key(hi);
