@@ -1609,12 +1609,13 @@ extern "C" int colinfer_max_active_clusters(int V, int dtype) {
 namespace {
 constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024;
 // More rows than SMs: two CTAs of 384 threads per SM, one of which reads while the other one is in its block-wide steps.  One of
-// 1,024 where two do not fit (penalty tables of vocabularies beyond some 330,000), and with histories beyond 216,000 logits for bf16
-// rows (a top_p close to 1 beside penalties overflows the lists of 384 threads with equal logits) and for up to two rows per SM (a row
-// alone on an SM gets through sooner with 1,024).  262,144 logits with histories of 2,048, one CTA per SM and two, us: 512 bf16 rows
-// mixed 312 and 493; 160 fp32 rows mixed 109 and 142, no filter 76 and 98, 512 of them mixed 250 and 222, top_p 416 and 354.
-// Without histories two are the faster everywhere but at 160 to 296 half greedy bf16 rows (56 and 60, 79 and 87): 512 bf16 rows
-// greedy 87 and 61, mixed 212 and 189, top_p 360 and 312, top_k 1000 217 and 142; under a mask top_p 465 and 388, top_k 1000 187 and 171.
+// 768 where two do not fit (penalty tables of vocabularies beyond some 330,000), and with histories beyond 216,000 logits for bf16
+// rows and for up to two rows per SM.  262,144 logits with histories of 2,048, one CTA per SM and two, us: bf16 rows mixed 121 and 166
+// (160 rows), 169 and 199 (296), 273 and 304 (512), top_p 234 and 202, 244 and 329, 463 and 398; fp32 rows mixed 107 and 144 (160),
+// 153 and 183 (296), half greedy 74 and 98, 105 and 132, top_p 215 and 181, 227 and 189.
+// Without histories two are the faster everywhere but at 160 to 296 half greedy bf16 rows (56 and 60, 79 and 87) and 296 mixed ones
+// (127 and 166): 512 bf16 rows greedy 87 and 61, mixed 212 and 189, top_p 360 and 312, top_k 1000 217 and 142; under a mask top_p 465
+// and 388, top_k 1000 187 and 171.
 constexpr int kTwoPerSm = 113 * 1024, kRowV = 216000;
 
 // The sets of instantiations: a CTA of 384 threads per row, two per SM (ROWS); a CTA of 1,024 threads per row (ROW); a cluster of
