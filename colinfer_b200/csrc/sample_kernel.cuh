@@ -2009,7 +2009,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
             };
             // The pivot by mass among the logits of [lo, hi], `above` being the mass beyond them: a pass per 256-fold narrowing of
             // the bracket.  A band of bf16 logits, which may hold thousands of equal ones, has at most 256 values: one pass.
-            // False when the pivot lies elsewhere.
+            // False when the pivot lies elsewhere.  A band of a single value takes no pass at all: the lists have counted its logits
+            // beyond what they hold, and so many masses of the value either reach the target or do not.
             auto bracket_select = [&](float lo, float hi, u64 target, u64 above, float& pivot) {
                 uint32_t klo = f2key(lo), khi = f2key(hi);
                 const bool coarse = ELT == 2 && !rw.pen_on;      // every logit is a bf16: one value among any 2^16 neighbouring keys
@@ -2019,7 +2020,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         uint32_t k = khi;
                         if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
                         pivot = key2f(k);
-                        return true;
+                        if (step) return true;
+                        u64 n = 0;
+                        for (int i = lane; i < GW; i += 32) n += (u64)g.at(sc, i / NW)->wn[i % NW];
+                        return target - above <= warp_sum_u64(n) * (u64)rw.mass(pivot);
                     }
                     const int sh = max(coarse ? 16 : 0, 24 - __clz(span));       // at most BINS bins
                     g.sync();

@@ -794,21 +794,23 @@ static __device__ bool radix_select(const Row& rw, int r_lo, int r_hi, const Mas
 // The pivot by mass among the effective logits of [lo, hi], `above` being the mass beyond them: a pass per 256-fold narrowing of the
 // bracket, over exact masses.  bf16 logits without penalties have at most one value among any 2^16 neighbouring keys: a band that holds
 // thousands of equal ones has a few dozen values and takes one pass.  False when the pivot lies elsewhere.
+// listed: how many logits the lists have counted in the bracket, beyond what they hold (-1: unknown).  Where it is known a bracket of
+// a single value takes no pass: so many masses of the value either reach the target or do not.
 // Only the band's logits add anything, and there are one to three passes instead of the radix select's four over all logits: 128 bf16
 // rows of 151,936 with mixed filters 630 -> 110 us, 128 fp32 rows of 262,144 929 -> 199 us.
-static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, int r_hi, const MassFn& mass, float lo, float hi, u64 target, u64 above, u64* bins, Sc* sc, float& pivot) {
+static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, int r_hi, const MassFn& mass, float lo, float hi, u64 target, u64 above, int listed, u64* bins, Sc* sc, float& pivot) {
     const int tid = threadIdx.x, lane = lane_id();
     uint32_t klo = f2key(lo), khi = f2key(hi);
     const bool coarse = rw.p16 != nullptr && !rw.pen_inline;
     for (int step = 0; step < 5; ++step) {
         const uint32_t span = khi - klo;
         if (klo > khi) return false;
-        if (span < (coarse ? 65536u : 1u)) {
+        if (span < (coarse ? 65536u : 1u) && (step || listed >= 0)) {
             // (the only bf16 among them, or none)
             uint32_t k = khi;
             if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
             pivot = key2f(k);
-            return true;
+            return step || target - above <= (u64)listed * (u64)mass(pivot);
         }
         const int sh = max(coarse ? 16 : 0, 24 - __clz(span));           // at most FB_NB bins of 2^sh keys, from the largest down
         for (int i = tid; i < FB_NB; i += NT) bins[i] = 0;
@@ -1661,7 +1663,8 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                             bool got = false;
 #pragma unroll 1
                             for (int all = inside && s_above < target ? 0 : 1; all < 2 && !got && s1 > 0; ++all)
-                                got = bracket_select(rw, r_lo, r_hi, mass, all ? lk : fmaxf(t_lo, lk), all ? L : fminf(t_hi, L), target, all ? 0ull : s_above, fb_hist, sc, lpiv);
+                                got = bracket_select(rw, r_lo, r_hi, mass, all ? lk : fmaxf(t_lo, lk), all ? L : fminf(t_hi, L), target, all ? 0ull : s_above,
+                                                     all || rw.has_pen ? -1 : sc->woffs[NWA], fb_hist, sc, lpiv);
                             if (got) lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
                             const float lk3 = fmaxf(lcut, -ST_FLT_MAX);
                             u64 acc = 0;
