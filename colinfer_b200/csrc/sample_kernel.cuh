@@ -1180,6 +1180,15 @@ static __device__ __noinline__ bool list_select(const View w, bool by_mass, cons
     return false;
 }
 
+// The mass of what the group's warps have listed, beyond what their lists hold too, where that is one value.
+template <bool CL>
+static __device__ __noinline__ u64 listed_mass(const Grp<CL> g, const RowS& rw, float value) {
+    Sc* sc = scratch();
+    uint32_t n = 0;
+    for (int i = lane_id(); i < NW * (CL ? g.C : 1); i += 32) n += (uint32_t)g.at(sc, i / NW)->wn[i % NW];
+    return (u64)__reduce_add_sync(0xffffffffu, n) * (u64)rw.mass(value);
+}
+
 // How a wide row is cut, from its histogram (summed over the CTAs of the cluster): by one warp of every CTA.  A lane holds 32
 // buckets; a rank or a share of the estimated mass is found by a scan over the lanes and one over the buckets of the lane it
 // falls into.  The estimated mass of a logit of bucket b is 2^min(0, e0 - b * e1) (of the last bucket, which holds everything
@@ -2021,9 +2030,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                         if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
                         pivot = key2f(k);
                         if (step) return true;
-                        u64 n = 0;
-                        for (int i = lane; i < GW; i += 32) n += (u64)g.at(sc, i / NW)->wn[i % NW];
-                        return target - above <= warp_sum_u64(n) * (u64)rw.mass(pivot);
+                        return target - above <= listed_mass(g, rw, pivot);
                     }
                     const int sh = max(coarse ? 16 : 0, 24 - __clz(span));       // at most BINS bins
                     g.sync();
