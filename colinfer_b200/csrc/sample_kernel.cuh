@@ -1209,6 +1209,14 @@ static __device__ __noinline__ Ranked ranked(const uint32_t* hist, int last, uin
     const int t = in ? __ffs(in) - 1 : 31;
     return Ranked{hit ? hl * 32 + t : -1, __shfl_sync(0xffffffffu, i - n, t), __shfl_sync(0xffffffffu, i, t)};
 }
+// The middle between the first bf16 >= x (below: the last one <= x) and the next one above: in a row of bf16 logits the edge of a set
+// of values.
+__device__ __forceinline__ float above_bf16(float x, bool below) {
+    int s = __float_as_int(x);
+    s = s < 0 ? (int)(0x80000000u - (uint32_t)s) : s;                    // in the order of the floats
+    s = ((s + (below ? 0 : 0xFFFF)) & ~0xFFFF) + 0x8000;
+    return s >= 0x7F800000 ? SM_POS_INF : __int_as_float(s < 0 ? (int)(0x80000000u - (uint32_t)s) : s);
+}
 template <bool CL>
 static __device__ __noinline__ void decide_row(const Grp<CL> g, RowS& rw, int elt, bool miss) {
     Sc* sc = scratch();
@@ -1306,7 +1314,13 @@ static __device__ __noinline__ void decide_row(const Grp<CL> g, RowS& rw, int el
             // hundred (bf16: four hundred, one value's logits are many), after a sample more, the more the further down.
             uint32_t x0 = 0, x1 = 0;
             const uint32_t rank = n0 + (uint32_t)(part * (float)(n1 - n0)), near = elt == 2 ? 400u : 100u;
-            const uint32_t side = full ? near : min(min((uint32_t)BAND_SIDE, 300u + (uint32_t)sc->V / 256), near + rank / 4);
+            uint32_t side = full ? near : min(min((uint32_t)BAND_SIDE, 300u + (uint32_t)sc->V / 256), near + rank / 4);
+            // bf16 logits there: from one to the next, in buckets.  (Four to a bucket and more: as good as evenly spread over it.)
+            const float x = href - ((float)(bp - hoff) + part) * width;
+            const float step = __int_as_float(max((__float_as_int(x) & 0x7F800000) - (7 << 23), 0)) * scw;
+            const bool coarse = elt == 2 && step > 0.25f;
+            // (less half of the logits that share a value, by which the band grows on average below; at least half of it)
+            if (coarse) side -= min((uint32_t)((float)(n1 - n0) * fminf(step, 1.0f)), side) / 2;
             auto logit_at = [&](uint32_t r, int& bb) {                   // about the r-th largest
                 bb = find_rank(r, x0, x1);
                 return href - ((float)(bb - hoff) + __fdividef((float)(r - x0), fmaxf((float)(x1 - x0), 1.0f))) * width;
@@ -1315,6 +1329,14 @@ static __device__ __noinline__ void decide_row(const Grp<CL> g, RowS& rw, int el
             if (rank > side) t_hi = logit_at(rank - side, band_top);
             t_lo = rank + side > total ? -SM_FLT_MAX : logit_at(rank + side, band_bot);
             if (!(t_lo > -SM_FLT_MAX)) band_bot = NB1 - 1;
+            if (coarse) {
+                // A bucket may hold a single value, of thousands of logits, which lies anywhere in it: the band ends between values,
+                // and reaches to the ends of its buckets where the next value lies beyond them.  300 rows of N(16, 1), 151,936
+                // logits: 245 -> 160 us at 150 rows in the launch, 551 -> 345 at 592 (191 of 300 bands missed the pivot, now none).
+                const float eps = 0.01f * width + fabsf(href) * 1e-6f;
+                if (t_hi < SM_POS_INF) t_hi = fminf(above_bf16(t_hi, false), above_bf16(edge(band_top) + eps, true));
+                if (t_lo > -SM_FLT_MAX) t_lo = -fminf(above_bf16(-t_lo, false), above_bf16(-(edge(band_bot + 1) - eps), true));
+            }
             const int cap = find_rank(500u, x0, x1);
             if (cap < 0 || cap > band_bot) {
                 band_top = 0; band_bot = cap < 0 ? NB1 - 1 : cap - 1;

@@ -57,3 +57,22 @@ def test_coarse_rows_are_cut_at_the_oracles_value(shape, form):
         sp = wl.sampler_params({k: v[at] for k, v in params.items()}, x.size(-1), "cuda")
         got = m["draw"](x[at].cuda(), sp, None, u=u[at].cuda(), flags=flags).cpu().numpy()
         check_tokens(got, want[at.numpy()], [info[i] for i in at.tolist()], f"{shape}, {form}, from {lo}")
+
+
+@pytest.mark.parametrize("rows,V,mean", [(150, 16_000, 16.0), (300, 16_000, -16.0), (60, 98_305, -3.0), (150, 16_000, 10.0), (300, 30_000, 5.0)])
+def test_the_estimated_band_of_coarse_rows_holds_the_pivot(rows, V, mean):
+    """Rows short enough for the lists to hold the few values of a band: it takes no exact select where the band holds the pivot.  (With
+    edges at a rank's place in its bucket, where a single value lies anywhere, a third of such rows took one.)"""
+    m = mods()
+    g = torch.Generator().manual_seed(rows + V)
+    n = torch.arange(rows)
+    x = (torch.randn(rows, 1, V, generator=g) + mean).bfloat16()
+    params = wl._params(rows, V, 0.5 + 0.7 * torch.rand(rows, generator=g), torch.full((rows,), V), 0.8 + 0.19 * torch.rand(rows, generator=g), torch.zeros(rows))
+    u = wl.open_unit(g, rows, 1)
+    got, st = m["draw"](x.cuda(), wl.sampler_params(params, V, "cuda"), None, u=u.cuda(), status=True, flags=_lib.KERNEL_AUTO)
+    few = n[:: rows // 12].tolist()
+    want, info = oracle_draw_rows(x[few].float().numpy(), {k: v[few] for k, v in np_params(params).items()}, None, u=u[few].numpy(), workers=1)
+    check_tokens(got.cpu().numpy()[few], want, info, f"{rows} x {V} around {mean}")
+    slow = int((st & _lib.ROW_SELECT_SLOW).ne(0).sum())
+    print(f"{slow} of {rows} rows slow")
+    assert slow <= rows // 30
