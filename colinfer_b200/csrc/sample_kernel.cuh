@@ -1269,6 +1269,7 @@ static __device__ __noinline__ void decide_row(const Grp<CL> g, RowS& rw, int el
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((href - rw.L) * __frcp_rn(rw.tc) * CI_LOG2E));
         all = all * e - cut_off;
     }
+    if (!CL && ready && rw.hist_full) all = mass;                        // (counted in full by a pass that does not sum)
     auto find_rank = [&](uint32_t rank, uint32_t& before, uint32_t& with) {
         const Ranked r = ranked(hist, last, inc_c, cnt, rank);
         before = r.before; with = r.with;

@@ -38,6 +38,20 @@ def test_every_size_of_a_top_k(rows, V, dtype):
     _draw(x, params, wl.open_unit(g, rows, 1), _lib.KERNEL_AUTO, f"top_k, {rows} x {V} {dtype}", list(range(14)) + [rows - 1])
 
 
+@pytest.mark.parametrize("rows,V", [(150, 40_003), (300, 33_000), (150, 151_936)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_top_k_that_removes_nothing_leaves_the_band_in_its_place(rows, V, dtype):
+    """A top_k beyond what one pass lists, of which fewer logits have any mass, and a top_p: the row is counted in full, cut by its mass
+    alone, and takes no exact select."""
+    g = torch.Generator().manual_seed(rows + 7)
+    x = (torch.randn(rows, 1, V, generator=g) * 2).to(getattr(torch, dtype))
+    n = torch.arange(rows)
+    T = (0.26 if V < 50_000 else 0.2) - 0.02 * (n % 3)
+    params = wl._params(rows, V, T, torch.full((rows,), 10_000), torch.tensor([0.95, 0.8, 0.99])[n // 3 % 3], torch.zeros(rows))
+    st = _draw(x, params, wl.open_unit(g, rows, 1), _lib.KERNEL_AUTO, f"top_k 10,000, {rows} x {V} {dtype}", list(range(9)) + [rows - 1])
+    assert int((st & _lib.ROW_SELECT_SLOW).ne(0).sum()) == 0
+
+
 @pytest.mark.parametrize("rows", [36, 150])
 def test_rows_that_mislead_the_sample(rows):
     """The sample is the first chunks of the warps and a quarter of all others; the mass that the first pass sums is relative to the
