@@ -119,8 +119,9 @@ struct RowS {
 enum { ROW_SAMPLED = 1, ROW_FASTK = 2, ROW_WIDE = 4 };
 enum { PATH_PURE = 0, PATH_LIST = 1, PATH_BAND = 2, PATH_FALLBACK = 3 };
 
-// A warp's ring between passes: chunks consumed, chunks under way, and of which row (index + 1; 0: none) they are.
-struct WarpRing { int cons, out, key; };
+// A warp's ring between passes: chunks consumed, chunks under way, and of which row (index + 1; 0: none) they are; whether the warp
+// asks for chunks, whether a wait of its own ran out (it then waits for nothing any more).
+struct WarpRing { int cons, out, key, asks, lost; };
 
 // Where the row after the one at hand lies (key 0: none).
 struct NextRow { const char* base; uint32_t end; int key, Nc; };
@@ -130,7 +131,7 @@ struct Sc {
     NextRow next[2];
     WarpRing ring[NW];
     int V, W, GW, rank;                // logits per row; mask words per row; warps that share a row; this CTA among them
-    int drop, dead;                    // test flag; a wait ran out
+    int dead;                          // a wait ran out
     __align__(16) uint4 clc; u64 clc_bar;   // the answer of the hardware's work queue, its barrier
     int cls_tot[3]; unsigned short cls_pre[3][NT];   // rows per cost class: all, before each thread's
     int pen_off;                       // offset of the penalty tables in shared memory
@@ -389,6 +390,38 @@ static __device__ __noinline__ void mend_edges(const RowS& rw, uint32_t st, int 
     __syncwarp();
 }
 
+__device__ __forceinline__ bool ring_test(uint32_t bar, uint32_t par, uint32_t ns) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(par), "r"(ns) : "memory");
+    return ok != 0;
+}
+// Waits on where a first test failed, with a limit; the warp calls, and learns whether it may still ask for chunks.  Every warp waits
+// for its own copies.  Where one does not come the row is lost, but the CTA goes on to its end, when another one gets its shared
+// memory: the warp asks for no more, and what else it has under way, the stages from that one on in turn, is let land first (with a
+// limit of its own; what was never asked for does not come either).
+template <int N>
+static __device__ __noinline__ bool ring_wait(uint32_t bar, uint32_t par) {
+    WarpRing& r = scratch()->ring[warp_id()];
+    if (*(volatile int*)&r.lost) return false;
+    auto wait = [&](uint32_t b, uint32_t p, long long t0) {
+        while (!__all_sync(0xffffffffu, ring_test(b, p, 20000u)))
+            if (__any_sync(0xffffffffu, clock64() - t0 > WAIT_CYCLES)) return false;
+        return true;
+    };
+    if (wait(bar, par, clock64())) return r.asks != 0;
+    const bool asked = r.asks != 0;
+    __syncwarp();
+    if (lane_id() == 0) { r.asks = 0; r.lost = 1; scratch()->dead = 1; }
+    if (asked) {
+        const uint32_t first = smem_u32(smem) + OFF_BARS + warp_id() * (8 * N), s = (bar - first) / 8;
+        const long long t0 = clock64();
+        for (uint32_t j = 0; j < N; ++j) wait(first + 8 * ((s + j) % N), s + j >= N ? par ^ 1u : par, t0);
+    }
+    __syncwarp();
+    return false;
+}
+
 // A warp's ring.  While a pass runs its state lives in registers, between passes in Sc.
 template <int ELT>
 struct Pipe {
@@ -401,9 +434,8 @@ struct Pipe {
         const int warp = warp_id();
         buf = smem_u32(smem) + warp * RING;
         bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
-        const Sc* sc = scratch();
-        cons = sc->ring[warp].cons; out = sc->ring[warp].out;
-        asks = !(sc->drop | sc->dead);
+        const WarpRing& r = scratch()->ring[warp];
+        cons = r.cons; out = r.out; asks = r.asks != 0;
     }
     __device__ __forceinline__ uint32_t conv() const { return buf + NST * CHB; }          // bf16: an fp32 copy of one chunk
     __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) % NST) * CHB; }
@@ -424,19 +456,7 @@ struct Pipe {
     // The bytes of the chunk j places from the next one to consume are there.
     __device__ __forceinline__ void wait(int j = 0) { wait_at(bar + 8 * ((uint32_t)(cons + j) % NST), ((uint32_t)(cons + j) / NST) & 1u); }
     __device__ __forceinline__ void wait_at(uint32_t b, uint32_t par) {
-        auto test = [&]() {
-            uint32_t ok;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok) : "r"(b), "r"(par), "r"(20000u) : "memory");
-            return ok != 0;
-        };
-        if (!test()) {
-            // (with the test flag nothing was asked for: the wait runs out, once per CTA and warp)
-            Sc* sc = scratch();
-            const long long t0 = clock64();
-            while (!test()) if (*(volatile int*)&sc->dead || clock64() - t0 > WAIT_CYCLES) { sc->dead = 1; asks = false; break; }
-        }
-        __syncwarp();
+        if (!__all_sync(0xffffffffu, ring_test(b, par, 20000u))) asks = ring_wait<NST>(b, par);
     }
     // Between passes: what was asked for ahead stays when it belongs to row `key`, else it is let land and dropped.
     __device__ __forceinline__ void expect(int key) {
@@ -1477,13 +1497,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     if (CL && warp == PW) next_words = load_params(a, blockIdx.x / a.cluster, lane);   // (before the logits keep the memory busy)
     if (tid == 0) {
         sc->V = V; sc->W = a.W; sc->GW = GW; sc->rank = g.rank;
-        sc->drop = (a.flags & COLINFER_TEST_DROP_COPY) != 0; sc->dead = 0;
+        sc->dead = 0;
         sc->pen_off = pen_offset(V, a.p.history != nullptr);
         sc->flags = 0; sc->nsel = sc->npush = 0; sc->sum_all = sc->sum_keep = 0;
     }
     if (lane == 0) {
         const uint32_t bar = smem_u32(smem) + OFF_BARS + warp * (8 * NST);
-        sc->ring[warp].cons = 0; sc->ring[warp].out = 0; sc->ring[warp].key = 0;
+        sc->ring[warp] = WarpRing{0, 0, 0, !((a.flags & COLINFER_TEST_DROP_COPY) && !(warp & 1)), 0};   // (test flag: every other warp asks for nothing)
         sc->wn[warp] = 0; sc->swf[warp] = CI_NEG_INF;
         for (int j = 0; j < NST; ++j) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * j) : "memory");
         fence_mbar_init();

@@ -82,6 +82,27 @@ def test_copies_that_never_arrive_end_the_launch(form):
     assert torch.equal(again, good) and torch.equal(st3, st) and int((st & _lib.ROW_TIMEOUT).sum()) == 0
 
 
+@pytest.mark.parametrize("rows,V,dtype", [(150, 151_936, "float32"), (444, 60_000, "float32"), (60, 151_936, "bfloat16"), (300, 151_937, "bfloat16")])
+def test_a_lost_copy_leaves_none_under_way(rows, V, dtype):
+    """With the test flag every other warp's copies never come: the others go on reading theirs to the end of the row, and of the rows
+    after it, so that none lands in shared memory that is another CTA's by then: launches on its heels, of rows of several passes, are
+    as without it."""
+    m = mods()
+    g = torch.Generator().manual_seed(rows)
+    x = (torch.randn(rows, 1, V, generator=g) * 2).to(getattr(torch, dtype)).cuda()
+    n = torch.arange(rows)
+    params = wl._params(rows, V, 0.8, torch.tensor([V, 40, 1000])[n % 3], torch.tensor([0.95, 1.0])[n % 2], 0.0)
+    sp = wl.sampler_params(params, V, "cuda")
+    u = wl.open_unit(g, rows, 1).cuda()
+    good, st = m["draw"](x, sp, None, u=u, status=True, flags=_lib.KERNEL_AUTO)
+    for _ in range(2):
+        _, lost = m["draw"](x, sp, None, u=u, status=True, flags=_lib.KERNEL_AUTO | _lib.TEST_DROP_COPY)
+        runs = [m["draw"](x, sp, None, u=u, status=True, flags=_lib.KERNEL_AUTO) for _ in range(3)]
+        assert (lost & _lib.ROW_TIMEOUT).ne(0).all()
+        for got, st2 in runs:
+            assert torch.equal(got, good) and torch.equal(st2, st)
+
+
 @pytest.mark.parametrize("rows,V", [(34, 98_320), (60, 98_307), (150, 20_000), (301, 4_099)])
 def test_random_rows_of_every_form_of_the_chunk_kernel(rows, V):
     """Random value shapes (ties, runs of -inf, dominant tokens, flat and wide rows), filters, masks and histories through the chunk
