@@ -1616,9 +1616,10 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
     // half of the CTAs they would go to every other SM in pairs.  So in such launches the second CTA of an SM starts a little later;
     // with rows of several passes by what the first pass takes alone (16 bytes a cycle).  432 top-p rows 187 -> 160 us, 360 without a
     // filter 113 -> 93, 1,024 mixed ones 212 -> 194, 1,024 greedy ones 109 -> 103.  (Mixed rows with penalties,
-    // whose passes take longer than their bytes, do not stay in step: 1,024 of them 259 us with the short delay, 263 with the long one.)
+    // whose passes take longer than their bytes, do not stay in step: 1,024 of them 259 us with the short delay, 263 with the long one.
+    // Rows that are not dealt have not been counted: the short delay.)
     if (!CL && CTAS_PER_SM == 2 && n_rows > 2 * NUM_SM && (n_rows - 1) % (2 * NUM_SM) < NUM_SM && (int)blockIdx.x >= NUM_SM && (int)blockIdx.x < 2 * NUM_SM) {
-        const bool wide = (int)blockIdx.x < sc->cls_tot[0] && (a.p.history == nullptr || 2 * sc->cls_tot[0] > n_rows);
+        const bool wide = dealt && (int)blockIdx.x < sc->cls_tot[0] && (a.p.history == nullptr || 2 * sc->cls_tot[0] > n_rows);
         const long long t0 = clock64(), d = (long long)V * ELT / (wide ? 16 : 48);
         while (clock64() - t0 < d) __nanosleep(200);
     }

@@ -93,6 +93,17 @@ def test_launches_whose_last_turn_is_half_full(rows):
     _draw(x, params, wl.open_unit(g, rows, 1), _lib.KERNEL_AUTO, f"{rows} rows", list(range(0, rows, 37)) + [rows - 1])
 
 
+# rows of 151,936 logits: the second CTA is late by 38,000 cycles (fp32) or 19,000; more rows than are dealt by cost (16,384)
+@pytest.mark.parametrize("rows,V,dtype", [(298, 151_936, "float32"), (432, 151_936, "bfloat16"), (16_385, 700, "float32"), (16_385, 700, "bfloat16")])
+def test_late_starts_of_long_rows_and_of_rows_that_are_not_dealt(rows, V, dtype):
+    g = torch.Generator().manual_seed(rows)
+    x = (torch.randn(rows, 1, V, generator=g) * 2).to(getattr(torch, dtype))
+    n = torch.arange(rows)
+    params = wl._params(rows, V, torch.where(n % 7 == 6, 0.0, 0.9), torch.tensor([V, V, 40])[n % 3], 0.95, 0.0)
+    few = sorted({0, 1, 2, 147, 148, 149, 150, 295, 296, 297, rows // 2, rows - 2, rows - 1})
+    _draw(x, params, wl.open_unit(g, rows, 1), _lib.KERNEL_AUTO, f"{rows} x {V} {dtype}", few)
+
+
 @pytest.mark.parametrize("dtype,levels,hist", [("bfloat16", 0, 0), ("bfloat16", 4, 0), ("float32", 8, 0), ("float32", 0, 0), ("bfloat16", 4, 200)])
 def test_the_streaming_kernels_band_of_thousands_of_equal_logits(dtype, levels, hist):
     """Bands that overflow the lists: the pivot by narrowing the band's keys, or all keys where the band is off it as well."""
