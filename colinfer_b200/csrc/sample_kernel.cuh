@@ -439,18 +439,18 @@ struct Pipe {
     }
     __device__ __forceinline__ uint32_t conv() const { return buf + NST * CHB; }          // bf16: an fp32 copy of one chunk
     __device__ __forceinline__ uint32_t stage(int j = 0) const { return buf + ((uint32_t)(cons + j) % NST) * CHB; }
-    // Copies `bytes` to `dst`, counted on `bar`.  The warp calls, one lane acts (unless a wait of its own ran out).
+    // Copies `bytes` to `dst`, counted on `bar`.  The warp calls, one lane acts (unless a wait of its own ran out).  None: the last
+    // chunk of the buffer's last row may hold less than a unit of 16 bytes, which comes by ordinary loads (mend_edges).
     __device__ __forceinline__ void copy(uint32_t dst, const char* p, uint32_t bytes, uint32_t bar, u64 pol) const {
         asm volatile("{\n\t.reg .pred e, a;\n\tsetp.ne.u32 a, %5, 0;\n\telect.sync _|e, 0xffffffff;\n\tand.pred e, e, a;\n\t"
-                     "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
+                     "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\tsetp.ne.and.u32 e, %2, 0, e;\n\t"
                      "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n\t}"
                      ::"r"(dst), "l"(p), "r"(bytes), "r"(bar), "l"(pol), "r"((uint32_t)asks) : "memory");
     }
     // skip: bytes at the start of the stage that are left out
     __device__ __forceinline__ void issue(const char* p, uint32_t bytes, u64 pol, uint32_t skip = 0) {
         const uint32_t s = (uint32_t)(cons + out) % NST;
-        if (bytes) copy(buf + s * CHB + skip, p, bytes, bar + 8 * s, pol);
-        else if (lane_id() == 0 && asks) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar + 8 * s) : "memory");
+        copy(buf + s * CHB + skip, p, bytes, bar + 8 * s, pol);
         ++out;
     }
     // The bytes of the chunk j places from the next one to consume are there.

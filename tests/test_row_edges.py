@@ -23,9 +23,23 @@ def test_copies_stay_inside_the_buffer(built_lib, elt, dtype):
                         assert b < lo + 16 and e > hi - 16               # at most part of a unit is left to ordinary loads
 
 
+# the last chunk of the buffer's last row holds less than a unit, and is beyond those that a warp asks for before its first one is read:
+# a CTA per row (33 chunks, 12 warps), clusters of two and of four (193 and 321 chunks, 32 and 64 warps)
+SHORT_TAILS = [(149, 16_385), (57, 98_305), (33, 163_841)]
+
+
+@pytest.mark.parametrize("rows,V", SHORT_TAILS)
+@pytest.mark.parametrize("elt,dtype", [(4, _lib.F32), (2, _lib.BF16)])
+def test_nothing_is_copied_of_a_chunk_without_a_whole_unit(built_lib, rows, V, elt, dtype):
+    begin, end = C.c_int64(), C.c_int64()
+    assert _lib.lib().colinfer_sample_copy_range(1 << 20, dtype, rows, V, rows - 1, C.byref(begin), C.byref(end)) == 0
+    lo, hi = (rows - 1) * V * elt // 16 * 16, rows * V * elt
+    assert end.value < hi and end.value == lo + (hi - lo - 1) // (512 * elt) * (512 * elt)
+
+
 # a CTA per row and a cluster per row; rows of less than a unit, around a chunk of 512, and an odd one of many chunks
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,V", [(150, 1), (151, 3), (150, 5), (149, 511), (150, 513), (301, 4097), (40, 98_307)])
+@pytest.mark.parametrize("rows,V", [(150, 1), (151, 3), (150, 5), (149, 511), (150, 513), (301, 4097), (40, 98_307)] + SHORT_TAILS)
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_rows_of_a_buffer_at_any_alignment_draw_the_same_tokens(rows, V, dtype):
     """The first and last logits of the buffer decide (they are among the largest of their rows), and infinities surround it."""
