@@ -76,3 +76,19 @@ def test_the_estimated_band_of_coarse_rows_holds_the_pivot(rows, V, mean):
     slow = int((st & _lib.ROW_SELECT_SLOW).ne(0).sum())
     print(f"{slow} of {rows} rows slow")
     assert slow <= rows // 30
+
+
+@pytest.mark.parametrize("rows,V", [(300, 262_144), (300, 216_064)])
+def test_bands_of_long_coarse_rows_fit_the_lists(rows, V):
+    """A few values to a bucket of the histogram, 300 logits to a value: what the edges of a band move out by to end between values has
+    to be made up for, or the lists of its warps overflow (5 of 160 rows of 262,144 did)."""
+    m = mods()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = (torch.randn(rows, 1, V, generator=g, device="cuda") * 2).bfloat16()
+    params = wl._params(rows, V, 0.8, V, 0.95, 0.0)
+    u = wl.open_unit(torch.Generator().manual_seed(1), rows, 1)
+    got, st = m["draw"](x, wl.sampler_params(params, V, "cuda"), None, u=u.cuda(), status=True, flags=_lib.KERNEL_AUTO)
+    few = torch.arange(0, rows, rows // 8).tolist()
+    want, info = oracle_draw_rows(x[few].float().cpu().numpy(), {k: v[few] for k, v in np_params(params).items()}, None, u=u[few].numpy(), workers=1)
+    check_tokens(got.cpu().numpy()[few], want, info, f"{rows} x {V}")
+    assert int((st & _lib.ROW_SELECT_SLOW).ne(0).sum()) <= 1
