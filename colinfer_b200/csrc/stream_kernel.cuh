@@ -797,7 +797,7 @@ static __device__ bool radix_select(const Row& rw, int r_lo, int r_hi, const Mas
 // listed: how many logits the lists have counted in the bracket, beyond what they hold (-1: unknown).  Where it is known a bracket of
 // a single value takes no pass: so many masses of the value either reach the target or do not.
 // Only the band's logits add anything, and there are one to three passes instead of the radix select's four over all logits: 128 bf16
-// rows of 151,936 with mixed filters 630 -> 110 us, 128 fp32 rows of 262,144 929 -> 199 us.
+// rows of 151,936 with mixed filters 630 -> 104 us, 128 fp32 rows of 262,144 929 -> 199 us.
 static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, int r_hi, const MassFn& mass, float lo, float hi, u64 target, u64 above, int listed, u64* bins, Sc* sc, float& pivot) {
     const int tid = threadIdx.x, lane = lane_id();
     uint32_t klo = f2key(lo), khi = f2key(hi);
@@ -815,24 +815,13 @@ static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, i
         const int sh = max(coarse ? 16 : 0, 24 - __clz(span));           // at most FB_NB bins of 2^sh keys, from the largest down
         for (int i = tid; i < FB_NB; i += NT) bins[i] = 0;
         __syncthreads();
-        for (int i0 = r_lo; i0 < r_hi; i0 += 512) {
-            float4 v[4];
+        for (int i0 = r_lo; i0 < r_hi; i0 += 128) {
+            const float4 x = rw.load4(i0 + lane * 4);
+            const float e[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                v[k] = make_float4(CI_NEG_INF, CI_NEG_INF, CI_NEG_INF, CI_NEG_INF);
-                if (i0 + k * 128 < r_hi) v[k] = rw.raw4(i0 + k * 128 + lane * 4);
-            }
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                if (i0 + k * 128 >= r_hi) break;
-                float4 x = k == 0 ? v[0] : k == 1 ? v[1] : k == 2 ? v[2] : v[3];
-                x = rw.fix4(x, i0 + k * 128 + lane * 4, rw.V);
-                const float e[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t f = f2key(e[j]);
-                    if (f >= klo && f <= khi) add64(&bins[(khi - f) >> sh], (u64)mass(e[j]));
-                }
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t f = f2key(e[j]);
+                if (f >= klo && f <= khi) add64(&bins[(khi - f) >> sh], (u64)mass(e[j]));
             }
         }
         __syncthreads();
@@ -1584,7 +1573,9 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                             __syncthreads();
                             n = sc->glist_n <= GLIST ? sc->glist_n : -1;
                         }
-                        bool ok = n >= 0 && s1 > 0, inside = n < 0;   // inside: the pivot may lie in the band
+                        // (n < 0 from here on: the pivot may lie in the band, the lists do not say where.  A variable of its own for that
+                        // slowed the first pass of bf16 rows, far from here: 128 rows of 151,936, top_k 50, 26 -> 29 us)
+                        bool ok = n >= 0 && s1 > 0;
                         float cut2 = lcut;
                         if (ok) {
                             u64 part = 0;
@@ -1592,7 +1583,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                             u64 s_band;
                             block_excl_scan(part, sc, s_band);
                             const u64 target = ceil_target(topp, s1);
-                            ok = inside = s_above < target && target <= s_above + s_band;   // the pivot lies inside the band
+                            ok = s_above < target && target <= s_above + s_band;   // the pivot lies inside the band
                             if (ok) {
                                 const float base = t_hi < ST_POS_INF ? t_hi : L;
                                 // (a small nucleus gathers everything above the cut: the bins span [cut, base], not [-max, base])
@@ -1604,6 +1595,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                                     cut2 = fmaxf(lcut, lower_logit_for(scale_logit(lp, tc), tc, lp));
                                     if (cut2 < t_lo) ok = false;          // a tie partner could lie below the band
                                 }
+                                if (!ok) n = -1;
                             }
                         }
                         if (ok) {
@@ -1620,7 +1612,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                             }
                         } else {
                             status |= COLINFER_ROW_SELECT_SLOW;
-                            if (attempt == 0 && !inside && s1 > 0) {
+                            if (attempt == 0 && n >= 0 && s1 > 0) {
                                 // The estimated band missed the pivot.  Exact masses of the WIN fine buckets next to the band,
                                 // on the side the pivot lies, give its bucket; the mass pass then runs again around it.
                                 constexpr int WIN = BINS + FB_NB;
@@ -1662,7 +1654,7 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                             const u64 target = ceil_target(topp, s1);
                             bool got = false;
 #pragma unroll 1
-                            for (int all = inside && s_above < target ? 0 : 1; all < 2 && !got && s1 > 0; ++all)
+                            for (int all = n < 0 && s_above < target ? 0 : 1; all < 2 && !got && s1 > 0; ++all)
                                 got = bracket_select(rw, r_lo, r_hi, mass, all ? lk : fmaxf(t_lo, lk), all ? L : fminf(t_hi, L), target, all ? 0ull : s_above,
                                                      all || rw.has_pen ? -1 : sc->woffs[NWA], fb_hist, sc, lpiv);
                             if (got) lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
