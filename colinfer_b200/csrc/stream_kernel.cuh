@@ -793,45 +793,53 @@ static __device__ bool radix_select(const Row& rw, int r_lo, int r_hi, const Mas
 
 // The pivot by mass among the effective logits of [lo, hi], `above` being the mass beyond them: a pass per 256-fold narrowing of the
 // bracket, over exact masses.  bf16 logits without penalties have at most one value among any 2^16 neighbouring keys: a band that holds
-// thousands of equal ones has a few dozen values and takes one pass.  False when the pivot lies elsewhere.
+// thousands of equal ones has a few dozen values and takes one pass.  band: the bracket may miss the pivot, which then is looked for
+// among all logits of [lk, L]; else false when the pivot lies elsewhere.
 // listed: how many logits the lists have counted in the bracket, beyond what they hold (-1: unknown).  Where it is known a bracket of
 // a single value takes no pass: so many masses of the value either reach the target or do not.
 // Only the band's logits add anything, and there are one to three passes instead of the radix select's four over all logits: 128 bf16
-// rows of 151,936 with mixed filters 630 -> 104 us, 128 fp32 rows of 262,144 929 -> 199 us.
-static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, int r_hi, const MassFn& mass, float lo, float hi, u64 target, u64 above, int listed, u64* bins, Sc* sc, float& pivot) {
+// rows of 151,936 with mixed filters 630 -> 105 us, 128 fp32 rows of 262,144 929 -> 199 us.
+static __device__ __forceinline__ bool bracket_select(const Row& rw, int r_lo, int r_hi, const MassFn& mass, float lo, float hi, float lk, float L, u64 target, u64 above, int listed, bool band, u64* bins, Sc* sc, float& pivot) {
     const int tid = threadIdx.x, lane = lane_id();
     uint32_t klo = f2key(lo), khi = f2key(hi);
     const bool coarse = rw.p16 != nullptr && !rw.pen_inline;
     for (int step = 0; step < 5; ++step) {
         const uint32_t span = khi - klo;
-        if (klo > khi) return false;
-        if (span < (coarse ? 65536u : 1u) && (step || listed >= 0)) {
-            // (the only bf16 among them, or none)
-            uint32_t k = khi;
-            if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
-            pivot = key2f(k);
-            return step || target - above <= (u64)listed * (u64)mass(pivot);
-        }
-        const int sh = max(coarse ? 16 : 0, 24 - __clz(span));           // at most FB_NB bins of 2^sh keys, from the largest down
-        for (int i = tid; i < FB_NB; i += NT) bins[i] = 0;
-        __syncthreads();
-        for (int i0 = r_lo; i0 < r_hi; i0 += 128) {
-            const float4 x = rw.load4(i0 + lane * 4);
-            const float e[4] = {x.x, x.y, x.z, x.w};
+        if (klo <= khi) {
+            if (span < (coarse ? 65536u : 1u) && (step || listed >= 0)) {
+                // (the only bf16 among them, or none)
+                uint32_t k = khi;
+                if (coarse) k = khi >= 0x80000000u && (khi & 0xFFFF0000u) >= klo ? khi & 0xFFFF0000u : ((khi + 1u) & 0xFFFF0000u) - 1u;
+                pivot = key2f(k);
+                if (step || target - above <= (u64)listed * (u64)mass(pivot)) return true;
+            } else {
+                const int sh = max(coarse ? 16 : 0, 24 - __clz(span));   // at most FB_NB bins of 2^sh keys, from the largest down
+                for (int i = tid; i < FB_NB; i += NT) bins[i] = 0;
+                __syncthreads();
+                for (int i0 = r_lo; i0 < r_hi; i0 += 128) {
+                    const float4 x = rw.load4(i0 + lane * 4);
+                    const float e[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t f = f2key(e[j]);
-                if (f >= klo && f <= khi) add64(&bins[(khi - f) >> sh], (u64)mass(e[j]));
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t f = f2key(e[j]);
+                        if (f >= klo && f <= khi) add64(&bins[(khi - f) >> sh], (u64)mass(e[j]));
+                    }
+                }
+                __syncthreads();
+                int b; u64 before, tot;
+                bins_find([&](int i) { return bins[i]; }, FB_NB, target - above, sc, b, before, tot);
+                __syncthreads();
+                if (b >= 0) {
+                    above += before;
+                    khi -= (uint32_t)b << sh;
+                    klo = max(klo, khi - ((1u << sh) - 1u));
+                    continue;
+                }
             }
         }
-        __syncthreads();
-        int b; u64 before, tot;
-        bins_find([&](int i) { return bins[i]; }, FB_NB, target - above, sc, b, before, tot);
-        __syncthreads();
-        if (b < 0) return false;
-        above += before;
-        khi -= (uint32_t)b << sh;
-        klo = max(klo, khi - ((1u << sh) - 1u));
+        if (!band) return false;
+        band = false;
+        klo = f2key(lk); khi = f2key(L); above = 0; listed = -1; step = -1;
     }
     return false;
 }
@@ -1652,11 +1660,9 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample_stream(const __grid_
                             float lpiv;
                             corr = false; rw.pen_inline = rw.has_pen;
                             const u64 target = ceil_target(topp, s1);
-                            bool got = false;
-#pragma unroll 1
-                            for (int all = n < 0 && s_above < target ? 0 : 1; all < 2 && !got && s1 > 0; ++all)
-                                got = bracket_select(rw, r_lo, r_hi, mass, all ? lk : fmaxf(t_lo, lk), all ? L : fminf(t_hi, L), target, all ? 0ull : s_above,
-                                                     all || rw.has_pen ? -1 : sc->woffs[NWA], fb_hist, sc, lpiv);
+                            const bool in_band = n < 0 && s_above < target;
+                            const bool got = s1 > 0 && bracket_select(rw, r_lo, r_hi, mass, in_band ? fmaxf(t_lo, lk) : lk, in_band ? fminf(t_hi, L) : L, lk, L, target, in_band ? s_above : 0ull,
+                                                                      in_band && !rw.has_pen ? sc->woffs[NWA] : -1, in_band, fb_hist, sc, lpiv);
                             if (got) lcut = fmaxf(lcut, lower_logit_for(scale_logit(lpiv, tc), tc, lpiv));
                             const float lk3 = fmaxf(lcut, -ST_FLT_MAX);
                             u64 acc = 0;
