@@ -1609,16 +1609,31 @@ extern "C" int colinfer_max_active_clusters(int V, int dtype) {
 namespace {
 constexpr int kChunkMaxV = 524288, kChunkMaxSmem = 226 * 1024;
 // More rows than SMs: two CTAs of 384 threads per SM, one of which reads while the other one is in its block-wide steps.  One of
-// 768 where two do not fit (penalty tables of vocabularies beyond some 330,000), and with histories beyond 216,000 logits for bf16
-// rows and for up to two rows per SM.  262,144 logits with histories of 2,048, one CTA per SM and two, us: bf16 rows mixed 121 and 166
-// (160 rows), 169 and 199 (296), 273 and 304 (512), top_p 234 and 202, 244 and 329, 463 and 398; fp32 rows mixed 107 and 144 (160),
-// 153 and 183 (296), half greedy 74 and 98, 105 and 132, top_p 215 and 181, 227 and 189.
-// Without histories two are the faster everywhere but at 160 to 296 half greedy bf16 rows (56 and 60, 79 and 87) and 296 mixed ones
-// (127 and 166): 512 bf16 rows greedy 87 and 61, mixed 212 and 189, top_p 360 and 312, top_k 1000 217 and 142; under a mask top_p 465
-// and 388, top_k 1000 187 and 171.
-constexpr int kTwoPerSm = 113 * 1024, kRowV = 216000;
+// 768 where two do not fit (penalty tables of vocabularies beyond some 330,000), and for long rows with histories (one_per_sm).
+// One CTA per SM over two, histories of 2,048, geometric mean of the times of mixed, top_p, top_k 1000, half greedy and top_k 50 rows:
+//   rows                160/180   210    240    296    360    512    700   1,024
+//   bf16  200,000         0.99                  1.04   0.99   1.14   1.11   1.14
+//         216,064         0.96   1.03   1.08   0.99   1.03   1.12   1.04   1.10
+//         262,144         0.95   1.01   1.05   0.94   0.99   1.09   1.07   1.09
+//         280,000         0.91   0.94   1.01   0.96   0.93   1.01   1.02
+//         300,000         0.91                 0.96   0.94   1.01   1.01
+//   fp32  200,000         1.02                 1.07   1.09   1.19   1.16   1.21
+//         216,064         1.01   1.05   1.12   1.07   1.05   1.17   1.14   1.19
+//         262,144         1.00   1.05   1.11   1.05   1.00   1.15   1.10   1.14
+//         280,000         0.94   1.01   1.05   0.99
+//         300,000         0.97                 0.99   0.96   1.06   1.04
+// The host does not see the filters, which differ: 262,144 bf16 logits, 160 rows, mixed 120 and 162 us, half greedy 77 and 110, top_p 228
+// and 198, top_k 1000 141 and 111.  Where the mean is even the mixed rows decide (280,000, 512 bf16 rows: 276 and 364).
+// Without histories two are the faster everywhere but for up to two rows per SM half greedy (200,000 to 262,144, either type: 0.80 to
+// 0.95), and mixed at 160 (0.85 to 0.91): over the five 1.07 to 1.26.
+constexpr int kTwoPerSm = 113 * 1024, kRowV = 216000, kLongRowV = 280000;
+bool one_per_sm(int V, int dtype, bool pen, long long rows, int sms) {
+    if (!pen || V <= kRowV) return false;
+    const bool bf16 = dtype == COLINFER_BF16;
+    return V >= kLongRowV ? bf16 || rows <= 2 * sms : rows <= (bf16 ? 2 * sms : sms * 5 / 4);
+}
 
-// The sets of instantiations: a CTA of 384 threads per row, two per SM (ROWS); a CTA of 1,024 threads per row (ROW); a cluster of
+// The sets of instantiations: a CTA of 384 threads per row, two per SM (ROWS); a CTA of 768 threads per row (ROW); a cluster of
 // CTAs per row (FEW).
 enum { ROWS = 0, FEW = 1, ROW = 2 };
 int chunk_index(int set, int dtype, bool mask) { return 4 * set + (dtype == COLINFER_F32 ? 0 : 2) + (mask ? 1 : 0); }
@@ -1700,7 +1715,7 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
         // and 96, 100; top_k 50 65, 83 and 37, 38; top_k 1000 126, 130 and 55, 61; half greedy 46, 47 and 45, 50; greedy 29, 31 and
         // 25, 29 (a wide row alone on an SM has a third of the threads here).  400 rows: mixed 117 and 104, top-p 184 and 158, no filter
         // 97 and 105; 592: 166 and 135, 245 and 197, 133 and 130.
-    } else if ((pen && V > kRowV && (dtype == COLINFER_BF16 || rows <= 2 * sms)) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
+    } else if (one_per_sm(V, dtype, pen, rows, sms) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
     const int smem = chunk_smem(set, V, pen), ki = chunk_index(set, dtype, mask != nullptr);
     if (smem > kChunkMaxSmem) return -1;
     {

@@ -1,5 +1,5 @@
-// sample_row.cu -- the fused kernel with one CTA of 1,024 threads per row and SM, for launches of more rows than SMs whose rows
-// want more shared memory than half an SM has, and for long rows with histories (kRowV in sample.cu).
+// sample_row.cu -- the fused kernel with one CTA of 768 threads per row and SM, for launches of more rows than SMs whose rows
+// want more shared memory than half an SM has, and for long rows with histories (one_per_sm in sample.cu).
 #define SMP_NAME smp_row
 #define SMP_THREADS 768
 #define SMP_CTAS 1

@@ -34,6 +34,9 @@ def _case(rows, V, dtype, seed, levels=0, head=0):
     (150, 511, "bfloat16", False, 300, 0, 0), (201, 8193, "float32", False, 700, 0, 20), (296, 1024, "bfloat16", True, 0, 0, 0),
     (298, 4099, "float32", True, 48, 0, 0), (151, 65536, "bfloat16", False, 0, 4, 0), (150, 65536, "bfloat16", False, 2500, 8, 0),
     (150, 65537, "float32", False, 0, 16, 0), (150, 229632, "bfloat16", False, 30, 0, 0), (150, 262144, "float32", False, 200, 0, 100),
+    # long rows with histories: the last ones with an SM of their own, the first ones that share it
+    (185, 216064, "float32", False, 200, 0, 0), (186, 216064, "float32", False, 200, 0, 0), (296, 216064, "bfloat16", False, 200, 0, 100),
+    (297, 262144, "bfloat16", False, 200, 0, 0), (297, 280000, "bfloat16", False, 200, 0, 0),
 ])
 def test_every_choice_of_kernel_draws_the_oracles_tokens(rows, V, dtype, mask, hist, levels, head):
     m = mods()
