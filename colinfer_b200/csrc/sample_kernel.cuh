@@ -1788,11 +1788,13 @@ __global__ void __launch_bounds__(NT, CTAS_PER_SM) k_sample(const __grid_constan
                     if (!count_hist) { tw = sure; in_klist = true; }
                     else if (rw.kk > 0 && rw.kk < V) {
                         // So does a row with a top-k, where the sample says how far down the k-th largest lies: four standard
-                        // deviations below that and no more than half of what the lists hold.
+                        // deviations below that, and so many logits as fill 65 % of the lists, or a warp's may not hold its share
+                        // (180 of 277 logits with two CTAs per SM; the share's standard deviation, the bound's included, is 20).  592 fp32
+                        // rows, one pass and two: 151,936 logits, top_k up to 1,500, 136 and 203 us; 262,144, up to 1,200, 163 and 272.
                         const float f = (float)min(2 * NW, share) / (float)share, want = (float)rw.kk / (float)g.C * f;
                         const int r = (int)(want + 4.0f * sqrtf(want)) + 8;
                         const float t3 = bound(r);
-                        if ((float)r < 0.55f * f * (float)(KCAPC * NW) && t3 > -SM_FLT_MAX) { count_hist = false; tw = fmaxf(t3, sure); in_klist = true; }
+                        if ((float)r < 0.65f * f * (float)(KCAPC * NW) && t3 > -SM_FLT_MAX) { count_hist = false; tw = fmaxf(t3, sure); in_klist = true; }
                     }
                 }
                 if (in_klist) { list = klist + warp * KCAPC; lcap = KCAPC; }
