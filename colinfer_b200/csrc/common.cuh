@@ -98,35 +98,37 @@ __device__ __forceinline__ u64 quotient2(u64 l, u64 ntc, u64 r) {
     return fma2(fma2(q0, ntc, l), r, q0);
 }
 
-// The masses of MassFn for pairs of logits, each as two floats: mass = (hi * 2^15 + lo * 2^-15) * 2^15 with hi a multiple of
+// The masses of MassFn for pairs of logits, each in two parts: mass = (hi * 2^15 + lo * 2^-15) * 2^15 with hi a multiple of
 // 2^-15 and lo an integer, |lo| <= 2^14.  The arithmetic is MassFn's, operation by operation, two logits per instruction;
 // rounding the exponential to a multiple of 2^-30 takes two rounding additions instead of a conversion, which would double
 // the load of the exponentials' pipe.  A logit of -inf gives NaN.
 struct Mass2 {
     u64 rinv, ntc, nm;
     __device__ __forceinline__ void init(const MassFn& f) { rinv = pk2(f.rinv, f.rinv); ntc = pk2(-f.tc, -f.tc); nm = pk2(-f.m, -f.m); }
-    __device__ __forceinline__ void operator()(float l0, float l1, u64& hi, u64& lo) const {
+    __device__ __forceinline__ void exponentials(float l0, float l1, float& e0, float& e1) const {
         const u64 z = quotient2(pk2(l0, l1), ntc, rinv);
-        float y0, y1, e0, e1;
+        float y0, y1;
         up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(y1));
+    }
+    // 12582912 + lo: what the exponential e is beyond hi, exactly, rounded to 2^-30.
+    static __device__ __forceinline__ u64 rest(u64 e, u64 hi) {
+        return fma2(fma2(hi, pk2(-1.0f, -1.0f), e), pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f));
+    }
+    __device__ __forceinline__ void parts(float l0, float l1, u64& hi, u64& w) const {
+        float e0, e1;
+        exponentials(l0, l1, e0, e1);
         const u64 e = pk2(e0, e1);
-        hi = add2(add2(e, pk2(384.0f, 384.0f)), pk2(-384.0f, -384.0f));        // e rounded to a multiple of 2^-15
-        const u64 r = fma2(hi, pk2(-1.0f, -1.0f), e);                           // the rest, exactly
-        lo = add2(fma2(r, pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f)), pk2(-12582912.0f, -12582912.0f));   // to the nearest 2^-30
+        hi = add2(add2(e, pk2(384.0f, 384.0f)), pk2(-384.0f, -384.0f));
+        w = rest(e, hi);
     }
     // The masses as whole numbers, 0 for logits below lk: the bits of the two rounding sums, put together.
     __device__ __forceinline__ void whole(float l0, float l1, float lk, uint32_t& m0, uint32_t& m1) const {
-        const u64 z = quotient2(pk2(l0, l1), ntc, rinv);
-        float y0, y1, e0, e1;
-        up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(y1));
+        float e0, e1;
+        exponentials(l0, l1, e0, e1);
         const u64 e = pk2(l0 >= lk ? e0 : 0.0f, l1 >= lk ? e1 : 0.0f);
-        const u64 t = add2(e, pk2(384.0f, 384.0f));
-        const u64 r = fma2(add2(t, pk2(-384.0f, -384.0f)), pk2(-1.0f, -1.0f), e);
-        const u64 w = fma2(r, pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f));
+        const u64 t = add2(e, pk2(384.0f, 384.0f)), w = rest(e, add2(t, pk2(-384.0f, -384.0f)));
         constexpr uint32_t ZERO = (0x43C00000u << 15) + 0x4B400000u;             // the bits of 384 and of 12582912
         m0 = ((uint32_t)t << 15) + (uint32_t)w - ZERO;
         m1 = ((uint32_t)(t >> 32) << 15) + (uint32_t)(w >> 32) - ZERO;

@@ -821,9 +821,9 @@ __device__ __forceinline__ float pass_hist(RowS& rw, const NextRow& nx, bool kee
 
 // The mass pass: per chunk the mass of the logits >= lk (BAND: of those above t_hi) into csum, and, BAND, the logits of
 // [tl, t_hi] into the warp's list and the mass of all logits >= lk.  MINP: lk may lie above the mass horizon.
-// The masses are MassFn's, operation by operation: rounded to a multiple of 2^-15 (t, a float at 384) and the rest to 2^-30 (w, at
-// 12582912), whose bits are summed as integers.  What bounds it is issue and the pipes about alike: two logits take 10 packed
-// instructions of two cycles, two exponentials of eight, and, BAND, 12 compares, selects and additions.
+// The masses come in two parts (Mass2): multiples of 2^-15, and the rest at 12582912, whose bits are summed as integers.  What bounds
+// it is issue and the pipes about alike: two logits take 10 packed instructions of two cycles, two exponentials of eight, and, BAND,
+// 12 compares, selects and additions.
 struct Masses { u64 all, keep; };
 // Above t_hi: the two parts of a mass to their sums; from tl on: the logit's bit to the mask.  Five instructions without a branch.
 __device__ __forceinline__ void band_add(float x, float t_hi, float tl, float hi, uint32_t lo, uint32_t bit, float& sh, uint32_t& sl, uint32_t& mk) {
@@ -833,7 +833,8 @@ __device__ __forceinline__ void band_add(float x, float t_hi, float tl, float hi
 }
 template <bool CL, int ELT, bool MASK, bool BAND, bool MINP>
 __device__ __forceinline__ Masses pass_mass(RowS& rw, const NextRow& nx, int then, MassFn mass, float lk, float t_hi, float tl, Cand* list, u64* csum) {
-    const u64 rinv = pk2(mass.rinv, mass.rinv), ntc = pk2(-mass.tc, -mass.tc), nm = pk2(-mass.m, -mass.m);
+    Mass2 m2;
+    m2.init(mass);
     u64 keep = 0;
     int all_h = 0, all_l = 0;
     run_pass<CL, ELT, MASK>(rw, nx, false, 0, then, [&](const auto& k) {
@@ -854,17 +855,13 @@ __device__ __forceinline__ Masses pass_mass(RowS& rw, const NextRow& nx, int the
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float x0 = h ? v.z : v.x, x1 = h ? v.w : v.y;
-                    const u64 z = quotient2(pk2(x0, x1), ntc, rinv);
-                    float y0, y1, e0, e1, h0, h1;
-                    up2(mul2(add2(z, nm), pk2(CI_LOG2E, CI_LOG2E)), y0, y1);
-                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(y0));
-                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(y1));
-                    const u64 e = pk2(e0, e1), hi = add2(add2(e, pk2(384.0f, 384.0f)), pk2(-384.0f, -384.0f));
-                    const u64 w = fma2(fma2(hi, pk2(-1.0f, -1.0f), e), pk2(CI_MASS_SCALE, CI_MASS_SCALE), pk2(12582912.0f, 12582912.0f));
+                    u64 hi, w;
+                    m2.parts(x0, x1, hi, w);
                     const uint32_t w0 = (uint32_t)w, w1 = (uint32_t)(w >> 32);
                     sh = add2(sh, hi);
                     sl += w0 + w1;
                     if (BAND) {
+                        float h0, h1;
                         up2(hi, h0, h1);
                         band_add(x0, t_hi, tl, h0, w0, 1u << (4 * j + 2 * h), ah, al, mk);
                         band_add(x1, t_hi, tl, h1, w1, 2u << (4 * j + 2 * h), ah, al, mk);

@@ -30,10 +30,10 @@ __global__ void k_masses(const float* tcs, const float* lmax, u64* bad) {
         const float l0 = L - 24.0f * tc * ((float)i / 1048576.0f), l1 = L - 24.0f * tc * ((float)(1048576 - i) / 1048576.0f);
         uint32_t a, b;
         g.whole(l0, l1, -1e30f, a, b);
-        u64 hi, lo;
-        g(l0, l1, hi, lo);
+        u64 hi, w;
+        g.parts(l0, l1, hi, w);
         float h0, h1, o0, o1;
-        up2(hi, h0, h1); up2(lo, o0, o1);
+        up2(hi, h0, h1); up2(add2(w, pk2(-12582912.0f, -12582912.0f)), o0, o1);
         const uint32_t c = (uint32_t)((double)h0 * 1073741824.0 + (double)o0), d = (uint32_t)((double)h1 * 1073741824.0 + (double)o1);
         n += a != f(l0) || b != f(l1) || c != f(l0) || d != f(l1);
     }
