@@ -1700,9 +1700,9 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
     if (rows <= sms) {
         // At most a row per SM, more than the cluster-resident kernel holds at once: a cluster of two or four CTAs per row, where
         // they all run at once.  From 75 rows on there is one CTA per row either way, and the streaming kernel's 1,024 threads get
-        // a row through sooner.  60 fp32 rows of 151,936 logits, streaming kernel (half of the SMs idle) and here: mixed filters 62
-        // and 54 us, top-p 61 and 54, top_k 50 36 and 27, top_k 1000 66 and 67, no filter 29 and 29 - 32, greedy 12 and 17; bf16 mixed 108
-        // and 58, top-p 77 and 56, no filter 29 and 29.  The host does not see the filters.
+        // a row through sooner.  60 fp32 rows of 151,936 logits, streaming kernel (half of the SMs idle) and here: mixed filters 61
+        // and 52 us, top-p 59 and 52, top_k 50 34 and 24, top_k 1000 67 and 65, no filter 27 and 28, greedy 11 and 16; bf16 mixed 97
+        // and 57, top-p 73 and 54, no filter 27 and 27.  The host does not see the filters.
         const int ki = chunk_index(FEW, dtype, mask != nullptr), smem = colinfer_few_smem(V, pen);
         if (smem > kChunkMaxSmem) return -1;
         const int rc = chunk_device(ki, &dev, &sms);
@@ -1711,10 +1711,10 @@ int launch_chunk(const void* logits, int dtype, const int32_t* mask, int mask_ro
             if (V >= 16384 * C && rows <= chunk_clusters(dev, ki, C, smem)) { set = FEW; break; }
         }
         if (set != FEW) return -1;
-        // More rows than SMs.  149 and 200 fp32 rows of 151,936, streaming kernel and here: mixed 66, 68 and 69, 72 us; top-p 125, 125
-        // and 96, 100; top_k 50 65, 83 and 37, 38; top_k 1000 126, 130 and 55, 61; half greedy 46, 47 and 45, 50; greedy 29, 31 and
-        // 25, 29 (a wide row alone on an SM has a third of the threads here).  400 rows: mixed 117 and 104, top-p 184 and 158, no filter
-        // 97 and 105; 592: 166 and 135, 245 and 197, 133 and 130.
+        // More rows than SMs.  149 and 200 fp32 rows of 151,936, streaming kernel and here: mixed 67, 68 and 69, 73 us; top-p 122, 124
+        // and 94, 99; top_k 50 60, 74 and 35, 37; top_k 1000 123, 127 and 56, 61; half greedy 46, 48 and 45, 50; greedy 29, 30 and
+        // 24, 28 (a wide row alone on an SM has a third of the threads here).  400 rows: mixed 120 and 103, top-p 187 and 158, no filter
+        // 99 and 103; 592: 168 and 135, 245 and 195, 133 and 130.
     } else if (one_per_sm(V, dtype, pen, rows, sms) || colinfer_rows_smem(V, pen) > kTwoPerSm) set = ROW;
     const int smem = chunk_smem(set, V, pen), ki = chunk_index(set, dtype, mask != nullptr);
     if (smem > kChunkMaxSmem) return -1;

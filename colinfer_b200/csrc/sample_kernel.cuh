@@ -8,12 +8,13 @@
 // sample_rows.cu, sample_row.cu and sample_few.cu say how many threads and CTAs per SM, and why.
 //
 // Rows start at any alignment: chunks are counted from the 16-byte boundary at or below the row's first logit ("position"
-// p = token + a), what lies outside the row reads as -inf.  Nothing outside the buffer is read (row_span).  History penalties are applied to a chunk in shared memory before
-// the pass reads it, the grammar mask to the registers it is read into; all passes then see effective logits.
+// p = token + a), what lies outside the row reads as -inf.  Nothing outside the buffer is read (row_span).  History penalties are
+// applied to a chunk in shared memory before the pass reads it, the grammar mask to the registers it is read into; all passes then
+// see effective logits.
 //
 //   greedy        one pass: maximum and its lowest index
-//   top_k <= 100  one pass.  The first chunk of every warp (the CTA's sample) bounds the k-th largest logit from below; the
-//                 pass lists what reaches the bound, the row is finished on the list
+//   top_k <= 100  one pass.  The first two chunks of every warp (the CTA's sample) bound the k-th largest logit from below;
+//                 the pass lists what reaches the bound, the row is finished on the list
 //   larger top_k  one pass as well where the sample says that the lists can hold the k largest; they are selected from there
 //                 exactly.  Else a full histogram gives the bucket of the k-th largest, and a second pass lists what reaches it
 //   top_p         pass 1 also sums the row's mass (approximately) and counts a histogram, laid out from the sample's maximum: of
@@ -28,13 +29,14 @@
 // band misses the pivot, an exact select over the 32-bit keys runs (slower, same result).
 //
 // What bounds it.  A pass over a row that is in HBM: bytes (592 greedy rows of 151,936 fp32 logits 64 us, of which 53 at the copy
-// rate).  A wide row: the second pass's instructions, and the chains of block-wide steps between the passes, a third of its
-// time, during which the SM's other row has the pipes to itself.  Hence masses two logits per instruction with rounding additions
+// rate).  A wide row: the second pass's instructions, and the chains of block-wide steps between the passes, three tenths of
+// its time, during which the SM's other row has the pipes to itself.  Hence masses two logits per instruction with rounding additions
 // instead of conversions, a histogram of a sample, one warp that decides and one that draws while searches are repeated by every warp
 // instead of published behind barriers.  A thread has 80 registers: with 64 (512 threads) the passes kept what a row needs in local
 // memory, which beside 226 KB of shared memory is L2, and two rows on an SM were slower than one after the other.
-// Before and now, one B200, 151,936 fp32 logits, us: 592 rows greedy 69 -> 64, without a filter 138 -> 125, top_p 203 -> 191,
-// top_k 50 81 -> 78, top_k 1000 251 -> 117; 296 rows top_k 1000 121 -> 67; 360 bf16 rows with mixed filters 159 -> 100.
+// The version with 512 threads, a full histogram and two passes for every top_k above 100, and now, one B200, 151,936 fp32 logits, us:
+// 592 rows greedy 69 -> 64, without a filter 138 -> 127, top_p 202 -> 194, top_k 50 82 -> 78, top_k 1000 190 -> 120; 360 bf16 rows with
+// mixed filters 123 -> 99, top_p 207 -> 154.
 #pragma once
 #include <stddef.h>
 
@@ -52,7 +54,7 @@ __device__ unsigned long long g_prof[16];
 #endif
 
 constexpr int NT = SMP_THREADS, NW = NT / 32;
-constexpr int NUM_SM = 148;          // (a B200's; only says from how many rows on their order matters)
+constexpr int NUM_SM = 148;          // (a B200's; says from how many rows on their order matters, and which CTAs start later)
 constexpr int CTAS_PER_SM = SMP_CTAS;
 constexpr int NST = SMP_STAGES;      // stages of a warp's ring
 constexpr int CHUNK = 512;           // logits per chunk: 16 per lane
@@ -93,8 +95,8 @@ using Args = colinfer_sample_args;
 template <bool B> struct BoolTag { static constexpr bool value = B; };
 struct Cand { uint32_t idx; float l; };
 
-// A row at hand.  What the phases of a row hand on lives here, not in registers: at 64 registers per thread anything that
-// stays alive across a pass is spilled, and with 226 KB of an SM's 256 in shared memory a spill is a round trip to L2.
+// A row at hand.  What the phases of a row hand on lives here, not in registers: at 80 registers per thread what stays alive
+// across a pass is spilled, and with 226 KB of an SM's 256 in shared memory a spill is a round trip to L2.
 struct RowS {
     const char* base; uint32_t end;    // the 16-byte boundary at or below its first logit; what of it is copied (row_span)
     int row, key;                      // its index, and that plus 1
@@ -478,8 +480,8 @@ __device__ __forceinline__ uint32_t chunk_bytes(const char* p, uint32_t end) {
     return left < (uint32_t)(CHUNK * ELT) ? left : (uint32_t)(CHUNK * ELT);
 }
 // Asks for the first chunks of row `key`, as far as they are not under way.  Every pass starts and ends with it: out of line where
-// a thread has 64 registers and what it needs would be spilled (200 fp32 rows of 151,936 without a filter 78 us inline, 74 us so),
-// inline in the kernels of clusters (21 rows of 217,408, top_k 50: 25 us out of line, 24 us so).
+// a thread has 80 registers and what it needs would be spilled (592 fp32 rows of 151,936 top_p 202 us inline, 194 us so, 200 without a
+// filter 65 and 63), inline in the kernels of clusters (21 rows of 217,408, top_k 50: 25 us out of line, 24 us so).
 template <int ELT>
 __device__ __forceinline__ void ring_start_here(int key, const char* base, uint32_t end, int Nc, int gw, int GW, bool keep) {
     Pipe<ELT> p;

@@ -1,6 +1,6 @@
 // sample_rows.cu -- the fused kernel with one CTA per row, for launches of more rows than SMs: two CTAs of 384 threads per SM, so
 // that one of them reads while the other one is in its block-wide steps.  384 and not 512 threads: 80 registers each instead of 64,
-// and 32 KB less of rings, which goes to the L1 (592 rows of 151,936 fp32 logits, greedy 80 -> 66 us, top_k 50 88 -> 80).
+// and 32 KB less of rings, which goes to the L1 (592 rows of 151,936 fp32 logits, greedy 78 -> 64 us, top_k 50 92 -> 78, top_p 208 -> 194).
 // Two chunks under way per warp: with three a launch is no faster (98,304 bytes per SM are enough to keep HBM busy).
 #define SMP_NAME smp_rows
 #define SMP_THREADS 384
