@@ -480,7 +480,7 @@ def run_sweep(torch, dev, lib, peak, reps: int):
     sp = wl.sampler_params(w["params"], VL, dev)
     logits, pos, mask = w["logits"].to(dev), w["pos"].to(dev), w["mask"].to(dev)
     med, best = per_launch_us(torch, lambda: draw(logits, sp, pos, mask=mask), flush, reps)
-    out["config4_bf16_512x262144"] = entry(med, best, 512, wl.bytes_per_row(VL, 2, True, 0), "k_sample (1,024 threads per row)", "row")
+    out["config4_bf16_512x262144"] = entry(med, best, 512, wl.bytes_per_row(VL, 2, True, 0), "k_sample (a CTA per row)", "row")
     del logits, mask, sp
     # speculative verify: k = 8 drafts per slot, temperature 0.8, top_p 0.95; one slot (latency) and 64 slots
     ver = {}
